@@ -380,24 +380,37 @@ class Transformer:
         D = cfg.head_dim
         Hq = lw.wo.w.shape[1] // D
         qkv = linear(x, lw.wqkv, xq, xs)
-        if lw.bqkv is not None:
-            qkv = qkv + lw.bqkv
         Hkv = (qkv.shape[1] // D - Hq) // 2
-        q = qkv[:, : Hq * D].reshape(T, Hq, D)
-        k = qkv[:, Hq * D: (Hq + Hkv) * D].reshape(T, Hkv, D)
-        v = qkv[:, (Hq + Hkv) * D:].reshape(T, Hkv, D)
-        if x.is_cuda and x.dtype == torch.bfloat16 and self.rope.cos.shape[1] * 2 == D:
-            # in-place RoPE kernel on the (copied, contiguous) query and key heads
-            q, k = q.contiguous(), k.contiguous()
-            fused.rope_q_(q, meta.positions, self.rope.cos, self.rope.sin, D, cfg.rope_interleaved)
-            fused.rope_q_(k, meta.positions, self.rope.cos, self.rope.sin, D, cfg.rope_interleaved)
-        else:
-            cos, sin = self.rope.cos[meta.positions.long()], self.rope.sin[meta.positions.long()]
-            q = ref.apply_rope(q, cos, sin, cfg.rope_interleaved)
-            k = ref.apply_rope(k, cos, sin, cfg.rope_interleaved)
         kvc = cache.latent(l)                           # [P, page, 2 * Hkv_total * D]; this rank's slice is cached
-        ref.kv_cache_write(kvc, torch.cat([k.reshape(T, -1), v.reshape(T, -1)], -1), meta.slot_mapping)
         window = cfg.sliding_window if (cfg.sliding_window and l % 2 == 0) else 0
+        if attn_ops.gqa_on_kernels(qkv, kvc, D, self.rope.cos):
+            # bias, rotation and cache write in one kernel; the queries stay in their columns of the projection
+            attn_ops.gqa_heads(qkv, lw.bqkv, meta.positions, self.rope.cos, self.rope.sin, meta.slot_mapping, kvc, Hq, Hkv, D,
+                               cfg.rope_interleaved)
+            q = qkv[:, : Hq * D].unflatten(1, (Hq, D))
+            if meta.mode == "prefill":
+                work = self._gqa_prefill_work(meta, window)
+                if attn_ops.gqa_prefill_on_kernel(kvc.shape[1], work.shape[0]):
+                    whole = meta.cu_seqlens[0] == 0 and meta.cu_seqlens[-1] == T      # else rows of no sequence stay zero
+                    out = (torch.empty if whole else torch.zeros)(T, Hq * D, dtype=x.dtype, device=x.device)
+                    attn_ops.gqa_prefill(q, kvc, meta.block_table, work, Hkv, cfg.softmax_scale, out, window=window, sinks=lw.sinks)
+                    return linear(out, lw.wo)
+        else:
+            if lw.bqkv is not None:
+                qkv = qkv + lw.bqkv
+            q = qkv[:, : Hq * D].reshape(T, Hq, D)
+            k = qkv[:, Hq * D: (Hq + Hkv) * D].reshape(T, Hkv, D)
+            v = qkv[:, (Hq + Hkv) * D:].reshape(T, Hkv, D)
+            if x.is_cuda and x.dtype == torch.bfloat16 and self.rope.cos.shape[1] * 2 == D:
+                # in-place RoPE kernel on the (copied, contiguous) query and key heads
+                q, k = q.contiguous(), k.contiguous()
+                fused.rope_q_(q, meta.positions, self.rope.cos, self.rope.sin, D, cfg.rope_interleaved)
+                fused.rope_q_(k, meta.positions, self.rope.cos, self.rope.sin, D, cfg.rope_interleaved)
+            else:
+                cos, sin = self.rope.cos[meta.positions.long()], self.rope.sin[meta.positions.long()]
+                q = ref.apply_rope(q, cos, sin, cfg.rope_interleaved)
+                k = ref.apply_rope(k, cos, sin, cfg.rope_interleaved)
+            ref.kv_cache_write(kvc, torch.cat([k.reshape(T, -1), v.reshape(T, -1)], -1), meta.slot_mapping)
         if meta.mode == "decode" and x.is_cuda:
             # paged flash-decoding kernel: lengths stay on the device (graph capturable)
             o = attn_ops.gqa_decode(q.contiguous(), kvc, meta.block_table, meta.seqlens, Hkv, cfg.softmax_scale,
@@ -419,6 +432,16 @@ class Transformer:
             out[a:b] = ref.gqa_attention(q[a:b], ks, vs, cfg.softmax_scale, q_start=ctx, window=window,
                                          sinks=lw.sinks)
         return linear(out.reshape(T, -1), lw.wo)
+
+    def _gqa_prefill_work(self, meta: AttnMeta, window: int) -> torch.Tensor:
+        """Tiles of the prompt kernel, the longest first; made once per step and window."""
+        from ..ops import talking
+        made = meta.__dict__.setdefault("_gqa_work", {})
+        key = (window, tuple(meta.cu_seqlens), tuple(meta.ctx_lens))
+        if key not in made:
+            rows = talking.prefill_work(meta.cu_seqlens, meta.ctx_lens, 0, 1, window)
+            made[key] = torch.tensor(rows, dtype=torch.int32, device=self.device).view(-1, 4)
+        return made[key]
 
     # ------------------------------------------------------------------ feed-forward
     def _moe(self, l: int, lw: LayerWeights, x, xq, xs, meta: AttnMeta) -> torch.Tensor:

@@ -87,6 +87,54 @@ def mla_out_absorb(o_lat: torch.Tensor, w_uv: torch.Tensor) -> torch.Tensor:
     return torch.bmm(o_lat.transpose(0, 1), w_uv.transpose(1, 2)).transpose(0, 1).reshape(T, -1)
 
 
+def gqa_on_kernels(qkv: torch.Tensor, cache: torch.Tensor, D: int, tables: torch.Tensor) -> bool:
+    """Whether ``gqa_heads`` takes these projections: bf16 heads of 64 or 128 columns that turn whole, a bf16 cache of plain rows."""
+    return (qkv.is_cuda and qkv.dtype == cache.dtype == torch.bfloat16 and D in (64, 128) and tables.shape[1] * 2 == D
+            and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and cache.is_contiguous()
+            and cache.data_ptr() % 16 == 0)
+
+
+def gqa_heads(qkv: torch.Tensor, bias: Optional[torch.Tensor], positions: torch.Tensor, cos_table: torch.Tensor,
+              sin_table: torch.Tensor, slot_mapping: torch.Tensor, cache: torch.Tensor, Hq: int, Hkv: int, D: int,
+              interleaved: bool) -> None:
+    """qkv [T, (Hq + 2 Hkv) D] bf16 projections (q | k | v heads; the rows are used up): bias, rotation of queries and keys, queries
+    back in place, keys and values to cache[slot] ([P, page, 2 Hkv D]; slot < 0 writes nothing)."""
+    assert gqa_on_kernels(qkv, cache, D, cos_table) and qkv.shape[1] == (Hq + 2 * Hkv) * D and cache.shape[2] == 2 * Hkv * D
+    positions, slot_mapping = positions.to(torch.int32).contiguous(), slot_mapping.to(torch.int64).contiguous()
+    assert cos_table.dtype == torch.float32 and cos_table.is_contiguous() and sin_table.is_contiguous()
+    bias = bias.to(torch.bfloat16).contiguous() if bias is not None else None
+    rc = _ext.lib().bg_gqa_heads(_ext.ptr(qkv), ctypes.c_longlong(qkv.stride(0)), _ext.ptr(bias), _ext.ptr(positions),
+                                 _ext.ptr(cos_table), _ext.ptr(sin_table), _ext.ptr(slot_mapping), _ext.ptr(cache),
+                                 ctypes.c_int(qkv.shape[0]), ctypes.c_int(Hq), ctypes.c_int(Hkv), ctypes.c_int(D),
+                                 ctypes.c_int(int(interleaved)), _ext.stream())
+    _ext.check(rc, "bg_gqa_heads")
+
+
+def gqa_prefill_on_kernel(page: int, tiles: int) -> bool:
+    """Pages the prompt kernel's copies can walk, and tiles within one grid."""
+    return page >= 16 and page & (page - 1) == 0 and 0 < tiles <= 65535
+
+
+def gqa_prefill(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, work: torch.Tensor, num_kv_heads: int,
+                scale: float, out: torch.Tensor, window: int = 0, sinks: Optional[torch.Tensor] = None) -> None:
+    """Causal attention of prompt pieces over cached rows, probabilities to 2^-17 of themselves.  q [T, Hq, D] bf16 turned queries (a
+    column view of the projections is fine); cache [P, page, 2 Hkv D] with the new rows written; ``work`` int32 rows of
+    ``talking.prefill_work`` -> out [T, Hq * D] for the rows that tiles cover."""
+    T, Hq, D = q.shape
+    P, page, row = cache.shape
+    assert q.dtype == out.dtype == cache.dtype == torch.bfloat16 and q.stride(2) == 1 and q.stride(1) == D and out.stride(1) == 1
+    assert row == 2 * num_kv_heads * D and cache.is_contiguous() and work.dtype == torch.int32 and work.is_contiguous()
+    block_table = block_table.to(torch.int32)
+    block_table = block_table if block_table.stride(1) == 1 else block_table.contiguous()
+    sinks = sinks.float().contiguous() if sinks is not None else None
+    rc = _ext.lib().bg_gqa_prompt_fine(
+        _ext.ptr(q), ctypes.c_int(q.stride(0)), _ext.ptr(cache), ctypes.c_int(P), ctypes.c_int(page), _ext.ptr(block_table),
+        ctypes.c_int(block_table.stride(0)), ctypes.c_int(block_table.shape[1]), _ext.ptr(work), ctypes.c_int(work.shape[0]),
+        ctypes.c_int(T), _ext.ptr(out), ctypes.c_int(out.stride(0)), ctypes.c_int(Hq), ctypes.c_int(num_kv_heads), ctypes.c_int(D),
+        ctypes.c_int(window), ctypes.c_float(scale), _ext.ptr(sinks), _ext.ptr(_ext.status_word(q.device)), _ext.stream())
+    _ext.check(rc, "bg_gqa_prompt_fine")
+
+
 _GQA_SCRATCH = {}
 
 

@@ -5,6 +5,16 @@
 //   S[q, k] = Q[q, :] . K[k, kv(h)]      (M = 128 queries, N = 64 keys; Q resident, K streamed, both K-major)
 //   O[q, :] += P[q, k] . V[k, kv(h)]     (V read N-major, P written by the softmax threads as a swizzled K-major tile)
 //
+// FINE form (bf16 projections; the models whose attention was computed in fp32 from bf16 operands): queries are read where the
+// projection left them, the scale meets the fp32 scores, and a probability goes into two bf16 parts, p = hi + lo with |p - hi - lo|
+// below 2^-17 p, whose products with V are both accumulated.  The parts are the A operand from TMEM: they take the 2 x 32 columns of the
+// scores they were made of, so P costs no shared memory and two CTAs fit an SM up to 128-wide heads; S(t + 1) then waits for
+// P.V(t - 1), whose operand it overwrites.  Value rows past a sequence's end are zeroed before the last product, so stale rows of
+// a page cannot reach it through 0 * inf.  Bound by exponentials (16 a clock and SM) at 64-wide heads, by the two products with V
+// at 128-wide ones.  Measured on whole prompt steps, against scores and probabilities as fp32 tensors in memory: two layers of 64
+// heads of 64 with 128 experts, three prompts of up to 2,047 tokens 29.9 -> 10.4 ms; two layers of 48 heads of 128 with 256 experts,
+// two prompts of up to 1,100 behind 333 cached tokens 7.94 -> 2.91 ms.
+//
 // A first kernel turns the queries, folds scale * log2(e) in and rounds them once to bf16.  One CTA = (tile of 128 queries of
 // one sequence, head).  K and V come straight from the paged cache by TMA (3-D map: column, token of the page, page) through a
 // ring each, so a key tile is free again as soon as its scores are done; a head's last 64-wide block may reach into the next
@@ -53,6 +63,7 @@ struct Params {
   const float* sinks;            // [H] scores of the sink, or null: zero
   int staged;                    // gates per element: rows leave through shared memory, a warp a row at a time
   int row_shift;                 // rows of Q = rows of out - row_shift
+  float score_scale;             // FINE: scale * log2(e), applied to the scores
   int smem_bytes;
   int* status;
 };
@@ -98,6 +109,15 @@ __device__ __forceinline__ bool vote_any_128(bool v) {      // barrier over the 
       : "memory");
   return r != 0;
 }
+// D[tmem] += A[tmem] * B[smem]: a row of A is a lane, its 16-bit elements lie two to a column
+__device__ __forceinline__ void mma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.u32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "}\n" ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* v) {
   tmem_ld_32x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(v));
 }
@@ -113,11 +133,12 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
       : "memory");
 }
 
-// shared memory: Q [KB] | K [stages][KB] | V [stages][VB] | P, all on 1,024-byte boundaries, then Shared
-__host__ __device__ inline int tile_bytes(int KB, int VB, int stages) {
-  return KB * kQBlockBytes + stages * (KB + VB) * kBlockBytes + kPBytes;
+// shared memory: Q [KB] | K [stages][KB] | V [stages][VB] | P (not FINE), all on 1,024-byte boundaries, then Shared
+__host__ __device__ inline int tile_bytes(int KB, int VB, int stages, bool fine) {
+  return KB * kQBlockBytes + stages * (KB + VB) * kBlockBytes + (fine ? 0 : kPBytes);
 }
 
+template <bool FINE>
 __global__ void __launch_bounds__(kThreads, 2)
 attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv, const Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -126,7 +147,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
   uint8_t* k_buf = q_buf + p.KB * kQBlockBytes;
   uint8_t* v_buf = k_buf + p.stages * p.KB * kBlockBytes;
   uint8_t* p_buf = v_buf + p.stages * p.VB * kBlockBytes;
-  Shared& ss = *reinterpret_cast<Shared*>(p_buf + kPBytes);
+  Shared& ss = *reinterpret_cast<Shared*>(p_buf + (FINE ? 0 : kPBytes));
   if (reinterpret_cast<uint8_t*>(&ss + 1) > smem_raw + p.smem_bytes) {      // a base that is off its boundary leaves no room
     if (threadIdx.x == 0 && p.status != nullptr) atomicMax(p.status, (int)kBadArgument);
     return;
@@ -252,7 +273,9 @@ attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
       };
       if (ok && n_tiles > 0) ok = issue_s(0);
       for (int t = 0; ok && t < n_tiles; ++t) {
-        // S of tile t + 1 goes into the buffer that the softmax of tile t - 1 has left (its P was handed over before PV(t-1))
+        // S of tile t + 1 goes into the buffer that the softmax of tile t - 1 has left (its P was handed over before PV(t-1)); FINE:
+        // PV(t - 1) reads P from it
+        if (FINE && t > 0 && t + 1 < n_tiles && !mbar_wait(&ss.o_done, (t - 1) & 1, abort_flag, kTimeoutMma)) { ok = false; break; }
         if (t + 1 < n_tiles && !issue_s(t + 1)) { ok = false; break; }
         const int s = t % ST;
         if (!mbar_wait(&ss.v_full[s], (t / ST) & 1, abort_flag, kTimeoutMma)) { ok = false; break; }
@@ -261,7 +284,11 @@ attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         const uint64_t pdesc = make_smem_desc_sw128(smem_u32(p_buf));
         const uint32_t v_base = smem_u32(v_buf + s * p.VB * kBlockBytes);
 #pragma unroll
-        for (int j = 0; j < BN / 16; ++j)
+        for (int j = 0; FINE && j < BN / 8; ++j)                    // high parts, then low parts
+          mma_f16_ta(tm_o, tmem_base + (t & 1) * BN + j * 8, desc_mn_sw128(v_base + (j & 3) * 2048, kBlockBytes, 1024), idesc_pv,
+                     (t > 0 || j > 0) ? 1u : 0u);
+#pragma unroll
+        for (int j = 0; !FINE && j < BN / 16; ++j)
           mma_f16(tm_o, pdesc + 2 * j, desc_mn_sw128(v_base + j * 2048, kBlockBytes, 1024), idesc_pv, (t > 0 || j > 0) ? 1u : 0u);
         tc_commit(&ss.v_empty[s]);
         tc_commit(&ss.o_done);
@@ -299,14 +326,27 @@ attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
       float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
       for (int j = 0; j < BN; ++j) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(sv[j]));
-      const float mt = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+      const float mt = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * (FINE ? p.score_scale : 1.f);
       const bool grow = mt > m_run + 8.f;
       const float m_new = grow ? mt : m_run;
       const float alpha = (grow && m_run != -INFINITY) ? ex2(m_run - m_new) : 1.f;
       const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
       float l4[4] = {0.f, 0.f, 0.f, 0.f};
+      uint32_t lo_part[FINE ? BN / 2 : 1];
+      if (FINE) {
 #pragma unroll
-      for (int j = 0; j < BN; j += 2) {
+        for (int j = 0; j < BN; j += 2) {
+          const float e0 = ex2(fmaf(__uint_as_float(sv[j]), p.score_scale, neg_m));
+          const float e1 = ex2(fmaf(__uint_as_float(sv[j + 1]), p.score_scale, neg_m));
+          const __nv_bfloat162 o = __floats2bfloat162_rn(e0, e1);
+          const __nv_bfloat162 rest = __floats2bfloat162_rn(e0 - __low2float(o), e1 - __high2float(o));
+          l4[(j >> 1) & 3] += e0 + e1;
+          sv[j >> 1] = *reinterpret_cast<const uint32_t*>(&o);
+          lo_part[j >> 1] = *reinterpret_cast<const uint32_t*>(&rest);
+        }
+      }
+#pragma unroll
+      for (int j = 0; !FINE && j < BN; j += 2) {
         const __nv_bfloat162 o = __floats2bfloat162_rn(ex2(__uint_as_float(sv[j]) + neg_m), ex2(__uint_as_float(sv[j + 1]) + neg_m));
         l4[(j >> 1) & 3] += __low2float(o) + __high2float(o);
         sv[j >> 1] = *reinterpret_cast<const uint32_t*>(&o);
@@ -326,8 +366,21 @@ attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       }
+      if (FINE) {
+        tmem_st32(tmem_base + lane_addr + (t & 1) * BN, *reinterpret_cast<const uint32_t(*)[32]>(sv));
+        tmem_st32(tmem_base + lane_addr + (t & 1) * BN + 32, *reinterpret_cast<const uint32_t(*)[32]>(lo_part));
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        const int real = last + 1 - kt;
+        if (!kept && real < BN) {                                  // uniform: the tile past whose end rows belong to nobody
+          if (vote_any_128(!mbar_wait(&ss.v_full[t % ST], (t / ST) & 1, abort_flag, kTimeoutEpilogue))) { ok = false; break; }
+          uint8_t* v_tile = v_buf + (t % ST) * p.VB * kBlockBytes;
+          const int n16 = (BN - real) * 8;                          // 16-byte pieces of a block's dead rows
+          for (int i = r; i < p.VB * n16; i += 128)
+            *reinterpret_cast<uint4*>(v_tile + (i / n16) * kBlockBytes + real * 128 + (i % n16) * 16) = make_uint4(0, 0, 0, 0);
+        }
+      }
 #pragma unroll
-      for (int c = 0; c < BN / 8; ++c)
+      for (int c = 0; !FINE && c < BN / 8; ++c)
         *reinterpret_cast<uint4*>(prow + ((c ^ (r & 7)) << 4)) = make_uint4(sv[4 * c], sv[4 * c + 1], sv[4 * c + 2], sv[4 * c + 3]);
       l_run = l_run * alpha + (l4[0] + l4[1]) + (l4[2] + l4[3]);
       m_run = m_new;
@@ -473,10 +526,145 @@ static int encode(CUtensorMap* m, int rank, const void* base, const cuuint64_t* 
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -2;
 }
 
+template <bool FINE>
+static int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, Params& p, int H, int n_work, cudaStream_t stream) {
+  // two CTAs an SM when two stages and half of TMEM are enough, otherwise one with as many stages as fit
+  const bool two = p.VB <= 2 && tile_bytes(p.KB, p.VB, 2, FINE) + (int)sizeof(Shared) <= kSmemTwo;
+  const int room = (two ? kSmemTwo : 226 * 1024) - (int)sizeof(Shared);
+  p.stages = 2;
+  while (p.stages < kMaxStages && tile_bytes(p.KB, p.VB, p.stages + 1, FINE) <= room) ++p.stages;
+  p.staged = p.gate != nullptr && p.gate_cols > 1 && tile_bytes(p.KB, p.VB, p.stages, FINE) >= BM * p.VB * 256;
+  p.tmem_cols = two ? 256 : 512;
+  p.smem_bytes = two ? kSmemTwo : 227 * 1024;
+  static bg::DeviceOnce once;
+  if (!bg::ensure_dynamic_smem(attn_kernel<FINE>, 227 * 1024, once)) return -13;
+  attn_kernel<FINE><<<dim3(H, n_work), kThreads, p.smem_bytes, stream>>>(tq, tk, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -14;
+}
+static int encode_cache(CUtensorMap* tk, const void* cache, int row, int page, int n_pages, long long page_stride, int box_rows) {
+  cuuint64_t dims[3] = {(cuuint64_t)row, (cuuint64_t)page, (cuuint64_t)n_pages};
+  cuuint64_t strides[2] = {(cuuint64_t)row * 2, (cuuint64_t)page_stride * 2};
+  cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
+  return encode(tk, 3, cache, dims, strides, box);
+}
+
+// Heads of a bf16 projection row [q of Hq | k of G | v of G] of D columns each: bias, rotation (fp32, rounded once), queries back
+// in place, keys and values to cache[slot] (slot < 0: nowhere).  A thread takes 8 pairs of channels that turn together (or 8
+// channels of a value).  One pass over the row: before, bias, copies of q and k, two rotations, the joining of k and v and the masked
+// write were nine launches.
+__global__ void __launch_bounds__(256)
+heads_kernel(__nv_bfloat16* __restrict__ qkv, long long ld, const __nv_bfloat16* __restrict__ bias, const int* __restrict__ positions,
+             const float* __restrict__ cos_t, const float* __restrict__ sin_t, const long long* __restrict__ slots,
+             __nv_bfloat16* __restrict__ cache, int Hq, int G, int D, int interleaved) {
+  bg::pdl_prologue((BG_FILE_TAG << 16) | __LINE__);
+  const int t = blockIdx.x, half = D / 2, per = half / 8;
+  __nv_bfloat16* x = qkv + (size_t)t * ld;
+  const long long slot = slots[t];
+  __nv_bfloat16* row = cache + (slot < 0 ? 0 : slot) * (2 * G * D);
+  const float* co = cos_t + (size_t)positions[t] * half;
+  const float* si = sin_t + (size_t)positions[t] * half;
+  auto load = [&](int c, float (&f)[8]) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(x + c);
+    const __nv_bfloat162* v = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { const float2 a = __bfloat1622float2(v[i]); f[2 * i] = a.x; f[2 * i + 1] = a.y; }
+    if (bias != nullptr) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] += __bfloat162float(bias[c + i]);
+    }
+  };
+  auto store = [&](__nv_bfloat16* dst, const float (&f)[8]) {
+    __align__(16) __nv_bfloat162 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(v);
+  };
+  for (int it = threadIdx.x; it < (Hq + G) * per; it += blockDim.x) {
+    const int h = it / per, i = it % per * 8;                      // pairs i .. i + 7 of head h
+    if (h >= Hq && slot < 0) continue;
+    const int c0 = h * D + (interleaved ? 2 * i : i), c1 = interleaved ? c0 + 8 : c0 + half;
+    float a[8], b[8], cs[8], sn[8];
+    load(c0, a);
+    load(c1, b);
+#pragma unroll
+    for (int j = 0; j < 8; j += 4) {
+      *reinterpret_cast<float4*>(cs + j) = *reinterpret_cast<const float4*>(co + i + j);
+      *reinterpret_cast<float4*>(sn + j) = *reinterpret_cast<const float4*>(si + i + j);
+    }
+    float ra[8], rb[8];
+    if (interleaved) {                                             // a: pairs 0 .. 3, b: pairs 4 .. 7
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        ra[2 * j] = a[2 * j] * cs[j] - a[2 * j + 1] * sn[j];
+        ra[2 * j + 1] = a[2 * j + 1] * cs[j] + a[2 * j] * sn[j];
+        rb[2 * j] = b[2 * j] * cs[4 + j] - b[2 * j + 1] * sn[4 + j];
+        rb[2 * j + 1] = b[2 * j + 1] * cs[4 + j] + b[2 * j] * sn[4 + j];
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        ra[j] = a[j] * cs[j] - b[j] * sn[j];
+        rb[j] = b[j] * cs[j] + a[j] * sn[j];
+      }
+    }
+    __nv_bfloat16* dst = h < Hq ? x : row - Hq * D;                // keys of head g = h - Hq start the cached row
+    store(dst + c0, ra);
+    store(dst + c1, rb);
+  }
+  if (slot < 0) return;
+  for (int i = threadIdx.x * 8; i < G * D; i += blockDim.x * 8) {
+    float f[8];
+    load((Hq + G) * D + i, f);
+    store(row + G * D + i, f);
+  }
+}
+
 }  // namespace gqapre
 }  // namespace bg
 
 extern "C" {
+
+// qkv [T, ld] bf16: heads q | k | v of D columns (D % 16 == 0); bias [(Hq + 2 G) D] bf16 or null; tables [*, D / 2] fp32; slots [T];
+// cache [slots, 2 G D] bf16.
+int bg_gqa_heads(void* qkv, long long ld, const void* bias, const int* positions, const float* cos_t, const float* sin_t,
+                 const long long* slots, void* cache, int T, int Hq, int G, int D, int interleaved, cudaStream_t stream) {
+  using namespace bg::gqapre;
+  if (T <= 0) return 0;
+  if (Hq <= 0 || G <= 0 || D <= 0 || D % 16 || ld % 8 || ld < (long long)(Hq + 2 * G) * D) return -1;
+  const int items = (Hq + G) * D / 16, threads = items >= 256 ? 256 : (items + 31) / 32 * 32;
+  bg::launch_pdl(heads_kernel, dim3(T), dim3(threads), 0, stream, reinterpret_cast<__nv_bfloat16*>(qkv), ld,
+                 reinterpret_cast<const __nv_bfloat16*>(bias), positions, cos_t, sin_t, slots, reinterpret_cast<__nv_bfloat16*>(cache), Hq, G,
+                 D, interleaved);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+// Causal prompt attention over cached heads, probabilities in two parts.  q [R, ldq] bf16 turned queries (H heads of D columns, D a
+// multiple of 64 up to 128); cache [pages, page, 2 G D] bf16; work as for bg_gqa_prompt; sinks [H] fp32 or null; out [R, ldo] bf16.
+int bg_gqa_prompt_fine(const void* q, int ldq, const void* cache, int n_pages, int page, const int* block_table, int bt_stride,
+                       int bt_cols, const int* work, int n_work, int R, void* out, int ldo, int H, int G, int D, int window,
+                       float scale, const float* sinks, int* status, cudaStream_t stream) {
+  using namespace bg::gqapre;
+  if (n_work <= 0) return 0;
+  if (H <= 0 || G <= 0 || H % G || (D != 64 && D != 128) || page < 16 || (page & (page - 1)) || ldq % 8 || ldo % 8 || bt_cols <= 0 ||
+      n_work > 65535 || window < 0 || !(scale > 0.f))
+    return -1;
+  const int box_rows = page < 64 ? page : 64, row = 2 * G * D;
+  CUtensorMap tq, tk;
+  cuuint64_t dims[2] = {(cuuint64_t)H * D, (cuuint64_t)R};
+  cuuint64_t strides[1] = {(cuuint64_t)ldq * 2};
+  cuuint32_t box[2] = {64, BM};
+  if (encode(&tq, 2, q, dims, strides, box) != 0) return -10;
+  if (encode_cache(&tk, cache, row, page, n_pages, (long long)page * row, box_rows) != 0) return -11;
+  Params p = {};
+  p.score_scale = scale * 1.4426950408889634f;
+  p.work = reinterpret_cast<const Work*>(work);
+  p.block_table = block_table; p.bt_stride = bt_stride; p.bt_cols = bt_cols; p.page = page; p.box_rows = box_rows;
+  p.KB = p.VB = D / 64; p.dp = p.dvp = D; p.v_col0 = G * D; p.rep = H / G; p.sink = sinks != nullptr;
+  p.window = window; p.out_scale = 1.f; p.out = reinterpret_cast<__nv_bfloat16*>(out); p.ldo = ldo; p.gate_cols = 1; p.sinks = sinks;
+  p.status = status;
+  return launch_attn<true>(tq, tk, p, H, n_work, stream);
+}
+
 
 // Queries of R rows: q fp32 [R, ldq], rope [R, 2 * half] or null -> out bf16 [R, H, kc] (kc = dp rounded up to
 // 64), times scale * log2(e).
@@ -512,31 +700,16 @@ int bg_gqa_prompt(const void* qf, const void* cache, long long page_stride, int 
     cuuint32_t box[2] = {64, BM};
     if (encode(&tq, 2, qf, dims, strides, box) != 0) return -10;
   }
-  {
-    cuuint64_t dims[3] = {(cuuint64_t)row, (cuuint64_t)page, (cuuint64_t)n_pages};
-    cuuint64_t strides[2] = {(cuuint64_t)row * 2, (cuuint64_t)page_stride * 2};
-    cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
-    if (encode(&tk, 3, cache, dims, strides, box) != 0) return -11;
-  }
+  if (encode_cache(&tk, cache, row, page, n_pages, page_stride, box_rows) != 0) return -11;
   Params p;
+  p.score_scale = 1.f;
   p.work = reinterpret_cast<const Work*>(work);
   p.block_table = block_table; p.bt_stride = bt_stride; p.bt_cols = bt_cols; p.page = page; p.box_rows = box_rows;
   p.KB = kc / 64; p.VB = (dvp + 63) / 64; p.dp = dp; p.dvp = dvp; p.v_col0 = G * dp; p.rep = H / G; p.chunk = chunk; p.sink = sink;
   p.window = window; p.keep = keep; p.out_scale = out_scale;
   p.out = reinterpret_cast<__nv_bfloat16*>(out); p.ldo = ldo; p.gate = gate; p.ld_gate = ld_gate; p.gate_cols = gate_cols; p.sinks = sinks; p.row_shift = row_shift;
   p.status = status;
-  // two CTAs an SM when two stages and half of TMEM are enough, otherwise one with as many stages as fit
-  const bool two = p.VB <= 2 && tile_bytes(p.KB, p.VB, 2) + (int)sizeof(Shared) <= kSmemTwo;
-  const int room = (two ? kSmemTwo : 226 * 1024) - (int)sizeof(Shared);
-  p.stages = 2;
-  while (p.stages < kMaxStages && tile_bytes(p.KB, p.VB, p.stages + 1) <= room) ++p.stages;
-  p.staged = gate != nullptr && gate_cols > 1 && tile_bytes(p.KB, p.VB, p.stages) >= BM * p.VB * 256;
-  p.tmem_cols = two ? 256 : 512;
-  p.smem_bytes = two ? kSmemTwo : 227 * 1024;
-  static bg::DeviceOnce once;
-  if (!bg::ensure_dynamic_smem(attn_kernel, 227 * 1024, once)) return -13;
-  attn_kernel<<<dim3(H, n_work), kThreads, p.smem_bytes, stream>>>(tq, tk, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -14;
+  return launch_attn<false>(tq, tk, p, H, n_work, stream);
 }
 
 }  // extern "C"

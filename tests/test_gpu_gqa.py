@@ -29,3 +29,74 @@ def test_gqa_decode(Hq, Hkv, D, window, use_sinks, splits):
     want = attention.gqa_decode(q.float(), cache.float(), bt, sl, Hkv, scale, window=window, sinks=sinks)
     err = ((got - want).norm() / want.norm()).item()
     assert err < 1.5e-2, err
+
+
+@pytest.mark.parametrize("Hq,Hkv,D,page,interleaved,bias", [(16, 2, 64, 64, False, False), (6, 6, 128, 16, True, True),
+                                                             (24, 2, 128, 128, False, True), (5, 1, 64, 32, True, False)])
+@pytest.mark.parametrize("window,use_sinks", [(0, False), (0, True), (100, True), (1, False), (64, False)])
+def test_gqa_prompt(Hq, Hkv, D, page, interleaved, bias, window, use_sinks):
+    """Projections to attention output: lengths at the edges of tiles and pages, cached context, rows without a slot, stale rows of
+    the last page that are not finite.  Operands are the bf16 numbers the kernels see, so what is left is the two-part
+    probabilities (2^-17) and the rounding of the output (8 significant bits: up to 2^-8 of a value)."""
+    from batchgen_b200.ops import _ext, attention, ref, talking
+    g = torch.Generator().manual_seed(Hq * D + page + window)
+    lens, ctx = [1, 63, 64, 65, 127, 128, 129, 300, 2], [0, 0, 64, 1, 0, 33, 500, 7, 1000]
+    n, T = len(lens), sum(lens)
+    need = [-(-(a + b) // page) for a, b in zip(lens, ctx)]
+    order = torch.randperm(sum(need), generator=g).tolist()
+    cache = torch.full((sum(need), page, 2 * Hkv * D), float("nan"), dtype=torch.bfloat16)
+    bt = torch.zeros(n, max(need) + 1, dtype=torch.int32)
+    pos, slots, old = [], [], []
+    for i in range(n):
+        bt[i, :need[i]] = torch.tensor([order.pop() for _ in range(need[i])], dtype=torch.int32)
+        p = torch.arange(ctx[i] + lens[i])
+        where = bt[i].long()[p // page] * page + p % page
+        past = torch.randn(ctx[i], 2 * Hkv * D, generator=g).bfloat16()
+        cache.view(-1, 2 * Hkv * D)[where[:ctx[i]]] = past
+        old.append(past)
+        pos.append(p[ctx[i]:])
+        slots.append(where[ctx[i]:])
+    pos, slots = torch.cat(pos).int(), torch.cat(slots)
+    qkv = torch.randn(T, (Hq + 2 * Hkv) * D, generator=g).bfloat16()
+    b = torch.randn(qkv.shape[1], generator=g).bfloat16() if bias else None
+    inv = ref.rope_inv_freq(D, 10000.0)
+    ang = torch.arange(2048, dtype=torch.float32).unsqueeze(1) * inv
+    cos, sin = ang.cos(), ang.sin()
+    cu = [0]
+    for m in lens:
+        cu.append(cu[-1] + m)
+    # what the heads kernel makes of the projections
+    x = qkv.double() + (b.double() if bias else 0)
+    turn = lambda t: ref.apply_rope(t.float(), cos[pos.long()], sin[pos.long()], interleaved)  # noqa: E731
+    want_q = turn(x[:, :Hq * D].view(T, Hq, D))
+    want_kv = torch.cat([turn(x[:, Hq * D:(Hq + Hkv) * D].view(T, Hkv, D)).reshape(T, -1), x[:, (Hq + Hkv) * D:].float()], 1)
+    dev, dc = qkv.cuda(), cache.cuda()
+    skip = slots.clone()
+    skip[0] = -1                                              # the only row of the first sequence: its key is written by hand below
+    attention.gqa_heads(dev, b.cuda() if bias else None, pos.cuda(), cos.cuda(), sin.cuda(), skip.cuda(), dc, Hq, Hkv, D, interleaved)
+    got_q, flat = dev[:, :Hq * D].cpu().view(T, Hq, D), dc.view(-1, 2 * Hkv * D)
+    assert not torch.isfinite(flat[slots[0].item()].float()).any()
+    flat[slots[0].item()] = want_kv[0].bfloat16().cuda()
+    got_kv = flat[slots.cuda()].cpu()
+    assert (got_q.float() - want_q).abs().max() <= want_q.abs().max() * 2 ** -8
+    assert (got_kv.float() - want_kv).abs().max() <= want_kv.abs().max() * 2 ** -8
+    work = torch.tensor(talking.prefill_work(cu, ctx, 0, 1, window), dtype=torch.int32).cuda()
+    out = torch.full((T, Hq * D), 7.0, dtype=torch.bfloat16, device="cuda")
+    sinks = torch.randn(Hq, generator=g) if use_sinks else None
+    attention.gqa_prefill(dev[:, :Hq * D].unflatten(1, (Hq, D)), dc, bt.cuda(), work, Hkv, D ** -0.5, out, window=window,
+                          sinks=sinks.cuda() if use_sinks else None)
+    torch.cuda.synchronize()
+    _ext.check_status()
+    for i in range(n):
+        a, e = cu[i], cu[i + 1]
+        rows = torch.cat([old[i], got_kv[a:e]]).double()
+        k, v = (t.view(-1, Hkv, D).repeat_interleave(Hq // Hkv, 1) for t in rows.split(Hkv * D, 1))
+        s = torch.einsum("nhd,lhd->hnl", got_q[a:e].double(), k) * D ** -0.5
+        at, key = pos[a:e].long().unsqueeze(1), torch.arange(rows.shape[0]).unsqueeze(0)
+        s = s.masked_fill((key > at) | ((key <= at - window) if window else torch.zeros_like(key > at)), float("-inf"))
+        if use_sinks:
+            s = torch.cat([s, sinks.double().view(Hq, 1, 1).expand(Hq, s.shape[1], 1)], -1)
+        o = torch.einsum("hnl,lhd->nhd", s.softmax(-1)[..., :rows.shape[0]], v).reshape(e - a, -1)
+        err = (out[a:e].cpu().double() - o).abs()
+        # a value rounded to 8 significant bits: 2^-8 of it; fp32 sums of up to 1,000 terms (1,000 * 2^-24) and p of 2^-17: 7e-5
+        assert (err <= o.abs() * 2 ** -8 + 7e-5 * v.abs().max()).all(), (i, err.max())
