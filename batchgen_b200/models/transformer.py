@@ -108,7 +108,7 @@ class Transformer:
             act = linear(x, w13, xq, xs, silu_mul=True)
         else:
             gu = linear(x, w13, xq, xs)
-            act = ref.swiglu_clamped(gu) if self.cfg.activation == "swiglu_clamped" else ref.silu_mul(gu)
+            act = moe_ops.activation(gu, self.cfg.activation if self.cfg.activation == "swiglu_clamped" else "silu")
         return linear(act, w2)
 
     def _norm(self, x, w, residual, quant):
@@ -485,8 +485,10 @@ class Transformer:
             if self.comm is not None and self.layout.ep_size > 1:
                 routed = self.comm.moe(h, idx, w, ew, cfg.n_routed_experts, num_valid=meta.num_valid)
             else:
-                routed = moe_ops.experts_forward(h, idx, w, ew, 0, cfg.n_routed_experts,
+                joined = shared is not None and not cfg.moe_latent_size      # the combine adds the shared expert's rows
+                routed = moe_ops.experts_forward(h, idx, w, ew, 0, cfg.n_routed_experts, extra=shared if joined else None,
                                                  num_valid=meta.num_valid, timer=tm)
+                shared = None if joined else shared
         if self.streamer is not None:
             self.streamer.release(l)               # the slot returns once the kernels queued above have run
         if cfg.moe_latent_size:

@@ -281,9 +281,61 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ y, int ldy, const int* __re
   }
 }
 
+// Gated activation of bf16 rows [gate | up] of 2 F columns -> [F], in fp32, rounded once.  KIND 0: SiLU(g) u; 1: GPT-OSS, g clamped above
+// and u on both sides at `limit`, (u + 1) g sigmoid(1.702 g); 2: the same clamps, SiLU(g) u.  Rows past *total_rows, and padding rows of
+// an expert's segment (row_src < 0), are skipped: blocks walk the rows, so a capacity far above the rows that are present costs
+// nothing.  Bound by reading 4 F and writing 2 F bytes a row.  As tensor operations it was some ten passes in fp32 over the whole capacity:
+// 4 us instead of some 1,000 us for one token and 4 of 128 experts of 3,072 columns (16,512 rows of capacity); 18,600 rows of the same
+// width take 97 us (3.5 TB/s, bound by the exponential and the division).
+// A clamp lets a NaN through, like the tensor operation does.
+template <int KIND>
+__global__ void __launch_bounds__(256)
+gated_rows_kernel(const __nv_bfloat16* __restrict__ z, long long ldz, __nv_bfloat16* __restrict__ out, int ldo, int rows, int F, float limit,
+                  const int* __restrict__ total_rows, const int* __restrict__ row_src) {
+  bg::pdl_prologue((BG_FILE_TAG << 16) | __LINE__);
+  const int n = total_rows != nullptr ? min(rows, *total_rows) : rows;
+  for (int r = blockIdx.x; r < n; r += gridDim.x) {
+    if (row_src != nullptr && row_src[r] < 0) continue;
+    const __nv_bfloat16* zr = z + (size_t)r * ldz;
+    for (int v = threadIdx.x; v < F / 8; v += blockDim.x) {
+      const uint4 graw = *reinterpret_cast<const uint4*>(zr + v * 8), uraw = *reinterpret_cast<const uint4*>(zr + F + v * 8);
+      const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&graw);
+      const __nv_bfloat162* up = reinterpret_cast<const __nv_bfloat162*>(&uraw);
+      auto one = [&](float g, float u) {
+        if (KIND != 0) {
+          g = g > limit ? limit : g;
+          u = u > limit ? limit : u < -limit ? -limit : u;
+        }
+        return KIND == 1 ? (u + 1.f) * g / (1.f + expf(-1.702f * g)) : g / (1.f + expf(-g)) * u;
+      };
+      __align__(16) __nv_bfloat162 o[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 g = __bfloat1622float2(gp[i]), u = __bfloat1622float2(up[i]);
+        o[i] = __floats2bfloat162_rn(one(g.x, u.x), one(g.y, u.y));
+      }
+      *reinterpret_cast<uint4*>(out + (size_t)r * ldo + v * 8) = *reinterpret_cast<const uint4*>(o);
+    }
+  }
+}
+
 }  // namespace bg
 
 extern "C" {
+
+// z [rows, ldz] bf16 -> out [rows, ldo]; F, ldz and ldo multiples of 8.  total_rows, row_src: device, or null.
+int bg_gated_rows(int kind, const void* z, long long ldz, void* out, int ldo, int rows, int F, float limit, const int* total_rows,
+                  const int* row_src, int num_sms, cudaStream_t stream) {
+  using namespace bg;
+  if (rows <= 0 || F <= 0) return 0;
+  if (F % 8 || ldz % 8 || ldo % 8 || ldz < 2ll * F || ldo < F || kind < 0 || kind > 2) return -1;
+  const dim3 grid(min(rows, num_sms * 16)), block(min(256, (F / 8 + 31) / 32 * 32));
+  auto Z = reinterpret_cast<const __nv_bfloat16*>(z);
+  auto O = reinterpret_cast<__nv_bfloat16*>(out);
+  auto kern = kind == 0 ? gated_rows_kernel<0> : kind == 1 ? gated_rows_kernel<1> : gated_rows_kernel<2>;
+  bg::launch_pdl(kern, grid, block, 0, stream, Z, ldz, O, ldo, rows, F, limit, total_rows, row_src);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
 
 // logits: rows of E values, ldl apart; norm: weights divided by their sum, 1 unless K is 1, 2 always; group_max: a group counts with
 // its best expert instead of its best two

@@ -187,6 +187,30 @@ def combine(y: torch.Tensor, pos: torch.Tensor, weights: torch.Tensor, extra: Op
     return out
 
 
+def activation_on_kernel(gate_up: torch.Tensor) -> bool:
+    """Rows that the activation kernel reads: bf16 pairs of whole 16-byte columns."""
+    I = gate_up.shape[-1] // 2
+    return (gate_up.is_cuda and gate_up.dtype == torch.bfloat16 and gate_up.dim() == 2 and gate_up.shape[-1] == 2 * I and I % 8 == 0
+            and gate_up.stride(1) == 1 and gate_up.stride(0) % 8 == 0 and gate_up.data_ptr() % 16 == 0)
+
+
+def activation(gate_up: torch.Tensor, kind: str, limit: float = 0.0, offsets: Optional[torch.Tensor] = None,
+               row_src: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Gated activation of rows [gate | up]: ``kind`` swiglu_clamped, silu_limit (with a ``limit``), else SiLU(gate) * up.  Grouped rows:
+    those past ``offsets[-1]`` and padding rows (``row_src`` < 0) may stay undefined."""
+    if not activation_on_kernel(gate_up):
+        return _activation(gate_up, kind, limit)
+    R, I = gate_up.shape[0], gate_up.shape[1] // 2
+    out = torch.empty(R, I, dtype=gate_up.dtype, device=gate_up.device)
+    k = 1 if kind == "swiglu_clamped" else 2 if kind == "silu_limit" and limit > 0 else 0
+    rc = _ext.lib().bg_gated_rows(ctypes.c_int(k), _ext.ptr(gate_up), ctypes.c_longlong(gate_up.stride(0)), _ext.ptr(out),
+                                  ctypes.c_int(I), ctypes.c_int(R), ctypes.c_int(I), ctypes.c_float(7.0 if k == 1 else limit),
+                                  _ext.ptr(offsets[-1:] if offsets is not None else None), _ext.ptr(row_src),
+                                  ctypes.c_int(_ext.num_sms(gate_up.device)), _ext.stream())
+    _ext.check(rc, "bg_gated_rows")
+    return out
+
+
 def _activation(gate_up: torch.Tensor, kind: str, limit: float = 0.0) -> torch.Tensor:
     if kind == "swiglu_clamped":
         return ref.swiglu_clamped(gate_up)
@@ -195,6 +219,11 @@ def _activation(gate_up: torch.Tensor, kind: str, limit: float = 0.0) -> torch.T
         g, u = gate_up[..., :I].float().clamp(max=limit), gate_up[..., I:].float().clamp(-limit, limit)
         return (torch.nn.functional.silu(g) * u).to(gate_up.dtype)
     return ref.silu_mul(gate_up)
+
+
+def _grouped_on_kernels(x: torch.Tensor, ew: ExpertWeights) -> bool:
+    """Unquantised experts on the grouped bf16 GEMM."""
+    return x.is_cuda and x.dtype == torch.bfloat16 and ew.w13.shape[2] % 64 == 0 and ew.w2.shape[2] % 64 == 0
 
 
 def grouped_experts(xq, xs, offsets: torch.Tensor, ew: ExpertWeights, x_dense: Optional[torch.Tensor] = None,
@@ -233,16 +262,15 @@ def grouped_experts(xq, xs, offsets: torch.Tensor, ew: ExpertWeights, x_dense: O
         else:
             with timer.timed("moe.s1_gemm"):
                 gu = grouped_w4(x, ew.w13, ew.w13_s, offsets)
-            act = _activation(gu, ew.activation, ew.act_limit).to(x.dtype)
+            act = activation(gu, ew.activation, ew.act_limit, offsets, row_src).to(x.dtype)
         with timer.timed("moe.s3_gemm"):
             return grouped_w4(act, ew.w2, ew.w2_s, offsets)
     # unquantised experts
     x = x_dense
-    if (x.is_cuda and x.dtype == torch.bfloat16 and counts is not None and ew.w13.shape[2] % 64 == 0
-            and ew.w2.shape[2] % 64 == 0):
+    if counts is not None and _grouped_on_kernels(x, ew):
         with timer.timed("moe.s1_gemm"):
             gu = gemm.grouped_bf16_gemm(x, ew.w13, offsets, counts)
-        act = _activation(gu, ew.activation, ew.act_limit).contiguous()
+        act = activation(gu, ew.activation, ew.act_limit, offsets, row_src).contiguous()
         with timer.timed("moe.s3_gemm"):
             return gemm.grouped_bf16_gemm(act, ew.w2, offsets, counts)
     out = torch.zeros(x.shape[0], ew.w2.shape[1], dtype=x.dtype, device=x.device)
@@ -271,6 +299,8 @@ def experts_forward(hidden: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.
         pairs = topk_idx.shape[0] * topk_idx.shape[1]
         if gemm.use_swapab(pairs / max(expert_hi - expert_lo, 1), ew.w13.shape[1], ew.w13.shape[2]):
             align = 32
+    elif ew.quant == "none" and _grouped_on_kernels(hidden, ew):
+        align = 8                          # the grouped bf16 GEMM takes real row counts: segments only need aligned rows
     with timer.timed("moe.permute"):
         src, pos, offsets = permute(topk_idx, expert_lo, expert_hi, num_valid, align=align)
     if ew.quant == "fp8_block":
@@ -281,9 +311,15 @@ def experts_forward(hidden: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.
                             row_src=src if counts is not None else None,
                             rows_hint=(hidden.shape[0] * topk_idx.shape[1] if counts is not None else None))
     else:
-        rows = hidden[src.clamp_min(0).long()]
-        rows = torch.where((src >= 0).unsqueeze(-1), rows, torch.zeros_like(rows))
-        y = grouped_experts(None, None, offsets, ew, x_dense=rows, counts=getattr(offsets, "real_counts", None))
+        if hidden.is_cuda and hidden.dtype == torch.bfloat16 and hidden.shape[1] % 8 == 0:
+            # a pair's row goes straight to its place; padding rows of a segment stay undefined (no kept row depends on another)
+            with timer.timed("moe.gather"):
+                rows, _ = residual.moe_gather(hidden.contiguous(), pos, topk_w.float().contiguous(), src.shape[0])
+        else:
+            rows = hidden[src.clamp_min(0).long()]
+            rows = torch.where((src >= 0).unsqueeze(-1), rows, torch.zeros_like(rows))
+        y = grouped_experts(None, None, offsets, ew, x_dense=rows, counts=getattr(offsets, "real_counts", None),
+                            row_src=src if rows.is_cuda else None)
     with timer.timed("moe.combine"):
         if before_combine is not None:
             before_combine()

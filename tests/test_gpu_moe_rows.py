@@ -1,0 +1,73 @@
+"""Grouped rows of unquantised and 4-bit experts: the activation kernel, and the expert stack around it."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _plain(z, kind, limit):
+    g, u = z.double().chunk(2, -1)
+    if kind == "silu":
+        return g * torch.sigmoid(g) * u
+    g, u = g.clamp(max=limit), u.clamp(-limit, limit)
+    return (u + 1) * g * torch.sigmoid(1.702 * g) if kind == "swiglu_clamped" else g * torch.sigmoid(g) * u
+
+
+@pytest.mark.parametrize("kind,limit", [("silu", 0.0), ("swiglu_clamped", 7.0), ("silu_limit", 2.5)])
+@pytest.mark.parametrize("rows,F,pad", [(1, 8, 0), (3, 72, 16), (300, 3072, 0), (4000, 264, 8)])
+def test_activation_rows(kind, limit, rows, F, pad):
+    from batchgen_b200.ops import moe
+    g = torch.Generator().manual_seed(rows + F)
+    z = (torch.randn(rows, 2 * F + pad, generator=g) * 4).bfloat16()
+    z[0, :4] = torch.tensor([float("nan"), float("inf"), -float("inf"), 100.0])
+    z[0, F:F + 4] = torch.tensor([1.0, 2.0, 3.0, float("nan")])
+    present = max(1, rows - 5)
+    src = torch.arange(rows, dtype=torch.int32)
+    src[1::7] = -1
+    offsets = torch.tensor([0, present], dtype=torch.int32)
+    d = z.cuda()[:, :2 * F]
+    want = _plain(z[:, :2 * F], kind, limit)
+    for off, s in ((None, None), (offsets.cuda(), src.cuda())):
+        got = moe.activation(d, kind, limit, off, s).double().cpu()
+        keep = torch.ones(rows, dtype=torch.bool) if off is None else (src >= 0) & (torch.arange(rows) < present)
+        a, b = got[keep], want[keep]
+        fine = torch.isfinite(b)
+        assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(a[~fine & ~torch.isnan(b)], b[~fine & ~torch.isnan(b)])
+        # one rounding to 8 significant bits, and fp32 arithmetic: a few 2^-24
+        assert ((a - b).abs()[fine] <= b.abs()[fine] * (2 ** -8 + 1e-5) + 1e-30).all()
+
+
+@pytest.mark.parametrize("T", [1, 5, 130])
+@pytest.mark.parametrize("quant", ["none", "mxfp4"])
+@pytest.mark.parametrize("kind", ["silu", "swiglu_clamped"])
+def test_expert_stack(T, quant, kind):
+    """Pairs of a few tokens over experts of which some stay empty, padding tokens, a row added at the sum."""
+    from batchgen_b200.ops import _ext, moe, mxfp4
+    E, K, H, I = 9, 3, 192, 128
+    g = torch.Generator().manual_seed(T)
+    w13, w2 = torch.randn(E, 2 * I, H, generator=g) * 0.1, torch.randn(E, H, I, generator=g) * 0.1
+    x, extra = torch.randn(T, H, generator=g).bfloat16(), torch.randn(T, H, generator=g).bfloat16()
+    idx = torch.stack([torch.randperm(E - 2, generator=g)[:K] for _ in range(T)]).int()
+    w = torch.rand(T, K, generator=g)
+    if quant == "none":
+        ew = moe.ExpertWeights(w13.bfloat16().cuda(), w2.bfloat16().cuda(), activation=kind)
+        f13, f2 = w13.bfloat16().double(), w2.bfloat16().double()
+    else:
+        q13, s13 = mxfp4.quantize(w13)
+        q2, s2 = mxfp4.quantize(w2)
+        f13, f2 = mxfp4.dequantize(q13, s13, torch.float32).double(), mxfp4.dequantize(q2, s2, torch.float32).double()
+        ew = moe.ExpertWeights(q13.cuda(), q2.cuda(), s13.cuda(), s2.cuda(), quant="mxfp4", activation=kind).to_device_layout()
+    valid = T - T // 3
+    got = moe.experts_forward(x.cuda(), torch.where(torch.arange(T).unsqueeze(1) < valid, idx, -1).int().cuda(), w.cuda(), ew, 0, E,
+                              extra=extra.cuda(), num_valid=torch.tensor([valid], dtype=torch.int32).cuda())
+    torch.cuda.synchronize()
+    _ext.check_status()
+    want = extra.double()
+    for t in range(valid):
+        for k in range(K):
+            e = int(idx[t, k])
+            z = _plain((x[t].double() @ f13[e].t()).bfloat16(), kind, 7.0).bfloat16().double()
+            want[t] += w[t, k].double() * (z @ f2[e].t()).bfloat16().double()
+    err = (got.double().cpu() - want).norm() / want.norm()
+    # four roundings to bf16 on the way (pre-activation, activation, expert row, sum), each some 2^-9 of its value
+    assert err < 4 * 2 ** -9, err
