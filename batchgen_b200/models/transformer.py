@@ -413,7 +413,7 @@ class Transformer:
             ref.kv_cache_write(kvc, torch.cat([k.reshape(T, -1), v.reshape(T, -1)], -1), meta.slot_mapping)
         if meta.mode == "decode" and x.is_cuda:
             # paged flash-decoding kernel: lengths stay on the device (graph capturable)
-            o = attn_ops.gqa_decode(q.contiguous(), kvc, meta.block_table, meta.seqlens, Hkv, cfg.softmax_scale,
+            o = attn_ops.gqa_decode(q, kvc, meta.block_table, meta.seqlens, Hkv, cfg.softmax_scale,
                                     window=window, sinks=lw.sinks)
             return linear(o.reshape(T, -1), lw.wo)
         out = torch.zeros(T, Hq, D, dtype=x.dtype, device=x.device)

@@ -135,9 +135,6 @@ def gqa_prefill(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor,
     _ext.check(rc, "bg_gqa_prompt_fine")
 
 
-_GQA_SCRATCH = {}
-
-
 def gqa_decode(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, seqlens: torch.Tensor, num_kv_heads: int,
                scale: float, window: int = 0, sinks: Optional[torch.Tensor] = None, num_splits: int = 0) -> torch.Tensor:
     """Paged GQA decode.  q [B, Hq, D]; cache [P, page, 2 * Hkv * D] (K heads then V heads per token);
@@ -157,30 +154,24 @@ def gqa_decode(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, 
             vs = kv[:, num_kv_heads * D:].reshape(L, num_kv_heads, D)
             out[b:b + 1] = ref.gqa_attention(q[b:b + 1], ks, vs, scale, q_start=L - 1, window=window, sinks=sinks)
         return out
-    q = q.contiguous()
+    if not (q.stride(2) == 1 and q.stride(1) == D and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0):
+        q = q.contiguous()
     if num_splits <= 0:
-        ctas = B * num_kv_heads
-        sms = _ext.num_sms(q.device)
-        max_tiles = max(1, (block_table.shape[1] * page) // 64)
-        if window > 0:
-            max_tiles = min(max_tiles, window // 64 + 2)
-        num_splits = max(1, min(16, -(-2 * sms // ctas), max_tiles))
-    out = torch.empty_like(q)
+        from . import talking
+        keys = block_table.shape[1] * page
+        num_splits = talking._ranges(B * num_kv_heads, min(keys, window) if window > 0 else keys, _ext.num_sms(q.device))
+    out = torch.empty(B, Hq, D, dtype=q.dtype, device=q.device)
     part_o = part_ml = None
     if num_splits > 1:
-        key = (str(q.device), B * Hq * num_splits, D)
-        buf = _GQA_SCRATCH.get(key)
-        if buf is None:
-            buf = (torch.empty(B * Hq * num_splits * D, dtype=torch.float32, device=q.device),
-                   torch.empty(B * Hq * num_splits * 2, dtype=torch.float32, device=q.device))
-            _GQA_SCRATCH[key] = buf
-        part_o, part_ml = buf
-    rc = _ext.lib().bg_gqa_decode(_ext.ptr(q), _ext.ptr(cache), _ext.ptr(block_table), ctypes.c_int(block_table.stride(0)),
-                                  _ext.ptr(seqlens), _ext.ptr(sinks.float().contiguous() if sinks is not None else None),
-                                  _ext.ptr(out), _ext.ptr(part_o), _ext.ptr(part_ml), ctypes.c_int(B), ctypes.c_int(Hq),
-                                  ctypes.c_int(num_kv_heads), ctypes.c_int(D), ctypes.c_int(page), ctypes.c_int(window),
-                                  ctypes.c_float(scale), ctypes.c_int(num_splits), _ext.stream())
-    _ext.check(rc, "bg_gqa_decode", kernels=2 if num_splits > 1 else 1)
+        part_o = torch.empty(B * num_splits * Hq * D, dtype=torch.float32, device=q.device)
+        part_ml = torch.empty(B * num_splits * Hq * 2, dtype=torch.float32, device=q.device)
+    sinks = sinks.float().contiguous() if sinks is not None else None
+    rc = _ext.lib().bg_gqa_rows(_ext.ptr(q), ctypes.c_int(q.stride(0)), _ext.ptr(cache), _ext.ptr(block_table),
+                                ctypes.c_int(block_table.stride(0)), _ext.ptr(seqlens), _ext.ptr(sinks), _ext.ptr(out),
+                                _ext.ptr(part_o), _ext.ptr(part_ml), ctypes.c_int(B), ctypes.c_int(Hq), ctypes.c_int(num_kv_heads),
+                                ctypes.c_int(D), ctypes.c_int(page), ctypes.c_int(window), ctypes.c_float(scale),
+                                ctypes.c_int(num_splits), _ext.stream())
+    _ext.check(rc, "bg_gqa_rows", kernels=2 if num_splits > 1 else 1)
     return out
 
 

@@ -6,6 +6,12 @@
 // folded in before the rounding) with the keys on the tensor cores (mma m16n8k16: with a handful of heads per key head the 128-row
 // tcgen05 shapes would be idle rows), takes the online softmax in registers and feeds the probabilities straight into P.V.
 // Memory-bound by design: every key and value byte is read once per key head.
+//
+// FINE form (models whose cached attention keeps fp32 probabilities): queries come in bf16 and go into the product as they are, the
+// scale meets the fp32 scores, and a probability is multiplied in two bf16 parts (2^-17 of it is lost).  The second product with V costs
+// nothing that shows next to the bytes.  It took the place of a kernel that did both products on the CUDA cores, a thread per key
+// and a block-wide barrier five times a tile: 160 rows of up to 4,096 tokens, 64 heads of 64 over 8 key heads, one layer of all keys and
+// one with a window of 128, 2,957 -> 255 us (the bytes take 135); one row of 900 tokens 69 -> 12 us.
 #pragma once
 
 namespace bg {
@@ -43,7 +49,7 @@ __host__ __device__ inline int shared_bytes(int dp, int dvp, int heads) {
 }
 
 // KD, VD: upper bounds of the 16-wide steps of a key / value head; HI: more than 8 heads in the CTA
-template <int KD, int VD, bool HI>
+template <int KD, int VD, bool HI, bool FINE>
 __global__ void __launch_bounds__(kRowWarps * 32, 2) gqa_rows_kernel(const Params p, int groups) {
   bg::pdl_prologue((BG_FILE_TAG << 16) | __LINE__);
   extern __shared__ __align__(16) char sm_raw[];
@@ -116,7 +122,10 @@ __global__ void __launch_bounds__(kRowWarps * 32, 2) gqa_rows_kernel(const Param
   for (int i = tid; i < 16 * kb / 16; i += kRowWarps * 32) {
     const int h = i * 16 / kb, e = i * 16 % kb / 2;                // 8 channels
     __align__(16) __nv_bfloat162 v[4] = {};
-    if (h < nh && e < dp) {
+    if (FINE) {
+      if (h < nh && e < dp)
+        *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(p.qb + (size_t)t * p.ldq + (h0 + h) * dp + e);
+    } else if (h < nh && e < dp) {
       const float* x = p.q + (size_t)t * p.ldq + (h0 + h) * dp;
       float f[8];
       load8(x + e, f);
@@ -159,12 +168,12 @@ __global__ void __launch_bounds__(kRowWarps * 32, 2) gqa_rows_kernel(const Param
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) s[n][j] += s2[n][j];
+      for (int j = 0; j < 4; ++j) s[n][j] = FINE ? (s[n][j] + s2[n][j]) * p.scale_log2 : s[n][j] + s2[n][j];
 #pragma unroll
       for (int j = 0; j < 2; ++j)
         if (!seen(pos + n * 8 + j)) s[n][j] = s[n][2 + j] = -INFINITY;
     }
-    uint32_t pa[4] = {0, 0, 0, 0};
+    uint32_t pa[4] = {0, 0, 0, 0}, pr[4] = {0, 0, 0, 0};           // FINE: pr is what the rounding of pa left
     float al[2] = {1.f, 1.f};
 #pragma unroll
     for (int i = 0; i < (HI ? 2 : 1); ++i) {
@@ -174,9 +183,18 @@ __global__ void __launch_bounds__(kRowWarps * 32, 2) gqa_rows_kernel(const Param
       const float mn = fmaxf(m[i], mt), sub = mn == -INFINITY ? 0.f : mn;
       al[i] = exp2f(m[i] - sub);
       m[i] = mn;
-      const __nv_bfloat162 lo = __floats2bfloat162_rn(exp2f(s[0][2 * i] - sub), exp2f(s[0][2 * i + 1] - sub));
-      const __nv_bfloat162 hi = __floats2bfloat162_rn(exp2f(s[1][2 * i] - sub), exp2f(s[1][2 * i + 1] - sub));
-      l[i] = l[i] * al[i] + (__low2float(lo) + __high2float(lo)) + (__low2float(hi) + __high2float(hi));
+      const float e0 = exp2f(s[0][2 * i] - sub), e1 = exp2f(s[0][2 * i + 1] - sub);
+      const float e2 = exp2f(s[1][2 * i] - sub), e3 = exp2f(s[1][2 * i + 1] - sub);
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(e0, e1), hi = __floats2bfloat162_rn(e2, e3);
+      if (FINE) {
+        const __nv_bfloat162 rl = __floats2bfloat162_rn(e0 - __low2float(lo), e1 - __high2float(lo));
+        const __nv_bfloat162 rh = __floats2bfloat162_rn(e2 - __low2float(hi), e3 - __high2float(hi));
+        pr[i] = *reinterpret_cast<const uint32_t*>(&rl);
+        pr[2 + i] = *reinterpret_cast<const uint32_t*>(&rh);
+        l[i] = l[i] * al[i] + (e0 + e1) + (e2 + e3);
+      } else {
+        l[i] = l[i] * al[i] + (__low2float(lo) + __high2float(lo)) + (__low2float(hi) + __high2float(hi));
+      }
       pa[i] = *reinterpret_cast<const uint32_t*>(&lo);
       pa[2 + i] = *reinterpret_cast<const uint32_t*>(&hi);
     }
@@ -196,6 +214,10 @@ __global__ void __launch_bounds__(kRowWarps * 32, 2) gqa_rows_kernel(const Param
         if (n0 + n < vsteps) {
           mma16816(o[2 * (n0 + n)], pa, vf[n][0], vf[n][1]);
           mma16816(o[2 * (n0 + n) + 1], pa, vf[n][2], vf[n][3]);
+          if (FINE) {
+            mma16816(o[2 * (n0 + n)], pr, vf[n][0], vf[n][1]);
+            mma16816(o[2 * (n0 + n) + 1], pr, vf[n][2], vf[n][3]);
+          }
         }
     }
     slot = slot + 1 == kStages ? 0 : slot + 1;
@@ -248,28 +270,29 @@ __global__ void __launch_bounds__(kRowWarps * 32, 2) gqa_rows_kernel(const Param
   }
 }
 
-template <int KD, int VD, bool HI>
+template <int KD, int VD, bool HI, bool FINE>
 static int launch_as(const Params& p, int R, int groups, cudaStream_t stream) {
   const size_t smem = shared_bytes(p.dp, p.dvp, min(16, p.H / p.G));
   static DeviceOnce once;
-  auto kern = gqa_rows_kernel<KD, VD, HI>;
+  auto kern = gqa_rows_kernel<KD, VD, HI, FINE>;
   if (!ensure_dynamic_smem(kern, shared_bytes(16 * KD, 16 * VD, 16), once)) return -4;
   bg::launch_pdl(kern, dim3(R, p.G * groups, p.n_splits), dim3(kRowWarps * 32), smem, stream, p, groups);
   if (p.n_splits > 1) bg::launch_pdl(merge_kernel<__nv_bfloat16>, dim3(R, p.H), dim3(64), 0, stream, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
-template <int KD, int VD>
+template <int KD, int VD, bool FINE>
 static int launch_heads(const Params& p, int R, int groups, cudaStream_t stream) {
-  return p.H / p.G > 8 ? launch_as<KD, VD, true>(p, R, groups, stream) : launch_as<KD, VD, false>(p, R, groups, stream);
+  return p.H / p.G > 8 ? launch_as<KD, VD, true, FINE>(p, R, groups, stream) : launch_as<KD, VD, false, FINE>(p, R, groups, stream);
 }
 static bool supported(const Params& p) {
   const int groups = (p.H / p.G + 15) / 16;
   return p.talk == nullptr && p.v_col0 == p.G * p.dp && p.dp <= kMaxWidth && p.dvp <= kMaxWidth && (long long)p.G * groups <= 65535;
 }
+template <bool FINE>
 static int launch(const Params& p, int R, cudaStream_t stream) {
   const int groups = (p.H / p.G + 15) / 16;
-  if (p.dp <= 64 && p.dvp <= 64) return launch_heads<4, 4>(p, R, groups, stream);
-  return launch_heads<8, 8>(p, R, groups, stream);
+  if (p.dp <= 64 && p.dvp <= 64) return launch_heads<4, 4, FINE>(p, R, groups, stream);
+  return launch_heads<8, 8, FINE>(p, R, groups, stream);
 }
 
 }  // namespace plain

@@ -52,7 +52,7 @@ struct Params {
   int ld_gate, gate_cols;       // columns of a head: 1 or dvp
   const float* sinks;           // [H] or null: all zero
   int v_col0;                   // first value column of a cache row
-  const __nv_bfloat16* qb;      // latent_rows.cuh: [R, H, row] queries
+  const __nv_bfloat16* qb;      // latent_rows.cuh: [R, H, row] queries; gqa_rows.cuh, FINE: [R, ldq] queries
   int* status;
 };
 
@@ -480,7 +480,7 @@ int bg_talk_rows(int dt, const float* q, int ldq, const float* talk, const void*
   const int ni = (items + kThreads - 1) / kThreads;
   if (ni > 8 && !(dt == 0 && plain::supported(p))) return -1;
   if (dt == 0) {
-    if (plain::supported(p)) return plain::launch(p, R, stream);
+    if (plain::supported(p)) return plain::launch<false>(p, R, stream);
     if (ni == 1) return launch_rows<__nv_bfloat16, 1>(p, R, stream);
     if (ni == 2) return launch_rows<__nv_bfloat16, 2>(p, R, stream);
     if (ni <= 4) return launch_rows<__nv_bfloat16, 4>(p, R, stream);
@@ -490,6 +490,25 @@ int bg_talk_rows(int dt, const float* q, int ldq, const float* talk, const void*
   if (ni == 2) return launch_rows<float, 2>(p, R, stream);
   if (ni <= 4) return launch_rows<float, 4>(p, R, stream);
   return launch_rows<float, 8>(p, R, stream);
+}
+
+// Decode attention of bf16 queries q [B, ldq] (H heads of D = 64 or 128 columns, turned and unscaled) over cached rows of G key heads,
+// then G value heads; up to 16 heads a key head; probabilities in two parts.  lens [B]: keys a row sees (0: zero output); window 0: all
+// of them; sinks [H] fp32 or null; scratch for n_splits > 1: part_o [B, n_splits, H, D], part_ml [B, n_splits, H, 2] fp32.
+int bg_gqa_rows(const void* q, int ldq, const void* cache, const int* block_table, int bt_stride, const int* lens, const float* sinks,
+                void* out, float* part_o, float* part_ml, int B, int H, int G, int D, int page, int window, float scale,
+                int n_splits, cudaStream_t stream) {
+  using namespace bg::talk;
+  if (B <= 0) return 0;
+  if ((D != 64 && D != 128) || G <= 0 || H % G || H / G > 16 || H > 65535 || ldq % 8 || ldq < H * D || page <= 0 || (64 % page && page % 64) ||
+      window < 0 || n_splits < 1 || n_splits > 65535 || (n_splits > 1 && (part_o == nullptr || part_ml == nullptr)))
+    return -1;
+  Params p = {};
+  p.qb = reinterpret_cast<const __nv_bfloat16*>(q); p.ldq = ldq; p.cache = cache; p.page = page; p.row = 2 * G * D;
+  p.page_stride = (long long)page * p.row; p.block_table = block_table; p.bt_stride = bt_stride; p.lens = lens; p.out = out; p.ldo = H * D;
+  p.part_o = part_o; p.part_ml = part_ml; p.H = H; p.G = G; p.dp = p.dvp = D; p.v_col0 = G * D; p.window = window; p.n_splits = n_splits;
+  p.sink = sinks != nullptr; p.sinks = sinks; p.scale_log2 = scale * kLog2e; p.out_scale = 1.f; p.gate_cols = 1;
+  return plain::launch<true>(p, B, stream);
 }
 
 int bg_talk_kv_write(int dt, const float* kv, int ld, const long long* slots, void* cache, long long page_stride, int page,

@@ -100,3 +100,40 @@ def test_gqa_prompt(Hq, Hkv, D, page, interleaved, bias, window, use_sinks):
         err = (out[a:e].cpu().double() - o).abs()
         # a value rounded to 8 significant bits: 2^-8 of it; fp32 sums of up to 1,000 terms (1,000 * 2^-24) and p of 2^-17: 7e-5
         assert (err <= o.abs() * 2 ** -8 + 7e-5 * v.abs().max()).all(), (i, err.max())
+
+
+@pytest.mark.parametrize("Hq,Hkv,D,page", [(16, 1, 64, 64), (12, 4, 128, 16), (24, 2, 128, 128), (7, 7, 64, 32)])
+@pytest.mark.parametrize("window,use_sinks,splits", [(0, False, 1), (0, True, 0), (33, True, 2), (1, False, 3), (700, False, 5)])
+def test_gqa_decode_fine(Hq, Hkv, D, page, window, use_sinks, splits):
+    """Rows of every length class, one without keys, queries in columns of a wider tensor, stale rows that are not finite."""
+    from batchgen_b200.ops import _ext, attention
+    g = torch.Generator().manual_seed(Hq + page + splits)
+    lens = [1, 15, 16, 17, 0, 64, 65, 700, 1023]
+    B = len(lens)
+    need = [-(-n // page) for n in lens]
+    order = torch.randperm(sum(need), generator=g).tolist()
+    cache = torch.full((sum(need), page, 2 * Hkv * D), float("nan"), dtype=torch.bfloat16)
+    bt = torch.zeros(B, max(need), dtype=torch.int32)
+    rows = []
+    for i, n in enumerate(lens):
+        bt[i, :need[i]] = torch.tensor([order.pop() for _ in range(need[i])], dtype=torch.int32)
+        p = torch.arange(n)
+        rows.append(torch.randn(n, 2 * Hkv * D, generator=g).bfloat16())
+        cache.view(-1, 2 * Hkv * D)[bt[i].long()[p // page] * page + p % page] = rows[-1]
+    wide = torch.randn(B, (Hq + 2) * D, generator=g).bfloat16()
+    sinks = torch.randn(Hq, generator=g) if use_sinks else None
+    got = attention.gqa_decode(wide.cuda()[:, :Hq * D].unflatten(1, (Hq, D)), cache.cuda(), bt.cuda(), torch.tensor(lens, dtype=torch.int32).cuda(),
+                               Hkv, D ** -0.5, window=window, sinks=sinks.cuda() if use_sinks else None, num_splits=splits).cpu().double()
+    _ext.check_status()
+    for i, n in enumerate(lens):
+        if n == 0:
+            assert (got[i] == 0).all()
+            continue
+        r = rows[i][max(0, n - window) if window else 0:].double()
+        k, v = (t.view(-1, Hkv, D).repeat_interleave(Hq // Hkv, 1) for t in r.split(Hkv * D, 1))
+        s = torch.einsum("hd,lhd->hl", wide[i, :Hq * D].view(Hq, D).double(), k) * D ** -0.5
+        if use_sinks:
+            s = torch.cat([s, sinks.double().view(Hq, 1)], -1)
+        o = torch.einsum("hl,lhd->hd", s.softmax(-1)[:, :r.shape[0]], v)
+        # a value rounded to 8 significant bits: 2^-8 of it; fp32 sums of up to 1,023 terms (1,023 * 2^-24) and p of 2^-17: 7e-5
+        assert ((got[i] - o).abs() <= o.abs() * 2 ** -8 + 7e-5 * v.abs().max()).all(), i
