@@ -2,7 +2,7 @@
 on q, k, v, L2-normalised q / k, a per-channel decay gate and a sigmoid-gated RMSNorm on the output.
 
 ``kda_forward`` serves prefill (packed sequences, optional continuation from a stored state) and decode (one
-token per sequence) alike.  On CUDA it launches ``csrc/kda.cu``; on CPU (and as the oracle of the tests) it
+token per sequence) alike.  On CUDA it launches ``csrc/kda.cu``: token by token, or for longer pieces in chunks of 64 tokens; on CPU (and as the oracle of the tests) it
 runs the recurrence in fp32.  State lives in two pools indexed by a sequence's state slot:
 
     conv_state [slots, 3 * H * D, 3] fp32   the last three raw inputs of each q / k / v channel, oldest first
@@ -98,6 +98,46 @@ def kda_chunk_ref(q, k, v, g, beta, S, scale: float, chunk: int = 64):
     return out
 
 
+CHUNK = 64
+CHUNK_MIN_TOKENS = 48                 # shorter pieces never go through the chunk form
+_CHUNK_FLOATS = (5 * CHUNK + 1) * 128   # scratch of a (chunk, head)
+_CHUNK_SCRATCH = 1 << 30              # bytes of scratch a round of chunks may take
+
+
+def chunk_form_pays(lens: Sequence[int], heads: int, sms: int) -> bool:
+    """Whether pieces of ``lens`` tokens are faster in chunks.  Token by token costs 2.0 us for each token of the longest piece, or 2.6 us a
+    token and round of CTAs (two fit an SM) when the (piece, head) pairs fill the SMs; chunks cost 0.57 us a (chunk, head) on 148 SMs and 110
+    us to start (32 heads of 128, tokens / chunks: 1 x 64 149 / 142 us, 1 x 4,096 8,086 / 1,228; 4 x 512 1,061 / 686; 8 x 1,024 2,501 /
+    2,249; 32 x 64 667 / 736; 200 x 32 1,810 / 3,859)."""
+    if not lens:
+        return False
+    tokens = 45 + max(2.0 * max(lens), 2.6 * heads * sum(lens) / (2 * sms))
+    return 110 + 0.57 * heads * sum(-(-n // CHUNK) for n in lens) * 148 / sms < tokens
+
+
+def chunk_plan(cu: Sequence[int], min_tokens: int, most_items: int):
+    """Rounds of chunks of the pieces of at least ``min_tokens``: a list of (items, seqs) with items (sequence, first token, tokens,
+    tokens of the piece before it) and seqs (sequence, first item, items, 1 at the start of a piece), at most ``most_items`` items a
+    round, a sequence's chunks in order.  Longer pieces first: their chains take longest."""
+    order = sorted((i for i in range(len(cu) - 1) if cu[i + 1] - cu[i] >= max(min_tokens, 1)), key=lambda i: cu[i] - cu[i + 1])
+    rounds, items, seqs = [], [], []
+    for i in order:
+        a, b = int(cu[i]), int(cu[i + 1])
+        t = a
+        while t < b:
+            if len(items) == most_items:
+                rounds.append((items, seqs))
+                items, seqs = [], []
+            n = min(most_items - len(items), -(-(b - t) // CHUNK))
+            seqs.append((i, len(items), n, int(t == a)))
+            for _ in range(n):
+                items.append((i, t, min(CHUNK, b - t), t - a))
+                t = min(t + CHUNK, b)
+    if items:
+        rounds.append((items, seqs))
+    return rounds
+
+
 def _forward_ref(qkv, f, beta, z, p: KDAParams, conv_state, rec_state, slots, cu, has_initial, H, D, scale, eps):
     T = qkv.shape[0]
     HD = H * D
@@ -146,11 +186,29 @@ def kda_forward(qkv: torch.Tensor, f: torch.Tensor, beta: torch.Tensor, z: torch
     hi_t = None if has_initial is None else (
         has_initial if isinstance(has_initial, torch.Tensor) else torch.tensor([int(x) for x in has_initial], dtype=torch.int32, device=dev))
     out = torch.empty(qkv.shape[0], H * D, dtype=torch.bfloat16, device=dev)
-    rc = _ext.lib().bg_kda_forward(
-        _ext.ptr(qkv), ctypes.c_int(qkv.stride(0)), _ext.ptr(f), ctypes.c_int(f.stride(0)), _ext.ptr(beta),
-        ctypes.c_int(beta.stride(0)), _ext.ptr(z), ctypes.c_int(z.stride(0)), _ext.ptr(p.conv_w), _ext.ptr(p.conv_b),
-        _ext.ptr(p.A_log), _ext.ptr(p.dt_bias), _ext.ptr(p.norm_w), _ext.ptr(conv_state), _ext.ptr(rec_state),
-        _ext.ptr(cu_t), _ext.ptr(slots), _ext.ptr(hi_t), _ext.ptr(out), ctypes.c_int(nseq), ctypes.c_int(H),
-        ctypes.c_int(D), ctypes.c_float(scale), ctypes.c_float(eps), _ext.stream())
-    _ext.check(rc, "bg_kda_forward")
+    rounds = []
+    if D == 128 and cu_seqlens is not None and not isinstance(cu_seqlens, torch.Tensor) and z.stride(0) % 4 == 0 and z.data_ptr() % 8 == 0:
+        long = [b - a for a, b in zip(cu_seqlens, cu_seqlens[1:]) if b - a >= CHUNK_MIN_TOKENS]
+        if chunk_form_pays(long, H, _ext.num_sms(dev)):
+            rounds = chunk_plan(cu_seqlens, CHUNK_MIN_TOKENS, max(1, _CHUNK_SCRATCH // (4 * _CHUNK_FLOATS * H)))
+    short = (1 << 31) - 1                                 # tokens of the longest piece that goes token by token
+    if rounds:
+        lens = [b - a for a, b in zip(cu_seqlens, cu_seqlens[1:])]
+        short = CHUNK_MIN_TOKENS - 1 if any(0 < n < CHUNK_MIN_TOKENS for n in lens) else 0
+        most = max(len(it) for it, _ in rounds)
+        scratch = torch.empty(most * H * _CHUNK_FLOATS, dtype=torch.float32, device=dev)
+        tables = torch.tensor([r for it, sq in rounds for r in it + sq], dtype=torch.int32, device=dev)
+    at = 0
+    for n, (it, sq) in enumerate(rounds or [((), ())]):
+        last = n == max(len(rounds), 1) - 1
+        rc = _ext.lib().bg_kda_forward(
+            _ext.ptr(qkv), ctypes.c_int(qkv.stride(0)), _ext.ptr(f), ctypes.c_int(f.stride(0)), _ext.ptr(beta),
+            ctypes.c_int(beta.stride(0)), _ext.ptr(z), ctypes.c_int(z.stride(0)), _ext.ptr(p.conv_w), _ext.ptr(p.conv_b),
+            _ext.ptr(p.A_log), _ext.ptr(p.dt_bias), _ext.ptr(p.norm_w), _ext.ptr(conv_state), _ext.ptr(rec_state),
+            _ext.ptr(cu_t), _ext.ptr(slots), _ext.ptr(hi_t), _ext.ptr(out), ctypes.c_int(nseq), ctypes.c_int(H),
+            ctypes.c_int(D), ctypes.c_float(scale), ctypes.c_float(eps), _ext.ptr(tables[at:] if it else None), ctypes.c_int(len(it)),
+            _ext.ptr(tables[at + len(it):] if it else None), ctypes.c_int(len(sq)), ctypes.c_int(short if last else 0),
+            _ext.ptr(scratch if it else None), _ext.stream())
+        _ext.check(rc, "bg_kda_forward", kernels=(3 if it else 0) + int(last and short > 0))
+        at += len(it) + len(sq)
     return out

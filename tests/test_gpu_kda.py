@@ -94,3 +94,78 @@ def test_model_with_kda_layers_on_gpu_matches_cpu():
     set_library_fallback(False)
     # prefill logits and the first decode step (same tokens fed as long as greedy picks agree; compare what is comparable)
     assert _rel(logits["cuda"][0], logits["cpu"][0]) < 0.06
+
+
+def _recurrence64(qkv, f, beta, z, p, conv, rec, slots, cu, has, H, D, scale, eps):
+    """The recurrence token by token in 64 bits; conv and rec [slots, ..] are updated."""
+    HD = H * D
+    out = torch.zeros(qkv.shape[0], HD, dtype=torch.float64)
+    d = lambda t: t.double().cpu()  # noqa: E731
+    w, b, A, dt, nw = d(p.conv_w), d(p.conv_b), d(p.A_log), d(p.dt_bias), d(p.norm_w)
+    for i, s in enumerate(slots):
+        a, e = cu[i], cu[i + 1]
+        if s < 0 or e <= a:
+            continue
+        if not has[i]:
+            conv[s].zero_()
+            rec[s].zero_()
+        full = torch.cat([conv[s].t(), d(qkv[a:e])], 0)
+        y = torch.nn.functional.silu(sum(full[j:j + e - a] * w[:, j] for j in range(4)) + b)
+        conv[s] = full[-3:].t()
+        q, k, v = (t.view(-1, H, D) for t in y.chunk(3, -1))
+        q = q * torch.rsqrt(q.square().sum(-1, keepdim=True) + 1e-6) * scale
+        k = k * torch.rsqrt(k.square().sum(-1, keepdim=True) + 1e-6)
+        g = (-A.exp().view(1, H, 1) * torch.nn.functional.softplus(d(f[a:e]) + dt).view(-1, H, D)).exp()
+        bt, S = d(beta[a:e]).sigmoid(), rec[s].clone()
+        o = torch.empty(e - a, H, D, dtype=torch.float64)
+        for t in range(e - a):
+            S *= g[t].unsqueeze(-1)
+            S += k[t].unsqueeze(-1) * (bt[t].unsqueeze(-1) * (v[t] - torch.einsum("hkv,hk->hv", S, k[t]))).unsqueeze(-2)
+            o[t] = torch.einsum("hkv,hk->hv", S, q[t])
+        rec[s] = S
+        o = o * torch.rsqrt(o.square().mean(-1, keepdim=True) + eps) * nw
+        out[a:e] = (o * d(z[a:e]).view(-1, H, D).sigmoid()).reshape(-1, HD)
+    return out
+
+
+@pytest.mark.parametrize("decay", ["slow", "mixed", "fast"])
+@pytest.mark.parametrize("scratch", [1 << 30, 7 << 20])
+def test_chunk_form_against_64_bits(decay, scratch, monkeypatch):
+    """Pieces at the edges of chunks and blocks, fresh and continued, one without a slot, several rounds; the chunk form is as near to
+    64 bits as the token-by-token form."""
+    from batchgen_b200.ops import kda
+    H, D = 3, 128
+    HD = H * D
+    g = torch.Generator().manual_seed(5)
+    lens = [1, 47, 48, 63, 64, 65, 3, 127, 128, 129, 300, 50, 80]
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    T, B = cu[-1], len(lens)
+    slots = [i if i != 11 else -1 for i in range(B)]
+    has = [i % 2 for i in range(B)]
+    qkv, z = torch.randn(T, 3 * HD, generator=g).bfloat16(), torch.randn(T, HD, generator=g).bfloat16()
+    f, beta = torch.randn(T, HD, generator=g).bfloat16(), (torch.randn(T, H, generator=g) * 2).bfloat16()
+    A = {"slow": torch.full((H,), -4.0), "mixed": torch.tensor([-3.0, 0.0, 2.7]), "fast": torch.full((H,), 4.5)}[decay]
+    p = kda.KDAParams(*(t.cuda() for t in (torch.randn(3 * HD, 4, generator=g) * 0.5, torch.randn(3 * HD, generator=g) * 0.1, A,
+                                           torch.randn(HD, generator=g) - 1, 1 + 0.1 * torch.randn(D, generator=g))))
+    conv0, rec0 = torch.randn(B, 3 * HD, 3, generator=g).bfloat16().float(), torch.randn(B, H, D, D, generator=g) * 0.3
+    conv64, rec64 = conv0.double(), rec0.double()
+    want = _recurrence64(qkv, f, beta, z, p, conv64, rec64, slots, cu, has, H, D, D ** -0.5, 1e-6)
+    monkeypatch.setattr(kda, "_CHUNK_SCRATCH", scratch)
+    monkeypatch.setattr(kda, "chunk_form_pays", lambda lens, heads, sms: bool(lens))
+    err = {}
+    for form, least in (("chunks", kda.CHUNK_MIN_TOKENS), ("tokens", 1 << 30)):
+        monkeypatch.setattr(kda, "CHUNK_MIN_TOKENS", least)
+        conv, rec = conv0.cuda(), rec0.cuda()
+        out = kda.kda_forward(qkv.cuda(), f.cuda(), beta.cuda(), z.cuda(), p, conv, rec, slots, cu, has, H, D, D ** -0.5, 1e-6)
+        torch.cuda.synchronize()
+        live = torch.ones(T, dtype=torch.bool)
+        live[cu[11]:cu[12]] = False
+        assert torch.equal(conv.cpu().double(), conv64)
+        assert torch.equal(rec[11].cpu(), rec0[11])
+        d = (out.cpu().double() - want)[live]
+        err[form] = ((rec.cpu().double() - rec64).norm() / rec64.norm()).item(), (d.norm() / want[live].norm()).item()
+        # a value rounded to 8 significant bits; the recurrence in fp32
+        assert (d.abs() <= want[live].abs() * 2 ** -8 + 2e-4).all(), (form, d.abs().max())
+    assert err["chunks"][0] <= 1.5 * err["tokens"][0] + 1e-7 and err["chunks"][1] <= 1.02 * err["tokens"][1], err

@@ -138,3 +138,27 @@ def test_chunked_prefill_advances_the_recurrent_state_in_every_piece():
     eng = mk(max_prefill_tokens=24)
     assert eng.generate(prompts, params) == want
     assert eng.stats.prefill_chunks > 0
+
+
+def test_chunk_plan_covers_every_long_piece_once_and_in_order():
+    for cu in ([0, 1, 48, 96, 96, 260], [0, 64], [0, 65, 130, 1000], [0, 47]):
+        for most in (1, 2, 3, 100):
+            rounds = kda.chunk_plan(cu, 48, most)
+            seen, begun = {}, set()
+            for items, seqs in rounds:
+                assert len(items) <= most and sum(s[2] for s in seqs) == len(items)
+                at = 0
+                for seq, first, n, start in seqs:
+                    assert first == at and n > 0 and start == (seq not in begun)
+                    begun.add(seq)
+                    for s, t0, cnt, before in items[first:first + n]:
+                        assert s == seq and t0 == seen.get(seq, cu[seq]) and before == t0 - cu[seq] and 0 < cnt <= kda.CHUNK
+                        seen[seq] = t0 + cnt
+                    at += n
+            assert seen == {i: cu[i + 1] for i in range(len(cu) - 1) if cu[i + 1] - cu[i] >= 48}
+
+
+def test_chunk_form_is_taken_where_it_was_the_faster_one():
+    pays = lambda n, tokens: kda.chunk_form_pays([tokens] * n, 32, 148)  # noqa: E731
+    assert pays(1, 4096) and pays(4, 512) and pays(8, 1024)
+    assert not pays(1, 48) and not pays(32, 64) and not pays(200, 48) and not kda.chunk_form_pays([], 32, 148)
