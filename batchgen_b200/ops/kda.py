@@ -105,14 +105,14 @@ _CHUNK_SCRATCH = 1 << 30              # bytes of scratch a round of chunks may t
 
 
 def chunk_form_pays(lens: Sequence[int], heads: int, sms: int) -> bool:
-    """Whether pieces of ``lens`` tokens are faster in chunks.  Token by token costs 2.0 us for each token of the longest piece, or 2.6 us a
-    token and round of CTAs (two fit an SM) when the (piece, head) pairs fill the SMs; chunks cost 0.57 us a (chunk, head) on 148 SMs and 110
+    """Whether pieces of ``lens`` tokens are faster in chunks.  Token by token costs 2.0 us for each token of the longest piece, or 2.8 us a
+    token and round of CTAs (two fit an SM) when the (piece, head) pairs fill the SMs; chunks cost 0.57 us a (chunk, head) on 148 SMs and 125
     us to start (32 heads of 128, tokens / chunks: 1 x 64 149 / 142 us, 1 x 4,096 8,086 / 1,228; 4 x 512 1,061 / 686; 8 x 1,024 2,501 /
     2,249; 32 x 64 667 / 736; 200 x 32 1,810 / 3,859)."""
     if not lens:
         return False
-    tokens = 45 + max(2.0 * max(lens), 2.6 * heads * sum(lens) / (2 * sms))
-    return 110 + 0.57 * heads * sum(-(-n // CHUNK) for n in lens) * 148 / sms < tokens
+    tokens = 45 + max(2.0 * max(lens), 2.8 * heads * sum(lens) / (2 * sms))
+    return 125 + 0.57 * heads * sum(-(-n // CHUNK) for n in lens) * 148 / sms < tokens
 
 
 def chunk_plan(cu: Sequence[int], min_tokens: int, most_items: int):
