@@ -84,6 +84,25 @@ def linear(x, lin: Linear, xq=None, xs=None, silu_mul: bool = False):
     return x @ lin.w.t()
 
 
+def expanded_parts(cu, ctx, block_rows: int):
+    """Sequences of a step with cached context in groups whose rows (cached and new) stay within ``block_rows``, or None when
+    the absorbed form should run (``Transformer._expanded_blocks``)."""
+    rows = [int(c) + int(b) - int(a) for a, b, c in zip(cu, cu[1:], ctx)]
+    new = [int(b) - int(a) for a, b in zip(cu, cu[1:])]
+    live = [i for i, n in enumerate(new) if n > 0]
+    pairs = sum(new[i] * int(ctx[i]) + new[i] * (new[i] + 1) // 2 for i in live)
+    if not live or max(rows[i] for i in live) > block_rows or pairs < 200 * sum(rows[i] for i in live):
+        return None
+    parts, held = [[]], 0
+    for i in live:
+        if parts[-1] and held + rows[i] > block_rows:
+            parts.append([])
+            held = 0
+        parts[-1].append(i)
+        held += rows[i]
+    return parts
+
+
 class Transformer:
     def __init__(self, cfg: ModelConfig, weights: ModelWeights, layout: Optional[ParallelLayout] = None,
                  comm=None, max_positions: int = 8192):
@@ -100,6 +119,7 @@ class Transformer:
         self.attn_request_parallel = False
         self.streamer = None          # models.streaming.StreamedExperts when the routed experts live in host memory
         self.overlap_shared_expert = os.environ.get("BG_OVERLAP_SHARED", "1") != "0"   # decode: shared expert on a side stream
+        self.expanded_block_rows = 16384         # rows of cached context and prompt whose keys and values are up-projected at a time
         self.expanded_prefill_min_tokens = 256   # below this the absorbed kernel is as fast and saves the kv_b GEMM
 
     # ------------------------------------------------------------------ helpers
@@ -146,23 +166,22 @@ class Transformer:
         with tm.timed("attn.kv_write_qnorm_qb_rope", l):
             self._mla_q(lw, q_a, kv_a, meta, cache, l)
         q, qn = self._q, self._qn
-        if (meta.mode == "prefill" and lw.w_kvb is not None and q.is_cuda and T >= self.expanded_prefill_min_tokens
-                and not any(meta.ctx_lens)):
-            # long fresh prompts: attention over up-projected keys / values (3.4x fewer FLOPs than the
-            # absorbed form); the latent rows were just written to the cache, read them back by slot
-            with tm.timed("attn.core_prefill", l):
-                lat = cache.latent(l).view(-1, cfg.kv_cache_dim)[meta.slot_mapping.clamp_min(0)]
-                kvb = gemm.bf16_gemm(lat[:, : cfg.kv_lora_rank].contiguous(), lw.w_kvb)
-                Hh = q.shape[1]
-                key = (tuple(meta.cu_seqlens), T)
-                if getattr(meta, "_mha_work_key", None) != key:
-                    meta._mha_work = attn_ops.mha_prefill_work(meta.cu_seqlens, meta.ctx_lens, meta.cu_seqlens[:-1]).to(q.device)
-                    meta._mha_work_key = key
-                o = attn_ops.mha_prefill(q, kvb.view(T, Hh, 256), lat[:, cfg.kv_lora_rank:], meta._mha_work,
-                                         cfg.softmax_scale)
-                if meta.cu_seqlens[-1] < T:
-                    o[meta.cu_seqlens[-1]:].zero_()      # padding rows of a sequence-parallel step belong to no sequence
-            return o.reshape(T, -1)
+        if meta.mode == "prefill" and lw.w_kvb is not None and q.is_cuda and T >= self.expanded_prefill_min_tokens:
+            blocks = self._expanded_blocks(meta, T, q.shape[1], cache.page_size)
+            if blocks:
+                # long prompts: attention over up-projected keys / values (3.4x fewer FLOPs than the absorbed form); the
+                # latent rows of the step were just written to the cache, all rows that are seen are read from there
+                with tm.timed("attn.core_prefill", l):
+                    flat = cache.latent(l).view(-1, cfg.kv_cache_dim)
+                    o = None
+                    for slots, work in blocks:
+                        lat = flat[slots]
+                        kvb = gemm.bf16_gemm(lat[:, : cfg.kv_lora_rank].contiguous(), lw.w_kvb)
+                        o = attn_ops.mha_prefill(q, kvb.view(-1, q.shape[1], 256), lat[:, cfg.kv_lora_rank:], work,
+                                                 cfg.softmax_scale, out=o)
+                    if meta.cu_seqlens[-1] < T:
+                        o[meta.cu_seqlens[-1]:].zero_()      # padding rows of a sequence-parallel step belong to no sequence
+                return o.reshape(T, -1)
         q_nope, q_pe = q[..., : cfg.qk_nope_head_dim], q[..., cfg.qk_nope_head_dim:]
         # absorb W_UK: [T, Hh, nope] x [Hh, nope, kv_lora] -> [T, Hh, kv_lora]
         rp = self._request_parallel(meta, T)
@@ -185,6 +204,44 @@ class Transformer:
         # out-absorb W_UV: [T, Hh, kv_lora] x [Hh, v, kv_lora]^T -> [T, Hh * v]
         with tm.timed("attn.out_absorb", l):
             return attn_ops.mla_out_absorb(o_lat, lw.w_uv)
+
+    def _expanded_blocks(self, meta: AttnMeta, T: int, heads: int, page: int):
+        """Blocks of sequences for attention over up-projected keys and values, made once per step: (cache slots of every row the
+        block's queries see, tiles of ``attn_ops.mha_prefill``); None when the absorbed form is the cheaper one.
+
+        Without cached context the step's own rows are one block.  A cached row costs its up-projection (some 50 ns with 128 heads:
+        33.5 MFLOP, 64 KB written and read), a query-key pair saves some 0.3 ns (measured rates: 621 TFLOP/s of 278 KFLOP absorbed,
+        575 TFLOP/s of 82 KFLOP expanded), so the pairs have to be some 160 times the rows; 200 leaves a margin.  Blocks bound the
+        expanded rows (64 KB each at 128 heads); a sequence that is longer than a block stays with the absorbed form, and so
+        does its step.  With context only geometries that the absorbed kernel takes are covered."""
+        key = (tuple(meta.cu_seqlens), tuple(meta.ctx_lens), T)
+        if getattr(meta, "_mha_key", None) == key:
+            return meta._mha_blocks
+        cu, ctx = list(meta.cu_seqlens), list(meta.ctx_lens)
+        dev = meta.positions.device
+        blocks = None
+        if not any(ctx):
+            work = attn_ops.mha_prefill_work(cu, ctx, cu[:-1]).to(dev)
+            blocks = [(meta.slot_mapping.clamp_min(0), work)]
+        else:
+            parts = expanded_parts(cu, ctx, self.expanded_block_rows) if heads % 8 == 0 and page == 64 else None
+            if parts is not None:
+                blocks = []
+                bt = meta.block_table.long()
+                for seqs in parts:
+                    rows = [ctx[i] + cu[i + 1] - cu[i] for i in seqs]
+                    starts = [0]
+                    for n in rows:
+                        starts.append(starts[-1] + n)
+                    of = torch.repeat_interleave(torch.tensor(seqs, device=dev), torch.tensor(rows, device=dev), output_size=starts[-1])
+                    pos = torch.cat([torch.arange(n, device=dev) for n in rows])
+                    slots = bt[of, pos // page] * page + pos % page
+                    tiles = [attn_ops.mha_prefill_work([cu[i], cu[i + 1]], [ctx[i]], [starts[k]]) for k, i in enumerate(seqs)]
+                    work = torch.cat(tiles)
+                    order = torch.argsort(-(work[:, 3] + work[:, 1]), stable=True)       # longest key ranges first
+                    blocks.append((slots, work[order].contiguous().to(dev)))
+        meta._mha_key, meta._mha_blocks = key, blocks
+        return blocks
 
     def _mla_q(self, lw, q_a, kv_a, meta, cache, l):
         cfg = self.cfg

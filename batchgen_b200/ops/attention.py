@@ -188,14 +188,15 @@ def mha_prefill_work(cu_seqlens: Sequence[int], ctx_lens: Sequence[int], k_start
     return torch.tensor(rows, dtype=torch.int32).view(-1, 4)
 
 
-def mha_prefill(q: torch.Tensor, kv: torch.Tensor, kpe: torch.Tensor, work: torch.Tensor, scale: float) -> torch.Tensor:
+def mha_prefill(q: torch.Tensor, kv: torch.Tensor, kpe: torch.Tensor, work: torch.Tensor, scale: float,
+                out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Causal varlen attention in the expanded MLA form.  q [Tq, H, 192] (nope | roped pe); kv [Tk, H, 256]
     (key nope | value, the kv_b projection of the latent rows); kpe [Tk, >= 64] (roped shared key part in the
-    first 64 columns, may be a strided view); ``work`` from ``mha_prefill_work`` -> [Tq, H, 128]."""
+    first 64 columns, may be a strided view); ``work`` from ``mha_prefill_work`` -> [Tq, H, 128] (rows that tiles cover; ``out``: into it)."""
     Tq, H, _ = q.shape
     Tk = kv.shape[0]
     if not (q.is_cuda and q.dtype == torch.bfloat16):
-        out = torch.zeros(Tq, H, 128, dtype=q.dtype)
+        out = out if out is not None else torch.zeros(Tq, H, 128, dtype=q.dtype)
         kf = torch.cat([kv[..., :128].float(), kpe[:, None, :64].float().expand(Tk, H, 64)], -1)
         vf = kv[..., 128:].float()
         for q0, nq, k0, kv0 in work.tolist():
@@ -205,7 +206,9 @@ def mha_prefill(q: torch.Tensor, kv: torch.Tensor, kpe: torch.Tensor, work: torc
                 out[q0 + i] = torch.einsum("hk,khd->hd", torch.softmax(s, -1), vf[k0:k0 + n]).to(q.dtype)
         return out
     assert q.is_contiguous() and kv.is_contiguous() and kpe.stride(1) == 1
-    out = torch.empty(Tq, H, 128, dtype=torch.bfloat16, device=q.device)
+    if out is None:
+        out = torch.empty(Tq, H, 128, dtype=torch.bfloat16, device=q.device)
+    assert out.is_contiguous() and out.shape == (Tq, H, 128)
     work = work.to(q.device)
     rc = _ext.lib().bg_mha_prefill(_ext.ptr(q), _ext.ptr(kv), _ext.ptr(kpe), ctypes.c_longlong(kpe.stride(0)), _ext.ptr(out),
                                    _ext.ptr(work), ctypes.c_int(work.shape[0]), ctypes.c_int(Tq), ctypes.c_int(Tk),
