@@ -213,8 +213,23 @@ def bf16_gemm(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = No
         out = torch.empty(T, N, dtype=torch.float32 if fp32_out else torch.bfloat16, device=x.device)
     if T == 0:
         return out
+    # three quarters of the SMs with a tile of 256 tokens x 128 outputs: the wider product moves fewer operand bytes per FLOP (4,096 x 16,576 x
+    # 2,304 332 -> 253 us, 6,200 x 32,768 x 512 299 -> 202, 1,024 x 4,096 x 2,880 27 -> 21; 300 x 2,304 x 4,096, where the other kernel
+    # splits K, 19 -> 23)
+    if (not fp32_out and not _hooks_pending and out.dtype == torch.bfloat16 and out.stride(1) == 1 and x.is_contiguous() and w.is_contiguous()
+            and K > 0 and K % 64 == 0 and 4 * (-(-T // 256)) * (-(-N // 128)) >= 3 * _ext.num_sms(x.device)):
+        _bf16_swap(x, w, out, None, None, 1, N)
+        return out
     _launch(KIND_BF16, EPI_STORE_F32 if fp32_out else EPI_STORE, x, None, 0, w, None, out, None, 1, T, N, K)
     return out
+
+
+def _bf16_swap(x: torch.Tensor, w2d: torch.Tensor, out: torch.Tensor, offsets, counts, groups: int, N: int) -> None:
+    rc = _ext.lib().bg_gemm_bf16_swap(_ext.ptr(x), _ext.ptr(w2d), _ext.ptr(out), ctypes.c_int(out.stride(0)), _ext.ptr(offsets),
+                                      _ext.ptr(counts), ctypes.c_int(groups), ctypes.c_int(x.shape[0]), ctypes.c_int(N),
+                                      ctypes.c_int(x.shape[1]), ctypes.c_int(_ext.num_sms(x.device)),
+                                      _ext.ptr(_ext.status_word(x.device)), _ext.stream())
+    _ext.check(rc, "bg_gemm_bf16_swap")
 
 
 def grouped_bf16_gemm(x: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, counts: torch.Tensor, relu2: bool = False) -> torch.Tensor:
@@ -222,7 +237,12 @@ def grouped_bf16_gemm(x: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, c
     positive part of the products); ``counts`` rows of each segment are present, the others stay undefined."""
     E, N, K = w.shape
     out = torch.empty(x.shape[0], N, dtype=torch.bfloat16, device=x.device)
-    if x.shape[0]:
+    # tokens as the MMA's N where segments have a hundred rows and more (256 matrices of 2,048 x 2,304, rows a segment on average: 128
+    # rows 527 -> 484 us, 156 rows 639 -> 511, 512 rows 1,328 -> 1,123; 32 rows 395 -> 442, 4 rows 371 -> 411: there the weights are
+    # streamed, and the 128 x 128 kernel has more of them in flight)
+    if x.shape[0] >= 104 * E and not relu2 and 0 < E <= 1024 and K > 0 and K % 64 == 0:
+        _bf16_swap(x.contiguous(), w.view(E * N, K), out, offsets, counts, E, N)
+    elif x.shape[0]:
         _launch(KIND_BF16, EPI_RELU2 if relu2 else EPI_STORE, x.contiguous(), None, 0, w.view(E * N, K), None, out, offsets, E, x.shape[0], N, K,
                 counts=counts)
     return out

@@ -71,3 +71,43 @@ def test_expert_stack(T, quant, kind):
     err = (got.double().cpu() - want).norm() / want.norm()
     # four roundings to bf16 on the way (pre-activation, activation, expert row, sum), each some 2^-9 of its value
     assert err < 4 * 2 ** -9, err
+
+
+@pytest.mark.parametrize("counts,align", [([1, 0, 17, 130], 8), ([256, 257, 5, 600], 8), ([15, 16, 31, 33], 16), ([3, 0, 0, 0], 8)])
+@pytest.mark.parametrize("N,K", [(128, 64), (200, 192), (384, 1024)])
+def test_grouped_bf16_token_tiles(counts, align, N, K):
+    """Segments at the edges of the token tiles (16 and 256 rows), rows past a segment's count not finite, weight rows that end inside
+    a tile."""
+    from batchgen_b200.ops import _ext, gemm
+    g = torch.Generator().manual_seed(N + sum(counts))
+    offs = [0]
+    for c in counts:
+        offs.append(offs[-1] + (c + align - 1) // align * align + align)
+    x = torch.full((offs[-1], K), float("nan")).bfloat16()
+    for e, c in enumerate(counts):
+        x[offs[e]:offs[e] + c] = torch.randn(c, K, generator=g).bfloat16()
+    w = torch.randn(len(counts), N, K, generator=g).bfloat16()
+    off, cnt = torch.tensor(offs, dtype=torch.int32).cuda(), torch.tensor(counts, dtype=torch.int32).cuda()
+    swapped = torch.empty(offs[-1], N, dtype=torch.bfloat16, device="cuda")
+    gemm._bf16_swap(x.cuda(), w.cuda(), swapped, off, cnt, len(counts), N)
+    for got in (swapped.cpu().double(), gemm.grouped_bf16_gemm(x.cuda(), w.cuda(), off, cnt).cpu().double()):
+        _ext.check_status()
+        for e, c in enumerate(counts):
+            xe, we = x[offs[e]:offs[e] + c].double(), w[e].double()
+            want = xe @ we.t()
+            # one rounding to 8 significant bits; fp32 sums of K exact products: K * 2^-24 of their magnitudes
+            assert ((got[offs[e]:offs[e] + c] - want).abs() <= want.abs() * 2 ** -8 + (xe.abs() @ we.abs().t()) * K * 2 ** -24).all(), e
+
+
+@pytest.mark.parametrize("T,N,K", [(1030, 3144, 128), (257, 14208, 64), (4096, 1000, 192)])
+def test_dense_bf16_token_tiles(T, N, K):
+    """Enough tiles of 256 tokens for the SMs, rows and outputs that end inside a tile, output rows inside a wider tensor."""
+    from batchgen_b200.ops import _ext, gemm
+    g = torch.Generator().manual_seed(T)
+    x, w = torch.randn(T, K, generator=g).bfloat16(), torch.randn(N, K, generator=g).bfloat16()
+    wide = torch.full((T, N + 24), 7.0, dtype=torch.bfloat16, device="cuda")
+    gemm.bf16_gemm(x.cuda(), w.cuda(), out=wide[:, 8:8 + N])
+    _ext.check_status()
+    got, want = wide.cpu().double(), x.double() @ w.double().t()
+    assert (got[:, :8] == 7).all() and (got[:, 8 + N:] == 7).all()
+    assert ((got[:, 8:8 + N] - want).abs() <= want.abs() * 2 ** -8 + (x.double().abs() @ w.double().abs().t()) * K * 2 ** -24).all()
