@@ -109,30 +109,9 @@ __device__ __forceinline__ bool vote_any_128(bool v) {      // barrier over the 
       : "memory");
   return r != 0;
 }
-// D[tmem] += A[tmem] * B[smem]: a row of A is a lane, its 16-bit elements lie two to a column
-__device__ __forceinline__ void mma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.u32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* v) {
   tmem_ld_32x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(v));
 }
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, "
-      "%25, %26, %27, %28, %29, %30, %31, %32};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-      "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
-      "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
-      "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-      : "memory");
-}
-
 // shared memory: Q [KB] | K [stages][KB] | V [stages][VB] | P (not FINE), all on 1,024-byte boundaries, then Shared
 __host__ __device__ inline int tile_bytes(int KB, int VB, int stages, bool fine) {
   return KB * kQBlockBytes + stages * (KB + VB) * kBlockBytes + (fine ? 0 : kPBytes);
@@ -362,14 +341,14 @@ attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 32; ++j) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * alpha);
-          tmem_st32(tm_o + c * 32, ov);
+          tmem_st_32x32(tm_o + c * 32, ov);
         }
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tmem_st_wait();
       }
       if (FINE) {
-        tmem_st32(tmem_base + lane_addr + (t & 1) * BN, *reinterpret_cast<const uint32_t(*)[32]>(sv));
-        tmem_st32(tmem_base + lane_addr + (t & 1) * BN + 32, *reinterpret_cast<const uint32_t(*)[32]>(lo_part));
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tmem_st_32x32(tmem_base + lane_addr + (t & 1) * BN, *reinterpret_cast<const uint32_t(*)[32]>(sv));
+        tmem_st_32x32(tmem_base + lane_addr + (t & 1) * BN + 32, *reinterpret_cast<const uint32_t(*)[32]>(lo_part));
+        tmem_st_wait();
         const int real = last + 1 - kt;
         if (!kept && real < BN) {                                  // uniform: the tile past whose end rows belong to nobody
           if (vote_any_128(!mbar_wait(&ss.v_full[t % ST], (t / ST) & 1, abort_flag, kTimeoutEpilogue))) { ok = false; break; }

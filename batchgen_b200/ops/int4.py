@@ -44,10 +44,10 @@ def dequantize(wq: torch.Tensor, ws: torch.Tensor, dtype=torch.float32) -> torch
     return (w * s).view(*lead, K).to(dtype)
 
 
-def _launch(epi, x, wq2d, ws2d, out, offsets, groups, M, N, K):
+def _launch(epi, x, wq2d, ws2d, out, offsets, groups, M, N, K, counts=None):
     rc = _ext.lib().bg_int4_gemm(
         ctypes.c_int(epi), _ext.ptr(x), _ext.ptr(wq2d), _ext.ptr(ws2d), _ext.ptr(out), ctypes.c_int(out.stride(0)),
-        _ext.ptr(offsets), ctypes.c_int(groups), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
+        _ext.ptr(offsets), _ext.ptr(counts), ctypes.c_int(groups), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
         ctypes.c_int(_ext.num_sms(x.device)), _ext.ptr(_ext.status_word(x.device)), _ext.stream())
     _ext.check(rc, "bg_int4_gemm")
 
@@ -64,9 +64,10 @@ def int4_gemm(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor) -> torch.Tens
 
 
 def grouped_int4_gemm(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor, offsets: torch.Tensor,
-                      silu_mul: bool = False) -> torch.Tensor:
-    """Ragged grouped GEMM (segment e = offsets[e]:offsets[e+1], 128-aligned starts on the GPU).  wq [E, N, K/2],
-    ws [E, N, K/32] bf16.  ``silu_mul``: rows interleaved gate/up in blocks of 32, output silu(gate) * up."""
+                      silu_mul: bool = False,
+                      counts: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Ragged grouped GEMM (segment e = offsets[e]:offsets[e+1]; ``counts``: rows present in every segment, the others
+    stay undefined).  wq [E, N, K/2], ws [E, N, K/32] bf16.  ``silu_mul``: rows interleaved gate/up in blocks of 32, output silu(gate) * up."""
     E, N, Kh = wq.shape
     K = Kh * 2
     R = x.shape[0]
@@ -85,5 +86,5 @@ def grouped_int4_gemm(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor, offse
     out = torch.empty(R, N // 2 if silu_mul else N, dtype=torch.bfloat16, device=x.device)
     if R:
         _launch(1 if silu_mul else 0, x.contiguous(), wq.view(E * N, Kh), ws.contiguous().view(E * N, K // GROUP), out,
-                offsets, E, R, N, K)
+                offsets, E, R, N, K, counts)
     return out

@@ -258,13 +258,13 @@ def grouped_experts(xq, xs, offsets: torch.Tensor, ew: ExpertWeights, x_dense: O
         x = x_dense
         if x.is_cuda and ew.interleaved:
             with timer.timed("moe.s1_gemm"):
-                act = grouped_w4(x, ew.w13, ew.w13_s, offsets, silu_mul=True)
+                act = grouped_w4(x, ew.w13, ew.w13_s, offsets, silu_mul=True, counts=counts)
         else:
             with timer.timed("moe.s1_gemm"):
-                gu = grouped_w4(x, ew.w13, ew.w13_s, offsets)
+                gu = grouped_w4(x, ew.w13, ew.w13_s, offsets, counts=counts)
             act = activation(gu, ew.activation, ew.act_limit, offsets, row_src).to(x.dtype)
         with timer.timed("moe.s3_gemm"):
-            return grouped_w4(act, ew.w2, ew.w2_s, offsets)
+            return grouped_w4(act, ew.w2, ew.w2_s, offsets, counts=counts)
     # unquantised experts
     x = x_dense
     if counts is not None and _grouped_on_kernels(x, ew):
@@ -299,8 +299,9 @@ def experts_forward(hidden: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.
         pairs = topk_idx.shape[0] * topk_idx.shape[1]
         if gemm.use_swapab(pairs / max(expert_hi - expert_lo, 1), ew.w13.shape[1], ew.w13.shape[2]):
             align = 32
-    elif ew.quant == "none" and _grouped_on_kernels(hidden, ew):
-        align = 8                          # the grouped bf16 GEMM takes real row counts: segments only need aligned rows
+    elif hidden.is_cuda and hidden.dtype == torch.bfloat16 and (ew.quant in ("mxfp4", "int4")
+                                                                or ew.quant == "none" and _grouped_on_kernels(hidden, ew)):
+        align = 8                          # these grouped GEMMs take real row counts: segments only need aligned rows
     with timer.timed("moe.permute"):
         src, pos, offsets = permute(topk_idx, expert_lo, expert_hi, num_valid, align=align)
     if ew.quant == "fp8_block":

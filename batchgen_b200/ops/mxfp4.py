@@ -1,7 +1,7 @@
 """MXFP4 (e2m1 values, one e8m0 scale per 32) expert weights: GEMMs and conversion.
 
 On CUDA the GEMMs run ``gemm_mxfp4.cu``: packed weights go from HBM to shared memory as 4-bit data and are
-expanded to bf16 inside the CTA, then multiplied on tcgen05 with fp32 accumulation.  On CPU the same
+expanded to bf16 on their way to TMEM, then multiplied on tcgen05 with fp32 accumulation.  On CPU the same
 contract is met by dequantising and multiplying in fp32.
 
 Reference parity: quantiser / layout batchgen/quantization/mxfp4.py:30 and
@@ -43,10 +43,10 @@ def dequantize(wq: torch.Tensor, ws: torch.Tensor, dtype=torch.bfloat16) -> torc
     return out.to(dtype)
 
 
-def _launch(epi, x, wq2d, ws2d, out, offsets, groups, M, N, K):
+def _launch(epi, x, wq2d, ws2d, out, offsets, groups, M, N, K, counts=None):
     rc = _ext.lib().bg_mxfp4_gemm(
         ctypes.c_int(epi), _ext.ptr(x), _ext.ptr(wq2d), _ext.ptr(ws2d), _ext.ptr(out), ctypes.c_int(out.stride(0)),
-        _ext.ptr(offsets), ctypes.c_int(groups), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
+        _ext.ptr(offsets), _ext.ptr(counts), ctypes.c_int(groups), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
         ctypes.c_int(_ext.num_sms(x.device)), _ext.ptr(_ext.status_word(x.device)), _ext.stream())
     _ext.check(rc, "bg_mxfp4_gemm")
 
@@ -65,9 +65,10 @@ def mxfp4_gemm(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor, out: Optiona
 
 
 def grouped_mxfp4_gemm(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor, offsets: torch.Tensor,
-                       silu_mul: bool = False, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """Ragged grouped GEMM over rows grouped by expert (segment e = offsets[e]:offsets[e+1], starts
-    128-aligned on the GPU path).  wq [E, N, K/2], ws [E, N, K/32].  ``silu_mul``: the rows of each expert
+                       silu_mul: bool = False, out: Optional[torch.Tensor] = None,
+                       counts: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Ragged grouped GEMM over rows grouped by expert (segment e = offsets[e]:offsets[e+1]; ``counts``: rows present in
+    every segment, the others stay undefined).  wq [E, N, K/2], ws [E, N, K/32].  ``silu_mul``: the rows of each expert
     are stored gate/up interleaved in blocks of 32 and the output is silu(gate) * up with N/2 columns."""
     E, N, Kh = wq.shape
     K = Kh * 2
@@ -91,5 +92,5 @@ def grouped_mxfp4_gemm(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor, offs
     if R:
         assert offsets.dtype == torch.int32 and offsets.is_cuda
         _launch(EPI_SILU_MUL if silu_mul else EPI_STORE, x.contiguous(), wq.view(E * N, Kh), ws.view(E * N, K // 32),
-                out, offsets, E, R, N, K)
+                out, offsets, E, R, N, K, counts)
     return out

@@ -96,3 +96,48 @@ def test_int4_grouped_gemm(silu):
             want = torch.nn.functional.silu(want[:, : N // 2]) * want[:, N // 2:]
         assert _rel(y[a:a + n], want) < 8e-3, e
     assert _rel(int4.int4_gemm(x[:40].cuda(), q[0].cuda(), s[0].cuda()).cpu(), x[:40].float() @ wd[0].t()) < 8e-3
+
+
+@pytest.mark.parametrize("counts", [[1, 0, 17, 130], [192, 193, 5, 400], [16, 15, 33, 64]])
+@pytest.mark.parametrize("fmt", ["mxfp4", "int4"])
+@pytest.mark.parametrize("N,K,silu", [(256, 64, True), (384, 192, False), (200, 320, False)])
+def test_w4_token_tiles_and_scales(counts, fmt, N, K, silu):
+    """Segments at the edges of the token tiles (16 and 192 rows), rows past a segment's count not finite, weight rows that end inside a
+    tile, scales from 2^-127 to above 2 (the largest ones beside ordinary ones)."""
+    from batchgen_b200.ops import _ext, int4, mxfp4
+    from batchgen_b200.ops.gemm import interleave_gate_up_rows
+    g = torch.Generator().manual_seed(N + sum(counts))
+    E = len(counts)
+    offs = [0]
+    for c in counts:
+        offs.append(offs[-1] + (c + 7) // 8 * 8 + 8)
+    x = torch.full((offs[-1], K), float("nan")).bfloat16()
+    for e, c in enumerate(counts):
+        x[offs[e]:offs[e] + c] = torch.randn(c, K, generator=g).bfloat16()
+    wq = torch.randint(0, 256, (E, N, K // 2), generator=g, dtype=torch.uint8)
+    if fmt == "mxfp4":
+        ws = torch.randint(120, 129, (E, N, K // 32), generator=g, dtype=torch.uint8)
+        ws[0, ::5] = 0
+        ws[1, 3::64] = 131
+        ws[2, 1::7, 0] = 150
+        w = mxfp4.dequantize(wq, ws, torch.float32).double()
+    else:
+        ws = (torch.rand(E, N, K // 32, generator=g) * 0.1).bfloat16()
+        w = int4.dequantize(wq, ws).bfloat16().double()
+    off, cnt = torch.tensor(offs, dtype=torch.int32).cuda(), torch.tensor(counts, dtype=torch.int32).cuda()
+    run = mxfp4.grouped_mxfp4_gemm if fmt == "mxfp4" else int4.grouped_int4_gemm
+    got = run(x.cuda(), wq.cuda(), ws.cuda(), off, silu_mul=silu, counts=cnt).cpu().double()
+    _ext.check_status()
+    for e, c in enumerate(counts):
+        xe = x[offs[e]:offs[e] + c].double()
+        want, mag = xe @ w[e].t(), xe.abs() @ w[e].abs().t()
+        if silu:
+            back = torch.argsort(interleave_gate_up_rows(N))
+            want, mag = want[:, back], mag[:, back]
+            a, u = want.chunk(2, -1)
+            am, um = mag.chunk(2, -1)
+            want = torch.nn.functional.silu(a) * u
+            mag = am * (u.abs() + 1) * 1.1 + um * a.abs()
+        # one rounding to 8 significant bits; fp32 sums of up to 320 exact products: 320 * 2^-24 of their magnitudes; products of
+        # subnormal weights may be flushed (below 1e-36)
+        assert ((got[offs[e]:offs[e] + c] - want).abs() <= want.abs() * 2 ** -8 + mag * 2e-5 + 1e-36).all(), e
