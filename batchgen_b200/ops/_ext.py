@@ -50,7 +50,9 @@ def ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
 
 
 def stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream of the current device, without building a stream object: that object was 30 % of the host time of a step
+    (some 5 us at every launch)."""
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def num_sms(device=None) -> int:

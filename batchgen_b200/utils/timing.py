@@ -18,6 +18,9 @@ from typing import Dict, List, Optional, Tuple
 import torch
 
 
+_OFF = contextlib.nullcontext()
+
+
 class TimingStats:
     def __init__(self, enabled: bool = True, cuda: Optional[bool] = None):
         self.enabled = enabled
@@ -28,11 +31,11 @@ class TimingStats:
         self.by_layer: Dict[Tuple[str, int], float] = defaultdict(float)
         self.steps = 0
 
-    @contextlib.contextmanager
     def timed(self, op: str, layer: int = -1):
-        if not self.enabled:
-            yield
-            return
+        return self._timed(op, layer) if self.enabled else _OFF       # no generator for the regions of an untimed step
+
+    @contextlib.contextmanager
+    def _timed(self, op: str, layer: int):
         if self.cuda:
             e0 = torch.cuda.Event(enable_timing=True)
             e1 = torch.cuda.Event(enable_timing=True)
