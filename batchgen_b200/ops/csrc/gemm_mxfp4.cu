@@ -30,6 +30,7 @@
 #include <cuda_fp4.h>
 
 #include "common.cuh"
+#include "w4_steps.h"
 
 namespace bg {
 namespace mx {
@@ -38,10 +39,9 @@ constexpr int BW = 128;                   // weight rows of a tile (MMA M)
 constexpr int BT = 192;                   // most tokens of a tile (MMA N)
 constexpr int kBox = 32;                  // token rows of one TMA box
 constexpr int BK = 64;                    // elements of K per step (one 128-byte swizzle atom of bf16)
-constexpr int kXStages = 6, kQStages = 4, kSlots = 4;
-constexpr int kGroups = 4;                // expansion groups of four warps, a TMEM slot each
+constexpr int kXStages = 6, kQStages = 4;
 constexpr int kThreads = 32 * (7 + 4 * kGroups);
-constexpr int kTmemCols = 512;            // two accumulators of BT columns, kSlots weight operands of 32
+constexpr int kTmemCols = 512;            // two accumulators of BT columns, kGroups weight operands of 32
 constexpr int kSlotCol = 2 * BT;
 constexpr int kMaxGroups = 1024;
 constexpr int kXBytes = BT * BK * 2;      // 24 KB
@@ -64,7 +64,7 @@ struct Params {
 struct Shared {
   uint64_t x_full[kXStages], x_empty[kXStages];
   uint64_t q_full[kQStages], q_empty[kQStages];      // empty: every expansion warp has read its part of the stage
-  uint64_t w_full[kSlots], w_empty[kSlots];          // weight operands in TMEM
+  uint64_t w_full[kGroups], w_empty[kGroups];        // weight operands in TMEM, one of each group
   uint64_t tmem_full[2], tmem_empty[2];
   uint32_t tmem_base;
   int abort_flag;
@@ -157,7 +157,7 @@ w4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kXStages; ++s) { mbar_init(&ss.x_full[s], 1); mbar_init(&ss.x_empty[s], 1); }
     for (int s = 0; s < kQStages; ++s) { mbar_init(&ss.q_full[s], 1); mbar_init(&ss.q_empty[s], 4 * kGroups); }
-    for (int s = 0; s < kSlots; ++s) { mbar_init(&ss.w_full[s], 4); mbar_init(&ss.w_empty[s], 1); }
+    for (int s = 0; s < kGroups; ++s) { mbar_init(&ss.w_full[s], 4); mbar_init(&ss.w_empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&ss.tmem_full[b], 1); mbar_init(&ss.tmem_empty[b], 4); }
     ss.abort_flag = 0;
     mbar_fence_init();
@@ -234,9 +234,9 @@ w4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         if (!mbar_wait(&ss.tmem_empty[buf], ((acc >> 1) & 1) ^ 1, abort_flag, kTimeoutMma)) { ok = false; break; }
         tc_fence_after();
         for (int kb = 0; kb < KB; ++kb, ++it) {
-          const int s = it % kXStages, slot = it % kSlots;
+          const int s = it % kXStages, slot = step_group(kb);
           if (!mbar_wait(&ss.x_full[s], (it / kXStages) & 1, abort_flag, kTimeoutMma) ||
-              !mbar_wait(&ss.w_full[slot], (it / kSlots) & 1, abort_flag, kTimeoutMma)) { ok = false; break; }
+              !mbar_wait(&ss.w_full[slot], slot_use(KB, acc, kb) & 1, abort_flag, kTimeoutMma)) { ok = false; break; }
           tc_fence_after();
           const uint64_t bdesc = make_smem_desc_sw128(smem_u32(x_tiles + s * kXBytes));
           const uint32_t w = tmem_base + kSlotCol + slot * 32;
@@ -257,7 +257,7 @@ w4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     const int sk = (p.K / 32) * kScaleBytes;                     // scale bytes per weight row
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
     uint32_t stage = 0;                      // stages of packed weights so far
-    for (int tile = blockIdx.x; ok && walk.get(tile, t); tile += gridDim.x) {
+    for (int tile = blockIdx.x; ok && walk.get(tile, t); tile += gridDim.x, ++acc) {
       const uint8_t* srow = p.ws + (size_t)(t.g * p.N + min(t.n0 + r, p.N - 1)) * sk;
       // the two scales of a 64-wide K step: 2 bytes (e8m0) or 4 bytes (bf16)
       auto load_scales = [&](int kb) -> uint32_t {
@@ -268,13 +268,11 @@ w4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       uint32_t sc[3];                                                // three own steps ahead
 #pragma unroll
       for (int i = 0; i < 3; ++i) sc[i] = load_scales(group + kGroups * i);
-      const uint32_t base = it;
       for (int kb = group; kb < KB + group; kb += kGroups, ++stage) {
-        it = base + kb;
         const uint32_t s2 = sc[0];
         sc[0] = sc[1]; sc[1] = sc[2];
         sc[2] = load_scales(kb + 3 * kGroups);
-        const int qs = stage % kQStages, slot = it % kSlots;
+        const int qs = stage % kQStages;
         if (!__all_sync(0xffffffffu, mbar_wait(&ss.q_full[qs], (stage / kQStages) & 1, abort_flag, kTimeoutEpilogue))) { ok = false; break; }
         const uint8_t* q = q_tiles + qs * kQBytes + r * 128;          // 16-byte chunk c of row r lies at c ^ (r & 7)
         const uint4 q0 = *reinterpret_cast<const uint4*>(q + (((2 * group) ^ (r & 7)) << 4));
@@ -302,15 +300,14 @@ w4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
             for (int c = 0; c < 8; ++c) expand8<QMODE, false>(words[c], c < 4 ? f0 | f0 << 16 : f1 | f1 << 16, o + 4 * c);
           }
         }
-        if (!__all_sync(0xffffffffu, mbar_wait(&ss.w_empty[slot], ((it / kSlots) & 1) ^ 1, abort_flag, kTimeoutEpilogue))) { ok = false; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait(&ss.w_empty[group], (slot_use(KB, acc, kb) & 1) ^ 1, abort_flag, kTimeoutEpilogue))) { ok = false; break; }
         tc_fence_after();
-        tmem_st_32x32(tmem_base + lane_addr + kSlotCol + slot * 32, o);
+        tmem_st_32x32(tmem_base + lane_addr + kSlotCol + group * 32, o);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&ss.w_full[slot]);
+        if (lane == 0) mbar_arrive(&ss.w_full[group]);
       }
-      it = base + KB;
     }
   } else {
     // ------------------------------------------------------------ epilogue: thread = weight row, columns = tokens

@@ -141,3 +141,44 @@ def test_w4_token_tiles_and_scales(counts, fmt, N, K, silu):
         # one rounding to 8 significant bits; fp32 sums of up to 320 exact products: 320 * 2^-24 of their magnitudes; products of
         # subnormal weights may be flushed (below 1e-36)
         assert ((got[offs[e]:offs[e] + c] - want).abs() <= want.abs() * 2 ** -8 + mag * 2e-5 + 1e-36).all(), e
+
+
+@pytest.mark.parametrize("counts", [[1, 0, 210, 40], [193, 7, 0, 385]])
+@pytest.mark.parametrize("fmt", ["mxfp4", "int4"])
+@pytest.mark.parametrize("K", [320, 384, 448, 512, 2880])
+@pytest.mark.parametrize("N,silu", [(640, False), (512, True)])
+def test_w4_many_tiles_a_cta(counts, fmt, K, N, silu, monkeypatch):
+    """Two CTAs walk all tiles, a dozen and more each: operand slots, rings and accumulators across tile borders, with K steps that are and
+    are not a multiple of the expansion groups."""
+    from batchgen_b200.ops import _ext, int4, mxfp4
+    from batchgen_b200.ops.gemm import interleave_gate_up_rows
+    g = torch.Generator().manual_seed(K + N + sum(counts))
+    E = len(counts)
+    offs = [0]
+    for c in counts:
+        offs.append(offs[-1] + (c + 7) // 8 * 8)
+    x = torch.randn(offs[-1], K, generator=g).bfloat16()
+    wq = torch.randint(0, 256, (E, N, K // 2), generator=g, dtype=torch.uint8)
+    if fmt == "mxfp4":
+        ws = torch.randint(120, 124, (E, N, K // 32), generator=g, dtype=torch.uint8)
+        w = mxfp4.dequantize(wq, ws, torch.float32).double()
+    else:
+        ws = (torch.rand(E, N, K // 32, generator=g) * 0.1).bfloat16()
+        w = int4.dequantize(wq, ws).bfloat16().double()
+    off, cnt = torch.tensor(offs, dtype=torch.int32).cuda(), torch.tensor(counts, dtype=torch.int32).cuda()
+    monkeypatch.setattr(_ext, "num_sms", lambda device=None: 2)
+    run = mxfp4.grouped_mxfp4_gemm if fmt == "mxfp4" else int4.grouped_int4_gemm
+    got = run(x.cuda(), wq.cuda(), ws.cuda(), off, silu_mul=silu, counts=cnt).cpu().double()
+    _ext.check_status()
+    for e, c in enumerate(counts):
+        xe = x[offs[e]:offs[e] + c].double()
+        want, mag = xe @ w[e].t(), xe.abs() @ w[e].abs().t()
+        if silu:
+            back = torch.argsort(interleave_gate_up_rows(N))
+            want, mag = want[:, back], mag[:, back]
+            a, u = want.chunk(2, -1)
+            am, um = mag.chunk(2, -1)
+            want = torch.nn.functional.silu(a) * u
+            mag = am * (u.abs() + 1) * 1.1 + um * a.abs()
+        # one rounding to 8 significant bits; fp32 sums of K exact products: K * 2^-24 of their magnitudes
+        assert ((got[offs[e]:offs[e] + c] - want).abs() <= want.abs() * 2 ** -8 + mag * K * 2 ** -24 + 1e-36).all(), e
