@@ -313,7 +313,9 @@ w4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
     // ------------------------------------------------------------ epilogue: thread = weight row, columns = tokens
     for (int tile = blockIdx.x; ok && walk.get(tile, t); tile += gridDim.x, ++acc) {
       const int buf = acc & 1;
-      if (!__all_sync(0xffffffffu, mbar_wait(&ss.tmem_full[buf], (acc >> 1) & 1, abort_flag, kTimeoutEpilogue))) { ok = false; break; }
+      const bool late = !mbar_wait(&ss.tmem_full[buf], (acc >> 1) & 1, abort_flag, kTimeoutEpilogue);
+      // with barriers between the warps below, a warp that gives up alone would leave the others waiting for it
+      if (EPI == EPI_SILU_MUL ? vote_any_128(late) : __any_sync(0xffffffffu, late)) { ok = false; break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + buf * BT;
       const int n_tok = t.m_end - t.m0;

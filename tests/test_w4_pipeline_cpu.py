@@ -1,8 +1,8 @@
 """The barriers of the 4-bit GEMM as a host model: its roles as actors that move one at a time in a random order, with the slot numbering of
 ``w4_steps.h``, the header the kernel includes.
 
-A weight operand carries the (tile, K step, row quarter) it was made of; the product checks all four when it completes.  A planted mistake shows that
-the model sees what it is for: slots that follow the running step."""
+A weight operand carries the (tile, K step, row quarter) it was made of; the product checks all four when it completes.  Two planted mistakes show that
+the model sees what it is for: slots that follow the running step, and epilogue warps that leave one by one."""
 import os
 import shutil
 import subprocess
@@ -203,7 +203,17 @@ def test_every_product_reads_its_own_weights(model):
     assert model(1, 48, 60) == (0, 0)
 
 
+def test_failed_waits_end_every_role(model):
+    """A role that gives up at any moment: every other one ends, with the barriers of the SiLU epilogue between its warps."""
+    wrong, stuck = model(1, 9, 400, aborts=1)
+    assert stuck == 0
+
+
 @pytest.mark.parametrize("steps", [5, 6, 7, 45])
 def test_model_sees_slots_that_follow_the_running_step(model, steps):
     wrong, stuck = model(steps, steps, 400, by_step=1)
     assert wrong + stuck > 0
+
+
+def test_model_sees_epilogue_warps_that_leave_one_by_one(model):
+    assert model(1, 9, 400, one_by_one=1, aborts=1)[1] > 0
