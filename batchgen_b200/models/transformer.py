@@ -206,42 +206,45 @@ class Transformer:
             return attn_ops.mla_out_absorb(o_lat, lw.w_uv)
 
     def _expanded_blocks(self, meta: AttnMeta, T: int, heads: int, page: int):
-        """Blocks of sequences for attention over up-projected keys and values, made once per step: (cache slots of every row the
-        block's queries see, tiles of ``attn_ops.mha_prefill``); None when the absorbed form is the cheaper one.
+        """Blocks of sequences for attention over up-projected keys and values: (cache slots of every row the block's queries see,
+        tiles of ``attn_ops.mha_prefill``); None when the absorbed form is the cheaper one.  The tiles and the rows' places in
+        their sequences depend on lengths alone and are made once per step; slots are read from ``meta`` at every call.
 
         Without cached context the step's own rows are one block.  A cached row costs its up-projection (some 50 ns with 128 heads:
         33.5 MFLOP, 64 KB written and read), a query-key pair saves some 0.3 ns (measured rates: 621 TFLOP/s of 278 KFLOP absorbed,
         575 TFLOP/s of 82 KFLOP expanded), so the pairs have to be some 160 times the rows; 200 leaves a margin.  Blocks bound the
         expanded rows (64 KB each at 128 heads); a sequence that is longer than a block stays with the absorbed form, and so
         does its step.  With context only geometries that the absorbed kernel takes are covered."""
-        key = (tuple(meta.cu_seqlens), tuple(meta.ctx_lens), T)
-        if getattr(meta, "_mha_key", None) == key:
-            return meta._mha_blocks
+        key = (tuple(meta.cu_seqlens), tuple(meta.ctx_lens), T, heads % 8 == 0, page, self.expanded_block_rows)
+        if getattr(meta, "_mha_key", None) != key:
+            meta._mha_key, meta._mha_plan = key, self._expanded_plan(meta, heads, page)
+        if meta._mha_plan is None:
+            return None
+        return [(meta.slot_mapping.clamp_min(0) if seq is None else torch.add(row, meta.block_table[seq, col].long(), alpha=page), work)
+                for seq, col, row, work in meta._mha_plan]
+
+    def _expanded_plan(self, meta: AttnMeta, heads: int, page: int):
+        """Per block: sequence, page of the sequence and row of the page of each key row (or None: the rows of the step), and the tiles."""
         cu, ctx = list(meta.cu_seqlens), list(meta.ctx_lens)
         dev = meta.positions.device
-        blocks = None
         if not any(ctx):
-            work = attn_ops.mha_prefill_work(cu, ctx, cu[:-1]).to(dev)
-            blocks = [(meta.slot_mapping.clamp_min(0), work)]
-        else:
-            parts = expanded_parts(cu, ctx, self.expanded_block_rows) if heads % 8 == 0 and page == 64 else None
-            if parts is not None:
-                blocks = []
-                bt = meta.block_table.long()
-                for seqs in parts:
-                    rows = [ctx[i] + cu[i + 1] - cu[i] for i in seqs]
-                    starts = [0]
-                    for n in rows:
-                        starts.append(starts[-1] + n)
-                    of = torch.repeat_interleave(torch.tensor(seqs, device=dev), torch.tensor(rows, device=dev), output_size=starts[-1])
-                    pos = torch.cat([torch.arange(n, device=dev) for n in rows])
-                    slots = bt[of, pos // page] * page + pos % page
-                    tiles = [attn_ops.mha_prefill_work([cu[i], cu[i + 1]], [ctx[i]], [starts[k]]) for k, i in enumerate(seqs)]
-                    work = torch.cat(tiles)
-                    order = torch.argsort(-(work[:, 3] + work[:, 1]), stable=True)       # longest key ranges first
-                    blocks.append((slots, work[order].contiguous().to(dev)))
-        meta._mha_key, meta._mha_blocks = key, blocks
-        return blocks
+            return [(None, None, None, attn_ops.mha_prefill_work(cu, ctx, cu[:-1]).to(dev))]
+        parts = expanded_parts(cu, ctx, self.expanded_block_rows) if heads % 8 == 0 and page == 64 else None
+        if parts is None:
+            return None
+        plan = []
+        for seqs in parts:
+            rows = [ctx[i] + cu[i + 1] - cu[i] for i in seqs]
+            starts = [0]
+            for n in rows:
+                starts.append(starts[-1] + n)
+            of = torch.repeat_interleave(torch.tensor(seqs, device=dev), torch.tensor(rows, device=dev), output_size=starts[-1])
+            pos = torch.cat([torch.arange(n, device=dev) for n in rows])
+            tiles = [attn_ops.mha_prefill_work([cu[i], cu[i + 1]], [ctx[i]], [starts[k]]) for k, i in enumerate(seqs)]
+            work = torch.cat(tiles)
+            order = torch.argsort(-(work[:, 3] + work[:, 1]), stable=True)       # longest key ranges first
+            plan.append((of, pos // page, pos % page, work[order].contiguous().to(dev)))
+        return plan
 
     def _mla_q(self, lw, q_a, kv_a, meta, cache, l):
         cfg = self.cfg

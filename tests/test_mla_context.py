@@ -13,6 +13,30 @@ def test_expanded_parts_group_sequences_within_a_block():
     assert expanded_parts([0, 0], [8000], 16384) is None
 
 
+@pytest.mark.parametrize("ctx", [[0, 0], [200, 0]])
+def test_slots_follow_the_pages_of_a_reused_step(ctx):
+    """A second step of the same lengths through one AttnMeta: the rows that are read are those of its pages then."""
+    from types import SimpleNamespace
+    from batchgen_b200.models.transformer import AttnMeta, Transformer
+    cu, page = [0, 300, 700], 64
+    need = [-(-(ctx[i] + cu[i + 1] - cu[i]) // page) for i in range(2)]
+    me = SimpleNamespace(expanded_block_rows=16384)
+    for name in ("_expanded_blocks", "_expanded_plan"):
+        if hasattr(Transformer, name):
+            setattr(me, name, getattr(Transformer, name).__get__(me))
+    meta = AttnMeta(mode="prefill", positions=torch.zeros(cu[-1], dtype=torch.int32), slot_mapping=torch.zeros(cu[-1], dtype=torch.int64),
+                    block_table=torch.zeros(2, max(need), dtype=torch.int32), cu_seqlens=cu, ctx_lens=ctx)
+    for seed in range(3):
+        order = torch.randperm(sum(need), generator=torch.Generator().manual_seed(seed)).int()
+        for i in range(2):
+            meta.block_table[i, :need[i]] = order[sum(need[:i]):sum(need[:i + 1])]
+        rows = [torch.arange(ctx[i] + cu[i + 1] - cu[i]) for i in range(2)]
+        want = [meta.block_table[i].long()[r // page] * page + r % page for i, r in enumerate(rows)]
+        meta.slot_mapping.copy_(torch.cat([w[ctx[i]:] for i, w in enumerate(want)]))
+        (slots, work), = me._expanded_blocks(meta, cu[-1], 8, page)
+        assert torch.equal(slots, torch.cat(want)), seed
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("block_rows", [16384, 1300])
 def test_pieces_with_cached_context_take_the_expanded_form(block_rows):
