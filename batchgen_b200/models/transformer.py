@@ -84,6 +84,9 @@ def linear(x, lin: Linear, xq=None, xs=None, silu_mul: bool = False):
     return x @ lin.w.t()
 
 
+EXPANDED_BLOCK_ROWS = 16384      # rows of cached context and prompt whose keys and values are up-projected at a time
+
+
 def expanded_parts(cu, ctx, block_rows: int):
     """Sequences of a step with cached context in groups whose rows (cached and new) stay within ``block_rows``, or None when
     the absorbed form should run (``Transformer._expanded_blocks``)."""
@@ -119,7 +122,7 @@ class Transformer:
         self.attn_request_parallel = False
         self.streamer = None          # models.streaming.StreamedExperts when the routed experts live in host memory
         self.overlap_shared_expert = os.environ.get("BG_OVERLAP_SHARED", "1") != "0"   # decode: shared expert on a side stream
-        self.expanded_block_rows = 16384         # rows of cached context and prompt whose keys and values are up-projected at a time
+        self.expanded_block_rows = EXPANDED_BLOCK_ROWS
         self.expanded_prefill_min_tokens = 256   # below this the absorbed kernel is as fast and saves the kv_b GEMM
 
     # ------------------------------------------------------------------ helpers

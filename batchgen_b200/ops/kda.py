@@ -115,6 +115,15 @@ def chunk_form_pays(lens: Sequence[int], heads: int, sms: int) -> bool:
     return 125 + 0.57 * heads * sum(-(-n // CHUNK) for n in lens) * 148 / sms < tokens
 
 
+def chunk_scratch_bytes(tokens: int, heads: int, dim: int) -> int:
+    """Most scratch that ``kda_forward`` takes for a step of ``tokens`` tokens: a record per (chunk, head) of a round of chunks."""
+    if dim != 128:
+        return 0
+    chunks = -(-tokens // CHUNK) + tokens // CHUNK_MIN_TOKENS        # every piece may end in a part of a chunk
+    most = max(1, _CHUNK_SCRATCH // (4 * _CHUNK_FLOATS * heads))      # of a round
+    return min(chunks, most) * heads * _CHUNK_FLOATS * 4
+
+
 def chunk_plan(cu: Sequence[int], min_tokens: int, most_items: int):
     """Rounds of chunks of the pieces of at least ``min_tokens``: a list of (items, seqs) with items (sequence, first token, tokens,
     tokens of the piece before it) and seqs (sequence, first item, items, 1 at the start of a piece), at most ``most_items`` items a

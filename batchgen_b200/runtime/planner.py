@@ -106,7 +106,7 @@ def plan_deployment(cfg: ModelConfig, ecfg: EngineConfig, machine: MachineProfil
     if cfg.is_layered:
         per_tok = layered_workspace_bytes(cfg)
     per_tok += cfg.num_experts_per_tok * (cfg.expert_hidden * 3 + cfg.moe_intermediate_size * 3) if cfg.n_routed_experts else 0
-    workspace = int(min(ecfg.max_prefill_tokens, 32768) * per_tok * 1.25) + 2 * GiB
+    workspace = int(min(ecfg.max_prefill_tokens, 32768) * per_tok * 1.25) + 2 * GiB + prompt_scratch_bytes(cfg, ecfg)
     graphs = int(0.5 * GiB + ecfg.cuda_graph_num_buckets * 64 * (1 << 20)) if ecfg.enable_cuda_graph else 0
     usable = int(machine.hbm_bytes * ecfg.gpu_memory_frac)
     kv = usable - dense - experts - workspace - graphs
@@ -142,6 +142,21 @@ def layered_workspace_bytes(cfg: ModelConfig) -> int:
     return most + (12 + 4 * max(cfg.streams, 1)) * cfg.hidden_size
 
 
+def prompt_scratch_bytes(cfg: ModelConfig, ecfg: EngineConfig) -> int:
+    """Scratch that one layer of a prefill micro-batch takes beside its activations: the records of KDA chunks, or the keys and values that
+    attention of later prompt pieces up-projects from cached rows (with the gathered rows and their contiguous latent part)."""
+    from ..models.transformer import EXPANDED_BLOCK_ROWS
+    from ..ops import kda
+    tp = max(1, ecfg.attn_tp_size)
+    need = 0
+    if cfg.has_kda:
+        need = kda.chunk_scratch_bytes(ecfg.max_prefill_tokens, max(1, cfg.kda_num_heads // tp), cfg.kda_head_dim)
+    if cfg.is_mla and not cfg.has_dsa and not cfg.is_layered and not cfg.is_v4:
+        heads = max(1, cfg.num_heads // tp)
+        need = max(need, EXPANDED_BLOCK_ROWS * 2 * (heads * (cfg.qk_nope_head_dim + cfg.v_head_dim) + cfg.kv_cache_dim + cfg.kv_lora_rank))
+    return need
+
+
 def state_pool_bytes(cfg: ModelConfig, ecfg: EngineConfig) -> int:
     """Device bytes of the per-sequence state pool (recurrent state of KDA layers, or the window rings and compressor
     windows of DeepSeek-V4): one slot per sequence that may be live at once."""
@@ -163,7 +178,8 @@ def size_kv_pool(cfg: ModelConfig, ecfg: EngineConfig, device: str, dtype) -> Tu
         return ecfg.num_gpu_pages, host_pages
     if str(device).startswith("cuda"):
         free, total = torch.cuda.mem_get_info(torch.device(device))
-        reserve = int(total * (1.0 - ecfg.gpu_memory_frac)) + 4 * GiB      # graphs + prefill workspace headroom
+        # graphs, activations of a prefill micro-batch, a layer's scratch
+        reserve = int(total * (1.0 - ecfg.gpu_memory_frac)) + 4 * GiB + prompt_scratch_bytes(cfg, ecfg)
         if cfg.has_state:                                       # per-sequence state slots come out of the same memory
             reserve += state_pool_bytes(cfg, ecfg)
         if cfg.is_layered:
