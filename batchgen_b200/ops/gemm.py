@@ -232,15 +232,22 @@ def _bf16_swap(x: torch.Tensor, w2d: torch.Tensor, out: torch.Tensor, offsets, c
     _ext.check(rc, "bg_gemm_bf16_swap")
 
 
-def grouped_bf16_gemm(x: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, counts: torch.Tensor, relu2: bool = False) -> torch.Tensor:
+def swap_grouped(rows: float, groups: int, K: int) -> bool:
+    """Tokens as the MMA's N for segments of ``rows`` expected rows: from 128 on, where half of them would need a second 128-row tile
+    (Poisson rows, 256 matrices of 2,048 x 2,304, swapped against the 128 x 128 kernel: 112 rows 489 / 432 us, 128 rows 522 / 514, 156
+    rows 540 / 613, 512 rows 1,104 / 1,267; of 2,304 x 1,024: 112 rows 269 / 241, 128 rows 273 / 293; 32 matrices of 2,048 x 2,304: 13 rows
+    67 / 57, 128 rows 74 / 73, 156 rows 75 / 81).  Below, the weights are streamed, and the 128 x 128 kernel has more of them in flight."""
+    return rows >= 128 and 0 < groups <= 1024 and K > 0 and K % 64 == 0
+
+
+def grouped_bf16_gemm(x: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, counts: torch.Tensor, relu2: bool = False,
+                      rows_hint: Optional[float] = None) -> torch.Tensor:
     """Ragged grouped bf16 GEMM on the GPU: x [R, K] rows grouped by expert, w [E, N, K] -> [R, N] bf16 (``relu2``: the squared
-    positive part of the products); ``counts`` rows of each segment are present, the others stay undefined."""
+    positive part of the products); ``counts`` rows of each segment are present, the others stay undefined.  ``rows_hint``: rows that
+    are expected to be present in all (the capacity x.shape[0] when None; it is far above them where other ranks hold most experts)."""
     E, N, K = w.shape
     out = torch.empty(x.shape[0], N, dtype=torch.bfloat16, device=x.device)
-    # tokens as the MMA's N where segments have a hundred rows and more (256 matrices of 2,048 x 2,304, rows a segment on average: 128
-    # rows 527 -> 484 us, 156 rows 639 -> 511, 512 rows 1,328 -> 1,123; 32 rows 395 -> 442, 4 rows 371 -> 411: there the weights are
-    # streamed, and the 128 x 128 kernel has more of them in flight)
-    if x.shape[0] >= 104 * E and not relu2 and 0 < E <= 1024 and K > 0 and K % 64 == 0:
+    if x.shape[0] and not relu2 and swap_grouped((x.shape[0] if rows_hint is None else rows_hint) / max(E, 1), E, K):
         _bf16_swap(x.contiguous(), w.view(E * N, K), out, offsets, counts, E, N)
     elif x.shape[0]:
         _launch(KIND_BF16, EPI_RELU2 if relu2 else EPI_STORE, x.contiguous(), None, 0, w.view(E * N, K), None, out, offsets, E, x.shape[0], N, K,

@@ -228,7 +228,7 @@ def _grouped_on_kernels(x: torch.Tensor, ew: ExpertWeights) -> bool:
 
 def grouped_experts(xq, xs, offsets: torch.Tensor, ew: ExpertWeights, x_dense: Optional[torch.Tensor] = None,
                     timer=None, counts: Optional[torch.Tensor] = None, row_src: Optional[torch.Tensor] = None,
-                    rows_hint: Optional[int] = None):
+                    rows_hint: Optional[float] = None):
     """Run gate/up -> activation -> down for rows already grouped by expert.  fp8 path takes
     (xq, xs); the unquantised path takes ``x_dense``.  Returns y [rows, Hout].  With ``counts`` (real rows
     per segment) and ``row_src`` (negative on padding rows) the padding rows are skipped end to end."""
@@ -269,10 +269,10 @@ def grouped_experts(xq, xs, offsets: torch.Tensor, ew: ExpertWeights, x_dense: O
     x = x_dense
     if counts is not None and _grouped_on_kernels(x, ew):
         with timer.timed("moe.s1_gemm"):
-            gu = gemm.grouped_bf16_gemm(x, ew.w13, offsets, counts)
+            gu = gemm.grouped_bf16_gemm(x, ew.w13, offsets, counts, rows_hint=rows_hint)
         act = activation(gu, ew.activation, ew.act_limit, offsets, row_src).contiguous()
         with timer.timed("moe.s3_gemm"):
-            return gemm.grouped_bf16_gemm(act, ew.w2, offsets, counts)
+            return gemm.grouped_bf16_gemm(act, ew.w2, offsets, counts, rows_hint=rows_hint)
     out = torch.zeros(x.shape[0], ew.w2.shape[1], dtype=x.dtype, device=x.device)
     off = offsets.tolist()
     for e in range(ew.num_experts):
@@ -286,8 +286,9 @@ def grouped_experts(xq, xs, offsets: torch.Tensor, ew: ExpertWeights, x_dense: O
 def experts_forward(hidden: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.Tensor, ew: ExpertWeights,
                     expert_lo: int, expert_hi: int, extra: Optional[torch.Tensor] = None,
                     num_valid: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
-                    timer=None, before_combine=None) -> torch.Tensor:
-    """Partial MoE output of one rank: sum over the (token, k) pairs whose expert is local (+ ``extra``).
+                    timer=None, before_combine=None, num_experts: Optional[int] = None) -> torch.Tensor:
+    """Partial MoE output of one rank: sum over the (token, k) pairs whose expert is local (+ ``extra``).  ``num_experts``: experts of
+    all ranks (None: the local ones are all), from which follows how many pairs are expected here.
     ``before_combine`` is called right before the combine reads ``extra`` (it may come from another stream)."""
     if timer is None:
         from ..utils.timing import null_timer
@@ -320,7 +321,8 @@ def experts_forward(hidden: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.
             rows = hidden[src.clamp_min(0).long()]
             rows = torch.where((src >= 0).unsqueeze(-1), rows, torch.zeros_like(rows))
         y = grouped_experts(None, None, offsets, ew, x_dense=rows, counts=getattr(offsets, "real_counts", None),
-                            row_src=src if rows.is_cuda else None)
+                            row_src=src if rows.is_cuda else None,
+                            rows_hint=topk_idx.shape[0] * topk_idx.shape[1] * (expert_hi - expert_lo) / max(num_experts or expert_hi - expert_lo, 1))
     with timer.timed("moe.combine"):
         if before_combine is not None:
             before_combine()

@@ -101,12 +101,12 @@ class NcclComm:
         per = num_experts // self.world
         lo, hi = self.rank * per, (self.rank + 1) * per
         if replicated:
-            part = moe_ops.experts_forward(hidden, topk_idx, topk_w, ew, lo, hi, num_valid=num_valid)
+            part = moe_ops.experts_forward(hidden, topk_idx, topk_w, ew, lo, hi, num_valid=num_valid, num_experts=num_experts)
             return self.tp_reduce(part)
         h = self.all_gather_rows(hidden)
         idx = self.all_gather_rows(topk_idx)
         w = self.all_gather_rows(topk_w)
-        part = moe_ops.experts_forward(h, idx, w, ew, lo, hi)
+        part = moe_ops.experts_forward(h, idx, w, ew, lo, hi, num_experts=num_experts)
         return self.reduce_scatter_rows(part)
 
 

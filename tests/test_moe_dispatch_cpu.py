@@ -1,0 +1,38 @@
+"""Which grouped bf16 kernel a step's experts take: by the rows that are expected on this rank, not by the capacity of the buffer."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from batchgen_b200.ops import gemm, moe
+from batchgen_b200.parallel import comm
+
+
+@pytest.mark.parametrize("capacity,hint,swapped", [(200, None, True), (100, None, False), (200, 127.0, False), (1000, 128.0, True), (1000, 13.0, False)])
+def test_grouped_kernel_by_expected_rows(capacity, hint, swapped, monkeypatch):
+    taken = []
+    monkeypatch.setattr(gemm, "_bf16_swap", lambda *a, **k: taken.append(True))
+    monkeypatch.setattr(gemm, "_launch", lambda *a, **k: taken.append(False))
+    E = 4
+    x, w = torch.empty(E * capacity, 64).bfloat16(), torch.empty(E, 32, 64).bfloat16()
+    gemm.grouped_bf16_gemm(x, w, None, None, rows_hint=None if hint is None else hint * E)
+    assert taken == [swapped]
+
+
+@pytest.mark.parametrize("replicated", [True, False])
+def test_expert_parallel_rank_expects_its_share(replicated, monkeypatch):
+    """8 ranks of 4 experts each: an eighth of the step's pairs."""
+    T, K, H, E, W = 64, 3, 16, 32, 8
+    seen = []
+
+    def grouped(xq, xs, offsets, ew, x_dense=None, rows_hint=None, **kw):
+        seen.append(rows_hint)
+        return torch.zeros(x_dense.shape[0], H)
+
+    monkeypatch.setattr(moe, "grouped_experts", grouped)
+    me = SimpleNamespace(world=W, rank=2, tp_reduce=lambda x: x, all_gather_rows=lambda x: x, reduce_scatter_rows=lambda x: x)
+    idx = torch.stack([torch.randperm(E)[:K] for _ in range(T)]).int()
+    ew = moe.ExpertWeights(torch.zeros(E // W, 2 * 8, H), torch.zeros(E // W, H, 8))
+    comm.NcclComm.moe(me, torch.randn(T, H), idx, torch.rand(T, K), ew, E, replicated=replicated)
+    moe.experts_forward(torch.randn(T, H), idx, torch.rand(T, K), moe.ExpertWeights(torch.zeros(E, 16, H), torch.zeros(E, H, 8)), 0, E)
+    assert seen == [T * K / W, T * K]
