@@ -11,6 +11,7 @@
 // row; two accumulators of 256 columns, so one is stored while the other is filled).  All waits are bounded.
 #define BG_FILE_TAG 31     // kernel-trace ids of this file are (tag << 16) | line
 #include "common.cuh"
+#include "token_tiles.cuh"
 
 namespace bg {
 namespace bswap {
@@ -40,38 +41,8 @@ struct Shared {
   uint64_t tmem_full[2], tmem_empty[2];
   uint32_t tmem_base;
   int abort_flag;
-  int offs[kMaxGroups + 1];
-  int cnt[kMaxGroups];
+  Segments<kMaxGroups> seg;
 };
-
-struct Tile { int g, n0, m0, m_end; };               // weight rows n0 .., tokens m0 .. m_end (at most BT)
-
-// Tiles in the order (group, weight tile, token tile): token tiles of one weight tile are neighbours.  Token tiles of a segment are equal
-// up to 16 rows.
-struct Walker {
-  const int* offs;
-  const int* cnt;
-  int groups, n_tiles, M, g, before;
-  __device__ Walker(const int* o, const int* c, int gr, int nt, int m) : offs(o), cnt(c), groups(gr), n_tiles(nt), M(m), g(0), before(0) {}
-  __device__ bool get(int tile, Tile& t) {
-    while (g < groups) {
-      const int rows = offs != nullptr ? cnt[g] : M;
-      const int cut = max(1, (rows + BT - 1) / BT), per = max(16, ((rows + cut - 1) / cut + 15) / 16 * 16);   // per <= BT
-      const int tt = (rows + per - 1) / per, here = tt * n_tiles;
-      if (tile < before + here) {
-        const int local = tile - before, base = offs != nullptr ? offs[g] : 0;
-        t.g = g; t.n0 = (local / tt) * BW; t.m0 = base + (local % tt) * per; t.m_end = min(t.m0 + per, base + rows);
-        return true;
-      }
-      before += here;
-      ++g;
-    }
-    return false;
-  }
-};
-
-// tokens of a tile as the MMA's N
-__device__ __forceinline__ int tile_cols(const Tile& t) { return (t.m_end - t.m0 + 15) / 16 * 16; }
 
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params p) {
@@ -92,13 +63,7 @@ gemm_bf16_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
     ss.abort_flag = 0;
     mbar_fence_init();
   }
-  if (p.offsets != nullptr) {
-    for (int i = threadIdx.x; i <= p.groups; i += kThreads) ss.offs[i] = p.offsets[i];
-    for (int i = threadIdx.x; i < p.groups; i += kThreads) {
-      const int whole = p.offsets[i + 1] - p.offsets[i];
-      ss.cnt[i] = p.counts != nullptr ? min(max(p.counts[i], 0), whole) : whole;
-    }
-  }
+  if (p.offsets != nullptr) load_segments<BT>(ss.seg, p.offsets, p.counts, p.groups);
   if (warp == 1) {
     tmem_alloc(&ss.tmem_base, kTmemCols);
     tmem_relinquish();
@@ -107,8 +72,8 @@ gemm_bf16_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
-  Walker walk(p.offsets != nullptr ? ss.offs : nullptr, ss.cnt, p.groups, n_tiles, p.M);
-  Tile t;
+  TokenWalker<BT, BW, kMaxGroups> walk(p.offsets != nullptr ? &ss.seg : nullptr, p.groups, n_tiles, p.M);
+  TokenTile t;
   uint32_t it = 0, acc = 0;
   bool ok = true;
 
