@@ -213,15 +213,25 @@ def bf16_gemm(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = No
         out = torch.empty(T, N, dtype=torch.float32 if fp32_out else torch.bfloat16, device=x.device)
     if T == 0:
         return out
-    # three quarters of the SMs with a tile of 256 tokens x 128 outputs: the wider product moves fewer operand bytes per FLOP (4,096 x 16,576 x
-    # 2,304 332 -> 253 us, 6,200 x 32,768 x 512 299 -> 202, 1,024 x 4,096 x 2,880 27 -> 21; 300 x 2,304 x 4,096, where the other kernel
-    # splits K, 19 -> 23)
     if (not fp32_out and not _hooks_pending and out.dtype == torch.bfloat16 and out.stride(1) == 1 and x.is_contiguous() and w.is_contiguous()
-            and K > 0 and K % 64 == 0 and 4 * (-(-T // 256)) * (-(-N // 128)) >= 3 * _ext.num_sms(x.device)):
+            and swap_dense(T, N, K, _ext.num_sms(x.device))):
         _bf16_swap(x, w, out, None, None, 1, N)
         return out
     _launch(KIND_BF16, EPI_STORE_F32 if fp32_out else EPI_STORE, x, None, 0, w, None, out, None, 1, T, N, K)
     return out
+
+
+def swap_dense(T: int, N: int, K: int, sms: int) -> bool:
+    """Tokens as the MMA's N: three quarters of the SMs with a tile of 256 tokens x 128 outputs, where the wider product moves fewer operand
+    bytes per FLOP (4,096 x 16,576 x 2,304 332 -> 253 us, 6,200 x 32,768 x 512 299 -> 202, 1,024 x 4,096 x 2,880 27 -> 21; 300 x 2,304 x 4,096,
+    where the other kernel splits K, 19 -> 23), down to one token (16,576 x 2,304: 1 token 26 -> 18, 24 tokens 22.5 -> 18.9, 160 tokens 25 ->
+    20.6).  Not for up to 128 tokens of 65,536 elements and more with K of 1,536 and more: one token tile in both kernels, which
+    stream the weights, and the 128 x 128 kernel has more of them in flight (swapped / 128 x 128: 16,576 x 2,304, 32 tokens 18.3 / 17.8 us; 32,768 x
+    2,304, 100 tokens 35.7 / 33.8; 16,384 x 7,168, 12 tokens 46.8 / 43.9, 8 tokens 46.4 / 57.3; 32,768 x 512, 32 tokens 9.9 / 12.5); why it is the
+    slower one below those 65,536 elements was not found."""
+    if K <= 0 or K % 64 or 4 * (-(-T // 256)) * (-(-N // 128)) < 3 * sms:
+        return False
+    return T > 128 or K < 1536 or T * K < 65536
 
 
 def _bf16_swap(x: torch.Tensor, w2d: torch.Tensor, out: torch.Tensor, offsets, counts, groups: int, N: int) -> None:

@@ -1,4 +1,5 @@
-"""Which grouped bf16 kernel a step's experts take: by the rows that are expected on this rank, not by the capacity of the buffer."""
+"""Which bf16 kernel a product takes: grouped ones by the rows that are expected on this rank, not by the capacity of the buffer; dense ones
+by their tiles, unless a few tokens stream the weights."""
 from types import SimpleNamespace
 
 import pytest
@@ -36,3 +37,11 @@ def test_expert_parallel_rank_expects_its_share(replicated, monkeypatch):
     comm.NcclComm.moe(me, torch.randn(T, H), idx, torch.rand(T, K), ew, E, replicated=replicated)
     moe.experts_forward(torch.randn(T, H), idx, torch.rand(T, K), moe.ExpertWeights(torch.zeros(E, 16, H), torch.zeros(E, H, 8)), 0, E)
     assert seen == [T * K / W, T * K]
+
+
+@pytest.mark.parametrize("T,N,K,swapped", [(4096, 16576, 2304, True), (1024, 4096, 2880, True), (300, 2304, 4096, False), (1, 14208, 2304, True),
+                                           (1, 14080, 2304, False), (28, 16576, 2304, True), (29, 16576, 2304, False), (128, 16576, 2304, False),
+                                           (129, 16576, 2304, True), (9, 16384, 7168, True), (10, 16384, 7168, False), (128, 32768, 512, True),
+                                           (64, 16384, 1472, True), (64, 16384, 1536, False), (512, 16384, 96, False)])
+def test_dense_kernel_by_tiles_and_tokens(T, N, K, swapped):
+    assert gemm.swap_dense(T, N, K, 148) == swapped
