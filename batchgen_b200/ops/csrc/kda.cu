@@ -203,8 +203,10 @@ __global__ void __launch_bounds__(2 * D, 2) kda_seq_kernel(const Params p) {
 //
 // `chunk_prepare` makes W, Q', Kd = K exp(G_last - G), UV and O0 of every (chunk, head) at once, from the raw projections; `chunk_chain`
 // walks the chunks of a (sequence, head, 32 value columns) with S in shared memory; `chunk_finish` norms and gates whole heads.  Every
-// exponent is a sum of log decays over a range of tokens, at most zero: running sums restart every 16 tokens, products of
-// different 16-token blocks meet at the border before the later one.
+// exponent is a sum of the log decays of its own range of tokens, at most zero, and never a difference of running sums: behind a strong
+// decay a difference would carry that decay's rounding into the weak ones after it (tokens of 2^-400 and of 2^-0.001 in turn: states off
+// by 1.3e-5 with differences, 1.2e-7 so, 1.4e-7 token by token).  Products of different 16-token blocks meet at the border before the
+// later one.
 //
 // The token-by-token kernel runs a barrier chain of some 2 us a token with a CTA per head.  Here the limit is what shared memory delivers to
 // the fp32 FMAs: about 75,000 a token and head, two thirds of them in the chain.  One prompt of 4,096 tokens, 32 heads: 8,086 -> 1,228
@@ -226,7 +228,8 @@ __device__ __forceinline__ float ex2(float x) {
 __device__ __forceinline__ float2 twice(float x) { return make_float2(x, x); }
 
 constexpr int kPrepThreads = 512;
-constexpr int kPrepareFloats = 4 * kChunk * kPad + (2 * kSub + 3 * kSub) * kPad + 2 * kChunk * kAStride + kChunk;
+constexpr int kBlocks = kChunk / kSub;
+constexpr int kPrepareFloats = 4 * kChunk * kPad + (2 * kSub + 3 * kSub) * kPad + 2 * kChunk * kAStride + kChunk + kBlocks * 128;
 
 // Sixteen warps, one CTA an SM: the steps are short and each waits for the one before, so more warps hide more of a step's latency.
 __global__ void __launch_bounds__(kPrepThreads, 1)
@@ -235,7 +238,7 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
   extern __shared__ __align__(16) float sm[];
   float* kn = sm;                              // [64][kPad] each
   float* qn = kn + kChunk * kPad;
-  float* lg = qn + kChunk * kPad;              // log2 decay, running inside blocks of 16
+  float* lg = qn + kChunk * kPad;              // log2 decay of each token
   float* vv = lg + kChunk * kPad;
   float* ke = vv + kChunk * kPad;              // [16], then [16], then [48]: one block row's decayed operands; later K exp(G), W
   float* qe = ke + kSub * kPad;
@@ -243,6 +246,7 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
   float* am = kd + 3 * kSub * kPad;            // [64][kAStride] M, then L = I + diag(b) M and its inverse, then T
   float* pm = am + kChunk * kAStride;          // [64][kAStride] P
   float* bs = pm + kChunk * kAStride;          // [64]
+  float* tot = bs + kChunk;                    // [kBlocks][128] log2 decay over a block
   const ChunkItem it = items[blockIdx.x];
   const int h = blockIdx.y, H = p.H, HD = H * D;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -290,11 +294,12 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
           win[0] = win[1]; win[1] = win[2]; win[2] = xi;
           dst[(b + i) * kPad] = in ? y : 0.f;
         } else {
-          // a decay of 2^-160 and less is zero, as it was
-          run += in ? fmaxf(neg_a * softplus(xi + dtb) * kLog2e, -160.f) : 0.f;
-          dst[(b + i) * kPad] = run;
+          const float g = in ? neg_a * softplus(xi + dtb) * kLog2e : 0.f;
+          run += g;
+          dst[(b + i) * kPad] = g;
         }
       }
+      if (part == 3) tot[b / 16 * 128 + j] = run;
     }
     if (tid < kChunk) bs[tid] = tid < it.n ? sigmoid(__bfloat162float(p.beta[(size_t)(it.t0 + tid) * p.beta_stride + h])) : 0.f;
   }
@@ -315,17 +320,18 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
   for (int i = warp; i < kChunk; i += 16) {
     const int b0 = i & ~(kSub - 1), r = i - b0;
     const float4 ki = *reinterpret_cast<const float4*>(kn + i * kPad + lane * 4), qi = *reinterpret_cast<const float4*>(qn + i * kPad + lane * 4);
-    const float4 li = *reinterpret_cast<const float4*>(lg + i * kPad + lane * 4);
+    float4 run = make_float4(0.f, 0.f, 0.f, 0.f);                   // of tokens j + 1 .. r
     float v[32];
 #pragma unroll
-    for (int j = 0; j < kSub; ++j) {
+    for (int j = kSub - 1; j >= 0; --j) {
       v[j] = v[16 + j] = 0.f;
       if (j <= r) {
         const float4 kj = *reinterpret_cast<const float4*>(kn + (b0 + j) * kPad + lane * 4);
         const float4 lj = *reinterpret_cast<const float4*>(lg + (b0 + j) * kPad + lane * 4);
-        const float4 e = make_float4(kj.x * ex2(li.x - lj.x), kj.y * ex2(li.y - lj.y), kj.z * ex2(li.z - lj.z), kj.w * ex2(li.w - lj.w));
+        const float4 e = make_float4(kj.x * ex2(run.x), kj.y * ex2(run.y), kj.z * ex2(run.z), kj.w * ex2(run.w));
         v[j] = j < r ? ki.x * e.x + ki.y * e.y + ki.z * e.z + ki.w * e.w : 0.f;
         v[16 + j] = qi.x * e.x + qi.y * e.y + qi.z * e.z + qi.w * e.w;
+        run.x += lj.x; run.y += lj.y; run.z += lj.z; run.w += lj.w;
       }
     }
 #pragma unroll
@@ -338,27 +344,29 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
       }
     }
     (lane < 16 ? am : pm)[i * kAStride + b0 + (lane & 15)] = v[0];
-    for (int j = b0 + kSub + lane; j < kChunk; j += 32) am[i * kAStride + j] = pm[i * kAStride + j] = 0.f;
   }
   // ---- block row a against the blocks before it, decays split at the border before block a; half of the threads for M, half for P
+  const int blk = tid >> 7, ch = tid & 127, walk = blk * kSub * kPad + ch;
 #pragma unroll 1
   for (int a = 1; a < kChunk / kSub; ++a) {
     __syncthreads();
-    for (int i = tid; i < (a + 1) * kSub * 32; i += kPrepThreads) {
-      const int r = i >> 5, c4 = (i & 31) * 4, b = r / kSub;
-      const float4 l = *reinterpret_cast<const float4*>(lg + r * kPad + c4), k = *reinterpret_cast<const float4*>(kn + r * kPad + c4);
-      if (b == a) {
-        const float4 q = *reinterpret_cast<const float4*>(qn + r * kPad + c4), e = make_float4(ex2(l.x), ex2(l.y), ex2(l.z), ex2(l.w));
-        *reinterpret_cast<float4*>(ke + (r - a * kSub) * kPad + c4) = make_float4(k.x * e.x, k.y * e.y, k.z * e.z, k.w * e.w);
-        *reinterpret_cast<float4*>(qe + (r - a * kSub) * kPad + c4) = make_float4(q.x * e.x, q.y * e.y, q.z * e.z, q.w * e.w);
-      } else {
-        float4 x = *reinterpret_cast<const float4*>(lg + (b * kSub + kSub - 1) * kPad + c4);
-        x.x -= l.x; x.y -= l.y; x.z -= l.z; x.w -= l.w;
-        for (int m = b + 1; m < a; ++m) {
-          const float4 y = *reinterpret_cast<const float4*>(lg + (m * kSub + kSub - 1) * kPad + c4);
-          x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
-        }
-        *reinterpret_cast<float4*>(kd + r * kPad + c4) = make_float4(k.x * ex2(x.x), k.y * ex2(x.y), k.z * ex2(x.z), k.w * ex2(x.w));
+    // a thread walks one channel of a block, up from the border in block a, down to it in the others
+    if (blk == a) {
+      float run = 0.f;
+#pragma unroll
+      for (int i = 0; i < kSub; ++i) {
+        run += lg[walk + i * kPad];
+        const float e = ex2(run);
+        ke[i * kPad + ch] = kn[walk + i * kPad] * e;
+        qe[i * kPad + ch] = qn[walk + i * kPad] * e;
+      }
+    } else if (blk < a) {
+      float run = 0.f;
+      for (int m = blk + 1; m < a; ++m) run += tot[m * 128 + ch];
+#pragma unroll
+      for (int i = kSub - 1; i >= 0; --i) {
+        kd[(blk * kSub + i) * kPad + ch] = kn[walk + i * kPad] * ex2(run);
+        run += lg[walk + i * kPad];
       }
     }
     __syncthreads();
@@ -382,8 +390,7 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
         (tid < 256 ? am : pm)[(a * kSub + i) * kAStride + b * kSub + jj] = (sum[b][0].x + sum[b][1].x) + (sum[b][0].y + sum[b][1].y);
   }
   __syncthreads();
-  // ---- diagonal blocks of (I + diag(b) M)^-1: a thread solves for one column (two warps); the others make K exp(G) over the block
-  // operands, Q exp(G) in place, Kd and exp(G_last)
+  // ---- diagonal blocks of (I + diag(b) M)^-1: a thread of the first two warps solves for one column
   if (warp < 2) {
     const int b0 = tid & ~(kSub - 1), col = tid & (kSub - 1);
     float x[kSub];
@@ -402,28 +409,30 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
     __syncwarp();                              // a block's 16 columns are lanes of one warp: M of the block is read
 #pragma unroll
     for (int i = 0; i < kSub; ++i) am[(b0 + i) * kAStride + b0 + col] = x[i];
-  } else {
-    for (int i = tid - 64; i < kChunk * 32; i += kPrepThreads - 64) {
-      const int r = i >> 5, c4 = (i & 31) * 4, a = r / kSub;
-      const float4 l = *reinterpret_cast<const float4*>(lg + r * kPad + c4), k = *reinterpret_cast<const float4*>(kn + r * kPad + c4);
-      float4 up = l, down = make_float4(-l.x, -l.y, -l.z, -l.w);
+  }
+  // ---- K exp(G) over the block operands, Q exp(G) in place, Kd and exp(G_last): a thread walks one channel of a block
+  {
+    float up = 0.f, down = 0.f;
+    for (int m = 0; m < blk; ++m) up += tot[m * 128 + ch];
+    for (int m = blk + 1; m < kBlocks; ++m) down += tot[m * 128 + ch];
 #pragma unroll
-      for (int m = 0; m < kChunk / kSub; ++m) {
-        const float4 y = *reinterpret_cast<const float4*>(lg + (m * kSub + kSub - 1) * kPad + c4);
-        if (m < a) { up.x += y.x; up.y += y.y; up.z += y.z; up.w += y.w; }
-        else { down.x += y.x; down.y += y.y; down.z += y.z; down.w += y.w; }
-      }
-      const float4 e = make_float4(ex2(up.x), ex2(up.y), ex2(up.z), ex2(up.w));
-      *reinterpret_cast<float4*>(ke + r * kPad + c4) = make_float4(k.x * e.x, k.y * e.y, k.z * e.z, k.w * e.w);
-      *reinterpret_cast<float4*>(out + 2 * kPart + r * D + c4) =
-          make_float4(k.x * ex2(down.x), k.y * ex2(down.y), k.z * ex2(down.z), k.w * ex2(down.w));
-      const float4 q = *reinterpret_cast<const float4*>(qn + r * kPad + c4);
-      *reinterpret_cast<float4*>(qn + r * kPad + c4) = make_float4(q.x * e.x, q.y * e.y, q.z * e.z, q.w * e.w);
-      if (r == kChunk - 1) *reinterpret_cast<float4*>(g_last + ((size_t)blockIdx.x * H + h) * D + c4) = e;
+    for (int i = kSub - 1; i >= 0; --i) {
+      out[2 * kPart + (blk * kSub + i) * D + ch] = kn[walk + i * kPad] * ex2(down);
+      down += lg[walk + i * kPad];
     }
+    float e = 1.f;
+#pragma unroll
+    for (int i = 0; i < kSub; ++i) {
+      up += lg[walk + i * kPad];
+      e = ex2(up);
+      ke[walk + i * kPad] = kn[walk + i * kPad] * e;
+      qn[walk + i * kPad] *= e;
+    }
+    if (blk == kBlocks - 1) g_last[((size_t)blockIdx.x * H + h) * D + ch] = e;
   }
   // ---- the blocks below: X_ab = -X_aa (sum over b <= m < a of diag(b) M_am X_mb), a block row at a time; the sums stand in the places of
-  // X_ab's transposed mirror above the diagonal, which is zeroed again
+  // X_ab's transposed mirror above the diagonal.  Here and below what lies above a diagonal is left out, not multiplied by zero: a token
+  // that is not finite stays out of the rows before it
 #pragma unroll 1
   for (int a = 1; a < kChunk / kSub; ++a) {
     __syncthreads();
@@ -440,14 +449,14 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
       float s = 0.f;
 #pragma unroll
       for (int m = 0; m < kSub; ++m)
-        s = fmaf(am[(a * kSub + i) * kAStride + a * kSub + m], am[(b * kSub + m) * kAStride + a * kSub + j], s);
+        if (m <= i) s = fmaf(am[(a * kSub + i) * kAStride + a * kSub + m], am[(b * kSub + m) * kAStride + a * kSub + j], s);
       am[(a * kSub + i) * kAStride + b * kSub + j] = -s;
     }
   }
   __syncthreads();
   for (int o = tid; o < kChunk * kChunk; o += kPrepThreads) {
     const int i = o >> 6, j = o & 63;
-    am[i * kAStride + j] = j / kSub > i / kSub ? 0.f : am[i * kAStride + j] * bs[j];
+    if (j <= i) am[i * kAStride + j] *= bs[j];
   }
   __syncthreads();
   // ---- rows 8 g .. 8 g + 7 of a lower-triangular [64, 64] times a [64, 128], 4 columns a lane; a warp per (g, matrix)
@@ -457,7 +466,7 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
 #pragma unroll
     for (int r = 0; r < 8; ++r) x[r][0] = x[r][1] = make_float2(0.f, 0.f);
 #pragma unroll 2
-    for (int j = 0; j < grp * 8 + 8; j += 4) {
+    for (int j = 0; j < grp * 8; j += 4) {
       float4 l[4];
 #pragma unroll
       for (int m = 0; m < 4; ++m) l[m] = *reinterpret_cast<const float4*>(mat + (j + m) * kPad);
@@ -471,6 +480,16 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
           x[r][0] = __ffma2_rn(t2, make_float2(l[m].x, l[m].y), x[r][0]);
           x[r][1] = __ffma2_rn(t2, make_float2(l[m].z, l[m].w), x[r][1]);
         }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {                                   // the group's own columns, up to each row's diagonal
+      const float4 l = *reinterpret_cast<const float4*>(mat + (grp * 8 + j) * kPad);
+#pragma unroll
+      for (int r = j; r < 8; ++r) {
+        const float2 t2 = twice(tri[(grp * 8 + r) * kAStride + grp * 8 + j]);
+        x[r][0] = __ffma2_rn(t2, make_float2(l.x, l.y), x[r][0]);
+        x[r][1] = __ffma2_rn(t2, make_float2(l.z, l.w), x[r][1]);
       }
     }
   };

@@ -169,3 +169,71 @@ def test_chunk_form_against_64_bits(decay, scratch, monkeypatch):
         # a value rounded to 8 significant bits; the recurrence in fp32
         assert (d.abs() <= want[live].abs() * 2 ** -8 + 2e-4).all(), (form, d.abs().max())
     assert err["chunks"][0] <= 1.5 * err["tokens"][0] + 1e-7 and err["chunks"][1] <= 1.02 * err["tokens"][1], err
+
+
+def _prompt(H, lens, seed, f=None):
+    """One set of pieces, fresh and continued in turn, heads of 128: inputs, parameters, states."""
+    from batchgen_b200.ops import kda
+    HD = H * 128
+    g = torch.Generator().manual_seed(seed)
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    T, B = cu[-1], len(lens)
+    qkv, z = torch.randn(T, 3 * HD, generator=g).bfloat16(), torch.randn(T, HD, generator=g).bfloat16()
+    if f is None:
+        f = torch.randn(T, HD, generator=g).bfloat16()
+    beta = (torch.randn(T, H, generator=g) * 2).bfloat16()
+    p = [torch.randn(3 * HD, 4, generator=g) * 0.5, torch.randn(3 * HD, generator=g) * 0.1, torch.full((H,), 4.5),
+         torch.zeros(HD), 1 + 0.1 * torch.randn(128, generator=g)]
+    conv, rec = torch.randn(B, 3 * HD, 3, generator=g).bfloat16().float(), torch.randn(B, H, 128, 128, generator=g) * 0.3
+    return cu, list(range(B)), [i % 2 for i in range(B)], qkv, z, f, beta, kda.KDAParams(*(t.cuda() for t in p)), conv, rec
+
+
+def _both_forms(monkeypatch, cu, slots, has, qkv, z, f, beta, p, conv0, rec0, H):
+    from batchgen_b200.ops import kda
+    monkeypatch.setattr(kda, "chunk_form_pays", lambda lens, heads, sms: bool(lens))
+    out = {}
+    for form, least in (("chunks", 48), ("tokens", 1 << 30)):
+        monkeypatch.setattr(kda, "CHUNK_MIN_TOKENS", least)
+        conv, rec = conv0.cuda(), rec0.cuda()
+        o = kda.kda_forward(qkv.cuda(), f.cuda(), beta.cuda(), z.cuda(), p, conv, rec, slots, cu, has, H, 128, 128 ** -0.5, 1e-6)
+        out[form] = o.cpu().double(), conv.cpu().double(), rec.cpu().double()
+    return out
+
+
+def test_chunk_form_with_strong_and_weak_decays_in_turn(monkeypatch):
+    """Channels where a token forgets everything (2^-400) beside ones that forget almost nothing (2^-0.001): the weak decays behind a strong
+    one count with their own precision, as token by token."""
+    H, lens = 3, [64, 129, 300]
+    g = torch.Generator().manual_seed(11)
+    shape = (sum(lens), H * 128)
+    f = torch.where(torch.rand(shape, generator=g) < 0.4, torch.rand(shape, generator=g) * 3 + 2, -8 - 6 * torch.rand(shape, generator=g)).bfloat16()
+    cu, slots, has, qkv, z, f, beta, p, conv0, rec0 = _prompt(H, lens, 12, f)
+    conv64, rec64 = conv0.double(), rec0.double()
+    want = _recurrence64(qkv, f, beta, z, p, conv64, rec64, slots, cu, has, H, 128, 128 ** -0.5, 1e-6)
+    err = {}
+    for form, (o, conv, rec) in _both_forms(monkeypatch, cu, slots, has, qkv, z, f, beta, p, conv0, rec0, H).items():
+        assert torch.equal(conv, conv64)
+        err[form] = ((rec - rec64).norm() / rec64.norm()).item(), ((o - want).norm() / want.norm()).item()
+    print(err)
+    assert err["chunks"][0] <= 1.5 * err["tokens"][0] + 1e-7 and err["chunks"][1] <= 1.02 * err["tokens"][1], err
+
+
+@pytest.mark.parametrize("where", ["f", "q", "k", "v", "beta"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("at", [0, 9, 15, 16, 40, 63, 64, 100])
+def test_chunk_form_keeps_what_is_not_finite_to_later_tokens(where, value, at, monkeypatch):
+    """A value that is not finite at one token: the tokens before it are what they are without it, and a NaN is passed on wherever it is token
+    by token.  (An infinite decay input forgets everything and harms nothing.)"""
+    H, lens = 2, [130]
+    cu, slots, has, qkv, z, f, beta, p, conv0, rec0 = _prompt(H, lens, 13)
+    p.A_log.fill_(-1.0)
+    clean = _both_forms(monkeypatch, cu, slots, has, qkv, z, f, beta, p, conv0, rec0, H)["chunks"][0]
+    {"f": f, "q": qkv[:, :256], "k": qkv[:, 256:512], "v": qkv[:, 512:], "beta": beta}[where][at, 1] = value
+    form = _both_forms(monkeypatch, cu, slots, has, qkv, z, f, beta, p, conv0, rec0, H)
+    (o, _, rec), (ot, _, rect) = form["chunks"], form["tokens"]
+    assert torch.equal(o[:at], clean[:at])
+    assert (torch.isnan(o) | ~torch.isnan(ot)).all() and (torch.isnan(rec) | ~torch.isnan(rect)).all()
+    if where == "f" and value == float("inf"):
+        assert torch.isfinite(o).all() and torch.isfinite(rec).all()
