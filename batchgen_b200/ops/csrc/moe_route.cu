@@ -304,7 +304,8 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ y, int ldy, const int* __re
 // an expert's segment (row_src < 0), are skipped: blocks walk the rows, so a capacity far above the rows that are present costs
 // nothing.  Bound by reading 4 F and writing 2 F bytes a row.  As tensor operations it was some ten passes in fp32 over the whole capacity:
 // 4 us instead of some 1,000 us for one token and 4 of 128 experts of 3,072 columns (16,512 rows of capacity); 18,600 rows of the same
-// width take 64 us (5.4 TB/s; 97 with an exact exponential and division, whose last bits the rounding to bf16 drops).
+// width take 97 us (3.5 TB/s), bound by the exponential and the division, which stay those of fp32: __expf and __fdividef took 64 us, but
+// their error grows with |g| (1.5e-6 of the value at 20) and their quotient is zero past 2^126.
 // A clamp lets a NaN through, like the tensor operation does.
 template <int KIND>
 __global__ void __launch_bounds__(256)
@@ -324,7 +325,7 @@ gated_rows_kernel(const __nv_bfloat16* __restrict__ z, long long ldz, __nv_bfloa
           g = g > limit ? limit : g;
           u = u > limit ? limit : u < -limit ? -limit : u;
         }
-        return KIND == 1 ? (u + 1.f) * __fdividef(g, 1.f + __expf(-1.702f * g)) : __fdividef(g, 1.f + __expf(-g)) * u;
+        return KIND == 1 ? (u + 1.f) * g / (1.f + expf(-1.702f * g)) : g / (1.f + expf(-g)) * u;
       };
       __align__(16) __nv_bfloat162 o[4];
 #pragma unroll

@@ -37,6 +37,25 @@ def test_activation_rows(kind, limit, rows, F, pad):
         assert ((a - b).abs()[fine] <= b.abs()[fine] * (2 ** -8 + 1e-5) + 1e-30).all()
 
 
+@pytest.mark.parametrize("kind,limit", [("silu", 0.0), ("swiglu_clamped", 7.0), ("silu_limit", 2.5)])
+def test_activation_keeps_fp32(kind, limit):
+    """The activation is computed in fp32 and rounded once, for gates down to where the exponential overflows: an output differs from the rounded 64-bit
+    value only where that value lies as near to the border between two bf16 numbers as fp32 arithmetic is exact."""
+    from batchgen_b200.ops import moe
+    g = torch.Generator().manual_seed(2)
+    F = 1 << 14
+    z = torch.cat([torch.rand(16, F, generator=g) * 95 - 87.5, torch.randn(16, F, generator=g)], 1).bfloat16()
+    z[:, 0] = -87.5
+    got, want = moe.activation(z.cuda(), kind, limit).double().cpu(), _plain(z, kind, limit)
+    near = want.float().bfloat16().double()
+    # expf 2 units of 2^-24, the sum, the quotient and two products half a unit each, of which 1.702 g moves the exponent: |1.702 g| 2^-24
+    slack = 2.0 ** -24 * (4 + (1.702 * z[:, :F].double().abs() if kind == "swiglu_clamped" else 0))
+    # an ulp of bf16 is 2^-7 to 2^-8 of the value: the border lies half of it away
+    step = torch.exp2(want.abs().clamp_min(1e-300).log2().floor() - 7)
+    border = ((want / step).abs() % 1 - 0.5).abs() * step
+    assert ((got == near) | ((border <= want.abs() * slack) & ((got - near).abs() <= step * 1.01)) | (want.abs() < 1e-35)).all()
+
+
 @pytest.mark.parametrize("T", [1, 5, 130])
 @pytest.mark.parametrize("quant", ["none", "mxfp4"])
 @pytest.mark.parametrize("kind", ["silu", "swiglu_clamped"])
