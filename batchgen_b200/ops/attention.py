@@ -117,7 +117,7 @@ def gqa_prefill_on_kernel(page: int, tiles: int) -> bool:
 
 def gqa_prefill(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, work: torch.Tensor, num_kv_heads: int,
                 scale: float, out: torch.Tensor, window: int = 0, sinks: Optional[torch.Tensor] = None) -> None:
-    """Causal attention of prompt pieces over cached rows, probabilities to 2^-17 of themselves.  q [T, Hq, D] bf16 turned queries (a
+    """Causal attention of prompt pieces over cached rows, fp32 probabilities whole (three bf16 parts).  q [T, Hq, D] bf16 turned queries (a
     column view of the projections is fine); cache [P, page, 2 Hkv D] with the new rows written; ``work`` int32 rows of
     ``talking.prefill_work`` -> out [T, Hq * D] for the rows that tiles cover."""
     T, Hq, D = q.shape

@@ -110,6 +110,14 @@ __device__ __forceinline__ bool vote_any_128(bool v) {      // named barrier 2 o
   return r != 0;
 }
 
+// The 8 leading significant bits of both floats as a pair of bf16, cut off and not rounded; e keeps the rest.  Three times this takes the 24
+// bits of a float whole: the parts of an fp32 operand for products on the tensor cores.
+__device__ __forceinline__ uint32_t cut_bf16x2(float2& e) {
+  const uint32_t x = __float_as_uint(e.x), y = __float_as_uint(e.y);
+  e = __ffma2_rn(make_float2(__uint_as_float(x & 0xffff0000u), __uint_as_float(y & 0xffff0000u)), make_float2(-1.f, -1.f), e);
+  return __byte_perm(x, y, 0x7632);
+}
+
 // ---------------------------------------------------------------- TMA (plain per-CTA tile loads only)
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0,
                                             int c1) {

@@ -6,14 +6,17 @@
 //   O[q, :] += P[q, k] . V[k, kv(h)]     (V read N-major, P written by the softmax threads as a swizzled K-major tile)
 //
 // FINE form (bf16 projections; the models whose attention was computed in fp32 from bf16 operands): queries are read where the
-// projection left them, the scale meets the fp32 scores, and a probability goes into two bf16 parts, p = hi + lo with |p - hi - lo|
-// below 2^-17 p, whose products with V are both accumulated.  The parts are the A operand from TMEM: they take the 2 x 32 columns of the
-// scores they were made of, so P costs no shared memory and two CTAs fit an SM up to 128-wide heads; S(t + 1) then waits for
+// projection left them, the scale meets the fp32 scores, and a probability goes whole into three bf16 parts of 8 bits, whose products with V
+// are all accumulated.  The first two are the A operand from TMEM: they take the 2 x 32 columns of the scores they were made of; the third goes
+// through shared memory, like P of the other form, so two CTAs fit an SM up to 128-wide heads.  S(t + 1) then waits for
 // P.V(t - 1), whose operand it overwrites.  Value rows past a sequence's end are zeroed before the last product, so stale rows of
 // a page cannot reach it through 0 * inf.  Bound by exponentials (16 a clock and SM) at 64-wide heads, by the two products with V
 // at 128-wide ones.  Measured on whole prompt steps, against scores and probabilities as fp32 tensors in memory: two layers of 64
 // heads of 64 with 128 experts, three prompts of up to 2,047 tokens 29.9 -> 10.4 ms; two layers of 48 heads of 128 with 256 experts,
 // two prompts of up to 1,100 behind 333 cached tokens 7.94 -> 2.91 ms.
+// The third part costs 4 to 6 % (4,650 tokens in three prompts, 64 heads of 64: 231 -> 242 us; 4,096 tokens, 48 heads of 128: 372 -> 393)
+// and is kept for the probabilities' sake: with two parts that lose 2^-17, 2e-3 of the outputs differ from the rounded 64-bit ones, with three
+// 3e-4 within a window (fp32 sums: 2e-4 to 3e-4) and up to 2e-3 over 2,000 keys, where the tensor cores' accumulation shows.
 //
 // A first kernel turns the queries, folds scale * log2(e) in and rounds them once to bf16.  One CTA = (tile of 128 queries of
 // one sequence, head).  K and V come straight from the paged cache by TMA (3-D map: column, token of the page, page) through a
@@ -98,9 +101,9 @@ __device__ __forceinline__ float ex2(float x) {
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* v) {
   tmem_ld_32x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(v));
 }
-// shared memory: Q [KB] | K [stages][KB] | V [stages][VB] | P (not FINE), all on 1,024-byte boundaries, then Shared
-__host__ __device__ inline int tile_bytes(int KB, int VB, int stages, bool fine) {
-  return KB * kQBlockBytes + stages * (KB + VB) * kBlockBytes + (fine ? 0 : kPBytes);
+// shared memory: Q [KB] | K [stages][KB] | V [stages][VB] | P (FINE: its last part), all on 1,024-byte boundaries, then Shared
+__host__ __device__ inline int tile_bytes(int KB, int VB, int stages) {
+  return KB * kQBlockBytes + stages * (KB + VB) * kBlockBytes + kPBytes;
 }
 
 template <bool FINE>
@@ -112,7 +115,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
   uint8_t* k_buf = q_buf + p.KB * kQBlockBytes;
   uint8_t* v_buf = k_buf + p.stages * p.KB * kBlockBytes;
   uint8_t* p_buf = v_buf + p.stages * p.VB * kBlockBytes;
-  Shared& ss = *reinterpret_cast<Shared*>(p_buf + (FINE ? 0 : kPBytes));
+  Shared& ss = *reinterpret_cast<Shared*>(p_buf + kPBytes);
   if (reinterpret_cast<uint8_t*>(&ss + 1) > smem_raw + p.smem_bytes) {      // a base that is off its boundary leaves no room
     if (threadIdx.x == 0 && p.status != nullptr) atomicMax(p.status, (int)kBadArgument);
     return;
@@ -249,12 +252,12 @@ attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         const uint64_t pdesc = make_smem_desc_sw128(smem_u32(p_buf));
         const uint32_t v_base = smem_u32(v_buf + s * p.VB * kBlockBytes);
 #pragma unroll
-        for (int j = 0; FINE && j < BN / 8; ++j)                    // high parts, then low parts
+        for (int j = 0; FINE && j < BN / 8; ++j)                    // first parts, then second parts
           mma_f16_ta(tm_o, tmem_base + (t & 1) * BN + j * 8, desc_mn_sw128(v_base + (j & 3) * 2048, kBlockBytes, 1024), idesc_pv,
                      (t > 0 || j > 0) ? 1u : 0u);
 #pragma unroll
-        for (int j = 0; !FINE && j < BN / 16; ++j)
-          mma_f16(tm_o, pdesc + 2 * j, desc_mn_sw128(v_base + j * 2048, kBlockBytes, 1024), idesc_pv, (t > 0 || j > 0) ? 1u : 0u);
+        for (int j = 0; j < BN / 16; ++j)
+          mma_f16(tm_o, pdesc + 2 * j, desc_mn_sw128(v_base + j * 2048, kBlockBytes, 1024), idesc_pv, (FINE || t > 0 || j > 0) ? 1u : 0u);
         tc_commit(&ss.v_empty[s]);
         tc_commit(&ss.o_done);
       }
@@ -297,18 +300,20 @@ attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
       const float alpha = (grow && m_run != -INFINITY) ? ex2(m_run - m_new) : 1.f;
       const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
       float l4[4] = {0.f, 0.f, 0.f, 0.f};
-      uint32_t lo_part[FINE ? BN / 2 : 1];
+      uint32_t second[FINE ? BN / 2 : 1], third[FINE ? BN / 2 : 1];
       if (FINE) {
+        const float2 scale = make_float2(p.score_scale, p.score_scale), shift = make_float2(neg_m, neg_m);
+        float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
         for (int j = 0; j < BN; j += 2) {
-          const float e0 = ex2(fmaf(__uint_as_float(sv[j]), p.score_scale, neg_m));
-          const float e1 = ex2(fmaf(__uint_as_float(sv[j + 1]), p.score_scale, neg_m));
-          const __nv_bfloat162 o = __floats2bfloat162_rn(e0, e1);
-          const __nv_bfloat162 rest = __floats2bfloat162_rn(e0 - __low2float(o), e1 - __high2float(o));
-          l4[(j >> 1) & 3] += e0 + e1;
-          sv[j >> 1] = *reinterpret_cast<const uint32_t*>(&o);
-          lo_part[j >> 1] = *reinterpret_cast<const uint32_t*>(&rest);
+          const float2 x = __ffma2_rn(make_float2(__uint_as_float(sv[j]), __uint_as_float(sv[j + 1])), scale, shift);
+          float2 e = make_float2(ex2(x.x), ex2(x.y));
+          l2[(j >> 1) & 1] = __fadd2_rn(l2[(j >> 1) & 1], e);
+          sv[j >> 1] = cut_bf16x2(e);
+          second[j >> 1] = cut_bf16x2(e);
+          third[j >> 1] = cut_bf16x2(e);
         }
+        l4[0] = l2[0].x; l4[1] = l2[0].y; l4[2] = l2[1].x; l4[3] = l2[1].y;
       }
 #pragma unroll
       for (int j = 0; !FINE && j < BN; j += 2) {
@@ -333,7 +338,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
       }
       if (FINE) {
         tmem_st_32x32(tmem_base + lane_addr + (t & 1) * BN, *reinterpret_cast<const uint32_t(*)[32]>(sv));
-        tmem_st_32x32(tmem_base + lane_addr + (t & 1) * BN + 32, *reinterpret_cast<const uint32_t(*)[32]>(lo_part));
+        tmem_st_32x32(tmem_base + lane_addr + (t & 1) * BN + 32, *reinterpret_cast<const uint32_t(*)[32]>(second));
         tmem_st_wait();
         const int real = last + 1 - kt;
         if (!kept && real < BN) {                                  // uniform: the tile past whose end rows belong to nobody
@@ -345,8 +350,10 @@ attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         }
       }
 #pragma unroll
-      for (int c = 0; !FINE && c < BN / 8; ++c)
-        *reinterpret_cast<uint4*>(prow + ((c ^ (r & 7)) << 4)) = make_uint4(sv[4 * c], sv[4 * c + 1], sv[4 * c + 2], sv[4 * c + 3]);
+      for (int c = 0; c < BN / 8; ++c) {
+        const uint32_t* x = (FINE ? third : sv) + 4 * c;
+        *reinterpret_cast<uint4*>(prow + ((c ^ (r & 7)) << 4)) = make_uint4(x[0], x[1], x[2], x[3]);
+      }
       l_run = l_run * alpha + (l4[0] + l4[1]) + (l4[2] + l4[3]);
       m_run = m_new;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -494,11 +501,11 @@ static int encode(CUtensorMap* m, int rank, const void* base, const cuuint64_t* 
 template <bool FINE>
 static int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, Params& p, int H, int n_work, cudaStream_t stream) {
   // two CTAs an SM when two stages and half of TMEM are enough, otherwise one with as many stages as fit
-  const bool two = p.VB <= 2 && tile_bytes(p.KB, p.VB, 2, FINE) + (int)sizeof(Shared) <= kSmemTwo;
+  const bool two = p.VB <= 2 && tile_bytes(p.KB, p.VB, 2) + (int)sizeof(Shared) <= kSmemTwo;
   const int room = (two ? kSmemTwo : 226 * 1024) - (int)sizeof(Shared);
   p.stages = 2;
-  while (p.stages < kMaxStages && tile_bytes(p.KB, p.VB, p.stages + 1, FINE) <= room) ++p.stages;
-  p.staged = p.gate != nullptr && p.gate_cols > 1 && tile_bytes(p.KB, p.VB, p.stages, FINE) >= BM * p.VB * 256;
+  while (p.stages < kMaxStages && tile_bytes(p.KB, p.VB, p.stages + 1) <= room) ++p.stages;
+  p.staged = p.gate != nullptr && p.gate_cols > 1 && tile_bytes(p.KB, p.VB, p.stages) >= BM * p.VB * 256;
   p.tmem_cols = two ? 256 : 512;
   p.smem_bytes = two ? kSmemTwo : 227 * 1024;
   static bg::DeviceOnce once;
@@ -603,7 +610,7 @@ int bg_gqa_heads(void* qkv, long long ld, const void* bias, const int* positions
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-// Causal prompt attention over cached heads, probabilities in two parts.  q [R, ldq] bf16 turned queries (H heads of D columns, D a
+// Causal prompt attention over cached heads, probabilities in three parts.  q [R, ldq] bf16 turned queries (H heads of D columns, D a
 // multiple of 64 up to 128); cache [pages, page, 2 G D] bf16; work as for bg_gqa_prompt; sinks [H] fp32 or null; out [R, ldo] bf16.
 int bg_gqa_prompt_fine(const void* q, int ldq, const void* cache, int n_pages, int page, const int* block_table, int bt_stride,
                        int bt_cols, const int* work, int n_work, int R, void* out, int ldo, int H, int G, int D, int window,

@@ -8,10 +8,12 @@
 // Memory-bound by design: every key and value byte is read once per key head.
 //
 // FINE form (models whose cached attention keeps fp32 probabilities): queries come in bf16 and go into the product as they are, the
-// scale meets the fp32 scores, and a probability is multiplied in two bf16 parts (2^-17 of it is lost).  The second product with V costs
-// nothing that shows next to the bytes.  It took the place of a kernel that did both products on the CUDA cores, a thread per key
-// and a block-wide barrier five times a tile: 160 rows of up to 4,096 tokens, 64 heads of 64 over 8 key heads, one layer of all keys and
-// one with a window of 128, 2,957 -> 255 us (the bytes take 135); one row of 900 tokens 69 -> 12 us.
+// scale meets the fp32 scores, and a probability is multiplied whole, as three bf16 parts of 8 bits.  Up to 8 heads in the CTA, the second
+// parts are the rows 8 to 15 of the first parts' product, which have no heads of their own: the products with V bound it (two each tile
+// and 16 columns 245 us where three took 306: 160 rows of up to 4,096 tokens, 64 heads of 64 over 8 key heads).  Outputs that differ from
+// the rounded 64-bit ones: 1e-4 to 4e-4 of them, like sums in fp32 (two rounded parts: 2e-3).  It took the place of a kernel that did both
+// products on the CUDA cores, a thread per key and a block-wide barrier five times a tile: the same rows, one layer of all keys and one with
+// a window of 128, 2,957 -> 255 us (the bytes take 135); one row of 900 tokens 69 -> 12 us.
 #pragma once
 
 namespace bg {
@@ -173,7 +175,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 2) gqa_rows_kernel(const Param
       for (int j = 0; j < 2; ++j)
         if (!seen(pos + n * 8 + j)) s[n][j] = s[n][2 + j] = -INFINITY;
     }
-    uint32_t pa[4] = {0, 0, 0, 0}, pr[4] = {0, 0, 0, 0};           // FINE: pr is what the rounding of pa left
+    uint32_t pa[4] = {0, 0, 0, 0}, pb[4] = {0, 0, 0, 0}, pc[4] = {0, 0, 0, 0};           // FINE: three parts of 8 bits
     float al[2] = {1.f, 1.f};
 #pragma unroll
     for (int i = 0; i < (HI ? 2 : 1); ++i) {
@@ -183,20 +185,24 @@ __global__ void __launch_bounds__(kRowWarps * 32, 2) gqa_rows_kernel(const Param
       const float mn = fmaxf(m[i], mt), sub = mn == -INFINITY ? 0.f : mn;
       al[i] = exp2f(m[i] - sub);
       m[i] = mn;
-      const float e0 = exp2f(s[0][2 * i] - sub), e1 = exp2f(s[0][2 * i + 1] - sub);
-      const float e2 = exp2f(s[1][2 * i] - sub), e3 = exp2f(s[1][2 * i + 1] - sub);
-      const __nv_bfloat162 lo = __floats2bfloat162_rn(e0, e1), hi = __floats2bfloat162_rn(e2, e3);
+      float2 e = make_float2(exp2f(s[0][2 * i] - sub), exp2f(s[0][2 * i + 1] - sub));
+      float2 f = make_float2(exp2f(s[1][2 * i] - sub), exp2f(s[1][2 * i + 1] - sub));
       if (FINE) {
-        const __nv_bfloat162 rl = __floats2bfloat162_rn(e0 - __low2float(lo), e1 - __high2float(lo));
-        const __nv_bfloat162 rh = __floats2bfloat162_rn(e2 - __low2float(hi), e3 - __high2float(hi));
-        pr[i] = *reinterpret_cast<const uint32_t*>(&rl);
-        pr[2 + i] = *reinterpret_cast<const uint32_t*>(&rh);
-        l[i] = l[i] * al[i] + (e0 + e1) + (e2 + e3);
+        l[i] = l[i] * al[i] + (e.x + e.y) + (f.x + f.y);
+        pa[i] = cut_bf16x2(e); pa[2 + i] = cut_bf16x2(f);
+        pb[i] = cut_bf16x2(e); pb[2 + i] = cut_bf16x2(f);
+        pc[i] = cut_bf16x2(e); pc[2 + i] = cut_bf16x2(f);
       } else {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(e.x, e.y), hi = __floats2bfloat162_rn(f.x, f.y);
         l[i] = l[i] * al[i] + (__low2float(lo) + __high2float(lo)) + (__low2float(hi) + __high2float(hi));
+        pa[i] = *reinterpret_cast<const uint32_t*>(&lo);
+        pa[2 + i] = *reinterpret_cast<const uint32_t*>(&hi);
       }
-      pa[i] = *reinterpret_cast<const uint32_t*>(&lo);
-      pa[2 + i] = *reinterpret_cast<const uint32_t*>(&hi);
+    }
+    if (FINE && !HI) {                                             // rows 8 to 15 have no heads: they take the second parts of rows 0 to 7
+      pa[1] = pb[0];
+      pa[3] = pb[2];
+      al[1] = al[0];
     }
     if (__any_sync(0xffffffffu, al[0] != 1.f || al[1] != 1.f)) {
 #pragma unroll
@@ -214,9 +220,13 @@ __global__ void __launch_bounds__(kRowWarps * 32, 2) gqa_rows_kernel(const Param
         if (n0 + n < vsteps) {
           mma16816(o[2 * (n0 + n)], pa, vf[n][0], vf[n][1]);
           mma16816(o[2 * (n0 + n) + 1], pa, vf[n][2], vf[n][3]);
+          if (FINE && HI) {
+            mma16816(o[2 * (n0 + n)], pb, vf[n][0], vf[n][1]);
+            mma16816(o[2 * (n0 + n) + 1], pb, vf[n][2], vf[n][3]);
+          }
           if (FINE) {
-            mma16816(o[2 * (n0 + n)], pr, vf[n][0], vf[n][1]);
-            mma16816(o[2 * (n0 + n) + 1], pr, vf[n][2], vf[n][3]);
+            mma16816(o[2 * (n0 + n)], pc, vf[n][0], vf[n][1]);
+            mma16816(o[2 * (n0 + n) + 1], pc, vf[n][2], vf[n][3]);
           }
         }
     }
@@ -241,7 +251,8 @@ __global__ void __launch_bounds__(kRowWarps * 32, 2) gqa_rows_kernel(const Param
       for (int n = 0; n < 2 * VD; ++n) {
         const int col = n * 8 + (lane & 3) * 2;
         if (col < dvp)
-          *reinterpret_cast<float2*>(red + ((size_t)warp * nh + row) * dvp + col) = make_float2(o[n][2 * i], o[n][2 * i + 1]);
+          *reinterpret_cast<float2*>(red + ((size_t)warp * nh + row) * dvp + col) =
+              FINE && !HI ? make_float2(o[n][0] + o[n][2], o[n][1] + o[n][3]) : make_float2(o[n][2 * i], o[n][2 * i + 1]);
       }
     }
   }

@@ -493,7 +493,7 @@ int bg_talk_rows(int dt, const float* q, int ldq, const float* talk, const void*
 }
 
 // Decode attention of bf16 queries q [B, ldq] (H heads of D = 64 or 128 columns, turned and unscaled) over cached rows of G key heads,
-// then G value heads; up to 16 heads a key head; probabilities in two parts.  lens [B]: keys a row sees (0: zero output); window 0: all
+// then G value heads; up to 16 heads a key head; probabilities in three parts.  lens [B]: keys a row sees (0: zero output); window 0: all
 // of them; sinks [H] fp32 or null; scratch for n_splits > 1: part_o [B, n_splits, H, D], part_ml [B, n_splits, H, 2] fp32.
 int bg_gqa_rows(const void* q, int ldq, const void* cache, const int* block_table, int bt_stride, const int* lens, const float* sinks,
                 void* out, float* part_o, float* part_ml, int B, int H, int G, int D, int page, int window, float scale,

@@ -36,8 +36,8 @@ def test_gqa_decode(Hq, Hkv, D, window, use_sinks, splits):
 @pytest.mark.parametrize("window,use_sinks", [(0, False), (0, True), (100, True), (1, False), (64, False)])
 def test_gqa_prompt(Hq, Hkv, D, page, interleaved, bias, window, use_sinks):
     """Projections to attention output: lengths at the edges of tiles and pages, cached context, rows without a slot, stale rows of
-    the last page that are not finite.  Operands are the bf16 numbers the kernels see, so what is left is the two-part
-    probabilities (2^-17) and the rounding of the output (8 significant bits: up to 2^-8 of a value)."""
+    the last page that are not finite.  Operands are the bf16 numbers the kernels see, so what is left is the fp32
+    sums and the rounding of the output (8 significant bits: up to 2^-8 of a value)."""
     from batchgen_b200.ops import _ext, attention, ref, talking
     g = torch.Generator().manual_seed(Hq * D + page + window)
     lens, ctx = [1, 63, 64, 65, 127, 128, 129, 300, 2], [0, 0, 64, 1, 0, 33, 500, 7, 1000]
@@ -98,7 +98,7 @@ def test_gqa_prompt(Hq, Hkv, D, page, interleaved, bias, window, use_sinks):
             s = torch.cat([s, sinks.double().view(Hq, 1, 1).expand(Hq, s.shape[1], 1)], -1)
         o = torch.einsum("hnl,lhd->nhd", s.softmax(-1)[..., :rows.shape[0]], v).reshape(e - a, -1)
         err = (out[a:e].cpu().double() - o).abs()
-        # a value rounded to 8 significant bits: 2^-8 of it; fp32 sums of up to 1,000 terms (1,000 * 2^-24) and p of 2^-17: 7e-5
+        # a value rounded to 8 significant bits: 2^-8 of it; fp32 sums of up to 1,000 terms (1,000 * 2^-24 = 6e-5): 7e-5
         assert (err <= o.abs() * 2 ** -8 + 7e-5 * v.abs().max()).all(), (i, err.max())
 
 
@@ -135,5 +135,42 @@ def test_gqa_decode_fine(Hq, Hkv, D, page, window, use_sinks, splits):
         if use_sinks:
             s = torch.cat([s, sinks.double().view(Hq, 1)], -1)
         o = torch.einsum("hl,lhd->hd", s.softmax(-1)[:, :r.shape[0]], v)
-        # a value rounded to 8 significant bits: 2^-8 of it; fp32 sums of up to 1,023 terms (1,023 * 2^-24) and p of 2^-17: 7e-5
+        # a value rounded to 8 significant bits: 2^-8 of it; fp32 sums of up to 1,023 terms (1,023 * 2^-24 = 6e-5): 7e-5
         assert ((got[i] - o).abs() <= o.abs() * 2 ** -8 + 7e-5 * v.abs().max()).all(), i
+
+
+@pytest.mark.parametrize("new,ctx", [(1, 899), (1, 3000), (700, 0), (300, 900)])
+@pytest.mark.parametrize("Hq,Hkv,D", [(16, 2, 64), (12, 2, 128), (24, 2, 64)])
+def test_gqa_probabilities_stay_whole(Hq, Hkv, D, new, ctx):
+    """Probabilities reach the product with V with all 24 bits (three bf16 parts).  Seen through the outputs' rounding to 8 bits: an output that differs
+    from the rounded 64-bit value had that value within its error of a border.  fp32 sums leave errors of some 1e-6 of an output, so some
+    2 * 1e-6 / 2^-7.5 = 4e-4 of the outputs differ; with two rounded parts (2^-17 of a probability) it were 2e-3."""
+    from batchgen_b200.ops import _ext, attention, talking
+    g = torch.Generator().manual_seed(new + ctx + D)
+    window, n, page = (128 if new > 1 else 0), new + ctx, 64
+    wrong = total = 0
+    for _ in range(2 if new > 1 else 40):
+        pages = torch.randperm(-(-n // page), generator=g)
+        pos = torch.arange(n)
+        rows = torch.randn(n, 2 * Hkv * D, generator=g).bfloat16()
+        cache = torch.zeros(len(pages), page, 2 * Hkv * D).bfloat16()
+        cache.view(-1, 2 * Hkv * D)[pages[pos // page] * page + pos % page] = rows
+        q = (torch.randn(new, Hq, D, generator=g) * 0.5).bfloat16().cuda()
+        c, bt = cache.cuda(), pages.int().view(1, -1).cuda()
+        if new > 1:
+            out = torch.empty(new, Hq * D, dtype=torch.bfloat16, device="cuda")
+            work = torch.tensor(talking.prefill_work([0, new], [ctx], 0, 1, window), dtype=torch.int32).cuda()
+            attention.gqa_prefill(q, c, bt, work, Hkv, D ** -0.5, out, window=window)
+            out = out.view(new, Hq, D)
+        else:
+            out = attention.gqa_decode(q, c, bt, torch.tensor([n], dtype=torch.int32).cuda(), Hkv, D ** -0.5)
+        k, v = (t.view(n, Hkv, D).double().cuda() for t in rows.split(Hkv * D, 1))
+        at, key = (ctx + torch.arange(new, device="cuda"))[:, None], torch.arange(n, device="cuda")[None]
+        hidden = (key > at) | ((key <= at - window) if window else torch.zeros_like(key > at))
+        for h in range(Hq):
+            s = (q[:, h].double() @ k[:, h // (Hq // Hkv)].t() * D ** -0.5).masked_fill(hidden, float("-inf"))
+            want = s.softmax(-1) @ v[:, h // (Hq // Hkv)]
+            wrong += (out[:, h] != want.float().bfloat16()).sum().item()
+            total += want.numel()
+    _ext.check_status()
+    assert wrong <= 8e-4 * total, wrong / total
