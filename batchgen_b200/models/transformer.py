@@ -282,12 +282,18 @@ class Transformer:
         conv, rec = cache.state.layer(l)
         if meta.state_slots is None:
             raise RuntimeError("a model with KDA layers needs AttnMeta.state_slots")
+        plan = None
+        if meta.mode == "prefill" and x.is_cuda:
+            key = (tuple(meta.cu_seqlens), Hh, D)         # lengths and heads: one plan for the layers of a step
+            if getattr(meta, "_kda_key", None) != key:
+                meta._kda_key, meta._kda_plan = key, kda_ops.step_plan(meta.cu_seqlens, Hh, D, x.device)
+            plan = meta._kda_plan
         with tm.timed("kda.core_" + meta.mode, l):
             o = kda_ops.kda_forward(proj[:, : 3 * HD], f, proj[:, 4 * HD + r: 4 * HD + r + Hh], proj[:, 3 * HD: 4 * HD],
                                     kda_ops.KDAParams(kw.conv_w, None, kw.A_log, kw.dt_bias, kw.o_norm), conv, rec,
                                     meta.state_slots, meta.cu_seqlens if meta.mode == "prefill" else None,
                                     meta.state_has_initial if meta.mode == "prefill" else None, Hh, D, D ** -0.5,
-                                    cfg.rms_eps)
+                                    cfg.rms_eps, plan=plan)
         with tm.timed("attn.o_proj", l):
             return linear(o, lw.wo)
 

@@ -147,6 +147,27 @@ def chunk_plan(cu: Sequence[int], min_tokens: int, most_items: int):
     return rounds
 
 
+@dataclass
+class StepPlan:
+    """What ``kda_forward`` needs of a prompt step's lengths on the device: the same for every layer of the step."""
+    cu: torch.Tensor                       # [nseq + 1] int32
+    rounds: list                           # of chunks: (items, sequence pieces) in ``tables``
+    tables: Optional[torch.Tensor]         # [.., 4] int32, round after round: items, then pieces
+    short: int                             # tokens of the longest piece that goes token by token
+
+
+def step_plan(cu_seqlens: Sequence[int], heads: int, dim: int, device) -> StepPlan:
+    cu = [int(c) for c in cu_seqlens]
+    lens = [b - a for a, b in zip(cu, cu[1:])]
+    rounds, tables, short = [], None, (1 << 31) - 1
+    if dim == 128 and chunk_form_pays([n for n in lens if n >= CHUNK_MIN_TOKENS], heads, _ext.num_sms(device)):
+        made = chunk_plan(cu, CHUNK_MIN_TOKENS, max(1, _CHUNK_SCRATCH // (4 * _CHUNK_FLOATS * heads)))
+        rounds = [(len(it), len(sq)) for it, sq in made]
+        tables = torch.tensor([r for it, sq in made for r in it + sq], dtype=torch.int32, device=device)
+        short = CHUNK_MIN_TOKENS - 1 if any(0 < n < CHUNK_MIN_TOKENS for n in lens) else 0
+    return StepPlan(torch.tensor(cu, dtype=torch.int32, device=device), rounds, tables, short)
+
+
 def _forward_ref(qkv, f, beta, z, p: KDAParams, conv_state, rec_state, slots, cu, has_initial, H, D, scale, eps):
     T = qkv.shape[0]
     HD = H * D
@@ -175,10 +196,12 @@ def _forward_ref(qkv, f, beta, z, p: KDAParams, conv_state, rec_state, slots, cu
 
 def kda_forward(qkv: torch.Tensor, f: torch.Tensor, beta: torch.Tensor, z: torch.Tensor, p: KDAParams,
                 conv_state: torch.Tensor, rec_state: torch.Tensor, slots, cu_seqlens: Optional[Sequence[int]],
-                has_initial: Optional[Sequence[int]], H: int, D: int, scale: float, eps: float) -> torch.Tensor:
+                has_initial: Optional[Sequence[int]], H: int, D: int, scale: float, eps: float,
+                plan: Optional[StepPlan] = None) -> torch.Tensor:
     """qkv [T, >= 3HD] (raw q | k | v, may be a column view), f / z [T, HD], beta [T, >= H] (views allowed; unit
     column stride).  ``slots``: int32 tensor (or list) [nseq], < 0 skips; ``cu_seqlens`` None = one token per
-    sequence; ``has_initial`` None = continue from the stored state.  Returns [T, HD] in qkv's dtype and
+    sequence; ``has_initial`` None = continue from the stored state; ``plan``: ``step_plan`` of these lengths and heads, made here
+    when None (CUDA: a blocking copy of its tables).  Returns [T, HD] in qkv's dtype and
     updates both pools."""
     nseq = len(slots)
     if not qkv.is_cuda or qkv.dtype != torch.bfloat16:
@@ -190,34 +213,30 @@ def kda_forward(qkv: torch.Tensor, f: torch.Tensor, beta: torch.Tensor, z: torch
         assert t.stride(1) == 1
     if not isinstance(slots, torch.Tensor):
         slots = torch.tensor(list(slots), dtype=torch.int32, device=dev)
-    cu_t = None if cu_seqlens is None else (
-        cu_seqlens if isinstance(cu_seqlens, torch.Tensor) else torch.tensor(list(cu_seqlens), dtype=torch.int32, device=dev))
     hi_t = None if has_initial is None else (
         has_initial if isinstance(has_initial, torch.Tensor) else torch.tensor([int(x) for x in has_initial], dtype=torch.int32, device=dev))
     out = torch.empty(qkv.shape[0], H * D, dtype=torch.bfloat16, device=dev)
-    rounds = []
-    if D == 128 and cu_seqlens is not None and not isinstance(cu_seqlens, torch.Tensor) and z.stride(0) % 4 == 0 and z.data_ptr() % 8 == 0:
-        long = [b - a for a, b in zip(cu_seqlens, cu_seqlens[1:]) if b - a >= CHUNK_MIN_TOKENS]
-        if chunk_form_pays(long, H, _ext.num_sms(dev)):
-            rounds = chunk_plan(cu_seqlens, CHUNK_MIN_TOKENS, max(1, _CHUNK_SCRATCH // (4 * _CHUNK_FLOATS * H)))
-    short = (1 << 31) - 1                                 # tokens of the longest piece that goes token by token
-    if rounds:
-        lens = [b - a for a, b in zip(cu_seqlens, cu_seqlens[1:])]
-        short = CHUNK_MIN_TOKENS - 1 if any(0 < n < CHUNK_MIN_TOKENS for n in lens) else 0
-        most = max(len(it) for it, _ in rounds)
-        scratch = torch.empty(most * H * _CHUNK_FLOATS, dtype=torch.float32, device=dev)
-        tables = torch.tensor([r for it, sq in rounds for r in it + sq], dtype=torch.int32, device=dev)
+    if isinstance(cu_seqlens, torch.Tensor):
+        plan = StepPlan(cu_seqlens, [], None, (1 << 31) - 1)
+    elif cu_seqlens is not None and plan is None:
+        plan = step_plan(cu_seqlens, H, D, dev)
+    rounds, short = (plan.rounds, plan.short) if plan is not None and cu_seqlens is not None else ([], (1 << 31) - 1)
+    if z.stride(0) % 4 or z.data_ptr() % 8:               # the chunk form reads four gates at a time
+        rounds, short = [], (1 << 31) - 1
+    cu_t = plan.cu if cu_seqlens is not None else None
+    assert cu_t is None or cu_t.shape[0] == nseq + 1
+    tables, scratch = (plan.tables, torch.empty(max(n for n, _ in rounds) * H * _CHUNK_FLOATS, dtype=torch.float32, device=dev)) if rounds else (None, None)
     at = 0
-    for n, (it, sq) in enumerate(rounds or [((), ())]):
+    for n, (items, pieces) in enumerate(rounds or [(0, 0)]):
         last = n == max(len(rounds), 1) - 1
         rc = _ext.lib().bg_kda_forward(
             _ext.ptr(qkv), ctypes.c_int(qkv.stride(0)), _ext.ptr(f), ctypes.c_int(f.stride(0)), _ext.ptr(beta),
             ctypes.c_int(beta.stride(0)), _ext.ptr(z), ctypes.c_int(z.stride(0)), _ext.ptr(p.conv_w), _ext.ptr(p.conv_b),
             _ext.ptr(p.A_log), _ext.ptr(p.dt_bias), _ext.ptr(p.norm_w), _ext.ptr(conv_state), _ext.ptr(rec_state),
             _ext.ptr(cu_t), _ext.ptr(slots), _ext.ptr(hi_t), _ext.ptr(out), ctypes.c_int(nseq), ctypes.c_int(H),
-            ctypes.c_int(D), ctypes.c_float(scale), ctypes.c_float(eps), _ext.ptr(tables[at:] if it else None), ctypes.c_int(len(it)),
-            _ext.ptr(tables[at + len(it):] if it else None), ctypes.c_int(len(sq)), ctypes.c_int(short if last else 0),
-            _ext.ptr(scratch if it else None), _ext.stream())
-        _ext.check(rc, "bg_kda_forward", kernels=(3 if it else 0) + int(last and short > 0))
-        at += len(it) + len(sq)
+            ctypes.c_int(D), ctypes.c_float(scale), ctypes.c_float(eps), _ext.ptr(tables[at:] if items else None), ctypes.c_int(items),
+            _ext.ptr(tables[at + items:] if items else None), ctypes.c_int(pieces), ctypes.c_int(short if last else 0),
+            _ext.ptr(scratch if items else None), _ext.stream())
+        _ext.check(rc, "bg_kda_forward", kernels=(3 if items else 0) + int(last and short > 0))
+        at += items + pieces
     return out

@@ -237,3 +237,43 @@ def test_chunk_form_keeps_what_is_not_finite_to_later_tokens(where, value, at, m
     assert (torch.isnan(o) | ~torch.isnan(ot)).all() and (torch.isnan(rec) | ~torch.isnan(rect)).all()
     if where == "f" and value == float("inf"):
         assert torch.isfinite(o).all() and torch.isfinite(rec).all()
+
+
+def test_one_plan_serves_the_layers_of_a_step(monkeypatch):
+    """Three KDA layers of a prompt step: its lengths go to the device once; another step makes its own plan."""
+    from batchgen_b200.config import get_model_config
+    from batchgen_b200.models import build_model
+    from batchgen_b200.models.transformer import AttnMeta
+    from batchgen_b200.ops import kda
+    from batchgen_b200.ops.policy import set_library_fallback
+    from batchgen_b200.runtime.kv_cache import PagedKVCache
+    cfg = get_model_config("tiny-kimi-linear", kda_head_dim=128, kda_num_heads=4)
+    made = []
+    inner = kda.step_plan
+    monkeypatch.setattr(kda, "step_plan", lambda cu, *a: made.append(list(cu)) or inner(cu, *a))
+    set_library_fallback(True)
+    try:
+        model = build_model(cfg, device="cuda", dtype=torch.bfloat16, seed=4)
+        kv = PagedKVCache(cfg, 16, 64, "cuda", torch.bfloat16, state_slots=2)
+        meta, got = None, []
+        for lens in ([200, 70], [200, 70], [20, 90]):
+            T = sum(lens)
+            pos = torch.cat([torch.arange(n) for n in lens]).int().cuda()
+            table = torch.arange(8, dtype=torch.int32).view(2, 4).cuda()
+            slots = torch.cat([table[i].cpu().long()[torch.arange(n) // 64] * 64 + torch.arange(n) % 64 for i, n in enumerate(lens)]).cuda()
+            new = dict(positions=pos, slot_mapping=slots, block_table=table, cu_seqlens=[0, lens[0], T], ctx_lens=[0, 0])
+            if meta is None:
+                meta = AttnMeta(mode="prefill", state_slots=torch.tensor([0, 1], dtype=torch.int32).cuda(),
+                                state_has_initial=torch.zeros(2, dtype=torch.int32).cuda(), **new)
+            for k, v in new.items():                     # the same AttnMeta, reused
+                setattr(meta, k, v)
+            ids = (torch.arange(T, dtype=torch.int32) % 50 + 2).cuda()
+            got.append(model.forward(ids, meta, kv).float().cpu())
+            alone = AttnMeta(mode="prefill", state_slots=meta.state_slots, state_has_initial=meta.state_has_initial, **new)
+            assert torch.equal(got[-1], model.forward(ids, alone, kv).float().cpu())
+        torch.cuda.synchronize()
+    finally:
+        set_library_fallback(False)
+    a, b = [0, 200, 270], [0, 20, 110]
+    assert made == [a, a, a, b, b], made                 # first step, its twin; twin of the second; third and its twin
+    assert torch.equal(got[0], got[1])
