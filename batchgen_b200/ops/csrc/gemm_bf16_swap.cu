@@ -9,7 +9,7 @@
 //
 // Roles (192 threads, one CTA per SM, persistent): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 2..5 epilogue (thread = weight
 // row; two accumulators of 256 columns, so one is stored while the other is filled).  All waits are bounded.
-#define BG_FILE_TAG 31     // kernel-trace ids of this file are (tag << 16) | line
+#define BG_FILE_TAG 33     // kernel-trace ids of this file are (tag << 16) | line
 #include "common.cuh"
 #include "token_tiles.cuh"
 
