@@ -1,4 +1,4 @@
-// Kimi Delta Attention (gated delta-rule linear attention), prefill and decode in one kernel.
+// Kimi Delta Attention (gated delta-rule linear attention): decode and short pieces token by token, longer pieces in chunks.
 //
 // Per head the layer keeps a state S [D keys x D values] (fp32) and the last three raw inputs of every
 // q/k/v channel (the window of the width-4 causal depthwise convolution).  For each token, in order:
