@@ -9,8 +9,9 @@
 //
 // FINE form (models whose cached attention keeps fp32 probabilities): queries come in bf16 and go into the product as they are, the
 // scale meets the fp32 scores, and a probability is multiplied whole, as three bf16 parts of 8 bits.  Up to 8 heads in the CTA, the second
-// parts are the rows 8 to 15 of the first parts' product, which have no heads of their own: the products with V bound it (two each tile
-// and 16 columns 245 us where three took 306: 160 rows of up to 4,096 tokens, 64 heads of 64 over 8 key heads).  Outputs that differ from
+// parts are the rows 8 to 15 of the first parts' product, which have no heads of their own (160 rows of up to 4,096 tokens, 64 heads of 64 over 8
+// key heads: 245 us, a product of their own 306).  Bound by the chain of a tile's steps with eight warps an SM: issue slots 58 % busy, DRAM 45 %,
+// tensor pipe 17 %.  Outputs that differ from
 // the rounded 64-bit ones: 1e-4 to 4e-4 of them, like sums in fp32 (two rounded parts: 2e-3).  It took the place of a kernel that did both
 // products on the CUDA cores, a thread per key and a block-wide barrier five times a tile: the same rows, one layer of all keys and one with
 // a window of 128, 2,957 -> 255 us (the bytes take 135); one row of 900 tokens 69 -> 12 us.

@@ -208,9 +208,10 @@ __global__ void __launch_bounds__(2 * D, 2) kda_seq_kernel(const Params p) {
 // by 1.3e-5 with differences, 1.2e-7 so, 1.4e-7 token by token).  Products of different 16-token blocks meet at the border before the
 // later one.
 //
-// The token-by-token kernel runs a barrier chain of some 2 us a token with a CTA per head.  Here the limit is what shared memory delivers to
-// the fp32 FMAs: about 75,000 a token and head, two thirds of them in the chain.  One prompt of 4,096 tokens, 32 heads: 8,086 -> 1,228
-// us a layer (prepare 607, chain 464, finish 42); with two thirds of the warps and a column-by-column inverse prepare took 833.
+// The token-by-token kernel runs a barrier chain of some 2 us a token with a CTA per head.  Here the chain's limit is what shared memory
+// delivers to the fp32 FMAs (86 % of its rate), of which a token and head has about 75,000, two thirds of them in the chain; prepare waits at its
+// short steps' barriers (shared memory 53 %, issue slots 42 %).  One prompt of 4,096 tokens, 32 heads: 8,086 -> 1,226
+// us a layer (prepare 605, chain 466, finish 42); with two thirds of the warps and a column-by-column inverse prepare took 833.
 constexpr int kChunk = 64, kSub = 16, kPad = 132, kCols = 32;      // kPad: rows of 128 floats that start 4 banks apart
 constexpr int kPart = kChunk * 128;                                // floats of one [64, 128] result
 constexpr int kItemFloats = 5 * kPart;                             // W | Q' | Kd | UV | O of a (chunk, head)

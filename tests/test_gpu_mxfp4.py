@@ -182,3 +182,41 @@ def test_w4_many_tiles_a_cta(counts, fmt, K, N, silu, monkeypatch):
             mag = am * (u.abs() + 1) * 1.1 + um * a.abs()
         # one rounding to 8 significant bits; fp32 sums of K exact products: K * 2^-24 of their magnitudes
         assert ((got[offs[e]:offs[e] + c] - want).abs() <= want.abs() * 2 ** -8 + mag * K * 2 ** -24 + 1e-36).all(), e
+
+
+SPARSE = {0: 3, 15: 1, 16: 200, 40: 17, 47: 385, 69: 5}           # rows of the segments that have any, of 70
+
+
+@pytest.mark.parametrize("only", [sorted(SPARSE), [69], [16], [0], []])
+@pytest.mark.parametrize("kernel", ["mxfp4", "swap"])
+def test_segments_that_are_passed_over(only, kernel, monkeypatch):
+    """70 segments of which few have rows, first and last and in blocks of 16 of their own: every row of theirs, and nothing else, is written."""
+    from batchgen_b200.ops import _ext, gemm, mxfp4
+    g = torch.Generator().manual_seed(len(only))
+    E, N, K = 70, 256, 192
+    counts = [SPARSE.get(e, 0) if e in only else 0 for e in range(E)]
+    offs = [0]
+    for c in counts:
+        offs.append(offs[-1] + (c + 7) // 8 * 8)
+    rows = max(offs[-1], 8)
+    x = torch.randn(rows, K, generator=g).bfloat16()
+    off, cnt = torch.tensor(offs, dtype=torch.int32).cuda(), torch.tensor(counts, dtype=torch.int32).cuda()
+    out = torch.full((rows, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    monkeypatch.setattr(_ext, "num_sms", lambda device=None: 3)
+    if kernel == "mxfp4":
+        wq = torch.randint(0, 256, (E, N, K // 2), generator=g, dtype=torch.uint8)
+        ws = torch.randint(120, 124, (E, N, K // 32), generator=g, dtype=torch.uint8)
+        w = mxfp4.dequantize(wq, ws, torch.float32).double()
+        mxfp4.grouped_mxfp4_gemm(x.cuda(), wq.cuda(), ws.cuda(), off, out=out, counts=cnt)
+    else:
+        wb = torch.randn(E, N, K, generator=g).bfloat16()
+        w = wb.double()
+        gemm._bf16_swap(x.cuda(), wb.cuda(), out, off, cnt, E, N)
+    _ext.check_status()
+    got, seen = out.cpu().double(), torch.zeros(rows, dtype=torch.bool)
+    for e, c in enumerate(counts):
+        xe = x[offs[e]:offs[e] + c].double()
+        # one rounding to 8 significant bits; fp32 sums of K exact products: K * 2^-24 of their magnitudes
+        assert ((got[offs[e]:offs[e] + c] - xe @ w[e].t()).abs() <= (xe @ w[e].t()).abs() * 2 ** -8 + xe.abs() @ w[e].abs().t() * K * 2 ** -24).all(), e
+        seen[offs[e]:offs[e] + c] = True
+    assert (got[~seen] == 7).all()
