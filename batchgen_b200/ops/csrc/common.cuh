@@ -95,20 +95,23 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
-__device__ __forceinline__ bool vote_any_128(bool v) {      // named barrier 2 over 128 threads, OR of a flag: all of them leave a loop, or none
+// OR of a flag over THREADS threads at named barrier 2: warps with barriers between them leave a loop together or not at all
+template <int THREADS>
+__device__ __forceinline__ bool vote_any(bool v) {
   uint32_t r;
   asm volatile(
       "{\n"
       ".reg .pred p, q;\n"
       "setp.ne.u32 q, %1, 0;\n"
-      "bar.red.or.pred p, 2, 128, q;\n"
+      "bar.red.or.pred p, 2, %2, q;\n"
       "selp.u32 %0, 1, 0, p;\n"
       "}\n"
       : "=r"(r)
-      : "r"(static_cast<uint32_t>(v))
+      : "r"(static_cast<uint32_t>(v)), "n"(THREADS)
       : "memory");
   return r != 0;
 }
+__device__ __forceinline__ bool vote_any_128(bool v) { return vote_any<128>(v); }
 
 // The 8 leading significant bits of both floats as a pair of bf16, cut off and not rounded; e keeps the rest.  Three times this takes the 24
 // bits of a float whole: the parts of an fp32 operand for products on the tensor cores.

@@ -298,7 +298,7 @@ gemm_fp8_swapab_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
           r[4 * q + 3] = fmaf(__uint_as_float(v[4 * q + 3]), s4.w * sw, r[4 * q + 3]);
         }
       }
-      if (!ok) break;
+      if (vote_any_128(!ok)) { ok = false; break; }           // there are barriers between these warps: none may leave alone
       const int n_tok = min(BT, t.m_end - t.m0);
       if (EPI == EPI_SILU_MUL) {
         // rows [64b, 64b + 32) of the tile are gate rows of output columns n0/2 + 32b + [0, 32), rows [64b + 32, 64b + 64)

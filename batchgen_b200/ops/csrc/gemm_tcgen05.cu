@@ -376,7 +376,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           r[33 + j] = b.y;
         }
       }
-      if (!ok) break;
+      // with barriers between the epilogue warps below, none may leave alone
+      if (S > 1 ? vote_any<kEpiWarps * 32>(!ok) : !ok) { ok = false; break; }
       if (S > 1) {
         const int et = ew * 32 + lane;                              // 0 .. 255 over the epilogue warps
         constexpr int kEpiThreads = kEpiWarps * 32;
