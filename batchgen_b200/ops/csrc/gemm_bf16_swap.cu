@@ -4,8 +4,9 @@
 // reads its weights twice, and one of a dozen pays for 128. Here a weight tile of 128 rows meets all tokens of its segment (up to
 // 256 at a time, cut evenly, rounded up to 16) in one product of that width, so weights cross L2 once and the padding is below 16
 // tokens.  Bound by the tensor cores at prompt sizes and by the weights' bytes below some hundred rows a segment, where the caller keeps the 128 x
-// 128 kernel.  256 matrices of 2,048 x 2,304: 128 rows each on average 527 -> 484 us (5.0 TB/s), 156 rows 639 -> 511; dense 4,096 x 16,576 x
-// 2,304 332 -> 253 us (1,238 TFLOP/s), 6,200 x 32,768 x 512 299 -> 202.
+// 128 kernel.  256 matrices of 2,048 x 2,304, Poisson rows, 128 x 128 kernel -> here: 112 rows 432 -> 489 us, 128 rows 514 -> 522, 156 rows 613 -> 540
+// (alone 468: DRAM 72 %, tensor cores 45 %), 512 rows 1,267 -> 1,104; dense 4,096 x 16,576 x 2,304 332 -> 253 us (1,238 TFLOP/s), 6,200 x 32,768 x 512
+// 299 -> 202.
 //
 // Roles (192 threads, one CTA per SM, persistent): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 2..5 epilogue (thread = weight
 // row; two accumulators of 256 columns, so one is stored while the other is filled).  All waits are bounded.

@@ -10,16 +10,17 @@
 // instead of a 128-row one, and a prompt expert's 150 tokens meet each weight once.
 //
 // A pair of nibbles becomes a pair of bf16 by a byte selection, one product for both shifts, a mask and one packed product: e2m1 bits placed
-// at bit 6 of a bf16 are the value times 2^-126, subnormals included, and the product with 2^126 times the scale is exact.  160 rows
-// through 128 experts of 3,072 columns (2,880 wide): 745 us a product with four warps that converted, multiplied in fp32 and rounded,
-// shared-memory operands and 128-row token tiles; 450 here (142 at copy bandwidth); prompts of 4,650 tokens 1,252 -> 559 us.  Bound by the
-// latency of a step's chain (expansion, TMEM store, product): some 580 clocks whatever the token count, the integer pipe 60 % busy.
+// at bit 6 of a bf16 are the value times 2^-126, subnormals included, and the product with 2^126 times the scale is exact.  128 experts of
+// 6,144 x 2,880 and of 2,880 x 3,072, four a token, cold weights, against four warps that converted, multiplied in fp32 and rounded, with
+// shared-memory operands and 128-row token tiles: one token 59 and 36 us -> 35 and 21, 160 tokens 997 and 504 -> 546 and 286 (184 and 92 at copy
+// bandwidth), 4,650 tokens 1,864 and 945 -> 731 and 374.  Bound by the latency of a step's chain (expansion, TMEM store, product): some 520
+// clocks at 160 tokens, issue slots 59 % and the integer pipe 54 % busy.
 //
 // Roles (736 threads, one CTA per SM, persistent over tiles):
 //   warp 0       TMA producer of the token tiles (swizzled), 6 stages
 //   warp 1       TMEM allocator + tcgen05.mma issuer
 //   warps 2..5   epilogue (thread = weight row), optional SiLU(gate) * up on interleaved rows
-//   warps 6..21  weight expansion, four groups of four warps on K steps in turn (two groups: 533 us instead of 463 a product)
+//   warps 6..21  weight expansion, four groups of four warps on K steps in turn, a TMEM slot each (two groups: 15 % slower)
 //   warp 22      TMA producer of the packed weights, 4 stages of 256 columns (whole 128-byte lines of a row)
 //
 // Replaces (by behaviour): the Marlin-tile MXFP4 grouped kernels
@@ -407,8 +408,8 @@ static int launch(const void* A, const void* Wq, const Params& p, int b_rows, in
 extern "C" {
 
 // A: [M, K] bf16 row-major; Wq: [groups * N, K / 2] packed e2m1 (low nibble = even k); Ws: [groups * N, K / 32]
-// e8m0; D: [M, ldd] bf16.  offsets == nullptr -> dense; counts: rows present in every segment, or null (rows past them stay undefined).  K % 64 == 0.  epi 1: rows of W interleaved
-// (32 gate, 32 up), D gets N / 2 columns.  Returns 0 on a successful launch.
+// e8m0; D: [M, ldd] bf16.  offsets == nullptr -> dense; counts: rows present in every segment, or null (rows past them stay
+// undefined).  K % 64 == 0.  epi 1: rows of W interleaved (32 gate, 32 up), D gets N / 2 columns.  Returns 0 on a successful launch.
 int bg_mxfp4_gemm(int epi, const void* A, const void* Wq, const void* Ws, void* D, int ldd, const int* offsets, const int* counts,
                   int groups, int M, int N, int K, int num_sms, int* status, cudaStream_t stream) {
   using namespace bg::mx;
