@@ -105,14 +105,21 @@ _CHUNK_SCRATCH = 1 << 30              # bytes of scratch a round of chunks may t
 
 
 def chunk_form_pays(lens: Sequence[int], heads: int, sms: int) -> bool:
-    """Whether pieces of ``lens`` tokens are faster in chunks.  Token by token costs 2.0 us for each token of the longest piece, or 2.8 us a
-    token and round of CTAs (two fit an SM) when the (piece, head) pairs fill the SMs; chunks cost 0.57 us a (chunk, head) on 148 SMs and 125
-    us to start (32 heads of 128, tokens / chunks: 1 x 64 149 / 142 us, 1 x 4,096 8,086 / 1,228; 4 x 512 1,061 / 686; 8 x 1,024 2,501 /
-    2,249; 32 x 64 667 / 736; 200 x 32 1,810 / 3,859)."""
+    """Whether pieces of ``lens`` tokens are faster in chunks.  In chunks: 90 us to start, 0.52 us a (chunk, head) and 0.25 us a (piece, head) for
+    its state, on 148 SMs.  Token by token a CTA serves a (piece, head): 1.6 to 2.0 us a token of the longest piece with a CTA on an SM, 2.42
+    with two, and 2.42 a token of every further round of two CTAs an SM.  Measured in us, chunks / tokens: 32 heads 1 x 64 100 / 131, 1 x
+    4,096 1,160 / 8,100, 4 x 512 648 / 1,044, 16 x 128 724 / 649, 8 x 1,024 2,183 / 2,485, 64 x 64 1,638 / 1,136, 64 x 128 2,657 / 2,200, 64 x 512
+    8,943 / 8,568; 8 heads 16 x 128 225 / 235, 64 x 512 2,255 / 2,472; 64 heads 16 x 512 4,554 / 4,643, 128 x 64 6,356 / 4,384."""
     if not lens:
         return False
-    tokens = 45 + max(2.0 * max(lens), 2.8 * heads * sum(lens) / (2 * sms))
-    return 125 + 0.57 * heads * sum(-(-n // CHUNK) for n in lens) * 148 / sms < tokens
+    pairs, longest, total = heads * len(lens), max(lens), sum(lens)
+    if pairs <= sms:
+        tokens = (1.6 + 0.4 * pairs / sms) * longest
+    elif pairs <= 2 * sms:
+        tokens = 2.42 * longest
+    else:
+        tokens = 2.42 * max(longest, heads * total / (2 * sms) + 0.3 * total / len(lens))
+    return 90 + (0.52 * heads * sum(-(-n // CHUNK) for n in lens) + 0.25 * pairs) * 148 / sms < 30 + tokens
 
 
 def chunk_scratch_bytes(tokens: int, heads: int, dim: int) -> int:

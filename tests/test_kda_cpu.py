@@ -162,3 +162,19 @@ def test_chunk_form_is_taken_where_it_was_the_faster_one():
     pays = lambda n, tokens: kda.chunk_form_pays([tokens] * n, 32, 148)  # noqa: E731
     assert pays(1, 4096) and pays(4, 512) and pays(8, 1024)
     assert not pays(1, 48) and not pays(32, 64) and not pays(200, 48) and not kda.chunk_form_pays([], 32, 148)
+
+
+def test_chunk_form_over_heads_and_pieces():
+    """Times of both forms in us, chunks and token by token, for (heads, pieces, tokens of each): the slower one is never taken where it is more than 3 %
+    slower."""
+    took = {(4, 1, 64): (107, 133), (4, 16, 128): (134, 235), (4, 64, 64): (253, 169), (4, 64, 128): (412, 316), (4, 64, 512): (1166, 1260),
+            (8, 1, 512): (151, 837), (8, 16, 128): (225, 235), (8, 64, 64): (482, 331), (8, 64, 128): (722, 652), (8, 64, 512): (2255, 2472),
+            (16, 16, 128): (409, 305), (16, 16, 512): (1164, 1264), (16, 8, 1024): (1188, 2061), (16, 64, 128): (1370, 1231),
+            (16, 64, 512): (4556, 4647), (16, 128, 64): (1638, 1139), (32, 1, 64): (100, 131), (32, 4, 512): (648, 1044), (32, 16, 128): (724, 649),
+            (32, 16, 512): (2247, 2480), (32, 64, 64): (1638, 1136), (32, 64, 128): (2657, 2200), (32, 64, 512): (8943, 8568),
+            (32, 128, 64): (3175, 2226), (32, 3, 1300): (1164, 2601), (64, 1, 64): (115, 130), (64, 4, 512): (1163, 1264),
+            (64, 16, 128): (1370, 1224), (64, 16, 512): (4554, 4643), (64, 8, 1024): (4429, 4899), (64, 64, 64): (3175, 2222),
+            (64, 64, 128): (5310, 4337), (64, 128, 64): (6356, 4384)}
+    for (heads, pieces, n), (chunks, tokens) in took.items():
+        taken = chunks if kda.chunk_form_pays([n] * pieces, heads, 148) else tokens
+        assert taken <= 1.03 * min(chunks, tokens), (heads, pieces, n)
