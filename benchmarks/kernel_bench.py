@@ -263,9 +263,10 @@ def main():
         conv = torch.zeros(B, 3 * HD, 3, device=dev)
         rec = torch.zeros(B, H, D, D, device=dev)
         slots = torch.arange(B, dtype=torch.int32, device=dev)
-        cu = None if L == 1 else torch.arange(B + 1, dtype=torch.int32, device=dev) * L
+        cu = None if L == 1 else [i * L for i in range(B + 1)]
+        plan = None if L == 1 else kda.step_plan(cu, H, D, dev)
         ms = timeit(lambda: kda.kda_forward(wide[:, : 3 * HD], f, wide[:, 4 * HD: 4 * HD + H], wide[:, 3 * HD: 4 * HD], p,
-                                            conv, rec, slots, cu, None, H, D, D ** -0.5, 1e-6), a.iters)
+                                            conv, rec, slots, cu, None, H, D, D ** -0.5, 1e-6, plan=plan), a.iters)
         byts = 2 * B * H * D * D * 4 + T * HD * 2 * 6
         out.update(shape=[B, H, L], ms=ms, gbs=byts / ms / 1e6, frac_of_hbm=byts / ms / 1e6 / hbm,
                    us_per_token=ms * 1e3 / L, peak_note=tag)
