@@ -316,7 +316,8 @@ def experts_forward(hidden: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.
         if hidden.is_cuda and hidden.dtype == torch.bfloat16 and hidden.shape[1] % 8 == 0:
             # a pair's row goes straight to its place; padding rows of a segment stay undefined (no kept row depends on another)
             with timer.timed("moe.gather"):
-                rows, _ = residual.moe_gather(hidden.contiguous(), pos, topk_w.float().contiguous(), src.shape[0])
+                whole = hidden if hidden.is_contiguous() and hidden.data_ptr() % 16 == 0 else hidden.clone(memory_format=torch.contiguous_format)
+                rows, _ = residual.moe_gather(whole, pos, topk_w.float().contiguous(), src.shape[0])      # rows in 16-byte pieces
         else:
             rows = hidden[src.clamp_min(0).long()]
             rows = torch.where((src >= 0).unsqueeze(-1), rows, torch.zeros_like(rows))

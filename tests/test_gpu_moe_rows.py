@@ -92,6 +92,27 @@ def test_expert_stack(T, quant, kind):
     assert err < 4 * 2 ** -9, err
 
 
+@pytest.mark.parametrize("quant", ["none", "mxfp4"])
+def test_expert_stack_takes_tokens_at_any_address(quant):
+    """Tokens that are a contiguous view at any element of a buffer: the same bits as their copy."""
+    from batchgen_b200.ops import _ext, moe, mxfp4
+    E, K, H, I, T = 4, 2, 192, 128, 7
+    g = torch.Generator().manual_seed(5)
+    w13, w2 = torch.randn(E, 2 * I, H, generator=g) * 0.1, torch.randn(E, H, I, generator=g) * 0.1
+    if quant == "none":
+        ew = moe.ExpertWeights(w13.bfloat16().cuda(), w2.bfloat16().cuda())
+    else:
+        (q13, s13), (q2, s2) = mxfp4.quantize(w13), mxfp4.quantize(w2)
+        ew = moe.ExpertWeights(q13.cuda(), q2.cuda(), s13.cuda(), s2.cuda(), quant="mxfp4").to_device_layout()
+    x = torch.randn(3 + T * H, generator=g).bfloat16().cuda()[3:].view(T, H)
+    assert x.is_contiguous() and x.data_ptr() % 16
+    idx = torch.randint(0, E, (T, K), generator=g).int().cuda()
+    w = torch.rand(T, K, generator=g).cuda()
+    got, want = (moe.experts_forward(h, idx, w, ew, 0, E) for h in (x, torch.stack(list(x))))
+    _ext.check_status()
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("counts,align", [([1, 0, 17, 130], 8), ([256, 257, 5, 600], 8), ([15, 16, 31, 33], 16), ([3, 0, 0, 0], 8)])
 @pytest.mark.parametrize("N,K", [(128, 64), (200, 192), (384, 1024)])
 def test_grouped_bf16_token_tiles(counts, align, N, K):
