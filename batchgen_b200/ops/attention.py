@@ -155,7 +155,7 @@ def gqa_decode(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, 
             out[b:b + 1] = ref.gqa_attention(q[b:b + 1], ks, vs, scale, q_start=L - 1, window=window, sinks=sinks)
         return out
     if not (q.stride(2) == 1 and q.stride(1) == D and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0):
-        q = q.contiguous()
+        q = q.clone(memory_format=torch.contiguous_format)      # rows are read in 16-byte pieces, also those of a view that is contiguous
     if num_splits <= 0:
         from . import talking
         keys = block_table.shape[1] * page

@@ -174,3 +174,22 @@ def test_gqa_probabilities_stay_whole(Hq, Hkv, D, new, ctx):
             total += want.numel()
     _ext.check_status()
     assert wrong <= 8e-4 * total, wrong / total
+
+
+@pytest.mark.parametrize("first", [1, 8, 3])
+@pytest.mark.parametrize("splits", [1, 2])
+def test_gqa_decode_takes_queries_at_any_address(first, splits):
+    """Queries that are a contiguous view at any element of a buffer: the same bits as their copy."""
+    from batchgen_b200.ops import _ext, attention
+    g = torch.Generator(device="cuda").manual_seed(first)
+    B, Hq, Hkv, D = 3, 16, 2, 64
+    cache = torch.randn(8, 64, 2 * Hkv * D, generator=g, device="cuda").bfloat16()
+    bt = torch.arange(6, dtype=torch.int32, device="cuda").view(3, 2) + 1
+    lens = torch.tensor([1, 70, 128], dtype=torch.int32, device="cuda")
+    buf = torch.randn(first + B * Hq * D, generator=g, device="cuda").bfloat16()
+    q = buf[first:].view(B, Hq, D)
+    assert q.is_contiguous() and (q.data_ptr() % 16 == 0) == (first == 8)
+    got = attention.gqa_decode(q, cache, bt, lens, Hkv, D ** -0.5, num_splits=splits)
+    want = attention.gqa_decode(torch.stack(list(q)), cache, bt, lens, Hkv, D ** -0.5, num_splits=splits)
+    _ext.check_status()
+    assert torch.equal(got, want)
