@@ -113,12 +113,18 @@ __device__ __forceinline__ bool vote_any(bool v) {
 }
 __device__ __forceinline__ bool vote_any_128(bool v) { return vote_any<128>(v); }
 
-// The 8 leading significant bits of both floats as a pair of bf16, cut off and not rounded; e keeps the rest.  Three times this takes the 24
-// bits of a float whole: the parts of an fp32 operand for products on the tensor cores.
+// Parts of fp32 operands for products on the tensor cores: three bf16 numbers of 8 bits that sum up to the float, all 24 bits of it.  Twice
+// cut_bf16x2, then last_bf16x2.  A part is cut off (not rounded) from the float one or two steps below e, and e keeps the rest: so every part of a
+// positive float is positive, and an infinite factor gives infinity three times, where a part of zero would make it NaN.  The rest of a part is at
+// most one unit of its last bit and one of e's; zero has parts of zero, and below 2^-126 the last parts may be zero.
 __device__ __forceinline__ uint32_t cut_bf16x2(float2& e) {
-  const uint32_t x = __float_as_uint(e.x), y = __float_as_uint(e.y);
+  const float2 below = __fmul2_rn(e, make_float2(0x1.fffffcp-1f, 0x1.fffffcp-1f));
+  const uint32_t x = __float_as_uint(below.x), y = __float_as_uint(below.y);
   e = __ffma2_rn(make_float2(__uint_as_float(x & 0xffff0000u), __uint_as_float(y & 0xffff0000u)), make_float2(-1.f, -1.f), e);
   return __byte_perm(x, y, 0x7632);
+}
+__device__ __forceinline__ uint32_t last_bf16x2(float2 e) {
+  return __byte_perm(__float_as_uint(e.x), __float_as_uint(e.y), 0x7632);
 }
 
 // ---------------------------------------------------------------- TMA (plain per-CTA tile loads only)

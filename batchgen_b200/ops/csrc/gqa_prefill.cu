@@ -17,6 +17,8 @@
 // The third part costs 4 to 6 % (4,650 tokens in three prompts, 64 heads of 64: 231 -> 242 us; 4,096 tokens, 48 heads of 128: 372 -> 393)
 // and is kept for the probabilities' sake: with two parts that lose 2^-17, 2e-3 of the outputs differ from the rounded 64-bit ones, with three
 // 3e-4 within a window (fp32 sums: 2e-4 to 3e-4) and up to 2e-3 over 2,000 keys, where the tensor cores' accumulation shows.
+// That no part of a probability is zero (cut_bf16x2), so that an infinite value gives infinity as in fp32, takes 64-wide heads 246 -> 268 us
+// (4,650 tokens; 113 -> 127 with a window of 128), 128-wide ones 234 -> 230 (4,096 tokens in two prompts).
 //
 // A first kernel turns the queries, folds scale * log2(e) in and rounds them once to bf16.  One CTA = (tile of 128 queries of
 // one sequence, head).  K and V come straight from the paged cache by TMA (3-D map: column, token of the page, page) through a
@@ -311,7 +313,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
           l2[(j >> 1) & 1] = __fadd2_rn(l2[(j >> 1) & 1], e);
           sv[j >> 1] = cut_bf16x2(e);
           second[j >> 1] = cut_bf16x2(e);
-          third[j >> 1] = cut_bf16x2(e);
+          third[j >> 1] = last_bf16x2(e);
         }
         l4[0] = l2[0].x; l4[1] = l2[0].y; l4[2] = l2[1].x; l4[3] = l2[1].y;
       }

@@ -10,11 +10,12 @@
 // FINE form (models whose cached attention keeps fp32 probabilities): queries come in bf16 and go into the product as they are, the
 // scale meets the fp32 scores, and a probability is multiplied whole, as three bf16 parts of 8 bits.  Up to 8 heads in the CTA, the second
 // parts are the rows 8 to 15 of the first parts' product, which have no heads of their own (160 rows of up to 4,096 tokens, 64 heads of 64 over 8
-// key heads: 245 us, a product of their own 306).  Bound by the chain of a tile's steps with eight warps an SM: issue slots 58 % busy, DRAM 45 %,
-// tensor pipe 17 %.  Outputs that differ from
-// the rounded 64-bit ones: 1e-4 to 4e-4 of them, like sums in fp32 (two rounded parts: 2e-3).  It took the place of a kernel that did both
-// products on the CUDA cores, a thread per key and a block-wide barrier five times a tile: the same rows, one layer of all keys and one with
-// a window of 128, 2,957 -> 255 us (the bytes take 135); one row of 900 tokens 69 -> 12 us.
+// key heads: 245 us, a product of their own 306).  No part of a probability is zero (cut_bf16x2), so an infinite value gives infinity, as in fp32;
+// for that the third parts are halved over both rows of a head (the same kind of step 210 -> 212 us).  Bound by the chain of a tile's steps with
+// eight warps an SM: issue slots 58 % busy, DRAM 45 %, tensor pipe 17 %.  Outputs that differ from the rounded 64-bit ones: 1e-4 to 4e-4 of them,
+// like sums in fp32 (two rounded parts: 2e-3).  It took the place of a kernel that did both products on the CUDA cores, a thread per key and
+// a block-wide barrier five times a tile: the same rows, one layer of all keys and one with a window of 128, 2,957 -> 255 us (the bytes take
+// 135); one row of 900 tokens 69 -> 12 us.
 #pragma once
 
 namespace bg {
@@ -192,7 +193,8 @@ __global__ void __launch_bounds__(kRowWarps * 32, 2) gqa_rows_kernel(const Param
         l[i] = l[i] * al[i] + (e.x + e.y) + (f.x + f.y);
         pa[i] = cut_bf16x2(e); pa[2 + i] = cut_bf16x2(f);
         pb[i] = cut_bf16x2(e); pb[2 + i] = cut_bf16x2(f);
-        pc[i] = cut_bf16x2(e); pc[2 + i] = cut_bf16x2(f);
+        if (!HI) { e = __fmul2_rn(e, make_float2(0.5f, 0.5f)); f = __fmul2_rn(f, make_float2(0.5f, 0.5f)); }
+        pc[i] = last_bf16x2(e); pc[2 + i] = last_bf16x2(f);
       } else {
         const __nv_bfloat162 lo = __floats2bfloat162_rn(e.x, e.y), hi = __floats2bfloat162_rn(f.x, f.y);
         l[i] = l[i] * al[i] + (__low2float(lo) + __high2float(lo)) + (__low2float(hi) + __high2float(hi));
@@ -200,9 +202,11 @@ __global__ void __launch_bounds__(kRowWarps * 32, 2) gqa_rows_kernel(const Param
         pa[2 + i] = *reinterpret_cast<const uint32_t*>(&hi);
       }
     }
-    if (FINE && !HI) {                                             // rows 8 to 15 have no heads: they take the second parts of rows 0 to 7
+    if (FINE && !HI) {            // rows 8 to 15 have no heads: they take the second parts of rows 0 to 7, and half of the third ones (no zeros)
       pa[1] = pb[0];
       pa[3] = pb[2];
+      pc[1] = pc[0];
+      pc[3] = pc[2];
       al[1] = al[0];
     }
     if (__any_sync(0xffffffffu, al[0] != 1.f || al[1] != 1.f)) {

@@ -193,3 +193,39 @@ def test_gqa_decode_takes_queries_at_any_address(first, splits):
     want = attention.gqa_decode(torch.stack(list(q)), cache, bt, lens, Hkv, D ** -0.5, num_splits=splits)
     _ext.check_status()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("new,ctx,at,splits", [(1, 199, 5, 1), (1, 199, 198, 3), (200, 100, 40, 0), (200, 0, 130, 0), (129, 64, 192, 0)])
+@pytest.mark.parametrize("Hq,Hkv,D", [(16, 2, 64), (12, 2, 128), (24, 2, 64)])
+def test_gqa_infinite_values_stay_infinite(Hq, Hkv, D, new, ctx, at, splits):
+    """An infinite value under probabilities above zero gives infinity in its column, as in fp32, whatever bits a probability has: the
+    key at ``at`` has the largest score, so where its tile is the first its probability is exactly one before the division."""
+    from batchgen_b200.ops import _ext, attention, talking
+    g = torch.Generator().manual_seed(new + at)
+    n, page = new + ctx, 64
+    rows = torch.randn(n, 2, Hkv, D, generator=g).bfloat16()
+    rows[:, 0, :, 0] = 0
+    rows[at, 0, :, :] = 0
+    rows[at, 0, :, 0] = 8
+    rows[at, 1, 0, 3], rows[at, 1, 1, 7] = float("inf"), -float("inf")
+    rows[0, 1, 0, 5] = float("inf")                                  # seen by all, a probability of any bits
+    q = (torch.randn(new, Hq, D, generator=g) * 0.2).bfloat16()
+    q[..., 0] = 4
+    cache = torch.zeros(-(-n // page) * page, 2 * Hkv * D).bfloat16()
+    cache[:n] = rows.view(n, -1)
+    c, bt = cache.view(-1, page, 2 * Hkv * D).cuda(), torch.arange(-(-n // page)).int().view(1, -1).cuda()
+    if new > 1:
+        out = torch.empty(new, Hq * D, dtype=torch.bfloat16, device="cuda")
+        work = torch.tensor(talking.prefill_work([0, new], [ctx], 0, 1, 0), dtype=torch.int32).cuda()
+        attention.gqa_prefill(q.cuda(), c, bt, work, Hkv, D ** -0.5, out)
+    else:
+        out = attention.gqa_decode(q.cuda(), c, bt, torch.tensor([n], dtype=torch.int32).cuda(), Hkv, D ** -0.5, num_splits=splits)
+    _ext.check_status()
+    out = out.view(new, Hq, D).float().cpu()
+    seen = torch.arange(new) + ctx >= at                              # rows before it: its tile's products may hold 0 * inf
+    G = Hq // Hkv
+    assert (out[seen, :G, 3] == float("inf")).all() and (out[seen, G:, 7] == -float("inf")).all()
+    assert (out[:, :G, 5] == float("inf")).all()
+    finite = torch.ones(Hq, D, dtype=torch.bool)
+    finite[:G, 3] = finite[:G, 5] = finite[G:, 7] = False
+    assert torch.isfinite(out[:, finite]).all()
