@@ -1,12 +1,8 @@
-// bf16 GEMM with the weights on the tensor-core M side and up to 256 tokens as N (D^T = W . X^T), dense and ragged grouped.
+// Dense bf16 GEMM with the weights on the tensor-core M side and up to 256 tokens as N (D^T = W . X^T), for products of few tiles.
 //
-// A mixture gives an expert anything from a token to a few hundred. With 128-row token tiles an expert of 140 tokens takes two tiles and
-// reads its weights twice, and one of a dozen pays for 128. Here a weight tile of 128 rows meets all tokens of its segment (up to
-// 256 at a time, cut evenly, rounded up to 16) in one product of that width, so weights cross L2 once and the padding is below 16
-// tokens.  Bound by the tensor cores at prompt sizes and by the weights' bytes below some hundred rows a segment, where the caller keeps the 128 x
-// 128 kernel.  256 matrices of 2,048 x 2,304, Poisson rows, 128 x 128 kernel -> here: 112 rows 432 -> 489 us, 128 rows 514 -> 522, 156 rows 613 -> 540
-// (alone 468: DRAM 72 %, tensor cores 45 %), 512 rows 1,267 -> 1,104; dense 4,096 x 16,576 x 2,304 332 -> 253 us (1,238 TFLOP/s), 6,200 x 32,768 x 512
-// 299 -> 202.
+// A weight tile of 128 rows meets all tokens (up to 256 at a time, cut evenly, rounded up to 16) in one product of that width.  From two
+// rounds of 256 x 256 tiles on, and for segments of rows, pairs of CTAs move fewer operand bytes (gemm_bf16_pair.cu); below, tiles of half
+// the size fill the SMs better: 1,024 x 4,096 x 2,880 25 us (pairs 27), 2,000 x 1,024 x 4,096 29 (31), 160 x 32,768 x 512 15 (17).
 //
 // Roles (192 threads, one CTA per SM, persistent): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 2..5 epilogue (thread = weight
 // row; two accumulators of 256 columns, so one is stored while the other is filled).  All waits are bounded.
@@ -24,16 +20,13 @@ constexpr int BK = 64;                    // elements of K per stage (one 128-by
 constexpr int kStages = 4;
 constexpr int kThreads = 192;
 constexpr int kTmemCols = 512;
-constexpr int kMaxGroups = 1024;
 constexpr int kWBytes = BW * BK * 2;      // 16 KB
 constexpr int kXBytes = BT * BK * 2;      // 32 KB
 
 struct Params {
   __nv_bfloat16* D;      // [M, ldd]
   int ldd;
-  const int* offsets;    // [groups + 1] segment starts; null = dense
-  const int* counts;     // [groups] rows present in a segment, or null: all of it
-  int groups, M, N, K;
+  int M, N, K;
   int* status;
 };
 
@@ -42,7 +35,6 @@ struct Shared {
   uint64_t tmem_full[2], tmem_empty[2];
   uint32_t tmem_base;
   int abort_flag;
-  Segments<kMaxGroups> seg;
 };
 
 __global__ void __launch_bounds__(kThreads, 1)
@@ -64,7 +56,6 @@ gemm_bf16_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
     ss.abort_flag = 0;
     mbar_fence_init();
   }
-  if (p.offsets != nullptr) load_segments<BT>(ss.seg, p.offsets, p.counts, p.groups);
   if (warp == 1) {
     tmem_alloc(&ss.tmem_base, kTmemCols);
     tmem_relinquish();
@@ -73,7 +64,7 @@ gemm_bf16_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
-  TokenWalker<BT, BW, kMaxGroups> walk(p.offsets != nullptr ? &ss.seg : nullptr, p.groups, n_tiles, p.M);
+  TokenWalker<BT, BW, 1> walk(nullptr, 1, n_tiles, p.M);
   TokenTile t;
   uint32_t it = 0, acc = 0;
   bool ok = true;
@@ -84,7 +75,7 @@ gemm_bf16_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
       tma_prefetch_desc(&tmW);
       tma_prefetch_desc(&tmX);
       for (int tile = blockIdx.x; ok && walk.get(tile, t); tile += gridDim.x) {
-        const int boxes = (tile_cols(t) + kBox - 1) / kBox, row = t.g * p.N + t.n0;
+        const int boxes = (tile_cols(t) + kBox - 1) / kBox, row = t.n0;
         for (int kb = 0; kb < KB; ++kb, ++it) {
           const int s = it % kStages;
           if (!mbar_wait(&ss.empty[s], ((it / kStages) & 1) ^ 1, abort_flag, kTimeoutProducer)) { ok = false; break; }
@@ -195,25 +186,20 @@ static int make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t co
 
 extern "C" {
 
-// X [M, K] bf16 tokens, W [groups * N, K] bf16 -> D [M, ldd] bf16.  K a multiple of 64.  offsets null: dense; counts: rows present in
-// every segment, or null (rows past them stay undefined).
-int bg_gemm_bf16_swap(const void* X, const void* W, void* D, int ldd, const int* offsets, const int* counts, int groups, int M, int N,
-                      int K, int num_sms, int* status, cudaStream_t stream) {
+// X [M, K] bf16 tokens, W [N, K] bf16 -> D [M, ldd] bf16.  K a multiple of 64.
+int bg_gemm_bf16_swap(const void* X, const void* W, void* D, int ldd, int M, int N, int K, int num_sms, int* status, cudaStream_t stream) {
   using namespace bg::bswap;
   if (M <= 0 || N <= 0) return 0;
-  if (K <= 0 || K % BK != 0 || groups > kMaxGroups || groups <= 0) return -1;
-  if (offsets == nullptr) groups = 1;
+  if (K <= 0 || K % BK != 0) return -1;
   Params p;
-  p.D = reinterpret_cast<__nv_bfloat16*>(D); p.ldd = ldd; p.offsets = offsets; p.counts = offsets != nullptr ? counts : nullptr;
-  p.groups = groups; p.M = M; p.N = N; p.K = K; p.status = status;
+  p.D = reinterpret_cast<__nv_bfloat16*>(D); p.ldd = ldd; p.M = M; p.N = N; p.K = K; p.status = status;
   CUtensorMap tw, tx;
-  if (make_map(&tw, W, (uint64_t)groups * N, (uint64_t)K, BW) != 0) return -11;
+  if (make_map(&tw, W, (uint64_t)N, (uint64_t)K, BW) != 0) return -11;
   if (make_map(&tx, X, (uint64_t)M, (uint64_t)K, kBox) != 0) return -12;
   static bg::DeviceOnce once;
   const size_t smem = kStages * (kWBytes + kXBytes) + sizeof(Shared) + 1024;
   if (!bg::ensure_dynamic_smem(gemm_bf16_swap_kernel, smem, once)) return -13;
-  const int n_tiles = (N + BW - 1) / BW;
-  long long grid = ((long long)M / BT + (offsets != nullptr ? groups : 1)) * n_tiles;      // an upper bound of the tiles
+  long long grid = ((long long)M / BT + 1) * ((N + BW - 1) / BW);      // an upper bound of the tiles
   if (grid > num_sms) grid = num_sms;
   bg::launch_pdl(gemm_bf16_swap_kernel, dim3((int)grid), dim3(kThreads), smem, stream, tw, tx, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -14;

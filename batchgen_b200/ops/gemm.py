@@ -234,19 +234,33 @@ def swap_dense(T: int, N: int, K: int, sms: int) -> bool:
     return T > 128 or K < 1536 or T * K < 65536
 
 
+def use_pairs(T: int, N: int, sms: int) -> bool:
+    """Pairs of CTAs on tiles of 256 x 256 for a dense product: from two rounds of such tiles on, unless they take more rounds than tiles of 256 x
+    128 do (pairs / one CTA, us: 700 x 16,576 x 2,304 50 / 54, 300 x 20,480 x 2,880 48 / 56, 8,000 x 2,304 x 4,096 105 / 121; under two rounds 2,500
+    x 2,304 x 4,096 54 / 52, 160 x 32,768 x 512 17 / 15; four rounds against three 4,650 x 2,880 x 4,096 93 / 82)."""
+    tokens, pairs = -(-T // 256), sms // 2
+    tiles = tokens * -(-N // 256)
+    return tiles >= 2 * pairs > 0 and -(-tiles // pairs) <= -(-tokens * -(-N // 128) // sms)
+
+
 def _bf16_swap(x: torch.Tensor, w2d: torch.Tensor, out: torch.Tensor, offsets, counts, groups: int, N: int) -> None:
-    rc = _ext.lib().bg_gemm_bf16_swap(_ext.ptr(x), _ext.ptr(w2d), _ext.ptr(out), ctypes.c_int(out.stride(0)), _ext.ptr(offsets),
-                                      _ext.ptr(counts), ctypes.c_int(groups), ctypes.c_int(x.shape[0]), ctypes.c_int(N),
-                                      ctypes.c_int(x.shape[1]), ctypes.c_int(_ext.num_sms(x.device)),
-                                      _ext.ptr(_ext.status_word(x.device)), _ext.stream())
+    """Weights as the MMA's M, tokens as its N; segments of tokens always on pairs of CTAs, where they are never behind."""
+    sms = _ext.num_sms(x.device)
+    tail = (ctypes.c_int(x.shape[0]), ctypes.c_int(N), ctypes.c_int(x.shape[1]), ctypes.c_int(sms), _ext.ptr(_ext.status_word(x.device)), _ext.stream())
+    if offsets is not None or use_pairs(x.shape[0], N, sms):
+        rc = _ext.lib().bg_gemm_bf16_pair(_ext.ptr(x), _ext.ptr(w2d), _ext.ptr(out), ctypes.c_int(out.stride(0)), _ext.ptr(offsets),
+                                          _ext.ptr(counts), ctypes.c_int(groups), *tail)
+        _ext.check(rc, "bg_gemm_bf16_pair")
+        return
+    rc = _ext.lib().bg_gemm_bf16_swap(_ext.ptr(x), _ext.ptr(w2d), _ext.ptr(out), ctypes.c_int(out.stride(0)), *tail)
     _ext.check(rc, "bg_gemm_bf16_swap")
 
 
 def swap_grouped(rows: float, groups: int, K: int) -> bool:
     """Tokens as the MMA's N for segments of ``rows`` expected rows: from 128 on, where half of them would need a second 128-row tile
-    (Poisson rows, 256 matrices of 2,048 x 2,304, swapped against the 128 x 128 kernel: 112 rows 489 / 432 us, 128 rows 522 / 514, 156
-    rows 540 / 613, 512 rows 1,104 / 1,267; of 2,304 x 1,024: 112 rows 269 / 241, 128 rows 273 / 293; 32 matrices of 2,048 x 2,304: 13 rows
-    67 / 57, 128 rows 74 / 73, 156 rows 75 / 81).  Below, the weights are streamed, and the 128 x 128 kernel has more of them in flight."""
+    (Poisson rows, 256 matrices of 2,048 x 2,304, pairs of CTAs against the 128 x 128 kernel: 64 rows 408 / 402 us, 112 rows 422 / 435, 128 rows
+    439 / 510; of 2,304 x 1,024: 64 rows 227 / 233, 128 rows 234 / 288; 32 matrices of 2,048 x 2,304: 13 rows 64 / 62, 128 rows 68 / 80).  Below, both
+    stream the weights and differ by a few percent either way."""
     return rows >= 128 and 0 < groups <= 1024 and K > 0 and K % 64 == 0
 
 

@@ -151,3 +151,24 @@ def test_dense_bf16_token_tiles(T, N, K):
     got, want = wide.cpu().double(), x.double() @ w.double().t()
     assert (got[:, :8] == 7).all() and (got[:, 8 + N:] == 7).all()
     assert ((got[:, 8:8 + N] - want).abs() <= want.abs() * 2 ** -8 + (x.double().abs() @ w.double().abs().t()) * K * 2 ** -24).all()
+
+
+@pytest.mark.parametrize("T,N,K,pad", [(1, 8, 64, 0), (33, 264, 192, 24), (256, 512, 1024, 3), (257, 300, 64, 0), (700, 1000, 128, 8)])
+def test_dense_bf16_pairs(T, N, K, pad):
+    """Products on pairs of CTAs: tokens and outputs that end inside a CTA's half, rows that are not 16-byte aligned; the one-CTA form's bits."""
+    import ctypes
+    from batchgen_b200.ops import _ext
+    g = torch.Generator().manual_seed(T)
+    x, w = torch.randn(T, K, generator=g).bfloat16().cuda(), torch.randn(N, K, generator=g).bfloat16().cuda()
+    outs = []
+    for fn, mid in (("bg_gemm_bf16_pair", (None, None, 1)), ("bg_gemm_bf16_swap", ())):
+        out = torch.full((T, N + pad), 7.0, dtype=torch.bfloat16, device="cuda")
+        mid = tuple(ctypes.c_void_p(0) if m is None else ctypes.c_int(m) for m in mid)
+        rc = getattr(_ext.lib(), fn)(_ext.ptr(x), _ext.ptr(w), _ext.ptr(out), ctypes.c_int(N + pad), *mid, ctypes.c_int(T), ctypes.c_int(N),
+                                     ctypes.c_int(K), ctypes.c_int(_ext.num_sms(x.device)), _ext.ptr(_ext.status_word(x.device)), _ext.stream())
+        assert rc == 0
+        _ext.check_status()
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and (outs[0][:, N:] == 7).all()
+    got, want = outs[0][:, :N].cpu().double(), (x.cpu().double() @ w.cpu().double().t())
+    assert ((got - want).abs() <= want.abs() * 2 ** -8 + (x.cpu().double().abs() @ w.cpu().double().abs().t()) * K * 2 ** -24).all()
