@@ -15,6 +15,8 @@
 // shared-memory operands and 128-row token tiles: one token 59 and 36 us -> 35 and 21, 160 tokens 997 and 504 -> 546 and 286 (184 and 92 at copy
 // bandwidth), 4,650 tokens 1,864 and 945 -> 731 and 374.  Bound by the latency of a step's chain (expansion, TMEM store, product): some 520
 // clocks at 160 tokens, issue slots 59 % and the integer pipe 54 % busy.
+// MXFP4 products of up to 80 rows a segment without the fused SiLU go to gemm_mxfp4_block.cu (160 tokens 287 and 176 us); from there on the expanded
+// form is ahead, and int4 weights, whose scales are not powers of two, stay here.
 //
 // Roles (736 threads, one CTA per SM, persistent over tiles):
 //   warp 0       TMA producer of the token tiles (swizzled), 6 stages

@@ -12,6 +12,7 @@
 // bit-reproducible run to run).
 #define BG_FILE_TAG 2      // kernel-trace ids of this file are (tag << 16) | line
 #include "common.cuh"
+#include "mx_parts.cuh"
 
 namespace bg {
 
@@ -307,10 +308,11 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ y, int ldy, const int* __re
 // width take 97 us (3.5 TB/s), bound by the exponential and the division, which stay those of fp32: __expf and __fdividef took 64 us, but
 // their error grows with |g| (1.5e-6 of the value at 20) and their quotient is zero past 2^126.
 // A clamp lets a NaN through, like the tensor operation does.
-template <int KIND>
+// PARTS: the rows leave as the 4-bit product's operand (mx_parts.cuh) instead of bf16, from the same rounded values.
+template <int KIND, bool PARTS>
 __global__ void __launch_bounds__(256)
 gated_rows_kernel(const __nv_bfloat16* __restrict__ z, long long ldz, __nv_bfloat16* __restrict__ out, int ldo, int rows, int F, float limit,
-                  const int* __restrict__ total_rows, const int* __restrict__ row_src) {
+                  const int* __restrict__ total_rows, const int* __restrict__ row_src, mxp::Parts parts) {
   bg::pdl_prologue((BG_FILE_TAG << 16) | __LINE__);
   const int n = total_rows != nullptr ? min(rows, *total_rows) : rows;
   for (int r = blockIdx.x; r < n; r += gridDim.x) {
@@ -333,9 +335,24 @@ gated_rows_kernel(const __nv_bfloat16* __restrict__ z, long long ldz, __nv_bfloa
         const float2 g = __bfloat1622float2(gp[i]), u = __bfloat1622float2(up[i]);
         o[i] = __floats2bfloat162_rn(one(g.x, u.x), one(g.y, u.y));
       }
-      *reinterpret_cast<uint4*>(out + (size_t)r * ldo + v * 8) = *reinterpret_cast<const uint4*>(o);
+      if (PARTS) {                               // F is a multiple of 32: a block's four lanes stay together
+        const mxp::Split<8> s(o);
+        s.store(parts, r, v * 8);
+      } else {
+        *reinterpret_cast<uint4*>(out + (size_t)r * ldo + v * 8) = *reinterpret_cast<const uint4*>(o);
+      }
     }
   }
+}
+
+template <bool PARTS>
+static int gated_rows(int kind, const void* z, long long ldz, void* out, int ldo, int rows, int F, float limit, const int* total_rows,
+                      const int* row_src, int num_sms, const mxp::Parts& parts, cudaStream_t stream) {
+  const dim3 grid(min(rows, num_sms * 16)), block(min(256, (F / 8 + 31) / 32 * 32));
+  auto kern = kind == 0 ? gated_rows_kernel<0, PARTS> : kind == 1 ? gated_rows_kernel<1, PARTS> : gated_rows_kernel<2, PARTS>;
+  bg::launch_pdl(kern, grid, block, 0, stream, reinterpret_cast<const __nv_bfloat16*>(z), ldz, reinterpret_cast<__nv_bfloat16*>(out), ldo, rows, F, limit,
+                 total_rows, row_src, parts);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 }  // namespace bg
@@ -348,12 +365,17 @@ int bg_gated_rows(int kind, const void* z, long long ldz, void* out, int ldo, in
   using namespace bg;
   if (rows <= 0 || F <= 0) return 0;
   if (F % 8 || ldz % 8 || ldo % 8 || ldz < 2ll * F || ldo < F || kind < 0 || kind > 2) return -1;
-  const dim3 grid(min(rows, num_sms * 16)), block(min(256, (F / 8 + 31) / 32 * 32));
-  auto Z = reinterpret_cast<const __nv_bfloat16*>(z);
-  auto O = reinterpret_cast<__nv_bfloat16*>(out);
-  auto kern = kind == 0 ? gated_rows_kernel<0> : kind == 1 ? gated_rows_kernel<1> : gated_rows_kernel<2>;
-  bg::launch_pdl(kern, grid, block, 0, stream, Z, ldz, O, ldo, rows, F, limit, total_rows, row_src);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return gated_rows<false>(kind, z, ldz, out, ldo, rows, F, limit, total_rows, row_src, num_sms, mxp::Parts{}, stream);
+}
+
+// The same rows as parts p [rows / 8 rounded up][2][8][F] and scales s [F / 128 rounded up][rows][4] of the 4-bit product; F a multiple of 32.
+int bg_gated_parts(int kind, const void* z, long long ldz, void* p, void* s, int rows, int F, float limit, const int* total_rows,
+                   const int* row_src, int num_sms, cudaStream_t stream) {
+  using namespace bg;
+  if (rows <= 0 || F <= 0) return 0;
+  if (F % 32 || ldz % 8 || ldz < 2ll * F || kind < 0 || kind > 2) return -1;
+  const mxp::Parts parts{reinterpret_cast<uint8_t*>(p), reinterpret_cast<uint8_t*>(s), rows, F};
+  return gated_rows<true>(kind, z, ldz, nullptr, 0, rows, F, limit, total_rows, row_src, num_sms, parts, stream);
 }
 
 // logits: rows of E values, ldl apart; norm: weights divided by their sum, 1 unless K is 1, 2 always; group_max: a group counts with

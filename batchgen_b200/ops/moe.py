@@ -10,12 +10,13 @@ and batchgen/moe/grouped_fp8_blockwise_moe.py.
 from __future__ import annotations
 
 import ctypes
+import functools
 from dataclasses import dataclass
 from typing import Optional, Tuple, Union
 
 import torch
 
-from . import _ext, fused, gemm, ref, residual
+from . import _ext, fused, gemm, mxfp4, ref, residual
 
 FP8 = torch.float8_e4m3fn
 ROW_ALIGN = 128  # grouped segments start on tile boundaries of the tcgen05 GEMM
@@ -194,6 +195,13 @@ def activation_on_kernel(gate_up: torch.Tensor) -> bool:
             and gate_up.stride(1) == 1 and gate_up.stride(0) % 8 == 0 and gate_up.data_ptr() % 16 == 0)
 
 
+def _activation_kind(kind: str, limit: float) -> Tuple[int, float]:
+    """The activation kernel's number and clamp."""
+    if kind == "swiglu_clamped":
+        return 1, 7.0
+    return (2, limit) if kind == "silu_limit" and limit > 0 else (0, limit)
+
+
 def activation(gate_up: torch.Tensor, kind: str, limit: float = 0.0, offsets: Optional[torch.Tensor] = None,
                row_src: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Gated activation of rows [gate | up]: ``kind`` swiglu_clamped, silu_limit (with a ``limit``), else SiLU(gate) * up.  Grouped rows:
@@ -202,9 +210,9 @@ def activation(gate_up: torch.Tensor, kind: str, limit: float = 0.0, offsets: Op
         return _activation(gate_up, kind, limit)
     R, I = gate_up.shape[0], gate_up.shape[1] // 2
     out = torch.empty(R, I, dtype=gate_up.dtype, device=gate_up.device)
-    k = 1 if kind == "swiglu_clamped" else 2 if kind == "silu_limit" and limit > 0 else 0
+    k, limit = _activation_kind(kind, limit)
     rc = _ext.lib().bg_gated_rows(ctypes.c_int(k), _ext.ptr(gate_up), ctypes.c_longlong(gate_up.stride(0)), _ext.ptr(out),
-                                  ctypes.c_int(I), ctypes.c_int(R), ctypes.c_int(I), ctypes.c_float(7.0 if k == 1 else limit),
+                                  ctypes.c_int(I), ctypes.c_int(R), ctypes.c_int(I), ctypes.c_float(limit),
                                   _ext.ptr(offsets[-1:] if offsets is not None else None), _ext.ptr(row_src),
                                   ctypes.c_int(_ext.num_sms(gate_up.device)), _ext.stream())
     _ext.check(rc, "bg_gated_rows")
@@ -250,19 +258,22 @@ def grouped_experts(xq, xs, offsets: torch.Tensor, ew: ExpertWeights, x_dense: O
         aq, as_ = ref.act_quant(act)
         return ref.grouped_fp8_gemm(aq, as_, ew.w2, ew.w2_s, offsets)
     if ew.quant in ("mxfp4", "int4"):
-        # W4A16, groups of 32: one tcgen05 kernel, two expansions (e2m1 x e8m0 scale, or offset-binary int4 x bf16 scale)
+        # W4A16, groups of 32: e2m1 x e8m0 scale on the block-scaled product, or offset-binary int4 x bf16 scale expanded to bf16
+        x = x_dense
         if ew.quant == "mxfp4":
-            from .mxfp4 import grouped_mxfp4_gemm as grouped_w4
+            grouped_w4 = functools.partial(mxfp4.grouped_mxfp4_gemm, rows_hint=rows_hint)
         else:
             from .int4 import grouped_int4_gemm as grouped_w4
-        x = x_dense
         if x.is_cuda and ew.interleaved:
             with timer.timed("moe.s1_gemm"):
                 act = grouped_w4(x, ew.w13, ew.w13_s, offsets, silu_mul=True, counts=counts)
         else:
             with timer.timed("moe.s1_gemm"):
                 gu = grouped_w4(x, ew.w13, ew.w13_s, offsets, counts=counts)
-            act = activation(gu, ew.activation, ew.act_limit, offsets, row_src).to(x.dtype)
+            if isinstance(x, mxfp4.Parts) and activation_on_kernel(gu) and mxfp4.block_scaled(ew.w2, ew.w2_s, rows_hint / ew.num_experts):
+                act = mxfp4.gated_parts(gu, *_activation_kind(ew.activation, ew.act_limit), offsets, row_src)
+            else:
+                act = activation(gu, ew.activation, ew.act_limit, offsets, row_src).to(x.dtype if isinstance(x, torch.Tensor) else torch.bfloat16)
         with timer.timed("moe.s3_gemm"):
             return grouped_w4(act, ew.w2, ew.w2_s, offsets, counts=counts)
     # unquantised experts
@@ -305,6 +316,7 @@ def experts_forward(hidden: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.
         align = 8                          # these grouped GEMMs take real row counts: segments only need aligned rows
     with timer.timed("moe.permute"):
         src, pos, offsets = permute(topk_idx, expert_lo, expert_hi, num_valid, align=align)
+    here = topk_idx.shape[0] * topk_idx.shape[1] * (expert_hi - expert_lo) / max(num_experts or expert_hi - expert_lo, 1)      # pairs expected on this rank
     if ew.quant == "fp8_block":
         counts = getattr(offsets, "real_counts", None)
         with timer.timed("moe.gather_quant"):
@@ -317,13 +329,16 @@ def experts_forward(hidden: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.
             # a pair's row goes straight to its place; padding rows of a segment stay undefined (no kept row depends on another)
             with timer.timed("moe.gather"):
                 whole = hidden if hidden.is_contiguous() and hidden.data_ptr() % 16 == 0 else hidden.clone(memory_format=torch.contiguous_format)
-                rows, _ = residual.moe_gather(whole, pos, topk_w.float().contiguous(), src.shape[0])      # rows in 16-byte pieces
+                if ew.quant == "mxfp4" and not ew.interleaved and mxfp4.block_scaled(ew.w13, ew.w13_s, here / max(ew.num_experts, 1)):
+                    rows = mxfp4.split(whole, pos, src.shape[0])
+                else:
+                    rows, _ = residual.moe_gather(whole, pos, topk_w.float().contiguous(), src.shape[0])      # rows in 16-byte pieces
         else:
             rows = hidden[src.clamp_min(0).long()]
             rows = torch.where((src >= 0).unsqueeze(-1), rows, torch.zeros_like(rows))
         y = grouped_experts(None, None, offsets, ew, x_dense=rows, counts=getattr(offsets, "real_counts", None),
                             row_src=src if rows.is_cuda else None,
-                            rows_hint=topk_idx.shape[0] * topk_idx.shape[1] * (expert_hi - expert_lo) / max(num_experts or expert_hi - expert_lo, 1))
+                            rows_hint=here)
     with timer.timed("moe.combine"):
         if before_combine is not None:
             before_combine()

@@ -1,8 +1,8 @@
 """MXFP4 (e2m1 values, one e8m0 scale per 32) expert weights: GEMMs and conversion.
 
-On CUDA the GEMMs run ``gemm_mxfp4.cu``: packed weights go from HBM to shared memory as 4-bit data and are
-expanded to bf16 on their way to TMEM, then multiplied on tcgen05 with fp32 accumulation.  On CPU the same
-contract is met by dequantising and multiplying in fp32.
+On CUDA the GEMMs run ``gemm_mxfp4_block.cu``: the weights and their scales are operands of the block-scaled tensor-core product, and a
+bf16 row is two e4m3 parts that sum up to it (``Parts``).  With the fused SiLU epilogue, for long segments and for shapes that its loads do not
+take they run ``gemm_mxfp4.cu``, which expands the weights to bf16 on their way to TMEM.  On CPU the same contract is met by dequantising and multiplying in fp32.
 
 Reference parity: quantiser / layout batchgen/quantization/mxfp4.py:30 and
 batchgen/models/moonshotai/kimi_linear/k3/mxfp4_layout.py:37-38,179-182; grouped GEMMs
@@ -11,7 +11,8 @@ batchgen_kernels/src/moe/mxfp4/marlin_grouped_gemm.cu and batchgen/moe/fused_moe
 from __future__ import annotations
 
 import ctypes
-from typing import Optional
+from dataclasses import dataclass
+from typing import Optional, Union
 
 import torch
 
@@ -51,6 +52,73 @@ def _launch(epi, x, wq2d, ws2d, out, offsets, groups, M, N, K, counts=None):
     _ext.check(rc, "bg_mxfp4_gemm")
 
 
+@dataclass
+class Parts:
+    """bf16 rows [rows, K] as the block-scaled product takes them: ``p`` uint8 [rows / 8 rounded up, 2, 8, K] (e4m3, eight rows' first parts and
+    then their second parts), ``s`` uint8 [K / 128 rounded up, rows, 4] (e8m0 of the first part, one per 32 elements; the second part's is five
+    less)."""
+    p: torch.Tensor
+    s: torch.Tensor
+
+    @property
+    def shape(self):
+        return self.s.shape[1], self.p.shape[3]
+
+    @property
+    def is_cuda(self) -> bool:
+        return self.p.is_cuda
+
+
+def _new_parts(rows: int, K: int, device) -> Parts:
+    return Parts(torch.empty(-(-rows // 8), 2, 8, K, dtype=torch.uint8, device=device), torch.empty(-(-K // 128), rows, 4, dtype=torch.uint8, device=device))
+
+
+def split(x: torch.Tensor, pos: Optional[torch.Tensor] = None, rows: Optional[int] = None) -> Parts:
+    """Rows of x [T, K] as parts; with ``pos`` (int32 [T, k]) token t goes to every row pos[t, j] >= 0 of ``rows``, the others stay undefined."""
+    T, K = x.shape
+    rows = T if rows is None else rows
+    out = _new_parts(rows, K, x.device)
+    rc = _ext.lib().bg_mx_split(_ext.ptr(x), ctypes.c_longlong(x.stride(0)), _ext.ptr(pos), ctypes.c_int(pos.shape[1] if pos is not None else 0),
+                                ctypes.c_int(T), _ext.ptr(out.p), _ext.ptr(out.s), ctypes.c_int(rows), ctypes.c_int(K),
+                                _ext.stream())
+    _ext.check(rc, "bg_mx_split")
+    return out
+
+
+def gated_parts(gate_up: torch.Tensor, kind: int, limit: float, offsets: Optional[torch.Tensor], row_src: Optional[torch.Tensor]) -> Parts:
+    """The gated activation of ``moe.activation`` (kind 0, 1, 2 of its kernel) with its rows as parts."""
+    R, I = gate_up.shape[0], gate_up.shape[1] // 2
+    out = _new_parts(R, I, gate_up.device)
+    rc = _ext.lib().bg_gated_parts(ctypes.c_int(kind), _ext.ptr(gate_up), ctypes.c_longlong(gate_up.stride(0)), _ext.ptr(out.p), _ext.ptr(out.s),
+                                   ctypes.c_int(R), ctypes.c_int(I), ctypes.c_float(limit),
+                                   _ext.ptr(offsets[-1:] if offsets is not None else None), _ext.ptr(row_src),
+                                   ctypes.c_int(_ext.num_sms(gate_up.device)), _ext.stream())
+    _ext.check(rc, "bg_gated_parts")
+    return out
+
+
+BLOCK_MAX_ROWS = 80
+
+
+def block_scaled(wq: torch.Tensor, ws: torch.Tensor, rows: float) -> bool:
+    """The block-scaled product takes weights wq [.., N, K / 2], ws [.., N, K / 32] for segments of ``rows`` expected rows: up to 80 of them (128 experts of
+    6,144 x 2,880, against weights expanded to bf16: 5 rows 287 / 553 us, 25 rows 369 / 559, 47 rows 461 / 573, 94 rows 643 / 605), K from 128 to
+    12,288, addresses and rows as its loads need them."""
+    return rows <= BLOCK_MAX_ROWS and bool(_ext.lib().bg_mxfp4_block_takes(_ext.ptr(wq), _ext.ptr(ws), ctypes.c_longlong(wq.shape[-2]),
+                                                                           ctypes.c_int(2 * wq.shape[-1])))
+
+
+def _block_gemm(x: Union[torch.Tensor, Parts], wq2d, ws2d, out, offsets, groups, M, N, K, counts, rows) -> None:
+    if isinstance(x, torch.Tensor):
+        x = x.contiguous()
+        x = split(x if x.data_ptr() % 16 == 0 else x.clone())
+    rc = _ext.lib().bg_mxfp4_block_gemm(
+        _ext.ptr(x.p), _ext.ptr(x.s), _ext.ptr(wq2d), _ext.ptr(ws2d), _ext.ptr(out), ctypes.c_int(out.stride(0)),
+        _ext.ptr(offsets), _ext.ptr(counts), ctypes.c_int(groups), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K), ctypes.c_float(rows),
+        ctypes.c_int(_ext.num_sms(out.device)), _ext.ptr(_ext.status_word(out.device)), _ext.stream())
+    _ext.check(rc, "bg_mxfp4_block_gemm")
+
+
 def mxfp4_gemm(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """[T, K] bf16 x MXFP4 [N, K] -> [T, N] bf16."""
     N, K = wq.shape[0], wq.shape[1] * 2
@@ -60,16 +128,20 @@ def mxfp4_gemm(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor, out: Optiona
     if out is None:
         out = torch.empty(T, N, dtype=torch.bfloat16, device=x.device)
     if T:
-        _launch(EPI_STORE, x.contiguous(), wq, ws, out, None, 1, T, N, K)
+        if block_scaled(wq, ws, T):
+            _block_gemm(x, wq, ws, out, None, 1, T, N, K, None, T)
+        else:
+            _launch(EPI_STORE, x.contiguous(), wq, ws, out, None, 1, T, N, K)
     return out
 
 
-def grouped_mxfp4_gemm(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor, offsets: torch.Tensor,
+def grouped_mxfp4_gemm(x: Union[torch.Tensor, Parts], wq: torch.Tensor, ws: torch.Tensor, offsets: torch.Tensor,
                        silu_mul: bool = False, out: Optional[torch.Tensor] = None,
-                       counts: Optional[torch.Tensor] = None) -> torch.Tensor:
+                       counts: Optional[torch.Tensor] = None, rows_hint: Optional[float] = None) -> torch.Tensor:
     """Ragged grouped GEMM over rows grouped by expert (segment e = offsets[e]:offsets[e+1]; ``counts``: rows present in
     every segment, the others stay undefined).  wq [E, N, K/2], ws [E, N, K/32].  ``silu_mul``: the rows of each expert
-    are stored gate/up interleaved in blocks of 32 and the output is silu(gate) * up with N/2 columns."""
+    are stored gate/up interleaved in blocks of 32 and the output is silu(gate) * up with N/2 columns.  ``x``: bf16 rows, or their
+    ``Parts`` (without ``silu_mul``); ``rows_hint``: rows that are expected to be present in all."""
     E, N, Kh = wq.shape
     K = Kh * 2
     R = x.shape[0]
@@ -88,9 +160,14 @@ def grouped_mxfp4_gemm(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor, offs
         return y.to(x.dtype)
     n_out = N // 2 if silu_mul else N
     if out is None:
-        out = torch.empty(R, n_out, dtype=torch.bfloat16, device=x.device)
+        out = torch.empty(R, n_out, dtype=torch.bfloat16, device=wq.device)
     if R:
         assert offsets.dtype == torch.int32 and offsets.is_cuda
-        _launch(EPI_SILU_MUL if silu_mul else EPI_STORE, x.contiguous(), wq.view(E * N, Kh), ws.view(E * N, K // 32),
-                out, offsets, E, R, N, K, counts)
+        wq2d, ws2d = wq.view(E * N, Kh), ws.view(E * N, K // 32)
+        rows = (R if rows_hint is None else rows_hint) / max(E, 1)
+        if isinstance(x, Parts) or not silu_mul and block_scaled(wq, ws, rows):
+            assert not silu_mul
+            _block_gemm(x, wq2d, ws2d, out, offsets, E, R, N, K, counts, rows)
+        else:
+            _launch(EPI_SILU_MUL if silu_mul else EPI_STORE, x.contiguous(), wq2d, ws2d, out, offsets, E, R, N, K, counts)
     return out

@@ -220,3 +220,80 @@ def test_segments_that_are_passed_over(only, kernel, monkeypatch):
         assert ((got[offs[e]:offs[e] + c] - xe @ w[e].t()).abs() <= (xe @ w[e].t()).abs() * 2 ** -8 + xe.abs() @ w[e].abs().t() * K * 2 ** -24).all(), e
         seen[offs[e]:offs[e] + c] = True
     assert (got[~seen] == 7).all()
+
+
+def _block_case(counts, lead, N, K, seed):
+    """Segments that start anywhere (``lead`` rows before each), rows of 20 binades, weights and scales of every size."""
+    g = torch.Generator().manual_seed(seed)
+    offs = [lead]
+    for c in counts:
+        offs.append(offs[-1] + c + lead)
+    x = torch.randn(offs[-1], K, generator=g) * torch.exp2(torch.randint(-10, 11, (offs[-1], K), generator=g).float())
+    wq = torch.randint(0, 256, (len(counts), N, K // 2), generator=g, dtype=torch.uint8)
+    ws = torch.randint(110, 135, (len(counts), N, K // 32), generator=g, dtype=torch.uint8)
+    return x.bfloat16(), wq, ws, torch.tensor(offs, dtype=torch.int32), torch.tensor(counts, dtype=torch.int32)
+
+
+@pytest.mark.parametrize("counts,lead", [([1, 0, 17, 40], 0), ([32, 33, 5, 3], 3), ([96, 97, 1, 8], 8), ([7, 31, 9, 64], 5)])
+@pytest.mark.parametrize("N,K,rows", [(256, 128, 10), (136, 192, 100), (200, 2880, 10), (640, 448, 40)])
+def test_block_scaled_products(counts, lead, N, K, rows, monkeypatch):
+    """Tiles of 32 and of 96 tokens whose segments start and end inside an eight of rows, weight rows that end inside a tile, the last half step of K,
+    output rows that are not 16-byte aligned; a few CTAs walk all tiles."""
+    from batchgen_b200.ops import _ext, mxfp4
+    x, wq, ws, off, cnt = _block_case(counts, lead, N, K, N + K + lead)
+    E = len(counts)
+    monkeypatch.setattr(_ext, "num_sms", lambda device=None: 3)
+    out = torch.full((x.shape[0] * (N + 8) + 1,), 7.0, dtype=torch.bfloat16, device="cuda")[1:].view(-1, N + 8)
+    mxfp4._block_gemm(x.cuda(), wq.cuda().view(E * N, -1), ws.cuda().view(E * N, -1), out, off.cuda(), E, x.shape[0], N, K, cnt.cuda(), rows)
+    _ext.check_status()
+    w, got, seen = mxfp4.dequantize(wq, ws, torch.float32).double(), out.cpu().double(), torch.zeros(x.shape[0], dtype=torch.bool)
+    for e, c in enumerate(counts):
+        a = int(off[e])
+        xe = x[a:a + c].double()
+        want, mag = xe @ w[e].t(), xe.abs() @ w[e].abs().t()
+        # what the parts leave out: 2^-22 of the largest of 32 elements, for each of them
+        tops = xe.abs().view(c, K // 32, 32).amax(-1, keepdim=True).expand(c, K // 32, 32).reshape(c, K)
+        lost = 2.0 ** -22 * (tops @ w[e].abs().t())
+        assert ((got[a:a + c, :N] - want).abs() <= want.abs() * 2 ** -8 + mag * K * 2 ** -24 + lost).all(), e
+        seen[a:a + c] = True
+    assert (got[~seen] == 7).all() and (got[:, N:] == 7).all()
+
+
+@pytest.mark.parametrize("what", [float("inf"), float("-inf"), float("nan")])
+def test_block_scaled_products_not_finite(what):
+    """An infinity or NaN in a row: what the product of bf16 operands gives, and nothing in other rows."""
+    from batchgen_b200.ops import _ext, mxfp4
+    x, wq, ws, off, cnt = _block_case([5, 20], 0, 256, 192, 3)
+    x[2, 7] = what
+    x[9, [3, 190]] = torch.tensor([what, -what]).bfloat16()
+    x[12, 100] = what
+    x[12, 64] = 3e38
+    args = (x.cuda(), wq.cuda().view(512, -1), ws.cuda().view(512, -1))
+    new, old = (torch.empty(25, 256, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    mxfp4._block_gemm(*args, new, off.cuda(), 2, 25, 256, 192, cnt.cuda(), 10)
+    mxfp4._launch(mxfp4.EPI_STORE, *args, old, off.cuda(), 2, 25, 256, 192, cnt.cuda())
+    _ext.check_status()
+    odd = ~torch.isfinite(old)
+    assert odd[2].all() and odd[9].all() and odd[12].all() and not odd[[0, 1, 3, 8, 10, 24]].any()
+    assert torch.equal(new[odd].nan_to_num(nan=1.0, posinf=2.0, neginf=3.0), old[odd].nan_to_num(nan=1.0, posinf=2.0, neginf=3.0))
+    assert torch.isfinite(new[~odd]).all()
+
+
+@pytest.mark.parametrize("kind", ["swiglu_clamped", "silu", "silu_limit"])
+def test_gated_parts(kind):
+    """The activation's rows as parts are the rows: every element but the ones far below their block's largest."""
+    from batchgen_b200.ops import _ext, moe, mxfp4
+    g = torch.Generator().manual_seed(1)
+    z = (torch.randn(37, 2 * 2880, generator=g) * 3).bfloat16().cuda()
+    src = torch.arange(37, dtype=torch.int32).cuda()
+    src[5] = -1
+    off = torch.tensor([0, 30], dtype=torch.int32).cuda()
+    want = moe.activation(z, kind, 2.0, off, src).cpu().double()
+    p = mxfp4.gated_parts(z, *moe._activation_kind(kind, 2.0), off, src)
+    _ext.check_status()
+    parts = p.p.view(torch.float8_e4m3fn).cpu().double().transpose(1, 2).reshape(-1, 2, 2880)
+    scale = torch.exp2(p.s.cpu().double().permute(1, 0, 2).reshape(37, -1)[:, :90] - 127).repeat_interleave(32, 1)
+    rows = [r for r in range(30) if r != 5]
+    got = scale[rows] * (parts[rows, 0] + parts[rows, 1] / 32)
+    top = want[rows].abs().view(-1, 90, 32).amax(-1).repeat_interleave(32, 1)
+    assert ((got - want[rows]).abs() <= top * 2.0 ** -22).all() and (got == want[rows])[want[rows].abs() > top * 2.0 ** -13].all()
