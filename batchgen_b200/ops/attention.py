@@ -176,14 +176,14 @@ def gqa_decode(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, 
 
 
 def mha_prefill_work(cu_seqlens: Sequence[int], ctx_lens: Sequence[int], k_starts: Sequence[int]) -> torch.Tensor:
-    """Work list of the expanded-prefill kernel: one row (q_row0, n_q, k_row0, kv0) per 128-query tile; query i
+    """Work list of the expanded-prefill kernel: one row (q_row0, n_q, k_row0, kv0) per 256-query tile; query i
     of a tile sees the first kv0 + i keys of its sequence, whose key rows start at ``k_starts[seq]``.  Longest
     key ranges first."""
     rows = []
     for i in range(len(cu_seqlens) - 1):
         a, b = int(cu_seqlens[i]), int(cu_seqlens[i + 1])
-        for q0 in range(a, b, 128):
-            rows.append((q0, min(128, b - q0), int(k_starts[i]), int(ctx_lens[i]) + (q0 - a) + 1))
+        for q0 in range(a, b, 256):
+            rows.append((q0, min(256, b - q0), int(k_starts[i]), int(ctx_lens[i]) + (q0 - a) + 1))
     rows.sort(key=lambda r: -(r[3] + r[1]))
     return torch.tensor(rows, dtype=torch.int32).view(-1, 4)
 

@@ -5,17 +5,22 @@
 // values).  This kernel is the flash-attention forward for that shape:
 //
 //   S[q, k] = Q[q, 0:192] . K[k, 0:192]          (M = 128 queries, N = 64 keys; both K-major via TMA)
-//   O[q, :] += P[q, k] . V[k, 0:128]             (M = 128, N = 128; V read N-major, P written by the softmax
-//                                                 threads as a swizzled K-major tile)
+//   O[q, :] += P[q, k] . V[k, 0:128]             (M = 128, N = 128; V read N-major, P from TMEM)
 //
-// One CTA = one (128-query tile, head).  Query row i of the tile sees the first kv0 + i keys of its
-// sequence's key range, which covers causal masking, cached context (kv0 > 1 for the first query) and the
-// boundary to the next sequence in the packed batch with a single comparison.  A thread owns a query row
-// (TMEM lane), so the online softmax needs no cross-thread reduction; the accumulator is rescaled only when
-// the running maximum grew by more than 2^8.  K/V tiles flow through a 3-stage TMA ring; S of tile t+1 is
-// issued before P.V of tile t.
+// One CTA = one (256-query tile, head): two halves of 128 queries with softmax warps of their own, so that the tensor cores work for one half
+// while the other's softmax runs, and each key / value tile is loaded once for both.  Query row i of the tile sees the first kv0 + i
+// keys of its sequence's key range, which covers causal masking, cached context (kv0 > 1 for the first query) and the boundary to
+// the next sequence in the packed batch with a single comparison.  A thread owns a query row (TMEM lane), so the online softmax
+// needs no cross-thread reduction; the accumulator is rescaled only when the running maximum grew by more than 2^8.  P goes back over
+// S in TMEM (two bf16 to a column) as the A operand of P.V.  K/V tiles flow through a 3-stage TMA ring; S of tile t+1 is issued before P.V of
+// tile t.
 //
-// Roles (192 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 2..5 softmax / epilogue.
+// With one 128-query tile a CTA and P through shared memory, the product of S, the softmax and P.V took turns.  One softmax warp's exponentials
+// take 512 of the tensor cores' 640 clocks for 128 queries x 64 keys.  128 heads: prompts of 2,048, 1,461, 874 and 1,000 tokens 654 -> 408 us
+// (813 TFLOP/s), 1,536 tokens behind 5,000 1,023 -> 654 (1,110); 32 heads, 4,096 tokens 293 -> 195.  What is left is each CTA's start and end,
+// some 4 us a tile, and the diagonal.
+//
+// Roles (384 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 4..7 and 8..11 softmax / epilogue of a half.
 // All waits are bounded (common.cuh).
 //
 // Replaces (by behaviour): FA2/FA3 varlen prefill as dispatched by batchgen/attention/varlen_dispatch.py and
@@ -29,16 +34,16 @@ constexpr int kDqk = 192, kDv = 128;
 constexpr int kKvRow = 256;                      // per head in the kv_b projection output: 128 key-nope dims | 128 value dims
 constexpr int BM = 128, BN = 64;
 constexpr int kStages = 3;
-constexpr int kThreads = 192;
-constexpr int kQBytes = 3 * BM * 128;            // 48 KB
+constexpr int kThreads = 384;
+constexpr int kQBytes = 3 * BM * 128;            // 48 KB, twice
 constexpr int kKBytes = 3 * BN * 128;            // 24 KB
 constexpr int kVBytes = 2 * BN * 128;            // 16 KB
-constexpr int kPBytes = BM * 128;                // 16 KB
-constexpr int kTmemCols = 256;                   // S: 2 x 64, O: 128
+constexpr int kTmemCols = 512;                   // each half: S (and P over it) 2 x 64, O 128
+constexpr int kHalfCols = 256;
 
 struct Work {
   int q_row0;    // first query row of the tile (rows of Q / out)
-  int n_q;       // queries in the tile (<= 128)
+  int n_q;       // queries in the tile (<= 256)
   int k_row0;    // first key row of the sequence (rows of K / V)
   int kv0;       // keys visible to query 0 of the tile (>= 1)
 };
@@ -47,9 +52,9 @@ struct Shared {
   uint64_t q_full;
   uint64_t kv_full[kStages];
   uint64_t kv_empty[kStages];
-  uint64_t s_full[2];
-  uint64_t p_full;
-  uint64_t o_done;
+  uint64_t s_full[2][2];     // [half][buffer]
+  uint64_t p_full[2];
+  uint64_t o_done[2];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -88,18 +93,6 @@ __device__ __forceinline__ float ex2(float x) {
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* v) {
   tmem_ld_32x32(taddr, *reinterpret_cast<uint32_t(*)[32]>(v));
 }
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* v) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, "
-      "%25, %26, %27, %28, %29, %30, %31, %32};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-      "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
-      "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
-      "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-      : "memory");
-}
-
 __global__ void __launch_bounds__(kThreads, 1)
 mha_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
                    const __grid_constant__ CUtensorMap tm_kpe, const Work* __restrict__ work,
@@ -107,23 +100,26 @@ mha_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* q_buf = smem;
-  uint8_t* k_buf = q_buf + kQBytes;
+  uint8_t* k_buf = q_buf + 2 * kQBytes;
   uint8_t* v_buf = k_buf + kStages * kKBytes;
-  uint8_t* p_buf = v_buf + kStages * kVBytes;
-  Shared& ss = *reinterpret_cast<Shared*>(p_buf + kPBytes);
+  Shared& ss = *reinterpret_cast<Shared*>(v_buf + kStages * kVBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* abort_flag = &ss.abort_flag;
   const Work w = work[blockIdx.x];
   const int h = blockIdx.y;
-  const int n_tiles = (w.kv0 + w.n_q - 1 + BN - 1) / BN;
+  // key tiles that a half sees: up to its last query's
+  const int tiles0 = (w.kv0 + min(w.n_q, BM) - 1 + BN - 1) / BN, tiles1 = w.n_q > BM ? (w.kv0 + w.n_q - 1 + BN - 1) / BN : 0;
+  const int n_tiles = max(tiles0, tiles1);
 
   if (threadIdx.x == 0) {
     mbar_init(&ss.q_full, 1);
     for (int s = 0; s < kStages; ++s) { mbar_init(&ss.kv_full[s], 1); mbar_init(&ss.kv_empty[s], 1); }
-    mbar_init(&ss.s_full[0], 1);
-    mbar_init(&ss.s_full[1], 1);
-    mbar_init(&ss.p_full, 128);
-    mbar_init(&ss.o_done, 1);
+    for (int x = 0; x < 2; ++x) {
+      mbar_init(&ss.s_full[x][0], 1);
+      mbar_init(&ss.s_full[x][1], 1);
+      mbar_init(&ss.p_full[x], 4);
+      mbar_init(&ss.o_done[x], 1);
+    }
     ss.abort_flag = 0;
     mbar_fence_init();
   }
@@ -139,8 +135,10 @@ mha_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      mbar_expect_tx(&ss.q_full, kQBytes);
-      for (int c = 0; c < 3; ++c) tma_load_2d(q_buf + c * BM * 128, &tm_q, &ss.q_full, h * kDqk + c * 64, w.q_row0);
+      mbar_expect_tx(&ss.q_full, tiles1 > 0 ? 2 * kQBytes : kQBytes);
+      for (int x = 0; x < (tiles1 > 0 ? 2 : 1); ++x)
+        for (int c = 0; c < 3; ++c)
+          tma_load_2d(q_buf + x * kQBytes + c * BM * 128, &tm_q, &ss.q_full, h * kDqk + c * 64, w.q_row0 + x * BM);
       bool ok = true;
       for (int t = 0; t < n_tiles; ++t) {
         const int s = t % kStages;
@@ -165,113 +163,125 @@ mha_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (elect_one()) {
       constexpr uint32_t idesc_s = idesc_bf16(BM, BN, 0);
       constexpr uint32_t idesc_pv = idesc_bf16(BM, kDv, 1);
-      const uint32_t tm_o = tmem_base + 2 * BN;
       bool ok = mbar_wait(&ss.q_full, 0, abort_flag, kTimeoutMma);
-      auto issue_s = [&](int t) -> bool {
-        const int s = t % kStages;
-        if (!mbar_wait(&ss.kv_full[s], (t / kStages) & 1, abort_flag, kTimeoutMma)) return false;
+      auto keys = [&](int t) { return mbar_wait(&ss.kv_full[t % kStages], (t / kStages) & 1, abort_flag, kTimeoutMma); };
+      auto issue_s = [&](int x, int t) {
         tc_fence_after();
-        const uint32_t tm_s = tmem_base + (t & 1) * BN;
+        const int s = t % kStages;
+        const uint32_t tm_s = tmem_base + x * kHalfCols + (t & 1) * BN;
         for (int c = 0; c < 3; ++c) {
-          const uint64_t adesc = make_smem_desc_sw128(smem_u32(q_buf + c * BM * 128));
+          const uint64_t adesc = make_smem_desc_sw128(smem_u32(q_buf + x * kQBytes + c * BM * 128));
           const uint64_t bdesc = make_smem_desc_sw128(smem_u32(k_buf + s * kKBytes + c * BN * 128));
 #pragma unroll
           for (int k = 0; k < 4; ++k) mma_f16(tm_s, adesc + 2 * k, bdesc + 2 * k, idesc_s, (c | k) ? 1u : 0u);
         }
-        tc_commit(&ss.s_full[t & 1]);
-        return true;
+        tc_commit(&ss.s_full[x][t & 1]);
       };
-      if (ok && n_tiles > 0) ok = issue_s(0);
+      ok = ok && keys(0);
+      if (ok) issue_s(0, 0);
+      if (ok && tiles1 > 0) issue_s(1, 0);
       for (int t = 0; ok && t < n_tiles; ++t) {
-        bool next_issued = true;
-        if (t + 1 < n_tiles) {
-          next_issued = mbar_probe(&ss.kv_full[(t + 1) % kStages], ((t + 1) / kStages) & 1);
-          if (next_issued && !issue_s(t + 1)) { ok = false; break; }
-        }
-        if (!mbar_wait(&ss.p_full, t & 1, abort_flag, kTimeoutMma)) { ok = false; break; }
-        tc_fence_after();
+        // S of a half's next tile before its P.V of this one, unless the keys are still on their way
+        const bool ready = t + 1 < n_tiles && mbar_probe(&ss.kv_full[(t + 1) % kStages], ((t + 1) / kStages) & 1);
         const int s = t % kStages;
-        const uint64_t pdesc = make_smem_desc_sw128(smem_u32(p_buf));
         const uint32_t v_base = smem_u32(v_buf + s * kVBytes);
+        for (int x = 0; ok && x < 2; ++x) {
+          const int mine = x ? tiles1 : tiles0;
+          if (t >= mine) continue;
+          if (ready && t + 1 < mine) issue_s(x, t + 1);
+          if (!mbar_wait(&ss.p_full[x], t & 1, abort_flag, kTimeoutMma)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t tm_p = tmem_base + x * kHalfCols + (t & 1) * BN, tm_o = tmem_base + x * kHalfCols + 2 * BN;
 #pragma unroll
-        for (int j = 0; j < BN / 16; ++j)
-          mma_f16(tm_o, pdesc + 2 * j, desc_mn_sw128(v_base + j * 2048, BN * 128, 1024), idesc_pv, (t > 0 || j > 0) ? 1u : 0u);
+          for (int j = 0; j < BN / 16; ++j)
+            mma_f16_ta(tm_o, tm_p + 8 * j, desc_mn_sw128(v_base + j * 2048, BN * 128, 1024), idesc_pv, (t > 0 || j > 0) ? 1u : 0u);
+          tc_commit(&ss.o_done[x]);
+        }
+        if (!ok) break;
         tc_commit(&ss.kv_empty[s]);
-        tc_commit(&ss.o_done);
-        if (!next_issued && !issue_s(t + 1)) { ok = false; break; }
+        if (!ready && t + 1 < n_tiles) {
+          ok = keys(t + 1);
+          for (int x = 0; ok && x < 2; ++x)
+            if (t + 1 < (x ? tiles1 : tiles0)) issue_s(x, t + 1);
+        }
       }
     }
-  } else {
-    // ------------------------------------------------------------ softmax / correction / epilogue: thread = query row
-    const int quad = warp & 3;
-    const int r = quad * 32 + lane;
-    const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t tm_o = tmem_base + 2 * BN + lane_addr;
-    const int visible = (r < w.n_q) ? (w.kv0 + r) : 0;       // keys this row may see
+  } else if (warp >= 4) {
+    // ------------------------------------------------------------ softmax / correction / epilogue of a half: thread = query row
+    const int quad = warp & 3, x = (warp - 4) >> 2, mine = x ? tiles1 : tiles0;
+    const int r = x * BM + quad * 32 + lane;
+    const uint32_t base = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + x * kHalfCols, tm_o = base + 2 * BN;
+    const int visible = w.kv0 + r, all_see = w.kv0 + x * BM + quad * 32;      // keys this row may see, keys every row of the warp may see
     float m_run = -INFINITY, l_run = 0.f;
-    uint8_t* prow = p_buf + (r >> 3) * 1024 + (r & 7) * 128;
     bool ok = true;
-    for (int t = 0; ok && t < n_tiles; ++t) {
-      if (vote_any_128(!mbar_wait(&ss.s_full[t & 1], (t >> 1) & 1, abort_flag, kTimeoutEpilogue))) { ok = false; break; }
+    for (int t = 0; ok && t < mine; ++t) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&ss.s_full[x][t & 1], (t >> 1) & 1, abort_flag, kTimeoutEpilogue))) { ok = false; break; }
       tc_fence_after();
+      const uint32_t tm_s = base + (t & 1) * BN;
       uint32_t sv[64];
-      tmem_ld32(tmem_base + lane_addr + (t & 1) * BN, sv);
-      tmem_ld32(tmem_base + lane_addr + (t & 1) * BN + 32, sv + 32);
+      tmem_ld32(tm_s, sv);
+      tmem_ld32(tm_s + 32, sv + 32);
       tmem_ld_wait();
-      const int n_ok = min(max(visible - t * BN, 0), BN);
-      float mt = -INFINITY;
+      if (all_see < (t + 1) * BN) {
+        const int n_ok = visible - t * BN;
 #pragma unroll
-      for (int j = 0; j < 64; ++j) {
-        const float v = (j < n_ok) ? __uint_as_float(sv[j]) * scale_log2 : -INFINITY;
-        sv[j] = __float_as_uint(v);
-        mt = fmaxf(mt, v);
+        for (int j = 0; j < 64; ++j)
+          if (j >= n_ok) sv[j] = 0xFF800000u;
       }
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int j = 0; j < 64; j += 2) {
+        const float2 v = __fmul2_rn(make_float2(__uint_as_float(sv[j]), __uint_as_float(sv[j + 1])), make_float2(scale_log2, scale_log2));
+        sv[j] = __float_as_uint(v.x);
+        sv[j + 1] = __float_as_uint(v.y);
+        mx[j & 2] = fmaxf(mx[j & 2], v.x);
+        mx[(j & 2) + 1] = fmaxf(mx[(j & 2) + 1], v.y);
+      }
+      const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       const bool grow = mt > m_run + 8.f;
       const float m_new = grow ? mt : m_run;
       const float alpha = (grow && m_run != -INFINITY) ? ex2(m_run - m_new) : 1.f;
-      if (t > 0 && vote_any_128(!mbar_wait(&ss.o_done, (t - 1) & 1, abort_flag, kTimeoutEpilogue))) { ok = false; break; }
-      tc_fence_after();
       if (t > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+        // P.V of the tile before this one (that of earlier ones was complete when S of this tile was)
+        if (!__all_sync(0xffffffffu, mbar_wait(&ss.o_done[x], (t - 1) & 1, abort_flag, kTimeoutEpilogue))) { ok = false; break; }
+        tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
           uint32_t ov[32];
-          tmem_ld32(tm_o + c * 32, ov);
+          tmem_ld_32x32(tm_o + c * 32, ov);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 32; ++j) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * alpha);
-          tmem_st32(tm_o + c * 32, ov);
+          tmem_st_32x32(tm_o + c * 32, ov);
         }
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       }
       float lsum = 0.f;
       const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
+      uint32_t pk[32];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        __align__(16) __nv_bfloat162 o[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float p0 = ex2(__uint_as_float(sv[c * 8 + 2 * q]) + neg_m);
-          const float p1 = ex2(__uint_as_float(sv[c * 8 + 2 * q + 1]) + neg_m);
-          o[q] = __floats2bfloat162_rn(p0, p1);
-          lsum += __low2float(o[q]) + __high2float(o[q]);
-        }
-        *reinterpret_cast<uint4*>(prow + ((c ^ (r & 7)) << 4)) = *reinterpret_cast<const uint4*>(o);
+      for (int j = 0; j < 32; ++j) {
+        const float2 e = __fadd2_rn(make_float2(__uint_as_float(sv[2 * j]), __uint_as_float(sv[2 * j + 1])), make_float2(neg_m, neg_m));
+        const __nv_bfloat162 o = __floats2bfloat162_rn(ex2(e.x), ex2(e.y));
+        pk[j] = *reinterpret_cast<const uint32_t*>(&o);
+        lsum += __uint_as_float(pk[j] << 16) + __uint_as_float(pk[j] & 0xffff0000u);
       }
+      tmem_st_32x32(tm_s, pk);
+      tmem_st_wait();
       l_run = l_run * alpha + lsum;
       m_run = m_new;
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       tc_fence_before();
-      mbar_arrive(&ss.p_full);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ss.p_full[x]);
     }
-    if (ok && n_tiles > 0) ok = !vote_any_128(!mbar_wait(&ss.o_done, (n_tiles - 1) & 1, abort_flag, kTimeoutEpilogue));
-    if (ok) {
+    if (ok && mine > 0) ok = __all_sync(0xffffffffu, mbar_wait(&ss.o_done[x], (mine - 1) & 1, abort_flag, kTimeoutEpilogue));
+    if (ok && mine > 0) {
       tc_fence_after();
       const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
       __nv_bfloat16* orow = out + ((size_t)(w.q_row0 + r) * H + h) * kDv;
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
         uint32_t ov[32];
-        tmem_ld32(tm_o + c * 32, ov);
+        tmem_ld_32x32(tm_o + c * 32, ov);
         tmem_ld_wait();
         if (r < w.n_q) {
 #pragma unroll
@@ -339,7 +349,7 @@ int bg_mha_prefill(const void* q, const void* kv, const void* kpe, long long kpe
   if (make_map(&tk, kv, (uint64_t)H * kKvRow, (uint64_t)Tk, (uint64_t)H * kKvRow, BN) != 0) return -11;
   if (make_map(&tv, kpe, 64, (uint64_t)Tk, (uint64_t)kpe_stride, BN) != 0) return -12;
   static bg::DeviceOnce attr_set;
-  const size_t smem = kQBytes + kStages * (kKBytes + kVBytes) + kPBytes + sizeof(Shared) + 1024;
+  const size_t smem = 2 * kQBytes + kStages * (kKBytes + kVBytes) + sizeof(Shared) + 1024;
   if (!bg::ensure_dynamic_smem(mha_prefill_kernel, smem, attr_set)) return -13;
   dim3 grid(n_work, H);
   mha_prefill_kernel<<<grid, kThreads, smem, stream>>>(tq, tk, tv, reinterpret_cast<const Work*>(work),

@@ -24,38 +24,11 @@ __device__ __forceinline__ uint32_t leader_addr(const void* p) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(out) : "r"(smem_u32(p)));
   return out;
 }
+// Arrive on a barrier in either CTA.  What the barriers of a pair hand over is TMEM (ordered by the tcgen05 fences) and tiles that the asynchronous
+// proxy writes and reads, nothing of this thread's own stores: release and acquire at cluster scope would only cost their fence, some
+// thousand clocks in every K block of the FP8 product.
 __device__ __forceinline__ void arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool try_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// mbar_wait for a barrier of this CTA on which the other CTA's threads, loads or products arrive too
-__device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int why) {
-  uint64_t t0 = 0;
-  for (uint32_t i = 0;; ++i) {
-    if (try_wait_cluster(bar, parity)) return true;
-    if ((i & 255u) == 255u) {
-      if (*abort_flag) return false;
-      if ((i & 0xFFFFu) == 0xFFFFu) {
-        const uint64_t t = global_timer_ns();
-        if (t0 == 0) t0 = t;
-        else if (t - t0 > kWaitBudgetNs) break;
-      }
-    }
-  }
-  if (*abort_flag == 0) *abort_flag = why;
-  return false;
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 // a tile load into this CTA whose bytes count on the barrier at shared::cluster address `bar`, in either CTA
@@ -113,14 +86,23 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&b);
 }
+// eight outputs of a row, `left` of them at most, in one piece where `wide` (rows on 16-byte boundaries)
+__device__ __forceinline__ void store_8(__nv_bfloat16* dst, const uint32_t (&w)[4], int left, bool wide) {
+  if (wide && left >= 8) {
+    *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (i < left) reinterpret_cast<uint16_t*>(dst)[i] = static_cast<uint16_t>(w[i / 2] >> (16 * (i & 1)));
+  }
+}
 __device__ __forceinline__ uint32_t transpose_8x8(uint32_t a) {
   uint32_t d;
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
   return d;
 }
 // 32 outputs x 8 tokens of a warp, x[b] the outputs 8 b + t / 4 of tokens 2 (t % 4) and the next: thread t stores the outputs 8 (t % 4) .. of
-// token t / 4 at row[0 .. 8), `left` of them at most (row: the thread's token, its first output; null: token not present), in one piece where
-// `wide` (rows on 16-byte boundaries)
+// token t / 4 at row[0 .. 8) as store_8 does (row: the thread's token, its first output; null: token not present)
 __device__ __forceinline__ void store_32x8(const uint32_t (&x)[4], __nv_bfloat16* row, int left, bool wide) {
   const bool e = threadIdx.x & 1, f = threadIdx.x & 2;
   uint32_t m[4];
@@ -134,14 +116,8 @@ __device__ __forceinline__ void store_32x8(const uint32_t (&x)[4], __nv_bfloat16
   const uint32_t x0 = e ? k1 : k0, x1 = e ? k0 : k1, y0 = e ? t1 : t0, y1 = e ? t0 : t1;
   const uint4 o = f ? make_uint4(y0, y1, x0, x1) : make_uint4(x0, x1, y0, y1);
   if (row == nullptr) return;
-  if (wide && left >= 8) {
-    *reinterpret_cast<uint4*>(row) = o;
-  } else {
-    const uint32_t w[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (i < left) reinterpret_cast<uint16_t*>(row)[i] = static_cast<uint16_t>(w[i / 2] >> (16 * (i & 1)));
-  }
+  const uint32_t w[4] = {o.x, o.y, o.z, o.w};
+  store_8(row, w, left, wide);
 }
 
 }  // namespace pair

@@ -86,6 +86,31 @@ def test_expanded_mla_prefill_attention(H):
     assert _rel(got, want) < 1.5e-2
 
 
+@pytest.mark.parametrize("lens,ctx", [([1, 128, 129, 64], [0, 0, 63, 1]), ([256, 257, 65], [64, 500, 0]), ([600], [191])])
+def test_expanded_mla_prefill_halves(lens, ctx):
+    """Tiles whose second half is missing, a single query or whole; queries whose keys end at, before and behind a key tile."""
+    from batchgen_b200.ops import _ext, attention
+    H, g = 3, torch.Generator().manual_seed(len(lens))
+    cu, k_starts, tk = [0], [], 0
+    for n, c in zip(lens, ctx):
+        cu.append(cu[-1] + n)
+        k_starts.append(tk)
+        tk += n + c
+    q, kv, kpe = (torch.randn(*shape, generator=g).to(torch.bfloat16) for shape in ((cu[-1], H, 192), (tk, H, 256), (tk, 64)))
+    work = attention.mha_prefill_work(cu, ctx, k_starts)
+    got = attention.mha_prefill(q.cuda(), kv.cuda(), kpe.cuda(), work, 0.1).cpu().double()
+    _ext.check_status()
+    for i, (n, c) in enumerate(zip(lens, ctx)):
+        a, k0 = cu[i], k_starts[i]
+        k = torch.cat([kv[k0:k0 + n + c, :, :128], kpe[k0:k0 + n + c, None].expand(-1, H, -1)], -1).double()
+        s = torch.einsum("nhd,lhd->nhl", q[a:a + n].double(), k) * 0.1
+        s.masked_fill_((torch.arange(n + c) > torch.arange(n).view(-1, 1) + c).unsqueeze(1), -float("inf"))
+        p, v = s.softmax(-1), kv[k0:k0 + n + c, :, 128:].double()
+        # probabilities and output rounded to 8 bits, exponents of fp32 sums of 192 products
+        bound = torch.einsum("nhl,lhd->nhd", p, v.abs()) * 2.0 ** -7 + 1e-6
+        assert ((got[a:a + n] - torch.einsum("nhl,lhd->nhd", p, v)).abs() <= bound).all(), i
+
+
 def test_model_prefill_uses_expanded_attention_and_matches_cpu():
     from batchgen_b200.config import get_model_config
     from batchgen_b200.models import build_model
