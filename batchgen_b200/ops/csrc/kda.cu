@@ -46,6 +46,7 @@ struct Params {
   int H;
   float scale, eps;
   int most;                  // sequences of more tokens are left to the chunk form
+  int whole;                 // rows of qkv and f in 16-byte pieces
 };
 
 __device__ __forceinline__ float silu(float x) { return x / (1.f + __expf(-x)); }
@@ -195,26 +196,28 @@ __global__ void __launch_bounds__(2 * D, 2) kda_seq_kernel(const Params p) {
 }
 
 // ---------------------------------------------------------------- prompts in chunk form
-// The recurrence of 64 tokens at a time, all in fp32.  With G the running sum of the log decay inside the chunk, M[i, j] =
+// The recurrence of 64 tokens at a time, all as precise as in fp32.  With G the running sum of the log decay inside the chunk, M[i, j] =
 // sum_c k_i k_j exp(G_i - G_j) for j < i and P the same of q_i and k_j for j <= i, the writes are U = T (V - (K exp(G)) S) with
 // T = (I + diag(b) M)^-1 diag(b), so that with W = T (K exp(G)), UV = T V, Q' = Q exp(G) - P W and O0 = P UV
 //
 //   U = UV - W S,   O = O0 + Q' S,   S <- exp(G_last) S + (K exp(G_last - G))^T U
 //
 // `chunk_prepare` makes W, Q', Kd = K exp(G_last - G), UV and O0 of every (chunk, head) at once, from the raw projections; `chunk_chain`
-// walks the chunks of a (sequence, head, 32 value columns) with S in shared memory; `chunk_finish` norms and gates whole heads.  Every
+// walks the chunks of a (sequence, head, 64 value columns) on the tensor cores with S in registers; `chunk_finish` norms and gates whole heads.  Every
 // exponent is a sum of the log decays of its own range of tokens, at most zero, and never a difference of running sums: behind a strong
 // decay a difference would carry that decay's rounding into the weak ones after it (tokens of 2^-400 and of 2^-0.001 in turn: states off
 // by 1.3e-5 with differences, 1.2e-7 so, 1.4e-7 token by token).  Products of different 16-token blocks meet at the border before the
 // later one.
 //
-// The token-by-token kernel runs a barrier chain of some 2 us a token with a CTA per head.  Here the chain's limit is what shared memory
-// delivers to the fp32 FMAs (86 % of its rate), of which a token and head has about 75,000, two thirds of them in the chain; prepare waits at its
-// short steps' barriers (shared memory 53 %, issue slots 42 %).  One prompt of 4,096 tokens, 32 heads: 8,086 -> 1,226
-// us a layer (prepare 605, chain 466, finish 42); with two thirds of the warps and a column-by-column inverse prepare took 833.
-constexpr int kChunk = 64, kSub = 16, kPad = 132, kCols = 32;      // kPad: rows of 128 floats that start 4 banks apart
-constexpr int kPart = kChunk * 128;                                // floats of one [64, 128] result
-constexpr int kItemFloats = 5 * kPart;                             // W | Q' | Kd | UV | O of a (chunk, head)
+// The token-by-token kernel runs a barrier chain of some 2 us a token with a CTA per head.  One prompt of 4,096 tokens, 32 heads: 8,024 us a layer
+// so, 913 in chunks (prepare 558, chain 328, finish 42); eight prompts of 300 to 1,024 tokens 1,014 (757, 224, 48).  With the chain in fp32
+// FMAs, which shared memory fed at 86 % of its rate, 478 and 573 us of it; with a thread walking the whole chunk for one channel of one input,
+// straight from global memory, prepare took 615 and 817, a third of that waiting for loads behind stores and branches.  Prepare has
+// one CTA an SM and short steps, each waiting for the one before: inputs 6,100 clocks, convolutions and decays 12,400, the diagonal
+// blocks of M and P 11,300, the others 18,200, the inverse 9,500, the products with P and T 12,700.
+constexpr int kChunk = 64, kSub = 16, kPad = 132;      // kPad: rows of 128 floats that start 4 banks apart
+constexpr int kPart = kChunk * 128;                                // elements of one [64, 128] result
+constexpr int kPartRows = 9 * kChunk;                              // of a (chunk, head): three bf16 parts of [W; Q'] (128 rows), then three of Kd
 constexpr int kAStride = 68;
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -226,15 +229,78 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// x / d for d from 1 to 2^60 and |x| at most as large: an approximate reciprocal and one correction by the residual (Markstein 1990), which rounds
+// like the division or to the number beside it at a third of its instructions
+__device__ __forceinline__ float quotient(float x, float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float q = x * r;
+  return fmaf(fmaf(-q, d, x), r, q);
+}
+__device__ __forceinline__ float silu_fast(float x) {
+  const float d = 1.f + __expf(-x);
+  float y = quotient(x, d);
+  if (!(fabsf(x) < 40.f)) y = x / d;          // d may be infinite, x may not be finite
+  return y;
+}
+// log(1 + e^x) = max(x, 0) + log(1 + e^-|x|), the logarithm as 2 artanh(s) with s = e / (2 + e) <= 1 / 3, whose series ends below 2^-26 of it with s^16;
+// e^-|x| is at most one and keeps its relative precision, which e^x loses towards 20
+__device__ __forceinline__ float softplus_series(float x) {
+  const float e = __expf(-fabsf(x)), s = quotient(e, 2.f + e), s2 = s * s;
+  float a = 2.f / 17.f;
+  a = fmaf(a, s2, 2.f / 15.f);
+  a = fmaf(a, s2, 2.f / 13.f);
+  a = fmaf(a, s2, 2.f / 11.f);
+  a = fmaf(a, s2, 2.f / 9.f);
+  a = fmaf(a, s2, 2.f / 7.f);
+  a = fmaf(a, s2, 2.f / 5.f);
+  a = fmaf(a, s2, 2.f / 3.f);
+  return fmaxf(x, 0.f) + fmaf(a * s2, s, 2.f * s);
+}
 __device__ __forceinline__ float2 twice(float x) { return make_float2(x, x); }
+// four neighbours as parts, rows of 128, `step` elements from part to part
+__device__ __forceinline__ void store_parts(__nv_bfloat16* dst, size_t step, float4 x) {
+  float2 a = make_float2(x.x, x.y), b = make_float2(x.z, x.w);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    *reinterpret_cast<uint2*>(dst + i * step) = i < 2 ? make_uint2(cut_bf16x2(a), cut_bf16x2(b)) : make_uint2(last_bf16x2(a), last_bf16x2(b));
+}
 
 constexpr int kPrepThreads = 512;
 constexpr int kBlocks = kChunk / kSub;
+constexpr int kRawRows = kChunk + 3;
 constexpr int kPrepareFloats = 4 * kChunk * kPad + (2 * kSub + 3 * kSub) * kPad + 2 * kChunk * kAStride + kChunk + kBlocks * 128;
+static_assert(4 * kRawRows * 128 * 2 <= ((2 * kSub + 3 * kSub) * kPad + 2 * kChunk * kAStride) * 4, "raw inputs stand where block operands, M and P come");
+
+__device__ __forceinline__ void cp16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+// Block row A of M (first 256 threads) and P (the others) against the A blocks before it: a thread has a row and one column of each.  A is known to
+// the compiler, or each block's loads would wait behind a branch (4,400 to 5,400 clocks a block row).
+template <int A>
+__device__ __forceinline__ void against(const float* ke, const float* qe, const float* kd, float* am, float* pm) {
+  const int tid = threadIdx.x, i = tid & 15, jj = (tid >> 4) & 15;
+  const float* left = (tid < 256 ? ke : qe) + i * kPad;
+  float2 sum[A][2] = {};
+#pragma unroll 8
+  for (int c = 0; c < 128; c += 4) {
+    const float4 x = *reinterpret_cast<const float4*>(left + c);
+#pragma unroll
+    for (int b = 0; b < A; ++b) {
+      const float4 d = *reinterpret_cast<const float4*>(kd + (b * kSub + jj) * kPad + c);
+      sum[b][0] = __ffma2_rn(make_float2(x.x, x.y), make_float2(d.x, d.y), sum[b][0]);
+      sum[b][1] = __ffma2_rn(make_float2(x.z, x.w), make_float2(d.z, d.w), sum[b][1]);
+    }
+  }
+#pragma unroll
+  for (int b = 0; b < A; ++b)
+    (tid < 256 ? am : pm)[(A * kSub + i) * kAStride + b * kSub + jj] = (sum[b][0].x + sum[b][1].x) + (sum[b][0].y + sum[b][1].y);
+}
 
 // Sixteen warps, one CTA an SM: the steps are short and each waits for the one before, so more warps hide more of a step's latency.
 __global__ void __launch_bounds__(kPrepThreads, 1)
-chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __restrict__ res, float* __restrict__ g_last) {
+chunk_prepare(const Params p, const ChunkItem* __restrict__ items, __nv_bfloat16* __restrict__ parts, float* __restrict__ res, float* __restrict__ g_last) {
   constexpr int D = 128;
   extern __shared__ __align__(16) float sm[];
   float* kn = sm;                              // [64][kPad] each
@@ -248,61 +314,81 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
   float* pm = am + kChunk * kAStride;          // [64][kAStride] P
   float* bs = pm + kChunk * kAStride;          // [64]
   float* tot = bs + kChunk;                    // [kBlocks][128] log2 decay over a block
+  __nv_bfloat16* raw = reinterpret_cast<__nv_bfloat16*>(ke);      // [4][3 + 64][128] raw q, k, v and f, from three tokens ahead of the chunk; until they are used
   const ChunkItem it = items[blockIdx.x];
   const int h = blockIdx.y, H = p.H, HD = H * D;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // ---- inputs: all of the chunk's on their way at once
+  if (p.whole) {
+    for (int i = tid; i < 4 * kRawRows * 16; i += kPrepThreads) {
+      const int part = i / (kRawRows * 16), t = i / 16 % kRawRows - 3, c = i % 16 * 8;
+      if (t >= it.n || t < (part < 3 ? -min(it.before, 3) : 0)) continue;
+      const __nv_bfloat16* src = part < 3 ? p.qkv + (ptrdiff_t)(it.t0 + t) * p.qkv_stride + part * HD : p.f + (size_t)(it.t0 + t) * p.f_stride;
+      cp16(raw + (part * kRawRows + t + 3) * D + c, src + h * D + c);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  } else {
+    for (int i = tid; i < 4 * kRawRows * D; i += kPrepThreads) {
+      const int part = i / (kRawRows * D), t = i / D % kRawRows - 3, c = i % D;
+      if (t >= it.n || t < (part < 3 ? -min(it.before, 3) : 0)) continue;
+      const __nv_bfloat16* src = part < 3 ? p.qkv + (ptrdiff_t)(it.t0 + t) * p.qkv_stride + part * HD : p.f + (size_t)(it.t0 + t) * p.f_stride;
+      raw[(part * kRawRows + t + 3) * D + c] = src[h * D + c];
+    }
+  }
   const int slot = p.slots[it.seq];
-  if (slot < 0) return;
-  float* out = res + ((size_t)blockIdx.x * H + h) * kItemFloats;
+  if (slot < 0) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    return;
+  }
+  float* out = res + ((size_t)blockIdx.x * H + h) * 2 * kPart;                     // UV | O
+  __nv_bfloat16* wq_out = parts + ((size_t)blockIdx.x * H + h) * kPartRows * D;     // [3][128][128]
+  __nv_bfloat16* kd_out = wq_out + 3 * 2 * kPart;                                   // [3][64][128]
 
-  // ---- convolutions, SiLU, log decays: a thread walks the chunk for one channel of q, k, v or f
+  // ---- convolutions, SiLU, log decays: a thread has one channel of a block's sixteen tokens, of q, k, v and f in turn; all of them are read before the
+  // first is stored: a store or a branch would hold up the loads behind it
   {
-    const int part = tid >> 7, j = tid & 127, c = h * D + j, ch = part * HD + c;
+    const int j = tid & 127, c = h * D + j, b = (tid >> 7) * kSub;
     const bool init = p.has_initial == nullptr || p.has_initial[it.seq] != 0;
-    const __nv_bfloat16* src = part < 3 ? p.qkv + (size_t)it.t0 * p.qkv_stride + ch : p.f + (size_t)it.t0 * p.f_stride + c;
-    const int stride = part < 3 ? p.qkv_stride : p.f_stride;
-    float win[3] = {0.f, 0.f, 0.f}, tap[4] = {0.f, 0.f, 0.f, 0.f}, bias = 0.f;
-    if (part < 3) {
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {            // the inputs 3, 2, 1 tokens ahead of the chunk: earlier tokens of the step, else the state
-        const int back = 3 - i;
-        if (it.before >= back) win[i] = __bfloat162float(src[-(ptrdiff_t)back * stride]);
-        else if (init) win[i] = p.conv_state[((size_t)slot * 3 * HD + ch) * 3 + i + it.before];
-      }
-      const float4 w = *reinterpret_cast<const float4*>(p.conv_w + (size_t)ch * 4);
-      tap[0] = w.x; tap[1] = w.y; tap[2] = w.z; tap[3] = w.w;
-      bias = p.conv_b ? p.conv_b[ch] : 0.f;
-    }
+    const float beta = tid < min(it.n, kChunk) ? __bfloat162float(p.beta[(size_t)(it.t0 + tid) * p.beta_stride + h]) : 0.f;
     const float neg_a = -__expf(p.A_log[h]), dtb = p.dt_bias[c];
-    float* dst = (part == 0 ? qn : part == 1 ? kn : part == 2 ? vv : lg) + j;
-    __nv_bfloat16 x[2][16];
-    auto load = [&](int b, __nv_bfloat16 (&v)[16]) {
+    float tap[3][4], bias[3], ahead[3][3] = {};                      // ahead: the three inputs before the block where the step does not have them
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = src[(size_t)min(b + i, it.n - 1) * stride];
-    };
-    load(0, x[0]);
+    for (int part = 0; part < 3; ++part) {
+      const int ch = part * HD + c;
+      const float4 w = *reinterpret_cast<const float4*>(p.conv_w + (size_t)ch * 4);
+      tap[part][0] = w.x; tap[part][1] = w.y; tap[part][2] = w.z; tap[part][3] = w.w;
+      bias[part] = p.conv_b ? p.conv_b[ch] : 0.f;
 #pragma unroll
-    for (int b = 0; b < kChunk; b += 16) {
-      if (b + 16 < kChunk) load(b + 16, x[(b / 16 + 1) & 1]);
-      const __nv_bfloat16 (&v)[16] = x[(b / 16) & 1];
-      float run = 0.f;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const bool in = b + i < it.n;
-        const float xi = __bfloat162float(v[i]);
-        if (part < 3) {
-          const float y = silu(bias + tap[0] * win[0] + tap[1] * win[1] + tap[2] * win[2] + tap[3] * xi);
-          win[0] = win[1]; win[1] = win[2]; win[2] = xi;
-          dst[(b + i) * kPad] = in ? y : 0.f;
-        } else {
-          const float g = in ? neg_a * softplus(xi + dtb) * kLog2e : 0.f;
-          run += g;
-          dst[(b + i) * kPad] = g;
-        }
-      }
-      if (part == 3) tot[b / 16 * 128 + j] = run;
+      for (int i = 0; i < 3; ++i)
+        if (b == 0 && it.before < 3 - i && init) ahead[part][i] = p.conv_state[((size_t)slot * 3 * HD + ch) * 3 + i + it.before];
     }
-    if (tid < kChunk) bs[tid] = tid < it.n ? sigmoid(__bfloat162float(p.beta[(size_t)(it.t0 + tid) * p.beta_stride + h])) : 0.f;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int part = 0; part < 3; ++part) {
+      const __nv_bfloat16* src = raw + (part * kRawRows + b) * D + j;
+      float* dst = (part == 0 ? qn : part == 1 ? kn : vv) + b * kPad + j;
+      float x[19], y[16];
+#pragma unroll
+      for (int i = 0; i < 19; ++i) x[i] = i < 3 && b == 0 && it.before < 3 - i ? ahead[part][i] : __bfloat162float(src[i * D]);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) y[i] = silu_fast(bias[part] + tap[part][0] * x[i] + tap[part][1] * x[i + 1] + tap[part][2] * x[i + 2] + tap[part][3] * x[i + 3]);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) dst[i * kPad] = b + i < it.n ? y[i] : 0.f;
+    }
+    const __nv_bfloat16* src = raw + (3 * kRawRows + 3 + b) * D + j;
+    float x[16], run = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = __bfloat162float(src[i * D]);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      x[i] = b + i < it.n ? neg_a * softplus_series(x[i] + dtb) * kLog2e : 0.f;
+      run += x[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) lg[(b + i) * kPad + j] = x[i];
+    tot[b / kSub * 128 + j] = run;
+    if (tid < kChunk) bs[tid] = tid < it.n ? sigmoid(beta) : 0.f;
   }
   __syncthreads();
   // ---- unit q (times scale) and k, four tokens a warp
@@ -371,24 +457,9 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
       }
     }
     __syncthreads();
-    const int i = tid & 15, jj = (tid >> 4) & 15;
-    const float* left = (tid < 256 ? ke : qe) + i * kPad;
-    float2 sum[3][2] = {};
-#pragma unroll 4
-    for (int c = 0; c < D; c += 4) {
-      const float4 x = *reinterpret_cast<const float4*>(left + c);
-#pragma unroll
-      for (int b = 0; b < 3; ++b)
-        if (b < a) {
-          const float4 d = *reinterpret_cast<const float4*>(kd + (b * kSub + jj) * kPad + c);
-          sum[b][0] = __ffma2_rn(make_float2(x.x, x.y), make_float2(d.x, d.y), sum[b][0]);
-          sum[b][1] = __ffma2_rn(make_float2(x.z, x.w), make_float2(d.z, d.w), sum[b][1]);
-        }
-    }
-#pragma unroll
-    for (int b = 0; b < 3; ++b)
-      if (b < a)
-        (tid < 256 ? am : pm)[(a * kSub + i) * kAStride + b * kSub + jj] = (sum[b][0].x + sum[b][1].x) + (sum[b][0].y + sum[b][1].y);
+    if (a == 1) against<1>(ke, qe, kd, am, pm);
+    else if (a == 2) against<2>(ke, qe, kd, am, pm);
+    else against<3>(ke, qe, kd, am, pm);
   }
   __syncthreads();
   // ---- diagonal blocks of (I + diag(b) M)^-1: a thread of the first two warps solves for one column
@@ -417,9 +488,18 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
     for (int m = 0; m < blk; ++m) up += tot[m * 128 + ch];
     for (int m = blk + 1; m < kBlocks; ++m) down += tot[m * 128 + ch];
 #pragma unroll
-    for (int i = kSub - 1; i >= 0; --i) {
-      out[2 * kPart + (blk * kSub + i) * D + ch] = kn[walk + i * kPad] * ex2(down);
+    for (int i = kSub - 2; i >= 0; i -= 2) {                        // two tokens: neighbours swap one, so that a thread stores both channels of the other
+      const float y1 = kn[walk + (i + 1) * kPad] * ex2(down);
+      down += lg[walk + (i + 1) * kPad];
+      const float y0 = kn[walk + i * kPad] * ex2(down);
       down += lg[walk + i * kPad];
+      const bool odd = ch & 1;
+      const float other = __shfl_xor_sync(0xffffffffu, odd ? y0 : y1, 1);
+      float2 y = odd ? make_float2(other, y1) : make_float2(y0, other);
+      uint32_t* dst = reinterpret_cast<uint32_t*>(kd_out + (blk * kSub + i + odd) * D + (ch & ~1));
+      dst[0] = cut_bf16x2(y);
+      dst[kPart / 2] = cut_bf16x2(y);
+      dst[kPart] = last_bf16x2(y);
     }
     float e = 1.f;
 #pragma unroll
@@ -460,9 +540,11 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
     if (j <= i) am[i * kAStride + j] *= bs[j];
   }
   __syncthreads();
-  // ---- rows 8 g .. 8 g + 7 of a lower-triangular [64, 64] times a [64, 128], 4 columns a lane; a warp per (g, matrix)
-  const int grp = warp >> 1;
-  float* mat = (warp & 1 ? vv : ke) + lane * 4;
+  // ---- rows 8 g .. 8 g + 7 of a lower-triangular [64, 64] times a [64, 128], 4 columns a lane; a warp per (g, matrix), g and 7 - g on one
+  // scheduler, so that all four have the same work
+  const int grp = warp & 4 ? 7 - (warp & 3) : warp & 3;
+  const bool second = warp & 8;
+  float* mat = (second ? vv : ke) + lane * 4;
   auto product = [&](const float* tri, float2 (&x)[8][2]) {
 #pragma unroll
     for (int r = 0; r < 8; ++r) x[r][0] = x[r][1] = make_float2(0.f, 0.f);
@@ -502,7 +584,8 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
     const int row = grp * 8 + r;
     const float4 y = make_float4(x[r][0].x, x[r][0].y, x[r][1].x, x[r][1].y);
     *reinterpret_cast<float4*>(mat + row * kPad) = y;
-    *reinterpret_cast<float4*>(out + (warp & 1 ? 3 : 0) * kPart + row * D + lane * 4) = y;
+    if (second) *reinterpret_cast<float4*>(out + row * D + lane * 4) = y;
+    else store_parts(wq_out + row * D + lane * 4, 2 * kPart, y);
   }
   __syncthreads();
   product(pm, x);                               // P W, P UV
@@ -510,134 +593,238 @@ chunk_prepare(const Params p, const ChunkItem* __restrict__ items, float* __rest
   for (int r = 0; r < 8; ++r) {
     const int row = grp * 8 + r;
     float4 y = make_float4(x[r][0].x, x[r][0].y, x[r][1].x, x[r][1].y);
-    if (!(warp & 1)) {
+    if (!second) {
       const float4 q = *reinterpret_cast<const float4*>(qn + row * kPad + lane * 4);
-      y = make_float4(q.x - y.x, q.y - y.y, q.z - y.z, q.w - y.w);
+      store_parts(wq_out + kPart + row * D + lane * 4, 2 * kPart, make_float4(q.x - y.x, q.y - y.y, q.z - y.z, q.w - y.w));
+    } else {
+      *reinterpret_cast<float4*>(out + kPart + row * D + lane * 4) = y;
     }
-    *reinterpret_cast<float4*>(out + (warp & 1 ? 4 : 1) * kPart + row * D + lane * 4) = y;
   }
 }
 
-constexpr int kChainFloats = 2 * 128 * kPad + kChunk * 128 + kCols * kPad + kChunk * kCols * 2;
+// ---- the chain on the tensor cores, every fp32 operand as three bf16 parts that sum up to it (common.cuh), all nine products.  Those of the leading
+// parts have two accumulators, one for each half of the reduction, the small ones accumulators of their own, added in fp32: states are as near to 64
+// bits as with fp32 FMAs or nearer (model-like decays 1.6e-7 against 1.7e-7; with the six largest products and one accumulator for the
+// leading one 1.9e-7).
+constexpr int kCols = 64;                                          // value columns of a CTA
+constexpr int kChainThreads = 320;
+constexpr int kTile = 64 * 128;                                    // bytes of 64 rows of 64 elements
+constexpr int kWqBytes = 3 * 4 * kTile, kKdBytes = 3 * 2 * kTile, kSBytes = 3 * 2 * kTile, kUBytes = 3 * kTile;
 
-__device__ __forceinline__ void cp16(float* dst, const float* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+struct ChainShared {
+  uint64_t wq_full, wq_empty, kd_full, kd_empty, s_ready, u_ready, d1_done, d2_done;
+  uint32_t tmem_base;
+  int abort_flag;
+};
+constexpr int kChainBytes = kWqBytes + kKdBytes + kSBytes + kUBytes + sizeof(ChainShared) + 1024;
+
+// tiles whose rows of 64 columns lie behind each other, the reduction running over the rows (16 a step); the next 64 columns are `next` bytes on
+__device__ __forceinline__ uint64_t desc_over_rows(uint32_t addr, uint32_t next) {
+  return static_cast<uint64_t>((addr & 0x3FFFFu) >> 4) | static_cast<uint64_t>(next >> 4) << 16 | static_cast<uint64_t>(1024 >> 4) << 32 |
+         static_cast<uint64_t>(1) << 46 | static_cast<uint64_t>(2) << 61;
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr)
+      : "memory");
+}
+// 32 columns of one row as parts into [part][rows][64] tiles (swizzled as a TMA load would)
+__device__ __forceinline__ void put_parts(uint8_t* tiles, int part_bytes, int row, int half, const float (&x)[32]) {
+  uint8_t* r = tiles + row * 128;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t w[3][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float2 e = make_float2(x[8 * c + 2 * i], x[8 * c + 2 * i + 1]);
+      w[0][i] = cut_bf16x2(e);
+      w[1][i] = cut_bf16x2(e);
+      w[2][i] = last_bf16x2(e);
+    }
+#pragma unroll
+    for (int m = 0; m < 3; ++m) *reinterpret_cast<uint4*>(r + m * part_bytes + (((4 * half + c) ^ (row & 7)) << 4)) = make_uint4(w[m][0], w[m][1], w[m][2], w[m][3]);
+  }
 }
 
-// grid (value columns / 32, H, sequence pieces): walks a piece's chunks, S of 32 value columns in shared memory as [column][key].
-// W and Q' of the next chunk and Kd of this one arrive under the products.
-__global__ void __launch_bounds__(256, 1)
-chunk_chain(const Params p, const ChunkItem* __restrict__ items, const ChunkSeq* __restrict__ seqs, float* __restrict__ res,
-            const float* __restrict__ g_last) {
+// grid (value columns / 64, H, sequence pieces): walks a piece's chunks.  Warps 0..7: a thread holds 32 value columns of one key of S, takes
+// U or O of one token's columns from the first product and the update from the second; warp 8 loads, warp 9 issues.
+// Bound by the products (3,456 clocks a chunk) and four hand-overs between threads and tensor cores, one after the other.
+__global__ void __launch_bounds__(kChainThreads, 1)
+chunk_chain(const __grid_constant__ CUtensorMap map, const Params p, const ChunkItem* __restrict__ items, const ChunkSeq* __restrict__ seqs,
+            float* __restrict__ res, const float* __restrict__ g_last, int* status) {
   constexpr int D = 128;
-  extern __shared__ __align__(16) float sm[];
-  float* wq2 = sm;                              // two of [128][kPad]: rows of W, then of Q'
-  float* kd = wq2 + 2 * 128 * kPad;                  // [64][128]
-  float* st = kd + kChunk * 128;                // [32][kPad]
-  float2* u2 = reinterpret_cast<float2*>(st + kCols * kPad);       // [64][32] (u, u)
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* wq = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));      // [3][2 key halves][128 rows]
+  uint8_t* kd = wq + kWqBytes;                  // [3][2 key halves][64 tokens]
+  uint8_t* st = kd + kKdBytes;                  // [3][128 keys]
+  uint8_t* ut = st + kSBytes;                   // [3][64 tokens]
+  ChainShared& ss = *reinterpret_cast<ChainShared*>(ut + kUBytes);
   const ChunkSeq sq = seqs[blockIdx.z];
   const int h = blockIdx.y, H = p.H, c0 = blockIdx.x * kCols;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = p.slots[sq.seq];
   if (slot < 0) return;
-  const bool init = !sq.first || p.has_initial == nullptr || p.has_initial[sq.seq] != 0;
-  float* Sg = p.rec_state + ((size_t)slot * H + h) * D * D + c0;
-  auto item = [&](int c) { return res + ((size_t)(sq.item0 + c) * H + h) * kItemFloats; };
-  auto fetch_wq = [&](int c) {
-    float* wq = wq2 + (c & 1) * 128 * kPad;
-    if (c < sq.items)
-      for (int i = tid; i < 128 * 32; i += 256) cp16(wq + (i >> 5) * kPad + (i & 31) * 4, item(c) + i * 4);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  auto fetch_kd = [&](int c) {
-    if (c < sq.items)
-      for (int i = tid; i < kChunk * 32; i += 256) cp16(kd + i * 4, item(c) + 2 * kPart + i * 4);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  fetch_wq(0);
-  fetch_kd(0);
-  for (int i = tid; i < D * kCols; i += 256) st[(i % kCols) * kPad + i / kCols] = init ? Sg[(size_t)(i / kCols) * D + i % kCols] : 0.f;
-  // first phase: rows 16 w + rg + 4 q (q < 4) of [W; Q'], columns cg + 8 q
-  const int rg = lane >> 3, cg = lane & 7;
-  // second phase: keys k0 .. k0 + 7, columns e0, e0 + 1
-  const int k0 = (warp & 3) * 32 + (lane >> 3) * 8, e0 = (warp >> 2) * 16 + (lane & 7) * 2;
-  for (int c = 0; c < sq.items; ++c) {
-    float* it = item(c);
-    float* add = it + (warp < 4 ? 3 : 4) * kPart + c0;               // UV or O0
-    const int r0 = (warp & 3) * 16 + rg;
-    float base[4][4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) base[q][e] = add[(size_t)(r0 + 4 * q) * D + cg + 8 * e];
-    const float* gl = g_last + ((size_t)(sq.item0 + c) * H + h) * D + k0;
-    const float4 ga = *reinterpret_cast<const float4*>(gl), gb = *reinterpret_cast<const float4*>(gl + 4);
-    asm volatile("cp.async.wait_group 1;" ::: "memory");             // W and Q' of this chunk; Kd may be under way
-    __syncthreads();
-    fetch_wq(c + 1);                                                 // into the buffer of the chunk before
-    {
-      float2 acc[4][4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[q][e] = make_float2(0.f, 0.f);
-      const float* wr = wq2 + (c & 1) * 128 * kPad + (warp * 16 + rg) * kPad;
-      const float* sr = st + cg * kPad;
-#pragma unroll 4
-      for (int k = 0; k < D; k += 4) {
-        float4 s[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) s[e] = *reinterpret_cast<const float4*>(sr + 8 * e * kPad + k);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float4 w = *reinterpret_cast<const float4*>(wr + 4 * q * kPad + k);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            acc[q][e] = __ffma2_rn(make_float2(w.x, w.y), make_float2(s[e].x, s[e].y), acc[q][e]);
-            acc[q][e] = __ffma2_rn(make_float2(w.z, w.w), make_float2(s[e].z, s[e].w), acc[q][e]);
-          }
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float d = acc[q][e].x + acc[q][e].y;
-          if (warp < 4) u2[(r0 + 4 * q) * kCols + cg + 8 * e] = twice(base[q][e] - d);
-          else add[(size_t)(r0 + 4 * q) * D + cg + 8 * e] = base[q][e] + d;
-        }
-    }
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();                                                 // U and Kd are there, the old S is read
-    {
-      float2 acc[4][2];
-#pragma unroll
-      for (int m = 0; m < 4; ++m) acc[m][0] = acc[m][1] = make_float2(0.f, 0.f);
-#pragma unroll 8
-      for (int i = 0; i < kChunk; ++i) {
-        const float4 a = *reinterpret_cast<const float4*>(kd + i * 128 + k0), b = *reinterpret_cast<const float4*>(kd + i * 128 + k0 + 4);
-        const float4 u = *reinterpret_cast<const float4*>(u2 + i * kCols + e0);
-        const float2 ua = make_float2(u.x, u.y), ub = make_float2(u.z, u.w);
-        acc[0][0] = __ffma2_rn(make_float2(a.x, a.y), ua, acc[0][0]); acc[0][1] = __ffma2_rn(make_float2(a.x, a.y), ub, acc[0][1]);
-        acc[1][0] = __ffma2_rn(make_float2(a.z, a.w), ua, acc[1][0]); acc[1][1] = __ffma2_rn(make_float2(a.z, a.w), ub, acc[1][1]);
-        acc[2][0] = __ffma2_rn(make_float2(b.x, b.y), ua, acc[2][0]); acc[2][1] = __ffma2_rn(make_float2(b.x, b.y), ub, acc[2][1]);
-        acc[3][0] = __ffma2_rn(make_float2(b.z, b.w), ua, acc[3][0]); acc[3][1] = __ffma2_rn(make_float2(b.z, b.w), ub, acc[3][1]);
-      }
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        float* s = st + (e0 + e) * kPad + k0;
-        float4 a = *reinterpret_cast<const float4*>(s), b = *reinterpret_cast<const float4*>(s + 4);
-        *reinterpret_cast<float4*>(s) = make_float4(fmaf(ga.x, a.x, acc[0][e].x), fmaf(ga.y, a.y, acc[0][e].y), fmaf(ga.z, a.z, acc[1][e].x),
-                                                    fmaf(ga.w, a.w, acc[1][e].y));
-        *reinterpret_cast<float4*>(s + 4) = make_float4(fmaf(gb.x, b.x, acc[2][e].x), fmaf(gb.y, b.y, acc[2][e].y),
-                                                        fmaf(gb.z, b.z, acc[3][e].x), fmaf(gb.w, b.w, acc[3][e].y));
-      }
-    }
-    __syncthreads();                                                 // the new S is there, Kd is read
-    fetch_kd(c + 1);
+  volatile int* abort_flag = &ss.abort_flag;
+  if (threadIdx.x == 0) {
+    mbar_init(&ss.wq_full, 1); mbar_init(&ss.wq_empty, 1);
+    mbar_init(&ss.kd_full, 1); mbar_init(&ss.kd_empty, 1);
+    mbar_init(&ss.s_ready, 8); mbar_init(&ss.u_ready, 8);
+    mbar_init(&ss.d1_done, 1); mbar_init(&ss.d2_done, 1);
+    ss.abort_flag = 0;
+    mbar_fence_init();
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  for (int i = tid; i < D * kCols; i += 256) Sg[(size_t)(i / kCols) * D + i % kCols] = st[(i % kCols) * kPad + i / kCols];
+  if (warp == 9) {
+    tmem_alloc(&ss.tmem_base, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tm = ss.tmem_base;             // both products: leading parts (two halves of the reduction), small ones (three)
+  bool ok = true;
+
+  if (warp == 8) {
+    if (elect_one()) {
+      tma_prefetch_desc(&map);
+      for (int c = 0; c < sq.items; ++c) {
+        const int row = ((sq.item0 + c) * H + h) * kPartRows;
+        if (!mbar_wait(&ss.wq_empty, (c & 1) ^ 1, abort_flag, kTimeoutProducer)) { ok = false; break; }
+        mbar_expect_tx(&ss.wq_full, kWqBytes);
+        for (int m = 0; m < 3; ++m)
+          for (int half = 0; half < 2; ++half)
+            for (int r = 0; r < 2; ++r)
+              tma_load_2d(wq + ((m * 2 + half) * 2 + r) * kTile, &map, &ss.wq_full, half * 64, row + m * 2 * kChunk + r * kChunk);
+        if (!mbar_wait(&ss.kd_empty, (c & 1) ^ 1, abort_flag, kTimeoutProducer)) { ok = false; break; }
+        mbar_expect_tx(&ss.kd_full, kKdBytes);
+        for (int m = 0; m < 3; ++m)
+          for (int half = 0; half < 2; ++half)
+            tma_load_2d(kd + (m * 2 + half) * kTile, &map, &ss.kd_full, half * 64, row + (6 + m) * kChunk);
+      }
+      if (ok) {                                 // the last copies are consumed
+        if (mbar_wait(&ss.wq_empty, (sq.items - 1) & 1, abort_flag, kTimeoutProducer))
+          mbar_wait(&ss.kd_empty, (sq.items - 1) & 1, abort_flag, kTimeoutProducer);
+      } else {
+        for (uint32_t i = 0; i < (1u << 16); ++i) __nanosleep(20);   // bounded grace period for copies in flight
+      }
+    }
+  } else if (warp == 9) {
+    if (elect_one()) {
+      // M = 128, bf16; the reduction of the first product lies along A's rows and down B's, of the second down both.  A's second and third part meet
+      // B's three side by side in columns 2 .. 4 (of 64), its first part the second and third of B there too and the first one in
+      // column 0 for the first half of the reduction, in 1 for the second
+      constexpr uint32_t down_b = 1u << 16, down_a = 1u << 15;
+      auto product = [&](int steps, auto a, uint32_t b, uint32_t next, uint32_t down) {
+#pragma unroll
+        for (int i = 1; i < 3; ++i)
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (k < steps)
+              mma_f16(tm + 2 * kCols, a(i, k), desc_over_rows(b + k * 2048, next), make_idesc(128, 3 * kCols, 1, 1) | down, i > 1 || k > 0 ? 1u : 0u);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (k < steps) {
+            mma_f16(tm + 2 * kCols, a(0, k), desc_over_rows(b + next + k * 2048, next), make_idesc(128, 2 * kCols, 1, 1) | down, 1u);
+            mma_f16(tm + (2 * k < steps ? 0 : kCols), a(0, k), desc_over_rows(b + k * 2048, next), make_idesc(128, kCols, 1, 1) | down,
+                    k == 0 || 2 * k == steps ? 0u : 1u);
+          }
+      };
+      for (int c = 0; c < sq.items; ++c) {
+        if (!mbar_wait(&ss.wq_full, c & 1, abort_flag, kTimeoutMma) || !mbar_wait(&ss.s_ready, c & 1, abort_flag, kTimeoutMma)) { ok = false; break; }
+        tc_fence_after();
+        product(D / 16, [&](int i, int k) { return make_smem_desc_sw128(smem_u32(wq) + (i * 2 + k / 4) * 2 * kTile) + 2 * (k % 4); }, smem_u32(st), 2 * kTile,
+                down_b);
+        tc_commit(&ss.wq_empty);
+        tc_commit(&ss.d1_done);
+        if (!mbar_wait(&ss.kd_full, c & 1, abort_flag, kTimeoutMma) || !mbar_wait(&ss.u_ready, c & 1, abort_flag, kTimeoutMma)) { ok = false; break; }
+        tc_fence_after();
+        product(kChunk / 16, [&](int i, int k) { return desc_over_rows(smem_u32(kd) + i * 2 * kTile + k * 2048, kTile); }, smem_u32(ut), kTile, down_b | down_a);
+        tc_commit(&ss.kd_empty);
+        tc_commit(&ss.d2_done);
+      }
+    }
+  } else {
+    const int half = warp >> 2, row = (warp & 3) * 32 + lane;        // row: a key of S; a row of [W; Q']
+    const uint32_t at = (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * 32;
+    const bool init = !sq.first || p.has_initial == nullptr || p.has_initial[sq.seq] != 0;
+    float* Sg = p.rec_state + (((size_t)slot * H + h) * D + row) * D + c0 + half * 32;
+    float S[32];
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+      const float4 x = init ? *reinterpret_cast<const float4*>(Sg + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      S[i] = x.x; S[i + 1] = x.y; S[i + 2] = x.z; S[i + 3] = x.w;
+    }
+    auto hand_over = [&](uint64_t* bar) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    auto done = [&](uint64_t* bar, int c) {
+      if (!__all_sync(0xffffffffu, mbar_wait(bar, c & 1, abort_flag, kTimeoutEpilogue))) return false;
+      tc_fence_after();
+      return true;
+    };
+    auto take = [&](float (&d)[32]) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {                                  // 16 columns at a time
+        uint32_t a[5][16];
+#pragma unroll
+        for (int i = 0; i < 5; ++i) tmem_ld16(tm + at + i * kCols + 16 * j, a[i]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float small = (__uint_as_float(a[2][i]) + __uint_as_float(a[3][i])) + __uint_as_float(a[4][i]);
+          d[16 * j + i] = (__uint_as_float(a[0][i]) + small) + __uint_as_float(a[1][i]);
+        }
+      }
+    };
+    put_parts(st, 2 * kTile, row, half, S);
+    hand_over(&ss.s_ready);
+    for (int c = 0; c < sq.items; ++c) {
+      const size_t item = (size_t)(sq.item0 + c) * H + h;
+      float* add = res + item * 2 * kPart + (size_t)row * D + c0 + half * 32;      // rows of UV, then of O
+      float x[32];
+#pragma unroll
+      for (int i = 0; i < 32; i += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(add + i);
+        x[i] = a.x; x[i + 1] = a.y; x[i + 2] = a.z; x[i + 3] = a.w;
+      }
+      const float g = g_last[item * D + row];
+      if (!done(&ss.d1_done, c)) { ok = false; break; }
+      float d[32];
+      take(d);
+      if (row < kChunk) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) x[i] -= d[i];
+        put_parts(ut, kTile, row, half, x);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; i += 4)
+          *reinterpret_cast<float4*>(add + i) = make_float4(x[i] + d[i], x[i + 1] + d[i + 1], x[i + 2] + d[i + 2], x[i + 3] + d[i + 3]);
+      }
+      hand_over(&ss.u_ready);
+      if (!done(&ss.d2_done, c)) { ok = false; break; }
+      take(d);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) S[i] = fmaf(g, S[i], d[i]);
+      if (c + 1 < sq.items) {
+        put_parts(st, 2 * kTile, row, half, S);
+        hand_over(&ss.s_ready);
+      }
+    }
+    if (ok)
+#pragma unroll
+      for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(Sg + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 9) tmem_dealloc(ss.tmem_base, 512);
+  if (threadIdx.x == 0 && ss.abort_flag != 0 && status != nullptr) atomicMax(status, ss.abort_flag);
 }
 
 // out = o / sqrt(mean(o^2) + eps) * w * sigmoid(z), a warp per token of (chunk, head); the last chunk of a sequence's last piece leaves the
@@ -651,7 +838,7 @@ chunk_finish(const Params p, const ChunkItem* __restrict__ items, const float* _
   if (slot < 0) return;
   const float4 w = *reinterpret_cast<const float4*>(p.norm_w + lane * 4);
   for (int t = warp; t < it.n; t += 8) {
-    const float4 o = *reinterpret_cast<const float4*>(res + ((size_t)blockIdx.x * H + h) * kItemFloats + 4 * kPart + t * D + lane * 4);
+    const float4 o = *reinterpret_cast<const float4*>(res + ((size_t)blockIdx.x * H + h) * 2 * kPart + kPart + t * D + lane * 4);
     const float rs = rsqrtf(warp_sum(o.x * o.x + o.y * o.y + o.z * o.z + o.w * o.w) / D + p.eps);
     const uint2 raw = *reinterpret_cast<const uint2*>(p.z + (size_t)(it.t0 + t) * p.z_stride + h * D + lane * 4);
     const float2 za = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
@@ -678,6 +865,32 @@ chunk_finish(const Params p, const ChunkItem* __restrict__ items, const float* _
   }
 }
 
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static EncodeTiledFn get_encode() {
+  static EncodeTiledFn fn = nullptr;
+  if (fn == nullptr) {
+    void* sym = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) == cudaSuccess &&
+        qres == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<EncodeTiledFn>(sym);
+  }
+  return fn;
+}
+// boxes of 64 rows of 64 elements out of rows of 128
+static int make_parts_map(CUtensorMap* m, void* base, uint64_t rows) {
+  EncodeTiledFn enc = get_encode();
+  if (enc == nullptr) return -1;
+  cuuint64_t dims[2] = {128, rows};
+  cuuint64_t strides[1] = {256};
+  cuuint32_t box[2] = {64, 64};
+  cuuint32_t es[2] = {1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -2;
+}
+
 }  // namespace kda
 }  // namespace bg
 
@@ -685,13 +898,13 @@ extern "C" {
 
 // See bg::kda::Params for the layouts.  D = 64 or 128; nseq sequences, H heads (this rank's).  Sequences of at most `longest_short` tokens go
 // token by token (0: none do); items [n_items, 4] and seqs [n_seqs, 4] (ChunkItem, ChunkSeq) list chunks of up to 64 tokens and the
-// pieces they make, with scratch of n_items * H * (5 * 64 + 1) * 128 floats.
+// pieces they make, with scratch of n_items * H * (417 * 128) floats, on a 16-byte boundary.
 int bg_kda_forward(const void* qkv, int qkv_stride, const void* f, int f_stride, const void* beta, int beta_stride,
                    const void* z, int z_stride, const float* conv_w, const float* conv_b, const float* A_log,
                    const float* dt_bias, const float* norm_w, float* conv_state, float* rec_state,
                    const int* cu_seqlens, const int* slots, const int* has_initial, void* out, int nseq, int H, int D,
                    float scale, float eps, const int* items, int n_items, const int* seqs, int n_seqs, int longest_short,
-                   float* scratch, cudaStream_t stream) {
+                   float* scratch, int* status, cudaStream_t stream) {
   using namespace bg::kda;
   if (nseq <= 0) return 0;
   if ((D != 64 && D != 128) || H <= 0) return -1;
@@ -710,15 +923,20 @@ int bg_kda_forward(const void* qkv, int qkv_stride, const void* f, int f_stride,
   p.out = reinterpret_cast<__nv_bfloat16*>(out);
   p.H = H; p.scale = scale; p.eps = eps;
   p.most = longest_short;
+  p.whole = qkv_stride % 8 == 0 && f_stride % 8 == 0 && reinterpret_cast<uintptr_t>(qkv) % 16 == 0 && reinterpret_cast<uintptr_t>(f) % 16 == 0;
   if (n_items > 0) {
     static bg::DeviceOnce once_p, once_c;
-    if (!bg::ensure_dynamic_smem(chunk_prepare, kPrepareFloats * 4, once_p) || !bg::ensure_dynamic_smem(chunk_chain, kChainFloats * 4, once_c))
-      return -3;
+    if (!bg::ensure_dynamic_smem(chunk_prepare, kPrepareFloats * 4, once_p) || !bg::ensure_dynamic_smem(chunk_chain, kChainBytes, once_c)) return -3;
     auto it = reinterpret_cast<const ChunkItem*>(items);
-    float* g_last = scratch + (size_t)n_items * H * kItemFloats;
-    chunk_prepare<<<dim3(n_items, H), kPrepThreads, kPrepareFloats * 4, stream>>>(p, it, scratch, g_last);
-    chunk_chain<<<dim3(128 / kCols, H, n_seqs), 256, kChainFloats * 4, stream>>>(p, it, reinterpret_cast<const ChunkSeq*>(seqs), scratch, g_last);
-    chunk_finish<<<dim3(n_items, H), 256, 0, stream>>>(p, it, scratch);
+    const size_t pairs = (size_t)n_items * H;
+    auto parts = reinterpret_cast<__nv_bfloat16*>(scratch);
+    float* res = scratch + pairs * kPartRows * 64;
+    float* g_last = res + pairs * 2 * kPart;
+    CUtensorMap tm;
+    if (make_parts_map(&tm, parts, pairs * kPartRows) != 0) return -4;
+    chunk_prepare<<<dim3(n_items, H), kPrepThreads, kPrepareFloats * 4, stream>>>(p, it, parts, res, g_last);
+    chunk_chain<<<dim3(128 / kCols, H, n_seqs), kChainThreads, kChainBytes, stream>>>(tm, p, it, reinterpret_cast<const ChunkSeq*>(seqs), res, g_last, status);
+    chunk_finish<<<dim3(n_items, H), 256, 0, stream>>>(p, it, res);
   }
   if (longest_short <= 0) return cudaGetLastError() == cudaSuccess ? 0 : -2;
   dim3 grid(H, nseq);

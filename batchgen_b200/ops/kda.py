@@ -100,7 +100,7 @@ def kda_chunk_ref(q, k, v, g, beta, S, scale: float, chunk: int = 64):
 
 CHUNK = 64
 CHUNK_MIN_TOKENS = 48                 # shorter pieces never go through the chunk form
-_CHUNK_FLOATS = (5 * CHUNK + 1) * 128   # scratch of a (chunk, head)
+_CHUNK_FLOATS = (9 * CHUNK // 2 + 2 * CHUNK + 1) * 128   # scratch of a (chunk, head): nine bf16 and two fp32 [64, 128] results, decays
 _CHUNK_SCRATCH = 1 << 30              # bytes of scratch a round of chunks may take
 
 
@@ -109,7 +109,9 @@ def chunk_form_pays(lens: Sequence[int], heads: int, sms: int) -> bool:
     its state, on 148 SMs.  Token by token a CTA serves a (piece, head): 1.6 to 2.0 us a token of the longest piece with a CTA on an SM, 2.42
     with two, and 2.42 a token of every further round of two CTAs an SM.  Measured in us, chunks / tokens: 32 heads 1 x 64 100 / 131, 1 x
     4,096 1,160 / 8,100, 4 x 512 648 / 1,044, 16 x 128 724 / 649, 8 x 1,024 2,183 / 2,485, 64 x 64 1,638 / 1,136, 64 x 128 2,657 / 2,200, 64 x 512
-    8,943 / 8,568; 8 heads 16 x 128 225 / 235, 64 x 512 2,255 / 2,472; 64 heads 16 x 512 4,554 / 4,643, 128 x 64 6,356 / 4,384."""
+    8,943 / 8,568; 8 heads 16 x 128 225 / 235, 64 x 512 2,255 / 2,472; 64 heads 16 x 512 4,554 / 4,643, 128 x 64 6,356 / 4,384.  The chunks have become
+    faster since (32 heads 1 x 64 67, 1 x 4,096 913, 4 x 512 404, 16 x 128 416, 8 x 1,024 1,014, 64 x 64 848, 64 x 128 1,543): the line still lies where both
+    took the same time then, so it leaves some short pieces to the tokens that chunks would now serve up to a third faster."""
     if not lens:
         return False
     pairs, longest, total = heads * len(lens), max(lens), sum(lens)
@@ -228,7 +230,7 @@ def kda_forward(qkv: torch.Tensor, f: torch.Tensor, beta: torch.Tensor, z: torch
     elif cu_seqlens is not None and plan is None:
         plan = step_plan(cu_seqlens, H, D, dev)
     rounds, short = (plan.rounds, plan.short) if plan is not None and cu_seqlens is not None else ([], (1 << 31) - 1)
-    if z.stride(0) % 4 or z.data_ptr() % 8:               # the chunk form reads four gates at a time
+    if z.stride(0) % 4 or z.data_ptr() % 8 or rec_state.data_ptr() % 16:      # the chunk form reads four gates, and four numbers of a state, at a time
         rounds, short = [], (1 << 31) - 1
     cu_t = plan.cu if cu_seqlens is not None else None
     assert cu_t is None or cu_t.shape[0] == nseq + 1
@@ -243,7 +245,7 @@ def kda_forward(qkv: torch.Tensor, f: torch.Tensor, beta: torch.Tensor, z: torch
             _ext.ptr(cu_t), _ext.ptr(slots), _ext.ptr(hi_t), _ext.ptr(out), ctypes.c_int(nseq), ctypes.c_int(H),
             ctypes.c_int(D), ctypes.c_float(scale), ctypes.c_float(eps), _ext.ptr(tables[at:] if items else None), ctypes.c_int(items),
             _ext.ptr(tables[at + items:] if items else None), ctypes.c_int(pieces), ctypes.c_int(short if last else 0),
-            _ext.ptr(scratch if items else None), _ext.stream())
+            _ext.ptr(scratch if items else None), _ext.ptr(_ext.status_word(dev)), _ext.stream())
         _ext.check(rc, "bg_kda_forward", kernels=(3 if items else 0) + int(last and short > 0))
         at += items + pieces
     return out

@@ -277,3 +277,29 @@ def test_one_plan_serves_the_layers_of_a_step(monkeypatch):
     a, b = [0, 200, 270], [0, 20, 110]
     assert made == [a, a, a, b, b], made                 # first step, its twin; twin of the second; third and its twin
     assert torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("lens,shift", [([64, 65], 0), ([130, 48, 200], 1), ([192], 4)])
+def test_chunk_form_of_unaligned_rows(lens, shift, monkeypatch):
+    """Inputs as columns of a wider projection: rows that are and are not in 16-byte pieces give the same numbers; the state's columns of both CTAs of a head."""
+    from batchgen_b200.ops import kda
+    H = 2
+    cu, slots, has, qkv, z, f, beta, p, conv0, rec0 = _prompt(H, lens, 21)
+    monkeypatch.setattr(kda, "chunk_form_pays", lambda lens, heads, sms: bool(lens))
+    got = []
+    for wide in (False, True):
+        conv, rec = conv0.cuda(), rec0.cuda()
+        q, ff = qkv.cuda(), f.cuda()
+        if wide:
+            q = torch.zeros(q.shape[0], q.shape[1] + 5 + shift, dtype=q.dtype, device="cuda")[:, shift:shift + q.shape[1]].copy_(q)
+            ff = torch.zeros(ff.shape[0], ff.shape[1] + 3, dtype=q.dtype, device="cuda")[:, 1:1 + ff.shape[1]].copy_(ff)
+        o = kda.kda_forward(q, ff, beta.cuda(), z.cuda(), p, conv, rec, slots, cu, has, H, 128, 128 ** -0.5, 1e-6)
+        got.append((o, conv, rec))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+    conv64, rec64 = conv0.double(), rec0.double()
+    want = _recurrence64(qkv, f, beta, z, p, conv64, rec64, slots, cu, has, H, 128, 128 ** -0.5, 1e-6)
+    o, _, rec = got[0]
+    # a value rounded to 8 significant bits; the recurrence in fp32
+    assert ((o.cpu().double() - want).abs() <= want.abs() * 2 ** -8 + 2e-4).all()
+    for half in (rec[..., :64], rec64.cuda()[..., :64]), (rec[..., 64:], rec64.cuda()[..., 64:]):
+        assert (half[0].double() - half[1]).norm() <= 5e-7 * half[1].norm()
