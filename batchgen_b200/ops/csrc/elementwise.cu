@@ -13,7 +13,7 @@
 // add_rmsnorm_fp8_quant.cu:243, batchgen_kernels/src/moe/fp8_blockwise/fp8_blockwise_ops.cu:39-445,
 // batchgen_kernels/src/attention/fused_kv_norm_rope_cache.cu:14, batchgen_kernels/triton/fp8_quantize.py.
 #define BG_FILE_TAG 1      // kernel-trace ids of this file are (tag << 16) | line
-#include "common.cuh"
+#include "quant_blocks.cuh"
 
 namespace bg {
 
@@ -30,134 +30,113 @@ __device__ __forceinline__ float block_sum_256(float v, float* red) {
   return t;
 }
 
-__device__ __forceinline__ float quant_scale(float amax, int pow2) {
-  float s = fmaxf(amax, 1e-4f) * (1.0f / 448.0f);
-  if (pow2) s = exp2f(ceilf(log2f(s)));
-  return s;
-}
-
-// One block per row.  Each thread owns vectors of 8 consecutive elements; 16 consecutive threads
-// cover one 128-wide quantisation block, so the block amax is a 16-lane shuffle reduction.
-template <bool ADD, bool QUANT>
+// One block per row.  Each thread owns NV vectors of 8 consecutive elements, all of them read before the first is used and kept in registers
+// between the two passes; 16 consecutive threads cover one 128-wide quantisation block, so the block amax is a 16-lane shuffle
+// reduction.  Bound by its bytes: with the row in shared memory, eight lanes on a bank, 4,739 rows of 7,168 with sum and quantisation took
+// 63.6 us, now 59 (floor 42); 1,536 rows 28.7, now 26.7; 256 and fewer as before (12).
+template <bool ADD, bool QUANT, int NV>
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ residual,
                const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out, uint8_t* __restrict__ out_q,
                float* __restrict__ out_s, int s_stride, int H, int ldx, int ldo, float eps, int pow2) {
   bg::pdl_prologue((BG_FILE_TAG << 16) | __LINE__);
-  extern __shared__ float row[];  // H floats
   __shared__ float red[32];
   const int t = blockIdx.x;
   const __nv_bfloat16* xr = x + (size_t)t * ldx;
   __nv_bfloat16* rr = ADD ? residual + (size_t)t * H : nullptr;
+  uint4 xv[NV], rv[ADD ? NV : 1];
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int v = threadIdx.x + n * kNormThreads;
+    if (v >= H / 8) continue;
+    xv[n] = *reinterpret_cast<const uint4*>(xr + v * 8);
+    if (ADD) rv[n] = *reinterpret_cast<const uint4*>(rr + v * 8);
+  }
   float ss = 0.f;
-  for (int v = threadIdx.x; v < H / 8; v += kNormThreads) {
-    uint4 raw = *reinterpret_cast<const uint4*>(xr + v * 8);
-    const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&raw);
-    float f[8];
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int v = threadIdx.x + n * kNormThreads;
+    if (v >= H / 8) continue;
+    __nv_bfloat162* xp = reinterpret_cast<__nv_bfloat162*>(&xv[n]);
+    if (ADD) {
+      const __nv_bfloat162* rp = reinterpret_cast<const __nv_bfloat162*>(&rv[n]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {         // the sum as stored (bf16) is what gets normalised
+        const float2 a = __bfloat1622float2(xp[i]), b = __bfloat1622float2(rp[i]);
+        xp[i] = __floats2bfloat162_rn(a.x + b.x, a.y + b.y);
+      }
+      *reinterpret_cast<uint4*>(rr + v * 8) = xv[n];
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      float2 a = __bfloat1622float2(xp[i]);
-      f[2 * i] = a.x;
-      f[2 * i + 1] = a.y;
-    }
-    if (ADD) {
-      uint4 rraw = *reinterpret_cast<const uint4*>(rr + v * 8);
-      const __nv_bfloat162* rp = reinterpret_cast<const __nv_bfloat162*>(&rraw);
-      __align__(16) __nv_bfloat162 o[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float2 a = __bfloat1622float2(rp[i]);
-        o[i] = __floats2bfloat162_rn(f[2 * i] + a.x, f[2 * i + 1] + a.y);
-        float2 b = __bfloat1622float2(o[i]);  // the sum as stored (bf16) is what gets normalised
-        f[2 * i] = b.x;
-        f[2 * i + 1] = b.y;
-      }
-      *reinterpret_cast<uint4*>(rr + v * 8) = *reinterpret_cast<const uint4*>(o);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      row[v * 8 + i] = f[i];
-      ss += f[i] * f[i];
+      const float2 a = __bfloat1622float2(xp[i]);
+      ss += a.x * a.x;
+      ss += a.y * a.y;
     }
   }
   const float total = block_sum_256(ss, red);
   const float rstd = rsqrtf(total / (float)H + eps);
-  for (int v = threadIdx.x; v < H / 8; v += kNormThreads) {
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    const int v = threadIdx.x + n * kNormThreads;
+    if (v >= H / 8) continue;               // H is a multiple of 128 where blocks are quantised: their lanes stay together
     uint4 wraw = *reinterpret_cast<const uint4*>(w + v * 8);
     const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&wraw);
+    const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&xv[n]);
     __align__(16) __nv_bfloat162 o[4];
     float y[8];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      float2 ww = __bfloat1622float2(wp[i]);
-      o[i] = __floats2bfloat162_rn(row[v * 8 + 2 * i] * rstd * ww.x, row[v * 8 + 2 * i + 1] * rstd * ww.y);
+      const float2 ww = __bfloat1622float2(wp[i]), a = __bfloat1622float2(xp[i]);
+      o[i] = __floats2bfloat162_rn(a.x * rstd * ww.x, a.y * rstd * ww.y);
       float2 b = __bfloat1622float2(o[i]);
       y[2 * i] = b.x;
       y[2 * i + 1] = b.y;
     }
     if (out != nullptr) *reinterpret_cast<uint4*>(out + (size_t)t * ldo + v * 8) = *reinterpret_cast<const uint4*>(o);
     if (QUANT) {
-      float amax = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(y[i]));
-#pragma unroll
-      for (int o2 = 8; o2 > 0; o2 >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o2));
-      const float s = quant_scale(amax, pow2);
-      const float inv = 1.0f / s;
-      __align__(8) uint16_t q[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) q[i] = to_e4m3x2(y[2 * i] * inv, y[2 * i + 1] * inv);
-      *reinterpret_cast<uint2*>(out_q + (size_t)t * H + v * 8) = *reinterpret_cast<const uint2*>(q);
+      const float s = quant_block(y, out_q + (size_t)t * H + v * 8, pow2, 0xffffu << (threadIdx.x & 16));
       if ((threadIdx.x & 15) == 0) out_s[(size_t)(v / 16) * s_stride + t] = s;
     }
   }
 }
 
-// Activation quantisation.  MODE 0: x [T, K].  MODE 1: x [T, 2K] = gate | up -> quantise silu(gate)*up.
-// One warp per (row, group of 128-blocks): 16 lanes per 128-block, two blocks per warp pass.
-template <int MODE>
+// Activation quantisation.  MODE 0: x [T, K].  MODE 1: x [T, 2K] = gate | up -> quantise silu(gate)*up.  Warps walk the rows (quant_blocks.cuh).
+template <int MODE, int U>
 __global__ void __launch_bounds__(256)
 act_quant_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ s, int s_stride,
                  int T, int K, int ldx, int pow2, const int* __restrict__ valid_rows,
                  const int* __restrict__ row_src) {
   bg::pdl_prologue((BG_FILE_TAG << 16) | __LINE__);
-  const int t = blockIdx.x;
-  if (valid_rows != nullptr && t >= *valid_rows) return;
-  if (row_src != nullptr && row_src[t] < 0) return;      // padding row of an expert segment: nothing reads it
-  const __nv_bfloat16* xr = x + (size_t)t * ldx;
-  for (int v = threadIdx.x; v < K / 8; v += blockDim.x) {
-    uint4 raw = *reinterpret_cast<const uint4*>(xr + v * 8);
-    const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&raw);
-    float f[8];
+  const int lane = threadIdx.x & 31, rows = valid_rows != nullptr ? min(T, *valid_rows) : T;
+  for (BlockWalk<U> walk(rows, K); walk.more(); walk.next()) {
+    const int t = walk.row;
+    if (row_src != nullptr && row_src[t] < 0) continue;    // padding row of an expert segment: nothing reads it
+    const __nv_bfloat16* xr = x + (size_t)t * ldx;
+    uint4 raw[U], up[MODE == 1 ? U : 1];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float2 a = __bfloat1622float2(xp[i]);
-      f[2 * i] = a.x;
-      f[2 * i + 1] = a.y;
+    for (int u = 0; u < U; ++u) {
+      const int kb = walk.block(u, lane);
+      if (kb * 128 >= K) continue;
+      raw[u] = *reinterpret_cast<const uint4*>(xr + kb * 128 + (lane & 15) * 8);
+      if (MODE == 1) up[u] = *reinterpret_cast<const uint4*>(xr + K + kb * 128 + (lane & 15) * 8);
     }
-    if (MODE == 1) {
-      uint4 uraw = *reinterpret_cast<const uint4*>(xr + K + v * 8);
-      const __nv_bfloat162* up = reinterpret_cast<const __nv_bfloat162*>(&uraw);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float2 u = __bfloat1622float2(up[i]);
+    for (int u = 0; u < U; ++u) {
+      const int kb = walk.block(u, lane);
+      if (kb * 128 >= K) continue;
+      float f[8];
+      unpack8(raw[u], f);
+      if (MODE == 1) {
+        float g[8];
+        unpack8(up[u], g);
         // round the activation to bf16 first: same bytes as silu_mul (bf16) followed by act_quant
-        f[2 * i] = __bfloat162float(__float2bfloat16(silu(f[2 * i]) * u.x));
-        f[2 * i + 1] = __bfloat162float(__float2bfloat16(silu(f[2 * i + 1]) * u.y));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = __bfloat162float(__float2bfloat16(silu(f[i]) * g[i]));
       }
+      const float sc = quant_block(f, q + (size_t)t * K + kb * 128 + (lane & 15) * 8, pow2, 0xffffu << (lane & 16));
+      if ((lane & 15) == 0) s[(size_t)kb * s_stride + t] = sc;
     }
-    float amax = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float sc = quant_scale(amax, pow2);
-    const float inv = 1.0f / sc;
-    __align__(8) uint16_t o4[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) o4[i] = to_e4m3x2(f[2 * i] * inv, f[2 * i + 1] * inv);
-    *reinterpret_cast<uint2*>(q + (size_t)t * K + v * 8) = *reinterpret_cast<const uint2*>(o4);
-    if ((threadIdx.x & 15) == 0) s[(size_t)(v / 16) * s_stride + t] = sc;
   }
 }
 
@@ -220,6 +199,50 @@ __global__ void rope_q_kernel(__nv_bfloat16* __restrict__ q, int H, int D, int r
   }
 }
 
+// The same, eight pairs a thread in 16-byte pieces (rope a multiple of 16, pieces on 16-byte boundaries).  Bound by
+// its bytes: two bytes an access took 63.5 us for 4,739 tokens of 128 heads with 64 rotated dims, now 34.8 (floor
+// 24 at the 32-byte sectors touched); 4 tokens 15, now 8.
+template <bool INTERLEAVED>
+__global__ void __launch_bounds__(256)
+rope_q_wide_kernel(__nv_bfloat16* __restrict__ q, int H, int D, int rope, const int* __restrict__ positions,
+                   const float* __restrict__ cos_t, const float* __restrict__ sin_t, long long ld_t) {
+  bg::pdl_prologue((BG_FILE_TAG << 16) | __LINE__);
+  const int t = blockIdx.x, half = rope / 2, per = rope / 16;
+  const float* ct = cos_t + (size_t)positions[t] * half;
+  const float* st = sin_t + (size_t)positions[t] * half;
+  for (int idx = threadIdx.x; idx < H * per; idx += blockDim.x) {
+    const int h = idx / per, i = (idx - h * per) * 8;                // pairs i .. i + 7
+    __nv_bfloat16* p = q + (size_t)t * ld_t + (size_t)h * D + (D - rope);
+    uint4* p0 = reinterpret_cast<uint4*>(p + (INTERLEAVED ? 2 * i : i));
+    uint4* p1 = reinterpret_cast<uint4*>(p + (INTERLEAVED ? 2 * i + 8 : i + half));
+    float x[8], y[8], c[8], s[8], a[8], b[8];
+    unpack8(*p0, x);
+    unpack8(*p1, y);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      c[j] = ct[i + j];
+      s[j] = st[i + j];
+      a[j] = INTERLEAVED ? (j < 4 ? x[2 * (j & 3)] : y[2 * (j & 3)]) : x[j];
+      b[j] = INTERLEAVED ? (j < 4 ? x[2 * (j & 3) + 1] : y[2 * (j & 3) + 1]) : y[j];
+    }
+    __align__(16) __nv_bfloat162 o[8];
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      const float u0 = a[j] * c[j] - b[j] * s[j], v0 = b[j] * c[j] + a[j] * s[j];
+      const float u1 = a[j + 1] * c[j + 1] - b[j + 1] * s[j + 1], v1 = b[j + 1] * c[j + 1] + a[j + 1] * s[j + 1];
+      if (INTERLEAVED) {
+        o[j] = __floats2bfloat162_rn(u0, v0);
+        o[j + 1] = __floats2bfloat162_rn(u1, v1);
+      } else {
+        o[j / 2] = __floats2bfloat162_rn(u0, u1);
+        o[4 + j / 2] = __floats2bfloat162_rn(v0, v1);
+      }
+    }
+    *p0 = reinterpret_cast<const uint4*>(o)[0];
+    *p1 = reinterpret_cast<const uint4*>(o)[1];
+  }
+}
+
 }  // namespace bg
 
 extern "C" {
@@ -232,14 +255,17 @@ int bg_rmsnorm(const void* x, void* residual, const void* w, void* out, void* ou
   using namespace bg;
   if (T <= 0) return 0;
   if (H % 8 != 0 || (out_q != nullptr && H % 128 != 0)) return -1;
-  const size_t smem = (size_t)H * sizeof(float);
+  if (H > 12256) return -1;                                    // within six vectors of eight a thread
   auto X = reinterpret_cast<const __nv_bfloat16*>(x);
   auto R = reinterpret_cast<__nv_bfloat16*>(residual);
   auto W = reinterpret_cast<const __nv_bfloat16*>(w);
   auto O = reinterpret_cast<__nv_bfloat16*>(out);
   auto Q = reinterpret_cast<uint8_t*>(out_q);
-#define BG_LAUNCH(ADD, QNT)                                                                                      \
-  bg::launch_pdl(rmsnorm_kernel<ADD, QNT>, dim3(T), dim3(kNormThreads), smem, stream, X, R, W, O, Q, out_s, s_stride, H, ldx, ldo, eps, pow2)
+  const int nv = (H + 8 * kNormThreads - 1) / (8 * kNormThreads);
+#define BG_LAUNCH(ADD, QNT)                                                                                                                        \
+  bg::launch_pdl(nv <= 1 ? rmsnorm_kernel<ADD, QNT, 1> : nv <= 2 ? rmsnorm_kernel<ADD, QNT, 2> : nv <= 4 ? rmsnorm_kernel<ADD, QNT, 4>            \
+                                                                                                        : rmsnorm_kernel<ADD, QNT, 6>,            \
+                 dim3(T), dim3(kNormThreads), 0, stream, X, R, W, O, Q, out_s, s_stride, H, ldx, ldo, eps, pow2)
   if (residual != nullptr && out_q != nullptr) BG_LAUNCH(true, true);
   else if (residual != nullptr) BG_LAUNCH(true, false);
   else if (out_q != nullptr) BG_LAUNCH(false, true);
@@ -255,11 +281,11 @@ int bg_act_quant(int mode, const void* x, void* q, float* s, int s_stride, int T
   using namespace bg;
   if (T <= 0) return 0;
   if (K % 128 != 0) return -1;
-  const int threads = K / 8 >= 256 ? 256 : ((K / 8 + 31) / 32) * 32;
   auto X = reinterpret_cast<const __nv_bfloat16*>(x);
   auto Q = reinterpret_cast<uint8_t*>(q);
-  if (mode == 0) bg::launch_pdl(act_quant_kernel<0>, dim3(T), dim3(threads), 0, stream, X, Q, s, s_stride, T, K, ldx, pow2, valid_rows, row_src);
-  else bg::launch_pdl(act_quant_kernel<1>, dim3(T), dim3(threads), 0, stream, X, Q, s, s_stride, T, K, ldx, pow2, valid_rows, row_src);
+  const bool many = many_blocks(T, K);
+  auto kern = mode == 0 ? (many ? act_quant_kernel<0, 4> : act_quant_kernel<0, 1>) : (many ? act_quant_kernel<1, 4> : act_quant_kernel<1, 1>);
+  bg::launch_pdl(kern, dim3(walk_grid(T, K, many ? 4 : 1)), dim3(256), 0, stream, X, Q, s, s_stride, T, K, ldx, pow2, valid_rows, row_src);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -278,8 +304,11 @@ int bg_rope_q(void* q, int T, int H, int D, int rope, const int* positions, cons
               int interleaved, long long ld_t, cudaStream_t stream) {
   using namespace bg;
   if (T <= 0) return 0;
-  bg::launch_pdl(rope_q_kernel, dim3(T), dim3(256), 0, stream, reinterpret_cast<__nv_bfloat16*>(q), H, D, rope, positions, cos_t, sin_t,
-                                       interleaved, ld_t);
+  auto Q = reinterpret_cast<__nv_bfloat16*>(q);
+  if (rope % 16 == 0 && D % 8 == 0 && ld_t % 8 == 0 && reinterpret_cast<uintptr_t>(q) % 16 == 0)
+    bg::launch_pdl(interleaved ? rope_q_wide_kernel<true> : rope_q_wide_kernel<false>, dim3(T), dim3(256), 0, stream, Q, H, D, rope, positions, cos_t, sin_t, ld_t);
+  else
+    bg::launch_pdl(rope_q_kernel, dim3(T), dim3(256), 0, stream, Q, H, D, rope, positions, cos_t, sin_t, interleaved, ld_t);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -13,6 +13,7 @@
 #define BG_FILE_TAG 2      // kernel-trace ids of this file are (tag << 16) | line
 #include "common.cuh"
 #include "mx_parts.cuh"
+#include "quant_blocks.cuh"
 
 namespace bg {
 
@@ -191,58 +192,88 @@ __global__ void moe_scatter_kernel(const int* __restrict__ topk_idx, int n_pairs
   }
 }
 
-// One block per grouped row: gather hidden[src_row[r]] (bf16) and quantise to e4m3 with 1x128
-// scales.  Padding rows (src < 0) become zeros with scale 0 so they produce exact zeros, or are left
-// untouched when `zero_padding` is 0 (the grouped GEMM is then given the real row counts).
+// Gather hidden[src_row[r]] (bf16) and quantise to e4m3 with 1x128 scales; warps walk the grouped rows (quant_blocks.cuh).  Padding rows
+// (src < 0) become zeros with scale 0 so they produce exact zeros, or are left untouched when `zero_padding` is 0 (the grouped GEMM is
+// then given the real row counts).
+template <int U>
 __global__ void __launch_bounds__(256)
 moe_gather_quant_kernel(const __nv_bfloat16* __restrict__ hidden, int ldh, const int* __restrict__ src_row,
                         const int* __restrict__ total_rows, uint8_t* __restrict__ q, float* __restrict__ s,
-                        int s_stride, int K, int pow2, int zero_padding) {
+                        int s_stride, int cap, int K, int pow2, int zero_padding) {
   bg::pdl_prologue((BG_FILE_TAG << 16) | __LINE__);
-  const int r = blockIdx.x;
-  if (r >= *total_rows) return;
-  const int src = src_row[r];
-  if (src < 0 && !zero_padding) return;
-  for (int v = threadIdx.x; v < K / 8; v += blockDim.x) {
-    float f[8];
-    if (src >= 0) {
-      uint4 raw = *reinterpret_cast<const uint4*>(hidden + (size_t)src * ldh + v * 8);
-      const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  const int lane = threadIdx.x & 31, rows = min(cap, *total_rows);
+  for (BlockWalk<U> walk(rows, K); walk.more(); walk.next()) {
+    const int r = walk.row, src = src_row[r];
+    if (src < 0 && !zero_padding) continue;
+    uint4 raw[U];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float2 a = __bfloat1622float2(xp[i]);
-        f[2 * i] = a.x;
-        f[2 * i + 1] = a.y;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] = 0.f;
+    for (int u = 0; u < U; ++u) {
+      const int kb = walk.block(u, lane);
+      raw[u] = src >= 0 && kb * 128 < K ? *reinterpret_cast<const uint4*>(hidden + (size_t)src * ldh + kb * 128 + (lane & 15) * 8) : make_uint4(0, 0, 0, 0);
     }
-    float amax = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    float sc = fmaxf(amax, 1e-4f) * (1.0f / 448.0f);
-    if (pow2) sc = exp2f(ceilf(log2f(sc)));
-    const float inv = 1.0f / sc;
-    __align__(8) uint16_t o4[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) o4[i] = to_e4m3x2(f[2 * i] * inv, f[2 * i + 1] * inv);
-    *reinterpret_cast<uint2*>(q + (size_t)r * K + v * 8) = *reinterpret_cast<const uint2*>(o4);
-    if ((threadIdx.x & 15) == 0) s[(size_t)(v / 16) * s_stride + r] = (src >= 0) ? sc : 0.f;
+    for (int u = 0; u < U; ++u) {
+      const int kb = walk.block(u, lane);
+      if (kb * 128 >= K) continue;
+      float f[8];
+      unpack8(raw[u], f);
+      const float sc = quant_block(f, q + (size_t)r * K + kb * 128 + (lane & 15) * 8, pow2, 0xffffu << (lane & 16));
+      if ((lane & 15) == 0) s[(size_t)kb * s_stride + r] = src >= 0 ? sc : 0.f;
+    }
   }
 }
 
-// out[t] = (extra[t] if given) + sum_k w[t,k] * y[pos[t,k]], k ascending.  Grid (token, 2,048-column chunk): a
-// thread owns 8 columns and has the top-k rows' loads in flight together, so a 48-token decode step still fills
-// the SMs instead of walking each row serially in 48 blocks.
+// The same by token: each is quantised once, its bytes and scales go to the row of every expert it has (pos [T, topk], < 0: none); padding rows
+// stay untouched.  Bound by its bytes: 4,739 tokens of 7,168 to eight rows each 84 us, quantised
+// again for every row 145 (floor 49); 256 tokens 11 against 18.
+template <int U>
 __global__ void __launch_bounds__(256)
+moe_spread_quant_kernel(const __nv_bfloat16* __restrict__ hidden, int ldh, const int* __restrict__ pos, int topk, uint8_t* __restrict__ q, float* __restrict__ s,
+                        int s_stride, int T, int K, int pow2) {
+  bg::pdl_prologue((BG_FILE_TAG << 16) | __LINE__);
+  const int lane = threadIdx.x & 31;
+  for (BlockWalk<U> walk(T, K); walk.more(); walk.next()) {
+    const int t = walk.row, mine = lane < topk ? pos[(size_t)t * topk + lane] : -1;
+    if (!__any_sync(0xffffffffu, mine >= 0)) continue;
+    uint4 raw[U];
+    uint2 bytes[U];
+    float sc[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int kb = walk.block(u, lane);
+      raw[u] = kb * 128 < K ? *reinterpret_cast<const uint4*>(hidden + (size_t)t * ldh + kb * 128 + (lane & 15) * 8) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float f[8];
+      unpack8(raw[u], f);
+      sc[u] = quant_block(f, reinterpret_cast<uint8_t*>(&bytes[u]), pow2, 0xffffu << (lane & 16));
+    }
+    for (int j = 0; j < topk; ++j) {
+      const int r = __shfl_sync(0xffffffffu, mine, j);
+      if (r < 0) continue;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int kb = walk.block(u, lane);
+        if (kb * 128 >= K) continue;
+        *reinterpret_cast<uint2*>(q + (size_t)r * K + kb * 128 + (lane & 15) * 8) = bytes[u];
+        if ((lane & 15) == 0) s[(size_t)kb * s_stride + r] = sc[u];
+      }
+    }
+  }
+}
+
+// out[t] = (extra[t] if given) + sum_k w[t,k] * y[pos[t,k]], k ascending.  A CTA per 1,024 columns of a
+// token: a thread owns 8 columns and has the top-k rows' loads in flight together, so a 48-token decode step still fills
+// the SMs instead of walking each row serially in 48 blocks.  256 threads with the chunks of a token
+// far apart in the grid took 148 us for 4,739 tokens of 7,168 with eight rows each, now 135 (floor 105 for its bytes); 256 tokens 16.5 either way.
+constexpr int kCombineThreads = 128;
+__global__ void __launch_bounds__(kCombineThreads)
 moe_combine_kernel(const __nv_bfloat16* __restrict__ y, int ldy, const int* __restrict__ pos,
                    const float* __restrict__ w, const __nv_bfloat16* __restrict__ extra, int lde,
                    __nv_bfloat16* __restrict__ out, int ldo, int K, int H, int out_fp32) {
   bg::pdl_prologue((BG_FILE_TAG << 16) | __LINE__);
-  const int t = blockIdx.x;
+  const int chunks = (H / 8 + kCombineThreads - 1) / kCombineThreads, t = blockIdx.x / chunks;
   __shared__ int p_s[kMaxTopK];
   __shared__ float w_s[kMaxTopK];
   if (threadIdx.x < K) {
@@ -250,7 +281,7 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ y, int ldy, const int* __re
     w_s[threadIdx.x] = w[(size_t)t * K + threadIdx.x];
   }
   __syncthreads();
-  const int v = blockIdx.y * blockDim.x + threadIdx.x;
+  const int v = (blockIdx.x - t * chunks) * kCombineThreads + threadIdx.x;
   if (v < H / 8) {
     float acc[8];
 #pragma unroll
@@ -391,6 +422,18 @@ int bg_router_topk(const float* logits, int ldl, const float* bias, int* idx, fl
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
+// hidden [T, ldh] quantised to the rows pos [T, topk] (negative: none) of q [.., K] and s; topk at most 32
+int bg_moe_spread_quant(const void* hidden, int ldh, const int* pos, int topk, void* q, float* s, int s_stride, int T, int K, int pow2,
+                        cudaStream_t stream) {
+  using namespace bg;
+  if (T <= 0) return 0;
+  if (K % 128 != 0 || topk <= 0 || topk > 32) return -1;
+  const bool many = many_blocks(T, K);
+  bg::launch_pdl(many ? moe_spread_quant_kernel<4> : moe_spread_quant_kernel<1>, dim3(walk_grid(T, K, many ? 4 : 1)), dim3(256), 0, stream,
+                 reinterpret_cast<const __nv_bfloat16*>(hidden), ldh, pos, topk, reinterpret_cast<uint8_t*>(q), s, s_stride, T, K, pow2);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
 // Builds offsets [El+1], pos [T*K], src_row [cap] (pre-filled with -1 here) for experts [lo, hi).
 int bg_moe_permute(const int* topk_idx, int T, int K, int lo, int hi, int align, int* offsets, int* cursor, int* pos,
                    int* src_row, int cap, const int* num_valid, cudaStream_t stream) {
@@ -410,8 +453,9 @@ int bg_moe_gather_quant(const void* hidden, int ldh, const int* src_row, const i
   using namespace bg;
   if (cap <= 0) return 0;
   if (K % 128 != 0) return -1;
-  bg::launch_pdl(moe_gather_quant_kernel, dim3(cap), dim3(256), 0, stream, reinterpret_cast<const __nv_bfloat16*>(hidden), ldh, src_row,
-                                                   total_rows, reinterpret_cast<uint8_t*>(q), s, s_stride, K, pow2, zero_padding);
+  const bool many = many_blocks(cap, K);
+  bg::launch_pdl(many ? moe_gather_quant_kernel<4> : moe_gather_quant_kernel<1>, dim3(walk_grid(cap, K, many ? 4 : 1)), dim3(256), 0, stream,
+                 reinterpret_cast<const __nv_bfloat16*>(hidden), ldh, src_row, total_rows, reinterpret_cast<uint8_t*>(q), s, s_stride, cap, K, pow2, zero_padding);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -420,7 +464,7 @@ int bg_moe_combine(const void* y, int ldy, const int* pos, const float* w, const
   using namespace bg;
   if (T <= 0) return 0;
   if (K > kMaxTopK || H % 8 != 0) return -1;
-  bg::launch_pdl(moe_combine_kernel, dim3(T, (H / 8 + 255) / 256), dim3(256), 0, stream, reinterpret_cast<const __nv_bfloat16*>(y), ldy, pos, w,
+  bg::launch_pdl(moe_combine_kernel, dim3(T * ((H / 8 + kCombineThreads - 1) / kCombineThreads)), dim3(kCombineThreads), 0, stream, reinterpret_cast<const __nv_bfloat16*>(y), ldy, pos, w,
                                             reinterpret_cast<const __nv_bfloat16*>(extra), lde,
                                             reinterpret_cast<__nv_bfloat16*>(out), ldo, K, H, out_fp32);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;

@@ -147,10 +147,10 @@ def permute(topk_idx: torch.Tensor, lo: int, hi: int, num_valid: Optional[torch.
 
 
 def gather_quant(hidden: torch.Tensor, src_row: torch.Tensor, offsets: torch.Tensor, pow2_scale: bool = False,
-                 zero_padding: bool = True):
+                 zero_padding: bool = True, pos: Optional[torch.Tensor] = None):
     """Gather hidden rows into expert-grouped order and quantise -> (q [cap, K] e4m3, s [cap, K/128]).
     Padding rows of a segment become zeros, or stay undefined with ``zero_padding=False`` (for a grouped
-    GEMM that is given the real row counts)."""
+    GEMM that is given the real row counts); then ``pos`` (int32 [T, k], the rows of every token) lets each token be quantised once."""
     K = hidden.shape[1]
     if not hidden.is_cuda:
         rows = hidden[src_row.clamp_min(0).long()].float()
@@ -159,6 +159,12 @@ def gather_quant(hidden: torch.Tensor, src_row: torch.Tensor, offsets: torch.Ten
     cap = src_row.shape[0]
     q = torch.empty(cap, K, dtype=FP8, device=hidden.device)
     s = fused._scale_buffer(cap, K // 128, hidden.device)
+    if pos is not None and not zero_padding and pos.shape[1] <= 32:
+        rc = _ext.lib().bg_moe_spread_quant(_ext.ptr(hidden), ctypes.c_int(hidden.stride(0)), _ext.ptr(pos), ctypes.c_int(pos.shape[1]), _ext.ptr(q),
+                                            _ext.ptr(s), ctypes.c_int(s.stride(1)), ctypes.c_int(pos.shape[0]), ctypes.c_int(K),
+                                            ctypes.c_int(int(pow2_scale)), _ext.stream())
+        _ext.check(rc, "bg_moe_spread_quant")
+        return q, s
     rc = _ext.lib().bg_moe_gather_quant(_ext.ptr(hidden), ctypes.c_int(hidden.stride(0)), _ext.ptr(src_row),
                                         _ext.ptr(offsets[-1:]), _ext.ptr(q), _ext.ptr(s), ctypes.c_int(s.stride(1)),
                                         ctypes.c_int(cap), ctypes.c_int(K), ctypes.c_int(int(pow2_scale)),
@@ -320,7 +326,7 @@ def experts_forward(hidden: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.
     if ew.quant == "fp8_block":
         counts = getattr(offsets, "real_counts", None)
         with timer.timed("moe.gather_quant"):
-            xq, xs = gather_quant(hidden, src, offsets, zero_padding=counts is None)
+            xq, xs = gather_quant(hidden, src, offsets, zero_padding=counts is None, pos=pos)
         y = grouped_experts(xq, xs, offsets, ew, timer=timer, counts=counts,
                             row_src=src if counts is not None else None,
                             rows_hint=(hidden.shape[0] * topk_idx.shape[1] if counts is not None else None))

@@ -172,3 +172,42 @@ def test_dense_bf16_pairs(T, N, K, pad):
     assert torch.equal(outs[0], outs[1]) and (outs[0][:, N:] == 7).all()
     got, want = outs[0][:, :N].cpu().double(), (x.cpu().double() @ w.cpu().double().t())
     assert ((got - want).abs() <= want.abs() * 2 ** -8 + (x.cpu().double().abs() @ w.cpu().double().abs().t()) * K * 2 ** -24).all()
+
+
+@pytest.mark.parametrize("T,K,local", [(1, 128, (0, 16)), (37, 640, (3, 9)), (700, 7168, (0, 16)), (1536, 2176, (12, 16))])
+def test_quantised_rows_of_tokens(T, K, local):
+    """A token's bytes and scales in the row of each of its local experts: those of the whole batch, by either walk."""
+    from batchgen_b200.ops import fused, moe, ref
+
+    torch.manual_seed(T)
+    x = (torch.randn(T, K + 8, device="cuda") * 3).to(torch.bfloat16)[:, 8:]
+    idx = torch.rand(T, 16, device="cuda").topk(5, -1)[1].to(torch.int32)
+    src, pos, offs = moe.permute(idx, *local)
+    assert ((pos >= 0) == ((idx >= local[0]) & (idx < local[1]))).all()
+    wq, ws = ref.act_quant(x.contiguous())
+    for kw in ({}, {"pos": pos}):
+        q, s = moe.gather_quant(x, src, offs, zero_padding=False, **kw)
+        rows = pos[pos >= 0].long()
+        token = torch.arange(T, device="cuda").unsqueeze(1).expand_as(pos)[pos >= 0]
+        fq, fs = fused.act_quant(x)
+        assert (q[rows].view(torch.uint8) == fq[token].view(torch.uint8)).all() and (s[rows] == fs[token]).all()
+        assert torch.allclose(s[rows], ws[token], rtol=1e-6, atol=0)          # the reference divides where the kernel multiplies: an ulp or two
+        assert (q[rows].view(torch.uint8) != wq[token].view(torch.uint8)).float().mean() < 2e-3     # as for whole batches: a byte at a rounding line
+
+
+@pytest.mark.parametrize("rope,D,pad", [(16, 24, 0), (64, 192, 8), (48, 128, 2), (24, 40, 0), (64, 64, 1)])
+def test_rotated_queries(rope, D, pad):
+    """Pieces of sixteen bytes where rows and dims allow them, pairs one by one elsewhere: the same rounding."""
+    from batchgen_b200.ops import fused, ref
+
+    torch.manual_seed(rope)
+    T, H = 19, 5
+    pos = torch.randint(0, 200, (T,), device="cuda", dtype=torch.int32)
+    ang = torch.rand(200, rope // 2, device="cuda") * 6
+    cos, sin = ang.cos(), ang.sin()
+    for inter in (True, False):
+        q = torch.randn(T, H * D + pad, device="cuda").to(torch.bfloat16)[:, pad:].unflatten(1, (H, D))
+        want = q.double().clone()
+        want[..., -rope:] = ref.apply_rope(q[..., -rope:].double(), cos[pos.long()].double(), sin[pos.long()].double(), inter).double()
+        bound = want.abs() * 2.0 ** -8 + q.double().abs().amax() * 2.0 ** -22         # one bf16 rounding of two fp32 products and a sum
+        assert ((fused.rope_q_(q.clone() if pad == 0 else q, pos, cos, sin, rope, inter).double() - want).abs() <= bound).all()
