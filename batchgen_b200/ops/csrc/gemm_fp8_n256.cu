@@ -15,6 +15,9 @@
 // accumulators and one 16-column read, and a warp of its own brings the scales, row times column block, to shared memory, four K
 // blocks at a time: loaded by the epilogue one block ahead they were spilled, and a spilled load waits for its whole latency in every
 // block.  6,144 x 4,096 x 7,168: 269 -> 216 us; 4,736 x 36,864 x 7,168: 1,363 -> 1,306 (power limited; 1,005 with an epilogue that reads nothing).
+// What a tile costs beside its K blocks is its stores, for the tensor cores stop two blocks into the next tile: four lanes swap the
+// pieces of their rows first and store whole sectors.  A row a lane and 16 bytes an access -> this: 5,900 x 24,576 x 1,536 394 us -> 315,
+// rows of 256 experts x 7,168 x 2,048 for 5,900 tokens 1,640 -> 1,400, 2,048 x 8,192 x 3,072 93 -> 85, 6,144 x 4,096 x 7,168 225 -> 209.
 //
 // Roles (640 threads, one CTA per SM, persistent): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warp 2 scales,
 // warps 4..19 epilogue.
@@ -115,6 +118,31 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* v) {
         "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
       : "r"(taddr)
       : "memory");
+}
+
+// sixteen bf16 of a row: a whole 32-byte sector in one store where it is aligned to one
+__device__ __forceinline__ void store16(__nv_bfloat16* dst, const uint32_t (&o)[8]) {
+  if ((reinterpret_cast<uintptr_t>(dst) & 31) == 0) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]),
+                 "r"(o[5]), "r"(o[6]), "r"(o[7])
+                 : "memory");
+  } else {
+    reinterpret_cast<uint4*>(dst)[0] = make_uint4(o[0], o[1], o[2], o[3]);
+    reinterpret_cast<uint4*>(dst)[1] = make_uint4(o[4], o[5], o[6], o[7]);
+  }
+}
+// Lanes `mask` apart: the upper one gives its first piece for the lower one's second.  Afterwards a and b are the same piece of two rows, so that
+// a warp's store covers whole runs of a row: with a row a lane it touches 32 lines.
+__device__ __forceinline__ void swap_pieces(uint32_t (&a)[8], uint32_t (&b)[8], int upper, int mask) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? a[i] : b[i], mask);
+    (upper ? a[i] : b[i]) = got;
+  }
+}
+__device__ __forceinline__ uint32_t bf16_pair(float2 v) {
+  const __nv_bfloat162 b = __floats2bfloat162_rn(v.x, v.y);
+  return *reinterpret_cast<const uint32_t*>(&b);
 }
 
 template <int EPI>
@@ -313,24 +341,35 @@ gemm_fp8_n256_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         }
       }
       if (!ok) break;
-      if (row_ok) {
-        if (EPI == EPI_SILU_MUL) {
-          const int col0 = gslice * 32;
-          const int n_out = p.N / 2;
-          __nv_bfloat16* dst = p.D + (size_t)row * p.ldd + col0;
+      if (EPI == EPI_SILU_MUL) {
+        __nv_bfloat16* dst = p.D + (size_t)row * p.ldd + gslice * 32;       // a row a lane: swapped pieces spill here, 10 % of the time
+        if (row_ok) {
 #pragma unroll
           for (int j = 0; j < 32; j += 8) {
-            if (col0 + j + 8 <= n_out) {
-              __align__(16) __nv_bfloat162 o[4];
+            __align__(16) __nv_bfloat162 o[4];
 #pragma unroll
-              for (int q = 0; q < 4; ++q)
-                o[q] = __floats2bfloat162_rn(silu(r2[j / 2 + q].x) * r2[16 + j / 2 + q].x,
-                                             silu(r2[j / 2 + q].y) * r2[16 + j / 2 + q].y);
-              *reinterpret_cast<uint4*>(dst + j) = *reinterpret_cast<const uint4*>(o);
-            }
+            for (int q = 0; q < 4; ++q)
+              o[q] = __floats2bfloat162_rn(silu(r2[j / 2 + q].x) * r2[16 + j / 2 + q].x, silu(r2[j / 2 + q].y) * r2[16 + j / 2 + q].y);
+            *reinterpret_cast<uint4*>(dst + j) = *reinterpret_cast<const uint4*>(o);
           }
-        } else {
-          const int col0 = gslice * 64;
+        }
+      } else {
+        const int col0 = gslice * 64;
+        if (p.row_map == nullptr && col0 + 64 <= p.N) {
+          uint32_t o[4][8];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) o[j / 8][j % 8] = bf16_pair(r2[j]);
+          const int piece = lane & 3;               // of the rows of four lanes
+          swap_pieces(o[0], o[2], lane & 2, 2);
+          swap_pieces(o[1], o[3], lane & 2, 2);
+          swap_pieces(o[0], o[1], lane & 1, 1);
+          swap_pieces(o[2], o[3], lane & 1, 1);
+          const int first_row = row - piece;
+          __nv_bfloat16* dst = p.D + (size_t)first_row * p.ldd + col0 + piece * 16;
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            if (first_row + r < t.m_end) store16(dst + (size_t)r * p.ldd, o[r]);
+        } else if (row_ok) {
           __nv_bfloat16* dst = p.D + (size_t)row * p.ldd + col0;
           if (p.row_map != nullptr) {
             const int2 rm = p.row_map[row];
@@ -340,10 +379,7 @@ gemm_fp8_n256_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 #pragma unroll
           for (int j = 0; j < 64; j += 8) {
             if (col0 + j + 8 <= p.N) {
-              __align__(16) __nv_bfloat162 o[4];
-#pragma unroll
-              for (int q = 0; q < 4; ++q) o[q] = __floats2bfloat162_rn(r2[j / 2 + q].x, r2[j / 2 + q].y);
-              *reinterpret_cast<uint4*>(dst + j) = *reinterpret_cast<const uint4*>(o);
+              *reinterpret_cast<uint4*>(dst + j) = make_uint4(bf16_pair(r2[j / 2]), bf16_pair(r2[j / 2 + 1]), bf16_pair(r2[j / 2 + 2]), bf16_pair(r2[j / 2 + 3]));
             } else {
               for (int q = 0; q < 8; ++q)
                 if (col0 + j + q < p.N) dst[j + q] = __float2bfloat16((q & 1) ? r2[(j + q) / 2].y : r2[(j + q) / 2].x);

@@ -165,6 +165,25 @@ def test_wide_tile_fp8_gemm_matches_reference(T, N, K, silu):
     assert _rel(narrow, want) < 1e-2 and _rel(got, narrow) < 2e-3
 
 
+@pytest.mark.parametrize("T,N,pad,silu", [(129, 320, 0, False), (131, 320, 8, False), (126, 256, 24, False), (3, 264, 8, False), (131, 256, 0, True), (129, 512, 8, True)])
+def test_wide_tile_stores(T, N, pad, silu):
+    """Row groups cut by the last row, column slices cut by N, rows that start inside a sector: the same values, nothing beside them."""
+    from batchgen_b200.ops import gemm, ref
+    g = torch.Generator().manual_seed(T + N)
+    xq, xs = ref.act_quant(torch.randn(T, 256, generator=g))
+    wq = (torch.randn(N, 256, generator=g) * 0.1).to(torch.float8_e4m3fn)
+    ws = torch.rand((N + 127) // 128, 2, generator=g) + 0.5
+    want = ref.fp8_gemm(xq, xs, wq, ws)
+    if silu:
+        want = ref.silu_mul(want)
+        wq = wq.view(torch.uint8)[gemm.interleave_gate_up_rows(N)].contiguous().view(torch.float8_e4m3fn)
+    n = want.shape[1]
+    buf = torch.full((T + 4, n + pad), 768.0, dtype=torch.bfloat16, device="cuda")
+    gemm.fp8_gemm(xq.cuda(), xs.cuda().t().contiguous().t(), wq.cuda(), ws.cuda(), out=buf[:T, pad:], silu_mul=silu, wide=True)
+    assert _rel(buf[:T, pad:].float().cpu(), want) < 1e-2              # as above: bf16 results of the same sums
+    assert (buf[T:] == 768).all() and (buf[:, :pad] == 768).all()
+
+
 def test_wide_tile_grouped_gemm_with_counts():
     from batchgen_b200.ops import _ext, gemm, ref
     FP8 = torch.float8_e4m3fn
