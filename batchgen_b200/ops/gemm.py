@@ -64,9 +64,13 @@ def hooks_pending() -> None:
     _hooks_pending = True
 
 
-def _use_wide(kind, D, M, N, wide) -> bool:
-    """128 x 256 tiles pay off when there are plenty of tiles to fill the SMs; GEMMs that consume collective
-    hooks (rows stored to peers, flag waits) and bf16 operands stay on the 128 x 128 kernel."""
+def _use_wide(kind, D, M, N, wide, dense) -> bool:
+    """128 x 256 tiles pay off as soon as a dense product has more than one round of 128 x 128 ones, for their K blocks take hardly
+    longer.  us, narrow and wide, K x N and rows: 16,384 x 7,168, 384 rows (168 narrow tiles) 105 and 78, 512 rows 132 and 78;
+    7,168 x 4,096, 651 rows (192) 58 and 41, 512 rows (128) 33 and 40; 7,168 x 2,112, 1,185 rows (170) 62 and 43, 1,024 rows (136) 35
+    and 43; 6,144 x 3,072, 900 rows (192) 50 and 35, 768 rows (144) 29 and 35.  Grouped products, whose tiles are an upper bound here,
+    keep two rounds.  GEMMs that consume collective hooks (rows stored to peers, flag waits) and bf16 operands stay on the 128 x 128
+    kernel, and in its second round rows that the wide one does not take (row stride no multiple of 8)."""
     global _hooks_pending
     if _hooks_pending:
         _hooks_pending = False
@@ -76,7 +80,8 @@ def _use_wide(kind, D, M, N, wide) -> bool:
     if wide is True or _WIDE == "1":
         return True
     tiles = -(-M // 128) * -(-N // 128)
-    return tiles >= 2 * _ext.num_sms(D.device)
+    sms = _ext.num_sms(D.device)
+    return tiles >= 2 * sms or dense and tiles > sms and D.stride(0) % 8 == 0
 
 
 def wide_enabled() -> bool:
@@ -123,7 +128,7 @@ def _launch(kind, epi, A, sA, sa_stride, B, sB, D, offsets, groups, M, N, K, wid
                                   base, ctypes.c_int(world), _ext.ptr(_ext.status_word(A.device)), _ext.stream())
         _ext.check(rc, "bg_gemm_fp8_swapab")
         return
-    if a_ready is not None or _use_wide(kind, D, M, N, wide):
+    if a_ready is not None or _use_wide(kind, D, M, N, wide, offsets is None):
         flag, epoch, base, world = a_ready if a_ready is not None else (ctypes.c_void_p(0), 0, ctypes.c_void_p(0), 1)
         rc = L.bg_gemm_fp8_n256(ctypes.c_int(epi), _ext.ptr(A), _ext.ptr(sA), ctypes.c_int(sa_stride), _ext.ptr(B),
                                 _ext.ptr(sB), _ext.ptr(D), ctypes.c_int(D.stride(0)), _ext.ptr(offsets), _ext.ptr(counts),

@@ -165,6 +165,20 @@ def test_wide_tile_fp8_gemm_matches_reference(T, N, K, silu):
     assert _rel(narrow, want) < 1e-2 and _rel(got, narrow) < 2e-3
 
 
+@pytest.mark.parametrize("T,N,wide", [(130, 9472, False), (130, 9600, True), (300, 6400, True), (600, 3840, True)])
+def test_tile_width_of_a_second_round(T, N, wide):
+    """Either side of one round of 128 x 128 tiles (148 SMs): the bytes of the kernel that the rule names."""
+    from batchgen_b200.ops import _ext, gemm, ref
+    if _ext.num_sms(torch.device("cuda")) != 148:
+        pytest.skip("rounds of 148 SMs")
+    xq, xs = ref.act_quant(torch.randn(T, 128))
+    wq, ws = (torch.randn(N, 128) * 0.1).to(torch.float8_e4m3fn), torch.rand((N + 127) // 128, 1) + 0.5
+    a = [v.cuda() for v in (xq, xs, wq, ws)]
+    got = gemm.fp8_gemm(*a)
+    assert torch.equal(got, gemm.fp8_gemm(*a, wide=wide))
+    assert _rel(got.float().cpu(), ref.fp8_gemm(xq, xs, wq, ws)) < 1e-2
+
+
 @pytest.mark.parametrize("T,N,pad,silu", [(129, 320, 0, False), (131, 320, 8, False), (126, 256, 24, False), (3, 264, 8, False), (131, 256, 0, True), (129, 512, 8, True)])
 def test_wide_tile_stores(T, N, pad, silu):
     """Row groups cut by the last row, column slices cut by N, rows that start inside a sector: the same values, nothing beside them."""
