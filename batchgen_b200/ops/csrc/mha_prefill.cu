@@ -15,6 +15,10 @@
 // S in TMEM (two bf16 to a column) as the A operand of P.V.  K/V tiles flow through a 3-stage TMA ring; S of tile t+1 is issued before P.V of
 // tile t.
 //
+// The warps of a half wait for nothing but their own tiles, so a fast one is up to a tile ahead of a slow one: it may store P of t+1 while the
+// other still rescales O for t.  So P has a barrier for each S buffer: a warp's next arrival there needs S of t+2, which follows P.V of t and
+// with it all four arrivals for t.
+//
 // With one 128-query tile a CTA and P through shared memory, the product of S, the softmax and P.V took turns.  One softmax warp's exponentials
 // take 512 of the tensor cores' 640 clocks for 128 queries x 64 keys.  128 heads: prompts of 2,048, 1,461, 874 and 1,000 tokens 654 -> 408 us
 // (813 TFLOP/s), 1,536 tokens behind 5,000 1,023 -> 654 (1,110); 32 heads, 4,096 tokens 293 -> 195.  What is left is each CTA's start and end,
@@ -53,7 +57,7 @@ struct Shared {
   uint64_t kv_full[kStages];
   uint64_t kv_empty[kStages];
   uint64_t s_full[2][2];     // [half][buffer]
-  uint64_t p_full[2];
+  uint64_t p_full[2][2];
   uint64_t o_done[2];
   uint32_t tmem_base;
   int abort_flag;
@@ -117,7 +121,8 @@ mha_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     for (int x = 0; x < 2; ++x) {
       mbar_init(&ss.s_full[x][0], 1);
       mbar_init(&ss.s_full[x][1], 1);
-      mbar_init(&ss.p_full[x], 4);
+      mbar_init(&ss.p_full[x][0], 4);
+      mbar_init(&ss.p_full[x][1], 4);
       mbar_init(&ss.o_done[x], 1);
     }
     ss.abort_flag = 0;
@@ -189,7 +194,7 @@ mha_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           const int mine = x ? tiles1 : tiles0;
           if (t >= mine) continue;
           if (ready && t + 1 < mine) issue_s(x, t + 1);
-          if (!mbar_wait(&ss.p_full[x], t & 1, abort_flag, kTimeoutMma)) { ok = false; break; }
+          if (!mbar_wait(&ss.p_full[x][t & 1], (t >> 1) & 1, abort_flag, kTimeoutMma)) { ok = false; break; }
           tc_fence_after();
           const uint32_t tm_p = tmem_base + x * kHalfCols + (t & 1) * BN, tm_o = tmem_base + x * kHalfCols + 2 * BN;
 #pragma unroll
@@ -271,7 +276,7 @@ mha_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       m_run = m_new;
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ss.p_full[x]);
+      if (lane == 0) mbar_arrive(&ss.p_full[x][t & 1]);
     }
     if (ok && mine > 0) ok = __all_sync(0xffffffffu, mbar_wait(&ss.o_done[x], (mine - 1) & 1, abort_flag, kTimeoutEpilogue));
     if (ok && mine > 0) {

@@ -1,5 +1,7 @@
 """Per-head batched GEMM (MLA absorb / out-absorb) and the grouped GEMM's real-row counts, against fp32
 references of the same ops."""
+import math
+
 import pytest
 import torch
 
@@ -109,6 +111,44 @@ def test_expanded_mla_prefill_halves(lens, ctx):
         # probabilities and output rounded to 8 bits, exponents of fp32 sums of 192 products
         bound = torch.einsum("nhl,lhd->nhd", p, v.abs()) * 2.0 ** -7 + 1e-6
         assert ((got[a:a + n] - torch.einsum("nhl,lhd->nhd", p, v)).abs() <= bound).all(), i
+
+
+def _uneven(n_q, ctx, H, seed):
+    """Queries behind ``ctx`` cached keys of which one group of 32 (one warp's rows) scores every tile of 64 keys 2^12 above the tile before, all others flat."""
+    g = torch.Generator().manual_seed(seed)
+    tk = n_q + ctx
+    q, kv, kpe = torch.zeros(n_q, H, 192), torch.zeros(tk, H, 256), torch.zeros(tk, 64)
+    steep = torch.arange(n_q) // 32 % 4 == seed % 4
+    q[steep, :, 0] = 1.0
+    kv[:, :, 0] = (12.0 * (torch.arange(tk) // 64)).view(-1, 1)
+    kv[:, :, 128:] = torch.randn(tk, H, 128, generator=g) + 1
+    return tuple(v.to(torch.bfloat16) for v in (q, kv, kpe))
+
+
+def _attention64(q, kv, ctx, scale):
+    """Softmax attention of one sequence in 64 bits, and the same of the values' magnitudes."""
+    k, v = kv[..., :128].double(), kv[..., 128:].double()
+    s = torch.einsum("nhd,lhd->nhl", q[..., :128].double(), k) * scale
+    s.masked_fill_((torch.arange(kv.shape[0]) > torch.arange(q.shape[0]).view(-1, 1) + ctx).unsqueeze(1), -float("inf"))
+    p = s.softmax(-1)
+    return torch.einsum("nhl,lhd->nhd", p, v), torch.einsum("nhl,lhd->nhd", p, v.abs())
+
+
+@pytest.mark.parametrize("n_q,ctx,seed", [(128, 1000, 0), (65, 640, 1), (100, 1900, 3), (256, 900, 2), (200, 576, 0), (700, 0, 1)])
+def test_expanded_mla_prefill_uneven_warps(n_q, ctx, seed):
+    """A warp that rescales at every tile beside three that never do: each tile's probabilities are multiplied when all four have stored theirs."""
+    from batchgen_b200.ops import _ext, attention
+    H, scale = 32, math.log(2.0)                        # scores in powers of two
+    q, kv, kpe = _uneven(n_q, ctx, H, seed)
+    work = attention.mha_prefill_work([0, n_q], [ctx], [0])
+    args = (q.cuda(), kv.cuda(), kpe.cuda(), work, scale)
+    got = attention.mha_prefill(*args)
+    again = [attention.mha_prefill(*args) for _ in range(4)]
+    _ext.check_status()
+    assert all(torch.equal(got, a) for a in again)
+    want, mag = _attention64(q, kv, ctx, scale)
+    # probabilities and output rounded to 8 bits; scores are exact, exponents up to 2^9 are fp32 sums
+    assert ((got.cpu().double() - want).abs() <= mag * 2.0 ** -7 + 1e-6).all()
 
 
 def test_model_prefill_uses_expanded_attention_and_matches_cpu():
