@@ -17,7 +17,8 @@
 //
 // The warps of a half wait for nothing but their own tiles, so a fast one is up to a tile ahead of a slow one: it may store P of t+1 while the
 // other still rescales O for t.  So P has a barrier for each S buffer: a warp's next arrival there needs S of t+2, which follows P.V of t and
-// with it all four arrivals for t.
+// with it all four arrivals for t.  The end of P.V likewise: a warp that does not rescale waits for none but the last, two phases after what its
+// last scores say is complete, where one barrier's parity is the same again.
 //
 // With one 128-query tile a CTA and P through shared memory, the product of S, the softmax and P.V took turns.  One softmax warp's exponentials
 // take 512 of the tensor cores' 640 clocks for 128 queries x 64 keys.  128 heads: prompts of 2,048, 1,461, 874 and 1,000 tokens 654 -> 408 us
@@ -58,7 +59,7 @@ struct Shared {
   uint64_t kv_empty[kStages];
   uint64_t s_full[2][2];     // [half][buffer]
   uint64_t p_full[2][2];
-  uint64_t o_done[2];
+  uint64_t o_done[2][2];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -123,7 +124,8 @@ mha_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       mbar_init(&ss.s_full[x][1], 1);
       mbar_init(&ss.p_full[x][0], 4);
       mbar_init(&ss.p_full[x][1], 4);
-      mbar_init(&ss.o_done[x], 1);
+      mbar_init(&ss.o_done[x][0], 1);
+      mbar_init(&ss.o_done[x][1], 1);
     }
     ss.abort_flag = 0;
     mbar_fence_init();
@@ -200,7 +202,7 @@ mha_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
           for (int j = 0; j < BN / 16; ++j)
             mma_f16_ta(tm_o, tm_p + 8 * j, desc_mn_sw128(v_base + j * 2048, BN * 128, 1024), idesc_pv, (t > 0 || j > 0) ? 1u : 0u);
-          tc_commit(&ss.o_done[x]);
+          tc_commit(&ss.o_done[x][t & 1]);
         }
         if (!ok) break;
         tc_commit(&ss.kv_empty[s]);
@@ -248,7 +250,7 @@ mha_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       const float alpha = (grow && m_run != -INFINITY) ? ex2(m_run - m_new) : 1.f;
       if (t > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
         // P.V of the tile before this one (that of earlier ones was complete when S of this tile was)
-        if (!__all_sync(0xffffffffu, mbar_wait(&ss.o_done[x], (t - 1) & 1, abort_flag, kTimeoutEpilogue))) { ok = false; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait(&ss.o_done[x][(t - 1) & 1], ((t - 1) >> 1) & 1, abort_flag, kTimeoutEpilogue))) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
@@ -278,7 +280,7 @@ mha_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       __syncwarp();
       if (lane == 0) mbar_arrive(&ss.p_full[x][t & 1]);
     }
-    if (ok && mine > 0) ok = __all_sync(0xffffffffu, mbar_wait(&ss.o_done[x], (mine - 1) & 1, abort_flag, kTimeoutEpilogue));
+    if (ok && mine > 0) ok = __all_sync(0xffffffffu, mbar_wait(&ss.o_done[x][(mine - 1) & 1], ((mine - 1) >> 1) & 1, abort_flag, kTimeoutEpilogue));
     if (ok && mine > 0) {
       tc_fence_after();
       const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;

@@ -151,6 +151,24 @@ def test_expanded_mla_prefill_uneven_warps(n_q, ctx, seed):
     assert ((got.cpu().double() - want).abs() <= mag * 2.0 ** -7 + 1e-6).all()
 
 
+@pytest.mark.parametrize("n_q,ctx,seed", [(1, 64, 0), (40, 200, 0), (128, 1025, 2), (129, 511, 3), (256, 0, 1), (512, 700, 0)])
+def test_expanded_mla_prefill_last_tiles(n_q, ctx, seed):
+    """Values that are zero but in the last two key tiles: a warp that ends first still waits for both."""
+    from batchgen_b200.ops import _ext, attention
+    H, scale = 48, math.log(2.0)
+    q, kv, kpe = _uneven(n_q, ctx, H, seed)
+    last = (n_q + ctx - 1) // 64
+    kv[:max(0, (last - 1) * 64), :, 128:] = 0
+    work = attention.mha_prefill_work([0, n_q], [ctx], [0])
+    args = (q.cuda(), kv.cuda(), kpe.cuda(), work, scale)
+    got = attention.mha_prefill(*args)
+    again = [attention.mha_prefill(*args) for _ in range(4)]
+    _ext.check_status()
+    assert all(torch.equal(got, a) for a in again)
+    want, mag = _attention64(q, kv, ctx, scale)
+    assert ((got.cpu().double() - want).abs() <= mag * 2.0 ** -7 + 1e-6).all()          # as above
+
+
 def test_model_prefill_uses_expanded_attention_and_matches_cpu():
     from batchgen_b200.config import get_model_config
     from batchgen_b200.models import build_model
