@@ -99,7 +99,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
         const uint32_t bytes = 2 * (kWBytes + half * kRowBytes);
         for (int kb = 0; kb < KB; ++kb, ++it) {
           const int s = it % kStages;
-          if (!mbar_wait(&ss.empty[s], ((it / kStages) & 1) ^ 1, abort_flag, kTimeoutProducer)) { ok = false; break; }
+          if (!pair::wait_cluster(&ss.empty[s], ((it / kStages) & 1) ^ 1, abort_flag, kTimeoutProducer)) { ok = false; break; }
           if (rank == 0) mbar_expect_tx(&ss.full[s], bytes);
           const uint32_t bar = pair::leader_addr(&ss.full[s]);
           uint8_t* x = x_tiles + s * kXBytes;
@@ -112,7 +112,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
       if (ok) {
         const uint32_t n = it < (uint32_t)kStages ? it : (uint32_t)kStages;
         for (uint32_t j = it - n; j < it; ++j)
-          if (!mbar_wait(&ss.empty[j % kStages], (j / kStages) & 1, abort_flag, kTimeoutProducer)) break;
+          if (!pair::wait_cluster(&ss.empty[j % kStages], (j / kStages) & 1, abort_flag, kTimeoutProducer)) break;
       } else {
         for (uint32_t i = 0; i < (1u << 16); ++i) __nanosleep(20);   // bounded grace period for copies in flight
       }
@@ -123,11 +123,11 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
       for (int tile = first; ok && walk.get(tile, t); tile += step, ++acc) {
         const int buf = acc & 1;
         const uint32_t idesc = make_idesc(BW, pair_cols(t), 1, 1);   // bf16 x bf16 -> fp32
-        if (!mbar_wait(&ss.tmem_empty[buf], ((acc >> 1) & 1) ^ 1, abort_flag, kTimeoutMma)) { ok = false; break; }
+        if (!pair::wait_cluster(&ss.tmem_empty[buf], ((acc >> 1) & 1) ^ 1, abort_flag, kTimeoutMma)) { ok = false; break; }
         tc_fence_after();
         for (int kb = 0; kb < KB; ++kb, ++it) {
           const int s = it % kStages;
-          if (!mbar_wait(&ss.full[s], (it / kStages) & 1, abort_flag, kTimeoutMma)) { ok = false; break; }
+          if (!pair::wait_cluster(&ss.full[s], (it / kStages) & 1, abort_flag, kTimeoutMma)) { ok = false; break; }
           tc_fence_after();
           const uint64_t adesc = make_smem_desc_sw128(smem_u32(w_tiles + s * kWBytes));
           const uint64_t bdesc = make_smem_desc_sw128(smem_u32(x_tiles + s * kXBytes));
@@ -144,7 +144,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
     const int side = (warp - 4) >> 2;
     for (int tile = first; ok && walk.get(tile, t); tile += step, ++acc) {
       const int buf = acc & 1;
-      if (!__all_sync(0xffffffffu, mbar_wait(&ss.tmem_full[buf], (acc >> 1) & 1, abort_flag, kTimeoutEpilogue))) { ok = false; break; }
+      if (!__all_sync(0xffffffffu, pair::wait_cluster(&ss.tmem_full[buf], (acc >> 1) & 1, abort_flag, kTimeoutEpilogue))) { ok = false; break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + buf * BT;
       const int n_tok = t.m_end - t.m0, row0 = t.n0 + rank * (BW / 2) + quad * 32, col = row0 + 8 * (lane & 3);

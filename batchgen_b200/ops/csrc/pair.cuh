@@ -24,11 +24,40 @@ __device__ __forceinline__ uint32_t leader_addr(const void* p) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(out) : "r"(smem_u32(p)));
   return out;
 }
-// Arrive on a barrier in either CTA.  What the barriers of a pair hand over is TMEM (ordered by the tcgen05 fences) and tiles that the asynchronous
-// proxy writes and reads, nothing of this thread's own stores: release and acquire at cluster scope would only cost their fence, some
-// thousand clocks.
+// Arrive on a barrier in either CTA, for a thread there that waits with wait_cluster: what the arriving thread has read is read before what
+// the waiting one issues, across CTAs only at cluster scope.
 __device__ __forceinline__ void arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool try_wait_cluster(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// mbar_wait for a barrier of this CTA on which the other CTA's threads, loads or products arrive too
+__device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int why) {
+  uint64_t t0 = 0;
+  for (uint32_t i = 0;; ++i) {
+    if (try_wait_cluster(bar, parity)) return true;
+    if ((i & 255u) == 255u) {
+      if (*abort_flag) return false;
+      if ((i & 0xFFFFu) == 0xFFFFu) {
+        const uint64_t t = global_timer_ns();
+        if (t0 == 0) t0 = t;
+        else if (t - t0 > kWaitBudgetNs) break;
+      }
+    }
+  }
+  if (*abort_flag == 0) *abort_flag = why;
+  return false;
 }
 
 // a tile load into this CTA whose bytes count on the barrier at shared::cluster address `bar`, in either CTA
