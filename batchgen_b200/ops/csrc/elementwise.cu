@@ -140,6 +140,29 @@ act_quant_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, f
   }
 }
 
+// MODE 1 for many blocks, a CTA a row.  Exponential and division bound it as much as its bytes, so resident warps count more than loads in flight:
+// 4,739 rows of 7,168 51 us, warps that walk the rows 60 with one block a half-warp and 80 with four, 2,400 rows of 4,096 20.5, 22.5 and 31; for
+// few blocks the walk's spread over the SMs wins, 256 rows of 7,168 12.3 against 10.2.
+__global__ void __launch_bounds__(256)
+silu_quant_rows_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ s, int s_stride, int K, int ldx, int pow2,
+                       const int* __restrict__ valid_rows, const int* __restrict__ row_src) {
+  bg::pdl_prologue((BG_FILE_TAG << 16) | __LINE__);
+  const int t = blockIdx.x;
+  if (valid_rows != nullptr && t >= *valid_rows) return;
+  if (row_src != nullptr && row_src[t] < 0) return;
+  const __nv_bfloat16* xr = x + (size_t)t * ldx;
+  for (int v = threadIdx.x; v < K / 8; v += blockDim.x) {            // K is a multiple of 128: a block's sixteen lanes stay together
+    float f[8], u[8];
+    unpack8(*reinterpret_cast<const uint4*>(xr + v * 8), f);
+    unpack8(*reinterpret_cast<const uint4*>(xr + K + v * 8), u);
+    // round the activation to bf16 first: same bytes as silu_mul (bf16) followed by act_quant
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = __bfloat162float(__float2bfloat16(silu(f[i]) * u[i]));
+    const float sc = quant_block(f, q + (size_t)t * K + v * 8, pow2, 0xffffu << (threadIdx.x & 16));
+    if ((threadIdx.x & 15) == 0) s[(size_t)(v / 16) * s_stride + t] = sc;
+  }
+}
+
 // MLA latent-KV producer.  One block (128 threads) per token:
 //   cache[slot, 0:kv_lora]        = rmsnorm(kv_a[t, 0:kv_lora]) * w
 //   cache[slot, kv_lora:+rope]    = rope(kv_a[t, kv_lora:], position[t])
@@ -284,7 +307,12 @@ int bg_act_quant(int mode, const void* x, void* q, float* s, int s_stride, int T
   auto X = reinterpret_cast<const __nv_bfloat16*>(x);
   auto Q = reinterpret_cast<uint8_t*>(q);
   const bool many = many_blocks(T, K);
-  auto kern = mode == 0 ? (many ? act_quant_kernel<0, 4> : act_quant_kernel<0, 1>) : (many ? act_quant_kernel<1, 4> : act_quant_kernel<1, 1>);
+  if (mode != 0 && many) {
+    const int threads = K / 8 >= 256 ? 256 : (K / 8 + 31) / 32 * 32;
+    bg::launch_pdl(silu_quant_rows_kernel, dim3(T), dim3(threads), 0, stream, X, Q, s, s_stride, K, ldx, pow2, valid_rows, row_src);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
+  auto kern = mode == 0 ? (many ? act_quant_kernel<0, 4> : act_quant_kernel<0, 1>) : act_quant_kernel<1, 1>;
   bg::launch_pdl(kern, dim3(walk_grid(T, K, many ? 4 : 1)), dim3(256), 0, stream, X, Q, s, s_stride, T, K, ldx, pow2, valid_rows, row_src);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

@@ -35,7 +35,8 @@ __device__ __forceinline__ float quant_block(const float (&f)[8], uint8_t* q, in
 
 // Rows of K elements in groups of 2 U blocks, a group a warp (a half-warp a block): all U loads of a lane are on their way together, and a
 // capacity above the rows that are present costs nothing.  A CTA a row kept one load in flight and cost its start for every padding row:
-// expert rows of 2,048 for 4,739 tokens (8 of 256 experts, segments of 128) 94 us, now 65; 4 tokens 14, now 8.  Few blocks (a decode step) take U = 1, so that they spread over the SMs.
+// expert rows of 2,048 for 4,739 tokens (8 of 256 experts, segments of 128) 94 us, now 65; 4 tokens 14, now 8.  Few blocks (a decode step) take U = 1, so
+// that they spread over the SMs.
 constexpr int kWalkBlocks = 148 * 8;
 inline bool many_blocks(long long rows, int K) { return rows * (K / 128) >= 148ll * 64 * 2; }
 inline int walk_grid(long long rows, int K, int U) {

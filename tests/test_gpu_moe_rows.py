@@ -211,3 +211,28 @@ def test_rotated_queries(rope, D, pad):
         want[..., -rope:] = ref.apply_rope(q[..., -rope:].double(), cos[pos.long()].double(), sin[pos.long()].double(), inter).double()
         bound = want.abs() * 2.0 ** -8 + q.double().abs().amax() * 2.0 ** -22         # one bf16 rounding of two fp32 products and a sum
         assert ((fused.rope_q_(q.clone() if pad == 0 else q, pos, cos, sin, rope, inter).double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("K", [128, 384, 2048, 7168])
+@pytest.mark.parametrize("padding", [False, True])
+def test_quantised_activation_of_few_and_many_rows(K, padding):
+    """SiLU * up quantised by warps that walk the rows and, from 18,944 blocks on, by a CTA a row: the same bytes."""
+    from batchgen_b200.ops import fused
+
+    T = -(-148 * 128 // (K // 128))                          # the first number of rows that takes the second form
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x = (torch.randn(T, 2 * K + 8, device="cuda", generator=g) * 3).to(torch.bfloat16)[:, 8:]
+    src = torch.arange(T, device="cuda", dtype=torch.int32)
+    kw = {}
+    if padding:
+        src[::7] = -1
+        kw = dict(valid_rows=torch.tensor([T - 3], dtype=torch.int32, device="cuda"), row_src=src)
+    kept = (src >= 0) & (torch.arange(T, device="cuda") < (T - 3 if padding else T))
+    q, s = fused.act_quant(x, silu_mul=True, **kw)
+    few = [fused.act_quant(x[a:b], silu_mul=True) for a, b in ((0, T // 2), (T // 2, T))]
+    assert (q.view(torch.uint8)[kept] == torch.cat([f[0].view(torch.uint8) for f in few])[kept]).all() and (s[kept] == torch.cat([f[1] for f in few])[kept]).all()
+    y = x.double()
+    want = (torch.nn.functional.silu(y[:, :K]) * y[:, K:])[kept]
+    step = s[kept].double().repeat_interleave(128, 1)
+    # a value rounded to 8 bits, then to 4, in units of the scale down to 2^-9 of it
+    assert ((q[kept].double() * step - want).abs() <= want.abs() * (2.0 ** -4 + 2.0 ** -8) + step * 2.0 ** -10).all()
