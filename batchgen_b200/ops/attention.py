@@ -212,7 +212,7 @@ def mha_prefill(q: torch.Tensor, kv: torch.Tensor, kpe: torch.Tensor, work: torc
     work = work.to(q.device)
     rc = _ext.lib().bg_mha_prefill(_ext.ptr(q), _ext.ptr(kv), _ext.ptr(kpe), ctypes.c_longlong(kpe.stride(0)), _ext.ptr(out),
                                    _ext.ptr(work), ctypes.c_int(work.shape[0]), ctypes.c_int(Tq), ctypes.c_int(Tk),
-                                   ctypes.c_int(H), ctypes.c_float(scale), _ext.ptr(_ext.status_word(q.device)),
-                                   _ext.stream())
+                                   ctypes.c_int(H), ctypes.c_float(scale), ctypes.c_int(_ext.num_sms(q.device)),
+                                   _ext.ptr(_ext.status_word(q.device)), _ext.stream())
     _ext.check(rc, "bg_mha_prefill")
     return out

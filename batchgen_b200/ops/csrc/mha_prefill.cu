@@ -25,6 +25,10 @@
 // (813 TFLOP/s), 1,536 tokens behind 5,000 1,023 -> 654 (1,110); 32 heads, 4,096 tokens 293 -> 195.  What is left is each CTA's start and end,
 // some 4 us a tile, and the diagonal.
 //
+// Where the halves of all tiles find an SM each, a half is a CTA by itself (grid z): two in one CTA would take turns beside idle SMs.  Heads x
+// tokens, one half a CTA / two / the kernel of one 128-query tile: 8 x 2,048 39 / 46 / 44 us, 1 x 4,096 59 / 77 / 72, 16 x 140 behind 4,000 66 / 80 / 78; past
+// one round two halves win, 64 x 300 23 / 18 / 20, 8 x 4,096 92 / 84 / 94.
+//
 // Roles (384 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 4..7 and 8..11 softmax / epilogue of a half.
 // All waits are bounded (common.cuh).
 //
@@ -110,8 +114,17 @@ mha_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   Shared& ss = *reinterpret_cast<Shared*>(v_buf + kStages * kVBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* abort_flag = &ss.abort_flag;
-  const Work w = work[blockIdx.x];
+  Work w = work[blockIdx.x];
   const int h = blockIdx.y;
+  if (gridDim.z > 1) {                    // one half of the tile
+    if (blockIdx.z > 0) {
+      w.q_row0 += BM;
+      w.kv0 += BM;
+      w.n_q -= BM;
+    }
+    w.n_q = min(w.n_q, BM);
+    if (w.n_q <= 0) return;
+  }
   // key tiles that a half sees: up to its last query's
   const int tiles0 = (w.kv0 + min(w.n_q, BM) - 1 + BN - 1) / BN, tiles1 = w.n_q > BM ? (w.kv0 + w.n_q - 1 + BN - 1) / BN : 0;
   const int n_tiles = max(tiles0, tiles1);
@@ -345,9 +358,9 @@ extern "C" {
 
 // q [Tq, H, 192] (nope | roped pe), kv [Tk, H, 256] (key nope | value: the kv_b projection of the latent rows),
 // kpe [Tk, kpe_stride] (roped shared key part in the first 64 columns), out [Tq, H, 128]: bf16.
-// work: n_work x 4 ints (q_row0, n_q, k_row0, kv0), one CTA per work item and head.
+// work: n_work x 4 ints (q_row0, n_q, k_row0, kv0), one CTA per work item and head, or two where all of them fit the SMs at once.
 int bg_mha_prefill(const void* q, const void* kv, const void* kpe, long long kpe_stride, void* out, const int* work,
-                   int n_work, int Tq, int Tk, int H, float scale, int* status, cudaStream_t stream) {
+                   int n_work, int Tq, int Tk, int H, float scale, int num_sms, int* status, cudaStream_t stream) {
   using namespace bg::mha;
   if (n_work <= 0 || H <= 0) return 0;
   if (kpe_stride % 8 != 0) return -1;
@@ -358,7 +371,7 @@ int bg_mha_prefill(const void* q, const void* kv, const void* kpe, long long kpe
   static bg::DeviceOnce attr_set;
   const size_t smem = 2 * kQBytes + kStages * (kKBytes + kVBytes) + sizeof(Shared) + 1024;
   if (!bg::ensure_dynamic_smem(mha_prefill_kernel, smem, attr_set)) return -13;
-  dim3 grid(n_work, H);
+  dim3 grid(n_work, H, 2ll * n_work * H <= num_sms ? 2 : 1);
   mha_prefill_kernel<<<grid, kThreads, smem, stream>>>(tq, tk, tv, reinterpret_cast<const Work*>(work),
                                                        reinterpret_cast<__nv_bfloat16*>(out), H,
                                                        scale * 1.4426950408889634f, status);

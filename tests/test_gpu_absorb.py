@@ -169,6 +169,27 @@ def test_expanded_mla_prefill_last_tiles(n_q, ctx, seed):
     assert ((got.cpu().double() - want).abs() <= mag * 2.0 ** -7 + 1e-6).all()          # as above
 
 
+@pytest.mark.parametrize("lens,ctx", [([1], [0]), ([128], [70]), ([129], [0]), ([255, 300, 64], [1, 64, 500]), ([1200], [63])])
+def test_expanded_mla_prefill_halves_as_ctas(lens, ctx):
+    """Few tiles take a CTA for each half of a tile: the bits of the same heads among so many that a CTA has both."""
+    from batchgen_b200.ops import _ext, attention
+    g = torch.Generator().manual_seed(sum(lens))
+    cu, k_starts, tk = [0], [], 0
+    for n, c in zip(lens, ctx):
+        cu.append(cu[-1] + n)
+        k_starts.append(tk)
+        tk += n + c
+    q, kv, kpe = (torch.randn(*shape, generator=g).to(torch.bfloat16).cuda() for shape in ((cu[-1], 2, 192), (tk, 2, 256), (tk, 64)))
+    work = attention.mha_prefill_work(cu, ctx, k_starts)
+    sms = _ext.num_sms(q.device)
+    assert 2 * work.shape[0] * 2 <= sms
+    many = sms // 2 + 1                                  # pairs of heads, all the same: one CTA an item and head
+    few = attention.mha_prefill(q, kv, kpe, work, 0.1)
+    all_ = attention.mha_prefill(q.repeat(1, many, 1), kv.repeat(1, many, 1), kpe, work, 0.1).view(cu[-1], many, 2, 128)
+    _ext.check_status()
+    assert (all_ == few.unsqueeze(1)).all()
+
+
 def test_model_prefill_uses_expanded_attention_and_matches_cpu():
     from batchgen_b200.config import get_model_config
     from batchgen_b200.models import build_model
