@@ -256,9 +256,15 @@ gemm_fp8_n256_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     uint32_t it = 0;
     bool ok = true, arrived = (p.a_ready == nullptr);
     for (int tile = blockIdx.x; ok && walk.get(tile, t); tile += gridDim.x) {
-      if (!arrived) {        // pushed scales are valid once every rank's arrival flag is up
-        for (int i = 0; ok && i < p.world; ++i) ok = __all_sync(0xffffffffu, wait_flag_ge(p.a_ready + i, epoch, p.status));
-        if (!ok) break;      // the TMA producer's wait for the same flags reports it
+      if (!arrived) {        // pushed scales are valid once every rank's arrival flag is up: one lane polls, its acquire holds for the warp behind the sync
+        if (lane == 0)
+          for (int i = 0; ok && i < p.world; ++i) ok = wait_flag_ge(p.a_ready + i, epoch, p.status);
+        __syncwarp();
+        ok = __shfl_sync(0xffffffffu, static_cast<int>(ok), 0) != 0;
+        if (!ok) {           // the TMA producer may have seen the flags in time: without this the epilogue would wait out its own budget
+          if (lane == 0 && *abort_flag == 0) *abort_flag = kTimeoutPeer;
+          break;
+        }
         arrived = true;
       }
       const int blk0 = min(EPI == EPI_SILU_MUL ? t.nt : 2 * t.nt, nblk - 1);
