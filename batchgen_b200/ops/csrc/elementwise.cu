@@ -203,6 +203,10 @@ mla_kv_write_kernel(const __nv_bfloat16* __restrict__ kv_a, int ld, const __nv_b
   }
 }
 
+// A pair turned by an angle, written out so that every kernel rounds alike: left to the compiler, two kernels contracted the second sum differently
+// (a query in 30,000 off by a bit of bf16 with its row's alignment).
+__device__ __forceinline__ float2 turn(float a, float b, float c, float s) { return make_float2(__fmaf_rn(a, c, -__fmul_rn(b, s)), __fmaf_rn(a, s, __fmul_rn(b, c))); }
+
 // In-place RoPE on the trailing `rope` dims of every head of q [T, H, D].
 __global__ void rope_q_kernel(__nv_bfloat16* __restrict__ q, int H, int D, int rope, const int* __restrict__ positions,
                               const float* __restrict__ cos_t, const float* __restrict__ sin_t, int interleaved,
@@ -216,9 +220,9 @@ __global__ void rope_q_kernel(__nv_bfloat16* __restrict__ q, int H, int D, int r
     __nv_bfloat16* p = q + (size_t)t * ld_t + (size_t)h * D + (D - rope);
     const float c = cos_t[(size_t)pos * half + i], s = sin_t[(size_t)pos * half + i];
     const int i0 = interleaved ? 2 * i : i, i1 = interleaved ? 2 * i + 1 : i + half;
-    const float a = __bfloat162float(p[i0]), b = __bfloat162float(p[i1]);
-    p[i0] = __float2bfloat16(a * c - b * s);
-    p[i1] = __float2bfloat16(b * c + a * s);
+    const float2 y = turn(__bfloat162float(p[i0]), __bfloat162float(p[i1]), c, s);
+    p[i0] = __float2bfloat16(y.x);
+    p[i1] = __float2bfloat16(y.y);
   }
 }
 
@@ -251,14 +255,13 @@ rope_q_wide_kernel(__nv_bfloat16* __restrict__ q, int H, int D, int rope, const 
     __align__(16) __nv_bfloat162 o[8];
 #pragma unroll
     for (int j = 0; j < 8; j += 2) {
-      const float u0 = a[j] * c[j] - b[j] * s[j], v0 = b[j] * c[j] + a[j] * s[j];
-      const float u1 = a[j + 1] * c[j + 1] - b[j + 1] * s[j + 1], v1 = b[j + 1] * c[j + 1] + a[j + 1] * s[j + 1];
+      const float2 y0 = turn(a[j], b[j], c[j], s[j]), y1 = turn(a[j + 1], b[j + 1], c[j + 1], s[j + 1]);
       if (INTERLEAVED) {
-        o[j] = __floats2bfloat162_rn(u0, v0);
-        o[j + 1] = __floats2bfloat162_rn(u1, v1);
+        o[j] = __floats2bfloat162_rn(y0.x, y0.y);
+        o[j + 1] = __floats2bfloat162_rn(y1.x, y1.y);
       } else {
-        o[j / 2] = __floats2bfloat162_rn(u0, u1);
-        o[4 + j / 2] = __floats2bfloat162_rn(v0, v1);
+        o[j / 2] = __floats2bfloat162_rn(y0.x, y1.x);
+        o[4 + j / 2] = __floats2bfloat162_rn(y0.y, y1.y);
       }
     }
     *p0 = reinterpret_cast<const uint4*>(o)[0];

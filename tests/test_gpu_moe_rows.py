@@ -236,3 +236,27 @@ def test_quantised_activation_of_few_and_many_rows(K, padding):
     step = s[kept].double().repeat_interleave(128, 1)
     # a value rounded to 8 bits, then to 4, in units of the scale down to 2^-9 of it
     assert ((q[kept].double() * step - want).abs() <= want.abs() * (2.0 ** -4 + 2.0 ** -8) + step * 2.0 ** -10).all()
+
+
+@pytest.mark.parametrize("interleaved", [True, False])
+def test_rotated_queries_do_not_depend_on_alignment(interleaved):
+    """Rows in 16-byte pieces and rows that start between them: the same bytes, those of a x cos - round(b x sin) and a x sin + round(b x cos)."""
+    from batchgen_b200.ops import fused
+
+    T, H, D, rope = 400, 16, 192, 64
+    g = torch.Generator(device="cuda").manual_seed(0)
+    pos = torch.randint(0, 4096, (T,), device="cuda", dtype=torch.int32, generator=g)
+    ang = torch.rand(4096, rope // 2, device="cuda", generator=g) * 6
+    cos, sin = ang.cos(), ang.sin()
+    q = torch.randn(T, H, D, device="cuda", generator=g).to(torch.bfloat16)
+    got = []
+    for shift in (0, 1):
+        rows = torch.zeros(T, H * D + 8, device="cuda", dtype=torch.bfloat16)[:, shift:shift + H * D].unflatten(1, (H, D)).copy_(q)
+        got.append(fused.rope_q_(rows, pos, cos, sin, rope, interleaved).clone())
+    assert torch.equal(got[0], got[1])
+    x = q[..., D - rope:].double()
+    a, b = (x[..., 0::2], x[..., 1::2]) if interleaved else (x[..., :rope // 2], x[..., rope // 2:])
+    c, s = (v[pos.long()].double().unsqueeze(1) for v in (cos, sin))
+    u, v = a * c - (b * s).float().double(), a * s + (b * c).float().double()
+    want = torch.stack([u, v], -1).flatten(-2) if interleaved else torch.cat([u, v], -1)
+    assert torch.equal(got[0][..., D - rope:], want.float().to(torch.bfloat16)) and torch.equal(got[0][..., :D - rope], q[..., :D - rope])
