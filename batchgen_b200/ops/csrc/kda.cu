@@ -632,9 +632,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* v) {
       : "r"(taddr)
       : "memory");
 }
-// 32 columns of one row as parts into [part][rows][64] tiles (swizzled as a TMA load would)
+// 32 columns of one row as parts into [part][rows][64] tiles (swizzled as a TMA load would).  An infinity is infinite three times: what is cut from it
+// leaves NaN, where its products with a finite number in fp32 are infinite.
 __device__ __forceinline__ void put_parts(uint8_t* tiles, int part_bytes, int row, int half, const float (&x)[32]) {
   uint8_t* r = tiles + row * 128;
+  auto piece = [&](int c) { return ((4 * half + c) ^ (row & 7)) << 4; };
+  float2 odd = make_float2(0.f, 0.f);           // NaN once a rest is
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     uint32_t w[3][4];
@@ -644,9 +647,16 @@ __device__ __forceinline__ void put_parts(uint8_t* tiles, int part_bytes, int ro
       w[0][i] = cut_bf16x2(e);
       w[1][i] = cut_bf16x2(e);
       w[2][i] = last_bf16x2(e);
+      odd = __ffma2_rn(e, make_float2(0.f, 0.f), odd);
     }
 #pragma unroll
-    for (int m = 0; m < 3; ++m) *reinterpret_cast<uint4*>(r + m * part_bytes + (((4 * half + c) ^ (row & 7)) << 4)) = make_uint4(w[m][0], w[m][1], w[m][2], w[m][3]);
+    for (int m = 0; m < 3; ++m) *reinterpret_cast<uint4*>(r + m * part_bytes + piece(c)) = make_uint4(w[m][0], w[m][1], w[m][2], w[m][3]);
+  }
+  if (!(odd.x + odd.y == 0.f)) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (fabsf(x[j]) == INFINITY)
+        for (int m = 0; m < 3; ++m) *reinterpret_cast<uint16_t*>(r + m * part_bytes + piece(j / 8) + j % 8 * 2) = x[j] > 0.f ? 0x7F80 : 0xFF80;
   }
 }
 

@@ -1,4 +1,6 @@
 """KDA kernel (conv + gated delta rule + gated norm, prefill and decode) against the fp32 reference."""
+import math
+
 import pytest
 import torch
 
@@ -303,3 +305,39 @@ def test_chunk_form_of_unaligned_rows(lens, shift, monkeypatch):
     assert ((o.cpu().double() - want).abs() <= want.abs() * 2 ** -8 + 2e-4).all()
     for half in (rec[..., :64], rec64.cuda()[..., :64]), (rec[..., 64:], rec64.cuda()[..., 64:]):
         assert (half[0].double() - half[1]).norm() <= 5e-7 * half[1].norm()
+
+
+def _one_write(H, bias_v, dt_bias, A_log, f_token, form, monkeypatch, last=None):
+    """A piece of 64 tokens of which the last alone has a key, the first unit vector with weight one, or (``f_token`` zero) a decay, on a state of zeros or
+    ones: afterwards row 0 of the state is SiLU(bias_v), or row i the decay of channel i.  ``last``: values of the last token itself, to which bias_v is added."""
+    from batchgen_b200.ops import kda
+    T, HD = 64, H * 128
+    monkeypatch.setattr(kda, "chunk_form_pays", lambda lens, heads, sms: bool(lens) and form == "chunks")
+    qkv = torch.zeros(T, 3 * HD, dtype=torch.bfloat16, device="cuda")
+    if f_token != 0:
+        qkv[-1, HD:2 * HD:128] = 32.0
+    if last is not None:
+        qkv[-1, 2 * HD:] = last.flatten().cuda()
+    w = torch.zeros(3 * HD, 4, device="cuda")
+    w[:, 3] = 1.0
+    bias = torch.zeros(3 * HD, device="cuda")
+    bias[2 * HD:] = bias_v.flatten().cuda()
+    f = torch.full((T, HD), -1e5, dtype=torch.bfloat16, device="cuda")           # no decay
+    f[-1] = f_token
+    p = kda.KDAParams(conv_w=w, conv_b=bias, A_log=A_log.cuda(), dt_bias=dt_bias.flatten().cuda(), norm_w=torch.ones(128, device="cuda"))
+    rec = torch.ones(1, H, 128, 128, device="cuda") if f_token == 0 else torch.zeros(1, H, 128, 128, device="cuda")
+    kda.kda_forward(qkv, f, torch.full((T, H), 100.0, dtype=torch.bfloat16, device="cuda"), torch.zeros(T, HD, dtype=torch.bfloat16, device="cuda"), p,
+                    torch.zeros(1, 3 * HD, 3, device="cuda"), rec, [0], [0, T], [1], H, 128, 1.0, 1e-6)
+    return rec[0].cpu()
+
+
+def test_silu_of_the_chunk_form_not_finite(monkeypatch):
+    """Infinities and NaN leave the formula as they leave the token form's division, and no other column is touched."""
+    x = torch.ones(1, 128)
+    x[0, 3], x[0, 70], x[0, 71], x[0, 90], x[0, 127] = float("inf"), float("nan"), -float("inf"), -300.0, 3e38
+    none = torch.zeros(1, 128)
+    a, b = (_one_write(1, none, none, torch.zeros(1), -1e5, form, monkeypatch, last=x)[0, 0] for form in ("chunks", "tokens"))
+    assert a[3] == b[3] == float("inf") and a[[70, 71]].isnan().all() and b[[70, 71]].isnan().all() and a[90] == b[90] == 0 and a[127] == b[127]
+    fine = torch.ones(128, dtype=torch.bool)
+    fine[[3, 70, 71, 90, 127]] = False
+    assert (a[fine] == a[0]).all() and abs(float(a[0]) - 0.7310586) < 1e-6
