@@ -229,8 +229,9 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// x / d for d from 1 to 2^60 and |x| at most as large: an approximate reciprocal and one correction by the residual (Markstein 1990), which rounds
-// like the division or to the number beside it at a third of its instructions
+// x / d for d from 1 to 2^60 and |x| up to 2^60: an approximate reciprocal and one correction by the residual (Markstein 1990), which rounds
+// like the division or to the number beside it at a third of its instructions (quotients whose residual is below the smallest float, as the
+// reciprocal gives them)
 __device__ __forceinline__ float quotient(float x, float d) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
@@ -664,8 +665,8 @@ __device__ __forceinline__ void put_parts(uint8_t* tiles, int part_bytes, int ro
 // U or O of one token's columns from the first product and the update from the second; warp 8 loads, warp 9 issues.
 // Bound by the products (3,456 clocks a chunk) and four hand-overs between threads and tensor cores, one after the other.
 __global__ void __launch_bounds__(kChainThreads, 1)
-chunk_chain(const __grid_constant__ CUtensorMap map, const Params p, const ChunkItem* __restrict__ items, const ChunkSeq* __restrict__ seqs,
-            float* __restrict__ res, const float* __restrict__ g_last, int* status) {
+chunk_chain(const __grid_constant__ CUtensorMap map, const Params p, const ChunkSeq* __restrict__ seqs, float* __restrict__ res,
+            const float* __restrict__ g_last, int* status) {
   constexpr int D = 128;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* wq = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));      // [3][2 key halves][128 rows]
@@ -945,7 +946,7 @@ int bg_kda_forward(const void* qkv, int qkv_stride, const void* f, int f_stride,
     CUtensorMap tm;
     if (make_parts_map(&tm, parts, pairs * kPartRows) != 0) return -4;
     chunk_prepare<<<dim3(n_items, H), kPrepThreads, kPrepareFloats * 4, stream>>>(p, it, parts, res, g_last);
-    chunk_chain<<<dim3(128 / kCols, H, n_seqs), kChainThreads, kChainBytes, stream>>>(tm, p, it, reinterpret_cast<const ChunkSeq*>(seqs), res, g_last, status);
+    chunk_chain<<<dim3(128 / kCols, H, n_seqs), kChainThreads, kChainBytes, stream>>>(tm, p, reinterpret_cast<const ChunkSeq*>(seqs), res, g_last, status);
     chunk_finish<<<dim3(n_items, H), 256, 0, stream>>>(p, it, res);
   }
   if (longest_short <= 0) return cudaGetLastError() == cudaSuccess ? 0 : -2;

@@ -331,6 +331,38 @@ def _one_write(H, bias_v, dt_bias, A_log, f_token, form, monkeypatch, last=None)
     return rec[0].cpu()
 
 
+def _arguments(n, seed):
+    """Floats around the borders of the formulas, and of every size."""
+    g = torch.Generator().manual_seed(seed)
+    edge = torch.tensor([0.0, 40.0, 20.0, 1.0, 0.6931472, 16.0, 88.0, 87.33, 86.0, 5.0, 2.0 ** -126, 2.0 ** -100, 2.0 ** -24, 2.0 ** -12, 1e-3, 64.0])
+    near = torch.cat([edge, torch.nextafter(edge, edge + 1), torch.nextafter(edge, edge - 1), edge * (1 + 2.0 ** -20)])
+    size = torch.exp2(torch.rand(n, generator=g) * 40 - 33)                      # up to 2^7
+    x = torch.cat([near, -near, size * (1 - 2 * torch.randint(0, 2, (n,), generator=g))])[:n]
+    x[0] = 64.0                                                                  # SiLU is the number itself
+    return x
+
+
+def test_silu_of_the_chunk_form(monkeypatch):
+    """The chunk form's quotient against the token form's division: the same float or its neighbour; both against 64 bits."""
+    H = 96
+    x = _arguments(H * 128, 1).view(H, 128)
+    x[:, 0] = 64.0
+    none, A = torch.zeros(H, 128), torch.zeros(H)
+    got = {form: _one_write(H, x, none, A, -1e5, form, monkeypatch)[:, 0] for form in ("chunks", "tokens")}
+    x64 = x.double()
+    want = x64 / (1 + (-x64).exp())
+    whole = want.abs() >= 2.0 ** -100             # all three parts of the state's number are normal floats
+    for y in got.values():
+        assert (y[:, 0] == 64).all()                                             # the key is exactly one
+        # e^-x off by 2 + 1.173 |x| units (CUDA's bound), the sum and the quotient by one each
+        rel = ((2 + 1.173 * x64.abs()) * (-x64).exp() / (1 + (-x64).exp()) + 2) * 2.0 ** -23
+        assert ((y.double() - want).abs()[whole] <= (rel * want.abs())[whole]).all()
+        assert ((y.double() - want).abs()[~whole] <= 2.0 ** -100).all()
+    a, b = got["chunks"][whole], got["tokens"][whole]
+    assert ((a == b) | (torch.nextafter(a, b) == b)).all()
+    assert whole.sum() > 0.9 * whole.numel()
+
+
 def test_silu_of_the_chunk_form_not_finite(monkeypatch):
     """Infinities and NaN leave the formula as they leave the token form's division, and no other column is touched."""
     x = torch.ones(1, 128)
@@ -341,3 +373,27 @@ def test_silu_of_the_chunk_form_not_finite(monkeypatch):
     fine = torch.ones(128, dtype=torch.bool)
     fine[[3, 70, 71, 90, 127]] = False
     assert (a[fine] == a[0]).all() and abs(float(a[0]) - 0.7310586) < 1e-6
+
+
+def test_softplus_of_the_chunk_form(monkeypatch):
+    """Decays of one token over 2^-110 to 2^12 of softplus: the series within the bounds of its exponential, and no further from 64 bits than log1p(e^x)."""
+    lo, hi = -110, 12
+    H = hi - lo
+    g = torch.Generator().manual_seed(2)
+    top = torch.exp2(torch.arange(lo, hi).double()).view(H, 1)
+    sp = top * (1 + torch.rand(H, 128, generator=g).double())                    # softplus wanted
+    x = torch.where(sp > 30, sp, torch.expm1(sp.clamp(max=30)).log()).float()
+    x64, a64 = x.double(), (4 - torch.arange(lo, hi).double()).view(H, 1) * math.log(2.0)                        # exponents of some 16 to 32
+    A = a64.float().flatten()
+    sp = x64.clamp_min(0) + torch.log1p((-x64.abs()).exp())
+    err = {}
+    for form in ("chunks", "tokens"):
+        S = _one_write(H, torch.zeros(H, 128), x, A, 0.0, form, monkeypatch)[:, :, 5].double()
+        e = (-S.log() / A.double().exp().view(H, 1) / sp - 1).abs()
+        part = torch.log1p((-x64.abs()).exp()) / sp                               # the exponential's share of the sum
+        # __expf off by 2 + 1.173 |x| units (CUDA's bound) in both places, eight roundings, ex2 off by two units of a state, which stands for 16 of the exponent
+        units = (2 + 1.173 * x64.abs()) * part + 2 + 1.173 * a64.abs() + 8 + 1
+        if form == "chunks":
+            assert (e <= units * 2.0 ** -23).all()
+        err[form] = e.square().mean().sqrt()
+    assert err["chunks"] <= 1.05 * err["tokens"]
