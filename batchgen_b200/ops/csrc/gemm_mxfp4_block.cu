@@ -449,8 +449,9 @@ int bg_mxfp4_block_gemm(const void* xp, const void* xs, const void* Wq, const vo
   p.xp = reinterpret_cast<const uint8_t*>(xp); p.xs = reinterpret_cast<const uint8_t*>(xs);
   p.D = reinterpret_cast<__nv_bfloat16*>(D); p.ldd = ldd; p.wide = reinterpret_cast<uintptr_t>(D) % 16 == 0;
   p.offsets = offsets; p.counts = offsets != nullptr ? counts : nullptr; p.groups = groups; p.M = M; p.N = N; p.K = K; p.status = status;
-  // 32 or 96 tokens a tile: 800 tokens of the figures above (25 rows an expert) 369 us with 32 and 410 with 96, 1,500 (47 rows) 590 and 461
-  return rows <= 24.f ? launch<40>(p, num_sms, stream) : launch<104>(p, num_sms, stream);
+  // 32 or 96 tokens a tile.  128 experts of 6,144 x 2,880, us: 24 rows each 334 / 401, 28 369 / 405, 30 412 / 412, 32 449 / 416, 47 602 / 449; of 2,880 x 3,072: 28
+  // 218 / 246, 30 234 / 248, 32 248 / 250, 36 275 / 257; 32 experts of 6,144 x 2,880: 28 113 / 119, 30 121 / 121, 36 148 / 123
+  return rows <= 30.f ? launch<40>(p, num_sms, stream) : launch<104>(p, num_sms, stream);
 }
 
 // x [T, ldx] bf16 -> parts p [rows / 8 rounded up][2][8][K], s [K / 128 rounded up][rows][4].  pos [T, topk]: the rows a token goes to (negative: none), or null: its

@@ -98,14 +98,25 @@ def gated_parts(gate_up: torch.Tensor, kind: int, limit: float, offsets: Optiona
 
 
 BLOCK_MAX_ROWS = 80
+BLOCK_NARROW_ROWS = 30                # rows of a segment up to which a tile has 32 tokens (gemm_mxfp4_block.cu)
 
 
-def block_scaled(wq: torch.Tensor, ws: torch.Tensor, rows: float) -> bool:
+def block_scaled(wq: torch.Tensor, ws: torch.Tensor, rows: float, split: bool = False) -> bool:
     """The block-scaled product takes weights wq [.., N, K / 2], ws [.., N, K / 32] for segments of ``rows`` expected rows: up to 80 of them (128 experts of
-    6,144 x 2,880, against weights expanded to bf16: 5 rows 287 / 553 us, 25 rows 369 / 559, 47 rows 461 / 573, 94 rows 643 / 605), K from 128 to
-    12,288, addresses and rows as its loads need them."""
-    return rows <= BLOCK_MAX_ROWS and bool(_ext.lib().bg_mxfp4_block_takes(_ext.ptr(wq), _ext.ptr(ws), ctypes.c_longlong(wq.shape[-2]),
-                                                                           ctypes.c_int(2 * wq.shape[-1])))
+    6,144 x 2,880, against weights expanded to bf16: 5 rows 287 / 553 us, 28 rows 369 / 559, 47 rows 449 / 573, 94 rows 643 / 605), K to 12,288, addresses and
+    rows as its loads need them.  K below 1,024 from one and a half rounds of tiles on: a tile of few steps is over before its start is paid
+    (layers, 16 rows: 16 experts of 512 x 768 55.4 / 53.3, of 2,048 x 768 67.6 / 72.6, 128 of 512 x 768 105.6 / 113.6).  Where the parts take a launch of their own (``split``), K beyond 2,048, and
+    beyond 4,096 with tiles of 96 tokens (dense, 24 tokens, 1,024 x 1,024 15.3 / 12.5, 4,096 x 1,024 15.3 / 14.4, 2,048 x 2,048 17.4 / 18.5, 2,880 x 3,072 19.4 / 22.6;
+    31 tokens, 2,880 x 3,072 23.6 / 22.5, 4,096 x 4,096 29.5 / 26.7, x 6,144 31.7 / 34.9).  With tiles of 96 tokens K to 10,112, past which shared memory has two
+    stages (40 tokens, 4,096 x 9,216 39.9 / 49.2, x 12,288 64.5 / 63.5, 80 tokens 68.6 / 65.5)."""
+    K, wide = 2 * wq.shape[-1], rows > BLOCK_NARROW_ROWS
+    if rows > BLOCK_MAX_ROWS or (wide and K > 10112):
+        return False
+    if split and K <= (4096 if wide else 2048):
+        return False
+    if K < 1024 and 2 * (wq.numel() // (wq.shape[-1] * wq.shape[-2])) * -(-wq.shape[-2] // 128) < 3 * _ext.num_sms(wq.device):
+        return False
+    return bool(_ext.lib().bg_mxfp4_block_takes(_ext.ptr(wq), _ext.ptr(ws), ctypes.c_longlong(wq.shape[-2]), ctypes.c_int(K)))
 
 
 def _block_gemm(x: Union[torch.Tensor, Parts], wq2d, ws2d, out, offsets, groups, M, N, K, counts, rows) -> None:
@@ -128,7 +139,7 @@ def mxfp4_gemm(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor, out: Optiona
     if out is None:
         out = torch.empty(T, N, dtype=torch.bfloat16, device=x.device)
     if T:
-        if block_scaled(wq, ws, T):
+        if block_scaled(wq, ws, T, split=True):
             _block_gemm(x, wq, ws, out, None, 1, T, N, K, None, T)
         else:
             _launch(EPI_STORE, x.contiguous(), wq, ws, out, None, 1, T, N, K)
@@ -165,7 +176,7 @@ def grouped_mxfp4_gemm(x: Union[torch.Tensor, Parts], wq: torch.Tensor, ws: torc
         assert offsets.dtype == torch.int32 and offsets.is_cuda
         wq2d, ws2d = wq.view(E * N, Kh), ws.view(E * N, K // 32)
         rows = (R if rows_hint is None else rows_hint) / max(E, 1)
-        if isinstance(x, Parts) or not silu_mul and block_scaled(wq, ws, rows):
+        if isinstance(x, Parts) or not silu_mul and block_scaled(wq, ws, rows, split=True):
             assert not silu_mul
             _block_gemm(x, wq2d, ws2d, out, offsets, E, R, N, K, counts, rows)
         else:

@@ -297,3 +297,45 @@ def test_gated_parts(kind):
     got = scale[rows] * (parts[rows, 0] + parts[rows, 1] / 32)
     top = want[rows].abs().view(-1, 90, 32).amax(-1).repeat_interleave(32, 1)
     assert ((got - want[rows]).abs() <= top * 2.0 ** -22).all() and (got == want[rows])[want[rows].abs() > top * 2.0 ** -13].all()
+
+
+@pytest.mark.parametrize("rows", [10, 31])
+def test_block_scaled_products_longest_rows(rows, monkeypatch):
+    """K of 12,288, the largest that the loads take: four stages beside tiles of 32 tokens, two beside tiles of 96."""
+    test_block_scaled_products([3, 40, 0, 97], 5, 136, 12288, rows, monkeypatch)
+
+
+def test_block_scaled_products_where_they_pay(monkeypatch):
+    """Which product runs on either side of the borders: short K, a launch for the parts alone, few stages, many rows; all of them the same numbers."""
+    from batchgen_b200.ops import _ext, mxfp4
+    calls = []
+    block, expand = mxfp4._block_gemm, mxfp4._launch
+    monkeypatch.setattr(mxfp4, "_block_gemm", lambda *a: (calls.append("block"), block(*a)))
+    monkeypatch.setattr(mxfp4, "_launch", lambda *a, **k: (calls.append("expand"), expand(*a, **k)))
+    g = torch.Generator().manual_seed(4)
+
+    def product(T, N, K, E=0):
+        calls.clear()
+        x = torch.randn(T, K, generator=g).bfloat16()
+        wq, ws = torch.randint(0, 256, (max(E, 1), N, K // 2), generator=g, dtype=torch.uint8), torch.randint(118, 124, (max(E, 1), N, K // 32), generator=g, dtype=torch.uint8)
+        w = mxfp4.dequantize(wq, ws, torch.float32).double()
+        if E:
+            off = torch.arange(0, T + 1, T // E, dtype=torch.int32)
+            rows = mxfp4.split(x.cuda()) if mxfp4.block_scaled(wq.cuda(), ws.cuda(), T / E) else x.cuda()
+            got = mxfp4.grouped_mxfp4_gemm(rows, wq.cuda(), ws.cuda(), off.cuda())
+            want = torch.cat([x[off[e]:off[e + 1]].double() @ w[e].t() for e in range(E)])
+            mag = torch.cat([x[off[e]:off[e + 1]].double().abs() @ w[e].abs().t() for e in range(E)])
+        else:
+            got = mxfp4.mxfp4_gemm(x.cuda(), wq[0].cuda(), ws[0].cuda())
+            want, mag = x.double() @ w[0].t(), x.double().abs() @ w[0].abs().t()
+        _ext.check_status()
+        assert ((got.cpu().double() - want).abs() <= want.abs() * 2 ** -8 + mag * (K * 2 ** -24 + 2.0 ** -12)).all()
+        return calls[0]
+
+    assert product(24, 256, 2048) == "expand" and product(24, 256, 2112) == "block"
+    assert product(31, 256, 4096) == "expand" and product(31, 256, 4160) == "block" and product(30, 256, 4096) == "block"
+    assert product(80, 256, 4160) == "block" and product(81, 256, 4160) == "expand"
+    assert product(31, 256, 10112) == "block" and product(31, 256, 10176) == "expand" and product(30, 256, 10176) == "block"
+    assert product(32, 256, 960, E=4) == "expand" and product(32, 256, 1024, E=4) == "block"
+    if _ext.num_sms(torch.device("cuda")) == 148:
+        assert product(8, 28 * 128, 192, E=8) == "block" and product(8, 27 * 128, 192, E=8) == "expand"
