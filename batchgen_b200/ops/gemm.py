@@ -68,7 +68,8 @@ def _use_wide(kind, D, M, N, wide, dense) -> bool:
     """128 x 256 tiles pay off as soon as a dense product has more than one round of 128 x 128 ones, for their K blocks take hardly
     longer.  us, narrow and wide, K x N and rows: 16,384 x 7,168, 384 rows (168 narrow tiles) 105 and 78, 512 rows 132 and 78;
     7,168 x 4,096, 651 rows (192) 58 and 41, 512 rows (128) 33 and 40; 7,168 x 2,112, 1,185 rows (170) 62 and 43, 1,024 rows (136) 35
-    and 43; 6,144 x 3,072, 900 rows (192) 50 and 35, 768 rows (144) 29 and 35.  Grouped products, whose tiles are an upper bound here,
+    and 43; 6,144 x 3,072, 900 rows (192) 50 and 35, 768 rows (144) 29 and 35; short K likewise, 900 x 3,072 with K of 128 13.3 and 11.2, 1,024
+    19.5 and 15.0, 2,048 29 and 20.  Grouped products, whose tiles are an upper bound here,
     keep two rounds.  GEMMs that consume collective hooks (rows stored to peers, flag waits) and bf16 operands stay on the 128 x 128
     kernel, and in its second round rows that the wide one does not take (row stride no multiple of 8)."""
     global _hooks_pending

@@ -258,6 +258,22 @@ def test_tile_width_of_a_second_round(T, N, wide):
     assert _rel(got.float().cpu(), ref.fp8_gemm(xq, xs, wq, ws)) < 1e-2
 
 
+def test_tile_width_rule(monkeypatch):
+    """Either side of each border of the rule itself: one round of narrow tiles for dense products, two for grouped ones, row strides, operands, hooks."""
+    from batchgen_b200.ops import _ext, gemm
+    monkeypatch.setattr(_ext, "num_sms", lambda device=None: 148)
+    monkeypatch.setattr(gemm, "_WIDE", "auto")
+    D = torch.empty(2, 16, dtype=torch.bfloat16, device="cuda")
+    odd = torch.empty(2, 12, dtype=torch.bfloat16, device="cuda")
+    use = lambda M, N, dense=True, D=D, kind=gemm.KIND_FP8, wide=None: gemm._use_wide(kind, D, M, N, wide, dense)  # noqa: E731
+    assert not use(128, 148 * 128) and use(128, 149 * 128) and use(129, 75 * 128) and not use(129, 74 * 128)
+    assert not use(128, 295 * 128, dense=False) and use(128, 296 * 128, dense=False)
+    assert not use(128, 200 * 128, D=odd) and use(128, 296 * 128, D=odd)
+    assert not use(128, 400 * 128, kind=gemm.KIND_BF16) and not use(128, 400 * 128, wide=False) and use(1, 128, wide=True)
+    gemm.hooks_pending()
+    assert not use(128, 400 * 128) and use(128, 400 * 128)
+
+
 @pytest.mark.parametrize("T,N,pad,silu", [(129, 320, 0, False), (131, 320, 8, False), (126, 256, 24, False), (3, 264, 8, False), (131, 256, 0, True), (129, 512, 8, True)])
 def test_wide_tile_stores(T, N, pad, silu):
     """Row groups cut by the last row, column slices cut by N, rows that start inside a sector: the same values, nothing beside them."""
