@@ -1,7 +1,8 @@
 // bf16 rows as two e4m3 parts with one power-of-two scale per 32 elements: the tokens' operand of the block-scaled 4-bit product.
 //
 // x = 2^s (p1 + 2^-5 p2) with 2^s such that the largest element of the 32 lies in [2^7, 2^8).  p1 takes the first four significant bits, p2 the
-// rest: a bf16 number has eight, so the sum is exact down to 2^-14 of the largest element and off by at most 2^-22 of it below.  An element that is not
+// rest: a bf16 number has eight, so the sum is exact down to 2^-14 of the largest element and off by at most 2^-22 of it below (from 2^-18 of it on
+// down bits are missing for good, and 2^-22 of it may become zero).  An element that is not
 // finite has the NaN of e4m3 as p1 and says what it was in p2 (0: NaN, else the sign of an infinity), for the product's epilogue.
 #pragma once
 #include "common.cuh"

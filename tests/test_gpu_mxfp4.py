@@ -339,3 +339,30 @@ def test_block_scaled_products_where_they_pay(monkeypatch):
     assert product(32, 256, 960, E=4) == "expand" and product(32, 256, 1024, E=4) == "block"
     if _ext.num_sms(torch.device("cuda")) == 148:
         assert product(8, 28 * 128, 192, E=8) == "block" and product(8, 27 * 128, 192, E=8) == "expand"
+
+
+@pytest.mark.parametrize("above", [8, 14, 16, 20])
+def test_parts_beside_an_outlier(above):
+    """A first element of every 32 that dwarfs the others: elements down to 2^-14 of it are whole, smaller ones within 2^-22 of it, and no output whose weight
+    for it is zero sees more than that."""
+    from batchgen_b200.ops import _ext, mxfp4
+    g = torch.Generator().manual_seed(above)
+    T, N, K = 40, 256, 1024
+    x = torch.randn(T, K, generator=g)
+    x[:, ::32] = 2.0 ** above * (1 + torch.rand(T, K // 32, generator=g))
+    x = x.bfloat16()
+    p = mxfp4.split(x.cuda())
+    parts = p.p.view(torch.float8_e4m3fn).cpu().double().transpose(1, 2).reshape(-1, 2, K)
+    scale = torch.exp2(p.s.cpu().double().permute(1, 0, 2).reshape(T, -1)[:, :K // 32] - 127).repeat_interleave(32, 1)
+    got, top = scale * (parts[:T, 0] + parts[:T, 1] / 32), x[:, ::32].double().repeat_interleave(32, 1)
+    assert (got == x.double())[x.double().abs() >= top * 2.0 ** -14].all() and ((got - x.double()).abs() <= top * 2.0 ** -22).all()
+    wq, ws = torch.randint(0, 256, (N, K // 2), generator=g, dtype=torch.uint8), torch.randint(118, 124, (N, K // 32), generator=g, dtype=torch.uint8)
+    wq.view(N, K // 32, 16)[:, :, 0] &= 0xF0
+    out = torch.empty(T, N, dtype=torch.bfloat16, device="cuda")
+    mxfp4._block_gemm(p, wq.cuda(), ws.cuda(), out, None, 1, T, N, K, None, T)
+    _ext.check_status()
+    w, x64 = mxfp4.dequantize(wq, ws, torch.float32).double(), x.double()
+    want, mag = x64 @ w.t(), x64.abs() @ w.abs().t()
+    small = torch.where(x64.abs() < top * 2.0 ** -14, top * 2.0 ** -22, 0.0)
+    # one rounding to 8 bits, fp32 sums of K products, and what the parts leave out of the small elements
+    assert ((out.cpu().double() - want).abs() <= want.abs() * 2 ** -8 + mag * K * 2 ** -24 + small @ w.abs().t()).all()
