@@ -410,9 +410,13 @@ template <int BT>
 static int launch(Params& p, int num_sms, cudaStream_t stream) {
   CUtensorMap tw, tail, t128, t16;
   const uint64_t wrows = (uint64_t)p.groups * p.N, kq = p.K / 2;
-  if (make_map(&tw, true, p.wq, wrows, p.K / BK * BK, kq, BW) != 0 || make_map(&tail, true, p.wq + (p.K - BK) / 2, wrows, BK, kq, BW) != 0) return -11;
+  if (make_map(&tw, true, p.wq, wrows, p.K / BK * BK, kq, BW) != 0) return -11;
+  tail = tw;                                                          // read only where K ends in half a step
+  if (p.K % BK != 0 && make_map(&tail, true, p.wq + (p.K - BK) / 2, wrows, BK, kq, BW) != 0) return -11;
   const uint64_t xrows = (uint64_t)(p.M + 7) / 8 * 16;
-  if (make_map(&t128, false, p.xp, xrows, p.K, p.K, 128) != 0 || make_map(&t16, false, p.xp, xrows, p.K, p.K, 16) != 0) return -12;
+  if (make_map(&t16, false, p.xp, xrows, p.K, p.K, 16) != 0) return -12;
+  t128 = t16;                                                         // read only by tiles of 128 rows of parts
+  if (2 * BT >= 128 && xrows >= 128 && make_map(&t128, false, p.xp, xrows, p.K, p.K, 128) != 0) return -12;
   static DeviceOnce once;
   auto kern = mxfp4_block_kernel<BT>;
   if (!ensure_dynamic_smem(kern, kMaxShared, once)) return -13;

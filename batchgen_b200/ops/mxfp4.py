@@ -11,7 +11,6 @@ batchgen_kernels/src/moe/mxfp4/marlin_grouped_gemm.cu and batchgen/moe/fused_moe
 from __future__ import annotations
 
 import ctypes
-from dataclasses import dataclass
 from typing import Optional, Union
 
 import torch
@@ -52,48 +51,72 @@ def _launch(epi, x, wq2d, ws2d, out, offsets, groups, M, N, K, counts=None):
     _ext.check(rc, "bg_mxfp4_gemm")
 
 
-@dataclass
+_P, _I = ctypes.c_void_p, ctypes.c_int
+# argument types are set once, so that plain integers pass: three of these calls a layer are host time of a decode step of few rows
+_ARGS = {
+    "bg_mx_split": (_P, ctypes.c_longlong, _P, _I, _I, _P, _P, _I, _I, _P),
+    "bg_gated_parts": (_I, _P, ctypes.c_longlong, _P, _P, _I, _I, ctypes.c_float, _P, _P, _I, _P),
+    "bg_mxfp4_block_gemm": (_P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, ctypes.c_float, _I, _P, _P),
+}
+
+
+def _call(name: str, *args) -> None:
+    fn = getattr(_ext.lib(), name)
+    if fn.argtypes is None:
+        fn.argtypes = _ARGS[name]
+    _ext.check(fn(*args, _ext.stream()), name)
+
+
+def _at(t: Optional[torch.Tensor]) -> Optional[int]:
+    return None if t is None else t.data_ptr()
+
+
 class Parts:
     """bf16 rows [rows, K] as the block-scaled product takes them: ``p`` uint8 [rows / 8 rounded up, 2, 8, K] (e4m3, eight rows' first parts and
     then their second parts), ``s`` uint8 [K / 128 rounded up, rows, 4] (e8m0 of the first part, one per 32 elements; the second part's is five
-    less)."""
-    p: torch.Tensor
-    s: torch.Tensor
+    less), in one allocation."""
+    __slots__ = ("shape", "data")
+
+    def __init__(self, rows: int, K: int, device):
+        self.shape = (rows, K)
+        self.data = torch.empty(self._scales_at() + -(-K // 128) * rows * 4, dtype=torch.uint8, device=device)
+
+    def _scales_at(self) -> int:
+        rows, K = self.shape
+        return -(-rows // 8) * 16 * K
 
     @property
-    def shape(self):
-        return self.s.shape[1], self.p.shape[3]
+    def p(self) -> torch.Tensor:
+        return self.data[:self._scales_at()].view(-1, 2, 8, self.shape[1])
+
+    @property
+    def s(self) -> torch.Tensor:
+        return self.data[self._scales_at():].view(-1, self.shape[0], 4)
 
     @property
     def is_cuda(self) -> bool:
-        return self.p.is_cuda
+        return self.data.is_cuda
 
-
-def _new_parts(rows: int, K: int, device) -> Parts:
-    return Parts(torch.empty(-(-rows // 8), 2, 8, K, dtype=torch.uint8, device=device), torch.empty(-(-K // 128), rows, 4, dtype=torch.uint8, device=device))
+    def pointers(self):
+        at = self.data.data_ptr()
+        return at, at + self._scales_at()
 
 
 def split(x: torch.Tensor, pos: Optional[torch.Tensor] = None, rows: Optional[int] = None) -> Parts:
     """Rows of x [T, K] as parts; with ``pos`` (int32 [T, k]) token t goes to every row pos[t, j] >= 0 of ``rows``, the others stay undefined."""
     T, K = x.shape
     rows = T if rows is None else rows
-    out = _new_parts(rows, K, x.device)
-    rc = _ext.lib().bg_mx_split(_ext.ptr(x), ctypes.c_longlong(x.stride(0)), _ext.ptr(pos), ctypes.c_int(pos.shape[1] if pos is not None else 0),
-                                ctypes.c_int(T), _ext.ptr(out.p), _ext.ptr(out.s), ctypes.c_int(rows), ctypes.c_int(K),
-                                _ext.stream())
-    _ext.check(rc, "bg_mx_split")
+    out = Parts(rows, K, x.device)
+    _call("bg_mx_split", x.data_ptr(), x.stride(0), _at(pos), pos.shape[1] if pos is not None else 0, T, *out.pointers(), rows, K)
     return out
 
 
 def gated_parts(gate_up: torch.Tensor, kind: int, limit: float, offsets: Optional[torch.Tensor], row_src: Optional[torch.Tensor]) -> Parts:
     """The gated activation of ``moe.activation`` (kind 0, 1, 2 of its kernel) with its rows as parts."""
     R, I = gate_up.shape[0], gate_up.shape[1] // 2
-    out = _new_parts(R, I, gate_up.device)
-    rc = _ext.lib().bg_gated_parts(ctypes.c_int(kind), _ext.ptr(gate_up), ctypes.c_longlong(gate_up.stride(0)), _ext.ptr(out.p), _ext.ptr(out.s),
-                                   ctypes.c_int(R), ctypes.c_int(I), ctypes.c_float(limit),
-                                   _ext.ptr(offsets[-1:] if offsets is not None else None), _ext.ptr(row_src),
-                                   ctypes.c_int(_ext.num_sms(gate_up.device)), _ext.stream())
-    _ext.check(rc, "bg_gated_parts")
+    out = Parts(R, I, gate_up.device)
+    _call("bg_gated_parts", kind, gate_up.data_ptr(), gate_up.stride(0), *out.pointers(), R, I, limit,
+          offsets.data_ptr() + 4 * (offsets.numel() - 1) if offsets is not None else None, _at(row_src), _ext.num_sms(gate_up.device))
     return out
 
 
@@ -105,8 +128,8 @@ def block_scaled(wq: torch.Tensor, ws: torch.Tensor, rows: float, split: bool = 
     """The block-scaled product takes weights wq [.., N, K / 2], ws [.., N, K / 32] for segments of ``rows`` expected rows: up to 80 of them (128 experts of
     6,144 x 2,880, against weights expanded to bf16: 5 rows 287 / 553 us, 28 rows 369 / 559, 47 rows 449 / 573, 94 rows 643 / 605), K to 12,288, addresses and
     rows as its loads need them.  K below 1,024 from one and a half rounds of tiles on: a tile of few steps is over before its start is paid
-    (layers, 16 rows: 16 experts of 512 x 768 55.4 / 53.3, of 2,048 x 768 67.6 / 72.6, 128 of 512 x 768 105.6 / 113.6).  Where the parts take a launch of their own (``split``), K beyond 2,048, and
-    beyond 4,096 with tiles of 96 tokens (dense, 24 tokens, 1,024 x 1,024 15.3 / 12.5, 4,096 x 1,024 15.3 / 14.4, 2,048 x 2,048 17.4 / 18.5, 2,880 x 3,072 19.4 / 22.6;
+    (layers, 16 rows: 16 experts of 512 x 768 55.4 / 53.3, of 2,048 x 768 67.6 / 72.6, 128 of 512 x 768 105.6 / 113.6).  Where the parts take a launch of their own
+    (``split``), K beyond 2,048, and beyond 4,096 with tiles of 96 tokens (dense, 24 tokens, 1,024 x 1,024 15.3 / 12.5, 4,096 x 1,024 15.3 / 14.4, 2,048 x 2,048 17.4 / 18.5, 2,880 x 3,072 19.4 / 22.6;
     31 tokens, 2,880 x 3,072 23.6 / 22.5, 4,096 x 4,096 29.5 / 26.7, x 6,144 31.7 / 34.9).  With tiles of 96 tokens K to 10,112, past which shared memory has two
     stages (40 tokens, 4,096 x 9,216 39.9 / 49.2, x 12,288 64.5 / 63.5, 80 tokens 68.6 / 65.5)."""
     K, wide = 2 * wq.shape[-1], rows > BLOCK_NARROW_ROWS
@@ -116,18 +139,16 @@ def block_scaled(wq: torch.Tensor, ws: torch.Tensor, rows: float, split: bool = 
         return False
     if K < 1024 and 2 * (wq.numel() // (wq.shape[-1] * wq.shape[-2])) * -(-wq.shape[-2] // 128) < 3 * _ext.num_sms(wq.device):
         return False
-    return bool(_ext.lib().bg_mxfp4_block_takes(_ext.ptr(wq), _ext.ptr(ws), ctypes.c_longlong(wq.shape[-2]), ctypes.c_int(K)))
+    # as bg_mxfp4_block_takes has it
+    return 128 <= K <= 12288 and K % 64 == 0 and wq.shape[-2] * (K // 32) % 16 == 0 and wq.data_ptr() % 32 == 0 and ws.data_ptr() % 16 == 0
 
 
 def _block_gemm(x: Union[torch.Tensor, Parts], wq2d, ws2d, out, offsets, groups, M, N, K, counts, rows) -> None:
     if isinstance(x, torch.Tensor):
         x = x.contiguous()
         x = split(x if x.data_ptr() % 16 == 0 else x.clone())
-    rc = _ext.lib().bg_mxfp4_block_gemm(
-        _ext.ptr(x.p), _ext.ptr(x.s), _ext.ptr(wq2d), _ext.ptr(ws2d), _ext.ptr(out), ctypes.c_int(out.stride(0)),
-        _ext.ptr(offsets), _ext.ptr(counts), ctypes.c_int(groups), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K), ctypes.c_float(rows),
-        ctypes.c_int(_ext.num_sms(out.device)), _ext.ptr(_ext.status_word(out.device)), _ext.stream())
-    _ext.check(rc, "bg_mxfp4_block_gemm")
+    _call("bg_mxfp4_block_gemm", *x.pointers(), wq2d.data_ptr(), ws2d.data_ptr(), out.data_ptr(), out.stride(0), _at(offsets), _at(counts), groups, M, N, K, rows,
+          _ext.num_sms(out.device), _ext.status_word(out.device).data_ptr())
 
 
 def mxfp4_gemm(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
