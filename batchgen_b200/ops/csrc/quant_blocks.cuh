@@ -37,8 +37,11 @@ __device__ __forceinline__ float quant_block(const float (&f)[8], uint8_t* q, in
 // capacity above the rows that are present costs nothing.  A CTA a row kept one load in flight and cost its start for every padding row:
 // expert rows of 2,048 for 4,739 tokens (8 of 256 experts, segments of 128) 94 us, now 65; 4 tokens 14, now 8.  Few blocks (a decode step) take U = 1, so
 // that they spread over the SMs.
-constexpr int kWalkBlocks = 148 * 8;
-inline bool many_blocks(long long rows, int K) { return rows * (K / 128) >= 148ll * 64 * 2; }
+// The line between the two is where a lane of every resident warp of 148 SMs has a block, us with U = 1 and 4: tokens of 7,168 to eight expert rows, 4,736 blocks
+// 8.2 / 10.3, 14,208 10.6 / 11.9, 18,944 12.4 / 12.2, 37,888 18.4 / 16.4, 150,000 51.4 / 47.1; rows alone 14,208 8.3 / 8.4, 18,944 9.0 / 8.4, 150,000 22.6 / 18.5.
+constexpr int kSms = 148;
+constexpr int kWalkBlocks = kSms * 8;
+inline bool many_blocks(long long rows, int K) { return rows * (K / 128) >= kSms * 64ll * 2; }
 inline int walk_grid(long long rows, int K, int U) {
   const long long warps = rows * ((K / 128 + 2 * U - 1) / (2 * U)), blocks = (warps + 7) / 8;
   return static_cast<int>(blocks < kWalkBlocks ? blocks : kWalkBlocks);

@@ -105,13 +105,13 @@ _CHUNK_SCRATCH = 1 << 30              # bytes of scratch a round of chunks may t
 
 
 def chunk_form_pays(lens: Sequence[int], heads: int, sms: int) -> bool:
-    """Whether pieces of ``lens`` tokens are faster in chunks.  In chunks: 90 us to start, 0.52 us a (chunk, head) and 0.25 us a (piece, head) for
-    its state, on 148 SMs.  Token by token a CTA serves a (piece, head): 1.6 to 2.0 us a token of the longest piece with a CTA on an SM, 2.42
-    with two, and 2.42 a token of every further round of two CTAs an SM.  Measured in us, chunks / tokens: 32 heads 1 x 64 100 / 131, 1 x
-    4,096 1,160 / 8,100, 4 x 512 648 / 1,044, 16 x 128 724 / 649, 8 x 1,024 2,183 / 2,485, 64 x 64 1,638 / 1,136, 64 x 128 2,657 / 2,200, 64 x 512
-    8,943 / 8,568; 8 heads 16 x 128 225 / 235, 64 x 512 2,255 / 2,472; 64 heads 16 x 512 4,554 / 4,643, 128 x 64 6,356 / 4,384.  The chunks have become
-    faster since (32 heads 1 x 64 67, 1 x 4,096 913, 4 x 512 404, 16 x 128 416, 8 x 1,024 1,014, 64 x 64 848, 64 x 128 1,543): the line still lies where both
-    took the same time then, so it leaves some short pieces to the tokens that chunks would now serve up to a third faster."""
+    """Whether pieces of ``lens`` tokens go through chunks.  Token by token a CTA serves a (piece, head): 1.6 to 2.0 us a token of the longest piece with a
+    CTA on an SM, 2.42 with two, and 2.42 a token of every further round of two CTAs an SM.  For chunks the line counts 90 us to start, 0.52 us a (chunk,
+    head) and 0.25 us a (piece, head) for its state, on 148 SMs, which is what they cost with their chain on CUDA cores.  They are faster now, and win
+    nearly everywhere: us, chunks / tokens, 32 heads 1 x 64 73 / 137, 4 x 48 83 / 107, 16 x 128 423 / 628, 4 x 512 413 / 1,030, 8 x 300 521 / 737, 8 x 1,024
+    1,519 / 2,460, 64 x 64 861 / 1,100, 64 x 128 1,574 / 2,166, 64 x 512 5,994 / 8,547, 1 x 4,096 929 / 8,100; 8 heads 16 x 128 138 / 266, 64 x 512 1,521 / 2,457; 64 heads 4 x
+    48 142 / 129, 8 x 300 974 / 1,446.  So the line sends to the tokens what chunks would serve up to 1.5 times as fast (of these points 32 heads 4 x 48, 8 x 300, 16 x
+    128, 64 x 64, 64 x 128 and 64 x 512): it lies where both took the same time with the older chain."""
     if not lens:
         return False
     pairs, longest, total = heads * len(lens), max(lens), sum(lens)
