@@ -132,22 +132,23 @@ def block_scaled(wq: torch.Tensor, ws: torch.Tensor, rows: float, split: bool = 
     (``split``), K beyond 2,048, and beyond 4,096 with tiles of 96 tokens (dense, 24 tokens, 1,024 x 1,024 15.3 / 12.5, 4,096 x 1,024 15.3 / 14.4, 2,048 x 2,048 17.4 / 18.5, 2,880 x 3,072 19.4 / 22.6;
     31 tokens, 2,880 x 3,072 23.6 / 22.5, 4,096 x 4,096 29.5 / 26.7, x 6,144 31.7 / 34.9).  With tiles of 96 tokens K to 10,112, past which shared memory has two
     stages (40 tokens, 4,096 x 9,216 39.9 / 49.2, x 12,288 64.5 / 63.5, 80 tokens 68.6 / 65.5)."""
-    K, wide = 2 * wq.shape[-1], rows > BLOCK_NARROW_ROWS
+    N, Kh = wq.shape[-2:]
+    K, wide = 2 * Kh, rows > BLOCK_NARROW_ROWS
     if rows > BLOCK_MAX_ROWS or (wide and K > 10112):
         return False
     if split and K <= (4096 if wide else 2048):
         return False
-    if K < 1024 and 2 * (wq.numel() // (wq.shape[-1] * wq.shape[-2])) * -(-wq.shape[-2] // 128) < 3 * _ext.num_sms(wq.device):
+    if K < 1024 and 2 * (wq.numel() // (N * Kh)) * -(-N // 128) < 3 * _ext.num_sms(wq.device):
         return False
     # as bg_mxfp4_block_takes has it
-    return 128 <= K <= 12288 and K % 64 == 0 and wq.shape[-2] * (K // 32) % 16 == 0 and wq.data_ptr() % 32 == 0 and ws.data_ptr() % 16 == 0
+    return 128 <= K <= 12288 and K % 64 == 0 and N * (K // 32) % 16 == 0 and wq.data_ptr() % 32 == 0 and ws.data_ptr() % 16 == 0
 
 
-def _block_gemm(x: Union[torch.Tensor, Parts], wq2d, ws2d, out, offsets, groups, M, N, K, counts, rows) -> None:
+def _block_gemm(x: Union[torch.Tensor, Parts], wq, ws, out, offsets, groups, M, N, K, counts, rows) -> None:
     if isinstance(x, torch.Tensor):
         x = x.contiguous()
         x = split(x if x.data_ptr() % 16 == 0 else x.clone())
-    _call("bg_mxfp4_block_gemm", *x.pointers(), wq2d.data_ptr(), ws2d.data_ptr(), out.data_ptr(), out.stride(0), _at(offsets), _at(counts), groups, M, N, K, rows,
+    _call("bg_mxfp4_block_gemm", *x.pointers(), wq.data_ptr(), ws.data_ptr(), out.data_ptr(), out.stride(0), _at(offsets), _at(counts), groups, M, N, K, rows,
           _ext.num_sms(out.device), _ext.status_word(out.device).data_ptr())
 
 
@@ -195,11 +196,12 @@ def grouped_mxfp4_gemm(x: Union[torch.Tensor, Parts], wq: torch.Tensor, ws: torc
         out = torch.empty(R, n_out, dtype=torch.bfloat16, device=wq.device)
     if R:
         assert offsets.dtype == torch.int32 and offsets.is_cuda
-        wq2d, ws2d = wq.view(E * N, Kh), ws.view(E * N, K // 32)
+        if not (wq.is_contiguous() and ws.is_contiguous()):          # the kernels take addresses
+            wq, ws = wq.view(E * N, Kh), ws.view(E * N, K // 32)
         rows = (R if rows_hint is None else rows_hint) / max(E, 1)
         if isinstance(x, Parts) or not silu_mul and block_scaled(wq, ws, rows, split=True):
             assert not silu_mul
-            _block_gemm(x, wq2d, ws2d, out, offsets, E, R, N, K, counts, rows)
+            _block_gemm(x, wq, ws, out, offsets, E, R, N, K, counts, rows)
         else:
-            _launch(EPI_SILU_MUL if silu_mul else EPI_STORE, x.contiguous(), wq2d, ws2d, out, offsets, E, R, N, K, counts)
+            _launch(EPI_SILU_MUL if silu_mul else EPI_STORE, x.contiguous(), wq, ws, out, offsets, E, R, N, K, counts)
     return out
