@@ -242,20 +242,24 @@ mha_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       tmem_ld32(tm_s, sv);
       tmem_ld32(tm_s + 32, sv + 32);
       tmem_ld_wait();
-      if (all_see < (t + 1) * BN) {
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      if (all_see < (t + 1) * BN) {             // masked after the scale, which may be zero or negative
         const int n_ok = visible - t * BN;
 #pragma unroll
-        for (int j = 0; j < 64; ++j)
-          if (j >= n_ok) sv[j] = 0xFF800000u;
-      }
-      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        for (int j = 0; j < 64; ++j) {
+          const float v = j < n_ok ? __uint_as_float(sv[j]) * scale_log2 : -INFINITY;
+          sv[j] = __float_as_uint(v);
+          mx[j & 3] = fmaxf(mx[j & 3], v);
+        }
+      } else {
 #pragma unroll
-      for (int j = 0; j < 64; j += 2) {
-        const float2 v = __fmul2_rn(make_float2(__uint_as_float(sv[j]), __uint_as_float(sv[j + 1])), make_float2(scale_log2, scale_log2));
-        sv[j] = __float_as_uint(v.x);
-        sv[j + 1] = __float_as_uint(v.y);
-        mx[j & 2] = fmaxf(mx[j & 2], v.x);
-        mx[(j & 2) + 1] = fmaxf(mx[(j & 2) + 1], v.y);
+        for (int j = 0; j < 64; j += 2) {
+          const float2 v = __fmul2_rn(make_float2(__uint_as_float(sv[j]), __uint_as_float(sv[j + 1])), make_float2(scale_log2, scale_log2));
+          sv[j] = __float_as_uint(v.x);
+          sv[j + 1] = __float_as_uint(v.y);
+          mx[j & 2] = fmaxf(mx[j & 2], v.x);
+          mx[(j & 2) + 1] = fmaxf(mx[(j & 2) + 1], v.y);
+        }
       }
       const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       const bool grow = mt > m_run + 8.f;

@@ -190,6 +190,22 @@ def test_expanded_mla_prefill_halves_as_ctas(lens, ctx):
     assert (all_ == few.unsqueeze(1)).all()
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.07, 0.07])
+@pytest.mark.parametrize("n_q,ctx", [(70, 0), (300, 40)])
+def test_expanded_mla_prefill_any_scale(n_q, ctx, scale):
+    """Keys behind a query stay out whatever the scale's sign; a scale of zero is the mean of the values."""
+    from batchgen_b200.ops import _ext, attention
+    H, g = 2, torch.Generator().manual_seed(n_q)
+    q, kv = (torch.randn(n, H, d, generator=g).to(torch.bfloat16) for n, d in ((n_q, 192), (n_q + ctx, 256)))
+    q[..., 128:] = 0
+    work = attention.mha_prefill_work([0, n_q], [ctx], [0])
+    got = attention.mha_prefill(q.cuda(), kv.cuda(), torch.zeros(n_q + ctx, 64, dtype=torch.bfloat16, device="cuda"), work, scale).cpu().double()
+    _ext.check_status()
+    want, mag = _attention64(q, kv, ctx, scale)
+    # probabilities and output rounded to 8 bits, exponents of fp32 sums of 128 products
+    assert ((got - want).abs() <= mag * 2.0 ** -7 + 1e-6).all()
+
+
 def test_model_prefill_uses_expanded_attention_and_matches_cpu():
     from batchgen_b200.config import get_model_config
     from batchgen_b200.models import build_model
