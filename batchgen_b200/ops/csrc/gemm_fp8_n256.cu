@@ -470,7 +470,7 @@ static int gemm_fp8_n256_impl(int epi, const void* A, const float* sA, int sa_st
                               int num_sms, bg::g256::Params p, cudaStream_t stream) {
   using namespace bg::g256;
   if (M <= 0 || N <= 0) return 0;
-  if (K % 128 != 0 || groups > kMaxGroups || (epi == EPI_SILU_MUL && (N % 256) != 0) || (ldd % 8) != 0) return -1;
+  if (K % 128 != 0 || groups > kMaxGroups || (epi == EPI_SILU_MUL && (N % 256) != 0) || (ldd % 8) != 0 || reinterpret_cast<uintptr_t>(D) % 16 != 0) return -1;
   if (p.row_map != nullptr && (epi != EPI_STORE || (N % 8) != 0)) return -1;
   if (offsets == nullptr) groups = 1;
   p.sA = sA; p.sa_stride = sa_stride; p.sB = sB; p.D = reinterpret_cast<__nv_bfloat16*>(D); p.ldd = ldd;

@@ -139,6 +139,9 @@ struct TileWalker {
   }
 };
 
+// rows of D may start anywhere (an odd row stride, a view): 16 bytes a store where the row allows it
+__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 template <int KIND, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
@@ -427,9 +430,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           const int col0 = t.nt * 64 + half * 32;
           const int n_out = p.N / 2;
           __nv_bfloat16* dst = out_base + out_row * p.ldd + col0;
+          const bool wide = aligned16(dst);
 #pragma unroll
           for (int j = 0; j < 32; j += 8) {
-            if (col0 + j + 8 <= n_out) {
+            if (wide && col0 + j + 8 <= n_out) {
               __align__(16) __nv_bfloat162 o[4];
 #pragma unroll
               for (int q = 0; q < 4; ++q) {
@@ -446,9 +450,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         } else if (EPI == EPI_STORE_F32) {
           const int col0 = t.nt * BN + half * 64;
           float* dst = reinterpret_cast<float*>(p.D) + out_row * p.ldd + col0;
+          const bool wide = aligned16(dst);
 #pragma unroll
           for (int j = 0; j < 64; j += 4) {
-            if (col0 + j + 4 <= p.N) {
+            if (wide && col0 + j + 4 <= p.N) {
               *reinterpret_cast<float4*>(dst + j) = make_float4(r[j], r[j + 1], r[j + 2], r[j + 3]);
             } else {
               for (int q = 0; q < 4; ++q)
@@ -465,9 +470,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
           const int col0 = t.nt * BN + half * 64;
           __nv_bfloat16* dst = out_base + out_row * p.ldd + col0;
+          const bool wide = aligned16(dst);
 #pragma unroll
           for (int j = 0; j < 64; j += 8) {
-            if (col0 + j + 8 <= p.N) {
+            if (wide && col0 + j + 8 <= p.N) {
               __align__(16) __nv_bfloat162 o[4];
 #pragma unroll
               for (int q = 0; q < 4; ++q) o[q] = __floats2bfloat162_rn(r[j + 2 * q], r[j + 2 * q + 1]);

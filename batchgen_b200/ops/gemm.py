@@ -71,7 +71,7 @@ def _use_wide(kind, D, M, N, wide, dense) -> bool:
     and 43; 6,144 x 3,072, 900 rows (192) 50 and 35, 768 rows (144) 29 and 35; short K likewise, 900 x 3,072 with K of 128 13.3 and 11.2, 1,024
     19.5 and 15.0, 2,048 29 and 20.  Grouped products, whose tiles are an upper bound here,
     keep two rounds.  GEMMs that consume collective hooks (rows stored to peers, flag waits) and bf16 operands stay on the 128 x 128
-    kernel, and in its second round rows that the wide one does not take (row stride no multiple of 8)."""
+    kernel, and in its second round rows that the wide one does not take (not in 16-byte pieces)."""
     global _hooks_pending
     if _hooks_pending:
         _hooks_pending = False
@@ -82,7 +82,7 @@ def _use_wide(kind, D, M, N, wide, dense) -> bool:
         return True
     tiles = -(-M // 128) * -(-N // 128)
     sms = _ext.num_sms(D.device)
-    return tiles >= 2 * sms or dense and tiles > sms and D.stride(0) % 8 == 0
+    return tiles >= 2 * sms or dense and tiles > sms and D.stride(0) % 8 == 0 and D.data_ptr() % 16 == 0
 
 
 def wide_enabled() -> bool:

@@ -274,6 +274,48 @@ def test_tile_width_of_a_second_round(T, N, wide):
     assert _rel(got.float().cpu(), ref.fp8_gemm(xq, xs, wq, ws)) < 1e-2
 
 
+@pytest.mark.parametrize("T,N,pad,off", [(40, 300, 0, 0), (130, 300, 3, 1), (40, 264, 8, 4), (257, 129, 0, 0), (1, 301, 0, 3), (40, 256, 0, 0)])
+@pytest.mark.parametrize("K", [256, 4096])
+def test_narrow_tile_rows_of_any_alignment(T, N, pad, off, K):
+    """Rows whose stride or start is no multiple of 16 bytes: the values, and nothing beside them, of every epilogue of the 128 x 128 kernel; split K too."""
+    from batchgen_b200.ops import _ext, gemm, ref
+    g = torch.Generator().manual_seed(T + N)
+    ld = N + pad
+
+    def into(rows, cols, dtype):
+        buf = torch.full((rows * ld + off + 8,), 768.0, dtype=dtype, device="cuda")
+        return buf, buf[off:off + rows * ld].view(rows, ld)[:, :cols]
+
+    def check(buf, view, want, rel):
+        _ext.check_status()
+        assert ((view.cpu().double() - want).abs() <= rel).all()
+        view.fill_(768.0)
+        assert (buf == 768).all()
+
+    x, w = torch.randn(T, K, generator=g).bfloat16(), (torch.randn(N, K, generator=g) * 0.1).bfloat16()
+    want, mag = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t() * K * 2.0 ** -24
+    buf, out = into(T, N, torch.bfloat16)
+    gemm._launch(gemm.KIND_BF16, gemm.EPI_STORE, x.cuda(), None, 0, w.cuda(), None, out, None, 1, T, N, K)
+    check(buf, out, want, want.abs() * 2.0 ** -8 + mag)
+    if ld % 4 == 0:
+        buf, out = into(T, N, torch.float32)
+        gemm.bf16_gemm(x.cuda(), w.cuda(), out=out, fp32_out=True)
+        check(buf, out, want, mag + want.abs() * 2.0 ** -23)
+    xq, xs = ref.act_quant(torch.randn(T, K, generator=g))
+    wq, ws = (torch.randn(N, K, generator=g) * 0.1).to(torch.float8_e4m3fn), torch.rand((N + 127) // 128, K // 128, generator=g) + 0.5
+    buf, out = into(T, N, torch.bfloat16)
+    gemm.fp8_gemm(xq.cuda(), xs.cuda(), wq.cuda(), ws.cuda(), out=out, wide=False)
+    want = ref.fp8_gemm(xq, xs, wq, ws).double()
+    _ext.check_status()
+    assert _rel(out.cpu(), want) < 1e-2
+    if N % 256 == 0:
+        out.fill_(768.0)
+        half = out[:, :N // 2]
+        perm = gemm.interleave_gate_up_rows(N)
+        gemm.fp8_gemm(xq.cuda(), xs.cuda(), wq.view(torch.uint8)[perm].contiguous().view(torch.float8_e4m3fn).cuda(), ws.cuda(), out=half, silu_mul=True, wide=False)
+        assert _rel(half.cpu(), ref.silu_mul(want.float())) < 1e-2 and (out[:, N // 2:] == 768).all()
+
+
 def test_tile_width_rule(monkeypatch):
     """Either side of each border of the rule itself: one round of narrow tiles for dense products, two for grouped ones, row strides, operands, hooks."""
     from batchgen_b200.ops import _ext, gemm
