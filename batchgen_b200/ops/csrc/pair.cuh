@@ -24,10 +24,11 @@ __device__ __forceinline__ uint32_t leader_addr(const void* p) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(out) : "r"(smem_u32(p)));
   return out;
 }
-// Arrive on a barrier in either CTA, for a thread there that waits with wait_cluster: what the arriving thread has read is read before what
-// the waiting one issues, across CTAs only at cluster scope.
+// Arrive on a barrier in either CTA, for a thread there that waits with wait_cluster.  At cluster scope, for the waiter is in another CTA; relaxed, for what
+// is handed over is TMEM, whose reads tcgen05.fence::before_thread_sync orders before the arrival, and nothing that this thread stored: a release
+// would also wait for the tile's stores to land (64 matrices of 2,304 x 512 with 300 rows 84 us, 66 so).
 __device__ __forceinline__ void arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ bool try_wait_cluster(uint64_t* bar, uint32_t parity) {
   uint32_t ok;

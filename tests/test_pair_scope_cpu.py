@@ -11,12 +11,17 @@ def _source(name):
     return re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
 
 
-def test_arrivals_in_another_cta_release_at_cluster_scope():
+def test_arrivals_in_another_cta_are_at_cluster_scope():
     for name in sorted(os.listdir(CSRC)):
         if name.endswith((".cu", ".cuh")):
             for ins in re.findall(r"mbarrier\.arrive[\w.:]*", _source(name)):
                 if "shared::cluster" in ins:
-                    assert ".release.cluster" in ins, (name, ins)
+                    assert re.search(r"\.(release|relaxed)\.cluster\.", ins), (name, ins)
+
+
+def test_relaxed_arrivals_stand_behind_the_fence_of_the_reads_they_report():
+    assert re.search(r"tc_fence_before\(\);\s*__syncwarp\(\);\s*if \(lane == 0\) pair::arrive_cluster\(", _source("gemm_bf16_pair.cu"))
+    assert _source("gemm_bf16_pair.cu").count("arrive_cluster(") == 1
 
 
 def test_waits_of_a_pair_acquire_at_cluster_scope():
