@@ -1,8 +1,11 @@
-// Dense bf16 GEMM with the weights on the tensor-core M side and up to 256 tokens as N (D^T = W . X^T), for products of few tiles.
+// bf16 GEMM with the weights on the tensor-core M side and up to 256 tokens as N (D^T = W . X^T), dense and ragged grouped, for products of few
+// tiles, short K or rows that start anywhere.
 //
-// A weight tile of 128 rows meets all tokens (up to 256 at a time, cut evenly, rounded up to 16) in one product of that width.  From two
-// rounds of 256 x 256 tiles on, and for segments of rows, pairs of CTAs move fewer operand bytes (gemm_bf16_pair.cu); below, tiles of half
-// the size fill the SMs better: 1,024 x 4,096 x 2,880 25 us (pairs 27), 2,000 x 1,024 x 4,096 29 (31), 160 x 32,768 x 512 15 (17).
+// A weight tile of 128 rows meets all tokens of its segment (up to 256 at a time, cut evenly, rounded up to 16) in one product of that width.
+// With enough 256 x 256 tiles and K from 512 on, pairs of CTAs move fewer operand bytes (gemm_bf16_pair.cu).  Below, tiles of half the size fill
+// the SMs better, us here and on pairs: 1,024 x 4,096 x 2,880 25 / 27, 2,000 x 1,024 x 4,096 29 / 31, 160 x 32,768 x 512 15 / 17; of short K a pair stores
+// a tile longer than it multiplies the next: 6,000 x 4,096 x 256 24.5 / 28.7, x 512 32.8 / 32.8; and two bytes a store do not mind where a row
+// starts: 1,100 x 20,004 x 1,024 51 / 139.
 //
 // Roles (192 threads, one CTA per SM, persistent): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 2..5 epilogue (thread = weight
 // row; two accumulators of 256 columns, so one is stored while the other is filled).  All waits are bounded.
@@ -20,13 +23,16 @@ constexpr int BK = 64;                    // elements of K per stage (one 128-by
 constexpr int kStages = 4;
 constexpr int kThreads = 192;
 constexpr int kTmemCols = 512;
+constexpr int kMaxGroups = 1024;
 constexpr int kWBytes = BW * BK * 2;      // 16 KB
 constexpr int kXBytes = BT * BK * 2;      // 32 KB
 
 struct Params {
   __nv_bfloat16* D;      // [M, ldd]
   int ldd;
-  int M, N, K;
+  const int* offsets;    // [groups + 1] segment starts; null = dense
+  const int* counts;     // [groups] rows present in a segment, or null: all of it
+  int groups, M, N, K;
   int* status;
 };
 
@@ -35,6 +41,7 @@ struct Shared {
   uint64_t tmem_full[2], tmem_empty[2];
   uint32_t tmem_base;
   int abort_flag;
+  Segments<kMaxGroups> seg;
 };
 
 __global__ void __launch_bounds__(kThreads, 1)
@@ -56,6 +63,7 @@ gemm_bf16_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
     ss.abort_flag = 0;
     mbar_fence_init();
   }
+  if (p.offsets != nullptr) load_segments<BT>(ss.seg, p.offsets, p.counts, p.groups);
   if (warp == 1) {
     tmem_alloc(&ss.tmem_base, kTmemCols);
     tmem_relinquish();
@@ -64,7 +72,7 @@ gemm_bf16_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
-  TokenWalker<BT, BW, 1> walk(nullptr, 1, n_tiles, p.M);
+  TokenWalker<BT, BW, kMaxGroups> walk(p.offsets != nullptr ? &ss.seg : nullptr, p.groups, n_tiles, p.M);
   TokenTile t;
   uint32_t it = 0, acc = 0;
   bool ok = true;
@@ -75,7 +83,7 @@ gemm_bf16_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
       tma_prefetch_desc(&tmW);
       tma_prefetch_desc(&tmX);
       for (int tile = blockIdx.x; ok && walk.get(tile, t); tile += gridDim.x) {
-        const int boxes = (tile_cols(t) + kBox - 1) / kBox, row = t.n0;
+        const int boxes = (tile_cols(t) + kBox - 1) / kBox, row = t.g * p.N + t.n0;
         for (int kb = 0; kb < KB; ++kb, ++it) {
           const int s = it % kStages;
           if (!mbar_wait(&ss.empty[s], ((it / kStages) & 1) ^ 1, abort_flag, kTimeoutProducer)) { ok = false; break; }
@@ -186,23 +194,32 @@ static int make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t co
 
 extern "C" {
 
-// X [M, K] bf16 tokens, W [N, K] bf16 -> D [M, ldd] bf16.  K a multiple of 64.
-int bg_gemm_bf16_swap(const void* X, const void* W, void* D, int ldd, int M, int N, int K, int num_sms, int* status, cudaStream_t stream) {
+// X [M, K] bf16 tokens, W [groups * N, K] bf16 -> D [M, ldd] bf16.  K a multiple of 64.  offsets null: dense; counts: rows present in
+// every segment, or null (rows past them stay undefined).
+int bg_gemm_bf16_swap_grouped(const void* X, const void* W, void* D, int ldd, const int* offsets, const int* counts, int groups, int M, int N, int K,
+                              int num_sms, int* status, cudaStream_t stream) {
   using namespace bg::bswap;
   if (M <= 0 || N <= 0) return 0;
-  if (K <= 0 || K % BK != 0) return -1;
+  if (K <= 0 || K % BK != 0 || groups > kMaxGroups || groups <= 0) return -1;
+  if (offsets == nullptr) groups = 1;
   Params p;
-  p.D = reinterpret_cast<__nv_bfloat16*>(D); p.ldd = ldd; p.M = M; p.N = N; p.K = K; p.status = status;
+  p.D = reinterpret_cast<__nv_bfloat16*>(D); p.ldd = ldd; p.offsets = offsets; p.counts = offsets != nullptr ? counts : nullptr;
+  p.groups = groups; p.M = M; p.N = N; p.K = K; p.status = status;
   CUtensorMap tw, tx;
-  if (make_map(&tw, W, (uint64_t)N, (uint64_t)K, BW) != 0) return -11;
+  if (make_map(&tw, W, (uint64_t)groups * N, (uint64_t)K, BW) != 0) return -11;
   if (make_map(&tx, X, (uint64_t)M, (uint64_t)K, kBox) != 0) return -12;
   static bg::DeviceOnce once;
   const size_t smem = kStages * (kWBytes + kXBytes) + sizeof(Shared) + 1024;
   if (!bg::ensure_dynamic_smem(gemm_bf16_swap_kernel, smem, once)) return -13;
-  long long grid = ((long long)M / BT + 1) * ((N + BW - 1) / BW);      // an upper bound of the tiles
+  long long grid = ((long long)M / BT + (offsets != nullptr ? groups : 1)) * ((N + BW - 1) / BW);      // an upper bound of the tiles
   if (grid > num_sms) grid = num_sms;
   bg::launch_pdl(gemm_bf16_swap_kernel, dim3((int)grid), dim3(kThreads), smem, stream, tw, tx, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -14;
+}
+
+// the dense form
+int bg_gemm_bf16_swap(const void* X, const void* W, void* D, int ldd, int M, int N, int K, int num_sms, int* status, cudaStream_t stream) {
+  return bg_gemm_bf16_swap_grouped(X, W, D, ldd, nullptr, nullptr, 1, M, N, K, num_sms, status, stream);
 }
 
 }  // extern "C"

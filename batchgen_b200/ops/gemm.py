@@ -240,26 +240,39 @@ def swap_dense(T: int, N: int, K: int, sms: int) -> bool:
     return T > 128 or K < 1536 or T * K < 65536
 
 
-def use_pairs(T: int, N: int, sms: int) -> bool:
+PAIR_MIN_K = 512       # of shorter products a pair stores a tile longer than it multiplies the next
+
+
+def use_pairs(T: int, N: int, sms: int, K: int = PAIR_MIN_K) -> bool:
     """Pairs of CTAs on tiles of 256 x 256 for a dense product: from two rounds of such tiles on, unless they take more rounds than tiles of 256 x
     128 do (pairs / one CTA, us: 700 x 16,576 x 2,304 50 / 54, 300 x 20,480 x 2,880 48 / 56, 8,000 x 2,304 x 4,096 105 / 121; under two rounds 2,500
-    x 2,304 x 4,096 54 / 52, 160 x 32,768 x 512 17 / 15; four rounds against three 4,650 x 2,880 x 4,096 93 / 82)."""
+    x 2,304 x 4,096 54 / 52, 160 x 32,768 x 512 17 / 15; four rounds against three 4,650 x 2,880 x 4,096 93 / 82), and from K of 512 on (1,100 x 20,000
+    x 256 27.6 / 22.5, x 384 28.8 / 28.6, x 512 30.8 / 32.7; 8,000 x 2,304 x 256 22.7 / 20.5, x 384 24.6 / 22.5, x 512 26.6 / 26.6, x 640 26.8 / 28.7)."""
     tokens, pairs = -(-T // 256), sms // 2
     tiles = tokens * -(-N // 256)
-    return tiles >= 2 * pairs > 0 and -(-tiles // pairs) <= -(-tokens * -(-N // 128) // sms)
+    return K >= PAIR_MIN_K and tiles >= 2 * pairs > 0 and -(-tiles // pairs) <= -(-tokens * -(-N // 128) // sms)
 
 
-def _bf16_swap(x: torch.Tensor, w2d: torch.Tensor, out: torch.Tensor, offsets, counts, groups: int, N: int) -> None:
-    """Weights as the MMA's M, tokens as its N; segments of tokens always on pairs of CTAs, where they are never behind."""
-    sms = _ext.num_sms(x.device)
-    tail = (ctypes.c_int(x.shape[0]), ctypes.c_int(N), ctypes.c_int(x.shape[1]), ctypes.c_int(sms), _ext.ptr(_ext.status_word(x.device)), _ext.stream())
-    if offsets is not None or use_pairs(x.shape[0], N, sms):
-        rc = _ext.lib().bg_gemm_bf16_pair(_ext.ptr(x), _ext.ptr(w2d), _ext.ptr(out), ctypes.c_int(out.stride(0)), _ext.ptr(offsets),
-                                          _ext.ptr(counts), ctypes.c_int(groups), *tail)
-        _ext.check(rc, "bg_gemm_bf16_pair")
-        return
-    rc = _ext.lib().bg_gemm_bf16_swap(_ext.ptr(x), _ext.ptr(w2d), _ext.ptr(out), ctypes.c_int(out.stride(0)), *tail)
-    _ext.check(rc, "bg_gemm_bf16_swap")
+def use_pairs_grouped(rows: float, groups: int, N: int, K: int, sms: int) -> bool:
+    """The same for segments of ``rows`` expected rows: from K of 512 (pairs / one CTA, us: 256 matrices of 2,048 x 256 with 256 rows 139 / 139, x 512 165 / 190; 16 of
+    4,096 x 256 with 600 46 / 41, x 512 50 / 53) and one round of tiles on, of K of 2,304 and more under one too (8 of 768 x 512 with 300 rows 15.5 / 14.6, x 1,536 21.4 /
+    20.5; 8 of 2,048 x 2,304 with 200 32.8 / 34.7, 3 of 1,000 x 7,168 with 260 47 / 53), and not where 256 outputs a tile pad to a further round (64 of 304 x 1,536
+    with 300 rows 51 / 47)."""
+    tokens, pairs = groups * max(1, -(-int(rows) // 256)), sms // 2
+    tiles = tokens * -(-N // 256)
+    return K >= PAIR_MIN_K and (tiles >= pairs or K >= 2304) and pairs > 0 and -(-tiles // pairs) <= -(-tokens * -(-N // 128) // sms)
+
+
+def _bf16_swap(x: torch.Tensor, w2d: torch.Tensor, out: torch.Tensor, offsets, counts, groups: int, N: int, rows: Optional[float] = None) -> None:
+    """Weights as the MMA's M, tokens as its N (``rows``: expected in a segment), on pairs of CTAs where they pay and rows of ``out`` are in 16-byte pieces
+    (1,100 x 20,004 x 1,024: a pair's scalar stores 139 us, one CTA's 51)."""
+    sms, (M, K) = _ext.num_sms(x.device), x.shape
+    tail = (ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K), ctypes.c_int(sms), _ext.ptr(_ext.status_word(x.device)), _ext.stream())
+    pairs = use_pairs(M, N, sms, K) if offsets is None else use_pairs_grouped(M / groups if rows is None else rows, groups, N, K, sms)
+    name = "bg_gemm_bf16_pair" if pairs and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 else "bg_gemm_bf16_swap_grouped"
+    rc = getattr(_ext.lib(), name)(_ext.ptr(x), _ext.ptr(w2d), _ext.ptr(out), ctypes.c_int(out.stride(0)), _ext.ptr(offsets), _ext.ptr(counts),
+                                   ctypes.c_int(groups), *tail)
+    _ext.check(rc, name)
 
 
 def swap_grouped(rows: float, groups: int, K: int) -> bool:
@@ -277,8 +290,9 @@ def grouped_bf16_gemm(x: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, c
     are expected to be present in all (the capacity x.shape[0] when None; it is far above them where other ranks hold most experts)."""
     E, N, K = w.shape
     out = torch.empty(x.shape[0], N, dtype=torch.bfloat16, device=x.device)
-    if x.shape[0] and not relu2 and swap_grouped((x.shape[0] if rows_hint is None else rows_hint) / max(E, 1), E, K):
-        _bf16_swap(x.contiguous(), w.view(E * N, K), out, offsets, counts, E, N)
+    rows = (x.shape[0] if rows_hint is None else rows_hint) / max(E, 1)
+    if x.shape[0] and not relu2 and swap_grouped(rows, E, K):
+        _bf16_swap(x.contiguous(), w.view(E * N, K), out, offsets, counts, E, N, rows)
     elif x.shape[0]:
         _launch(KIND_BF16, EPI_RELU2 if relu2 else EPI_STORE, x.contiguous(), None, 0, w.view(E * N, K), None, out, offsets, E, x.shape[0], N, K,
                 counts=counts)

@@ -260,3 +260,46 @@ def test_rotated_queries_do_not_depend_on_alignment(interleaved):
     u, v = a * c - (b * s).float().double(), a * s + (b * c).float().double()
     want = torch.stack([u, v], -1).flatten(-2) if interleaved else torch.cat([u, v], -1)
     assert torch.equal(got[0][..., D - rope:], want.float().to(torch.bfloat16)) and torch.equal(got[0][..., :D - rope], q[..., :D - rope])
+
+
+@pytest.mark.parametrize("pairs", [True, False])
+@pytest.mark.parametrize("counts,align", [([1, 0, 17, 130], 8), ([256, 257, 5, 600], 8), ([15, 16, 31, 33], 16), ([3, 0, 0, 0], 8)])
+@pytest.mark.parametrize("N,K", [(128, 64), (200, 192), (384, 1024)])
+def test_grouped_bf16_forms(pairs, counts, align, N, K, monkeypatch):
+    """Segments on pairs of CTAs and on one, whichever the rule would take."""
+    from batchgen_b200.ops import gemm
+    monkeypatch.setattr(gemm, "use_pairs_grouped", lambda *a: pairs)
+    test_grouped_bf16_token_tiles(counts, align, N, K)
+
+
+@pytest.mark.parametrize("pad,off", [(0, 0), (4, 0), (0, 4), (3, 1)])
+@pytest.mark.parametrize("counts", [None, [130, 0, 300, 7]])
+def test_bf16_rows_that_are_not_in_16_byte_pieces(counts, pad, off, monkeypatch):
+    """Such rows stay on one CTA even where pairs pay; the same bits, nothing beside them."""
+    from batchgen_b200.ops import _ext, gemm
+    g = torch.Generator().manual_seed(1)
+    N, K, E = 520, 704, 1 if counts is None else len(counts)
+    offs = [0]
+    for c in counts or [437]:
+        offs.append(offs[-1] + c)
+    M = offs[-1]
+    monkeypatch.setattr(gemm, "use_pairs", lambda *a: True)
+    monkeypatch.setattr(gemm, "use_pairs_grouped", lambda *a: True)
+    names = []
+    lib = _ext.lib()
+    monkeypatch.setattr(_ext, "lib", lambda: type("L", (), {"__getattr__": lambda self, n: (names.append(n), getattr(lib, n))[1]})())
+    x, w = torch.randn(M, K, generator=g).bfloat16().cuda(), torch.randn(E, N, K, generator=g).bfloat16().cuda()
+    tables = [None, None] if counts is None else [torch.tensor(v, dtype=torch.int32, device="cuda") for v in (offs, counts)]
+    whole = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    gemm._bf16_swap(x, w.view(E * N, K), whole, *tables, E, N)
+    buf = torch.full((M * (N + pad) + off,), 7.0, dtype=torch.bfloat16, device="cuda")
+    out = buf[off:].view(M, N + pad)[:, :N]
+    gemm._bf16_swap(x, w.view(E * N, K), out, *tables, E, N)
+    _ext.check_status()
+    assert names == ["bg_gemm_bf16_pair", "bg_gemm_bf16_swap_grouped" if pad % 8 or off % 8 else "bg_gemm_bf16_pair"] and torch.equal(out, whole)
+    out.fill_(7.0)
+    assert (buf == 7).all()
+    xe = x.double().cpu()
+    want = torch.cat([xe[offs[e]:offs[e + 1]] @ w[e].double().cpu().t() for e in range(E)])
+    mag = torch.cat([xe[offs[e]:offs[e + 1]].abs() @ w[e].double().cpu().abs().t() for e in range(E)])
+    assert ((whole.cpu().double() - want).abs() <= want.abs() * 2 ** -8 + mag * K * 2 ** -24).all()

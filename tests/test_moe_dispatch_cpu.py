@@ -45,3 +45,16 @@ def test_expert_parallel_rank_expects_its_share(replicated, monkeypatch):
                                            (64, 16384, 1472, True), (64, 16384, 1536, False), (512, 16384, 96, False)])
 def test_dense_kernel_by_tiles_and_tokens(T, N, K, swapped):
     assert gemm.swap_dense(T, N, K, 148) == swapped
+
+
+@pytest.mark.parametrize("T,N,K,pairs", [(4096, 16576, 2304, True), (4096, 16576, 512, True), (4096, 16576, 448, False), (2500, 2304, 4096, False), (4650, 2880, 4096, False),
+                                         (37 * 256, 1024, 704, True), (36 * 256, 1024, 704, False)])
+def test_dense_pairs_by_tiles_and_k(T, N, K, pairs):
+    assert gemm.use_pairs(T, N, 148, K) == pairs
+
+
+@pytest.mark.parametrize("rows,groups,N,K,pairs", [(128, 256, 2048, 2304, True), (128, 256, 2304, 512, True), (128, 256, 2304, 448, False), (200, 8, 2048, 2304, True),
+                                                   (200, 8, 2048, 2240, False), (300, 64, 304, 1536, False), (256, 37, 512, 1024, True), (256, 36, 512, 1024, False),
+                                                   (257, 19, 512, 1024, True)])
+def test_grouped_pairs_by_tiles_and_k(rows, groups, N, K, pairs):
+    assert gemm.use_pairs_grouped(rows, groups, N, K, 148) == pairs
