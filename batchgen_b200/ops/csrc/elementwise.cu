@@ -228,7 +228,8 @@ __global__ void rope_q_kernel(__nv_bfloat16* __restrict__ q, int H, int D, int r
 
 // The same, eight pairs a thread in 16-byte pieces (rope a multiple of 16, pieces on 16-byte boundaries).  Bound by
 // its bytes: two bytes an access took 63.5 us for 4,739 tokens of 128 heads with 64 rotated dims, now 34.8 (floor
-// 24 at the 32-byte sectors touched); 4 tokens 15, now 8.
+// 24 at the 32-byte sectors touched); 4 tokens 15, now 8.  Where a token has a pair a thread at most, and few tokens keep the SMs waiting for one
+// round of loads, the other kernel's shorter chain is faster: 64 tokens of 8 heads x 64 dims 1.58 us, here 1.73; 4,000 tokens 12.3, here 10.2.
 template <bool INTERLEAVED>
 __global__ void __launch_bounds__(256)
 rope_q_wide_kernel(__nv_bfloat16* __restrict__ q, int H, int D, int rope, const int* __restrict__ positions,
@@ -336,7 +337,8 @@ int bg_rope_q(void* q, int T, int H, int D, int rope, const int* positions, cons
   using namespace bg;
   if (T <= 0) return 0;
   auto Q = reinterpret_cast<__nv_bfloat16*>(q);
-  if (rope % 16 == 0 && D % 8 == 0 && ld_t % 8 == 0 && reinterpret_cast<uintptr_t>(q) % 16 == 0)
+  const bool few = (long long)H * (rope / 2) <= 256 && T <= 1024;
+  if (!few && rope % 16 == 0 && D % 8 == 0 && ld_t % 8 == 0 && reinterpret_cast<uintptr_t>(q) % 16 == 0)
     bg::launch_pdl(interleaved ? rope_q_wide_kernel<true> : rope_q_wide_kernel<false>, dim3(T), dim3(256), 0, stream, Q, H, D, rope, positions, cos_t, sin_t, ld_t);
   else
     bg::launch_pdl(rope_q_kernel, dim3(T), dim3(256), 0, stream, Q, H, D, rope, positions, cos_t, sin_t, interleaved, ld_t);

@@ -239,11 +239,11 @@ def test_quantised_activation_of_few_and_many_rows(K, padding):
 
 
 @pytest.mark.parametrize("interleaved", [True, False])
-def test_rotated_queries_do_not_depend_on_alignment(interleaved):
+@pytest.mark.parametrize("T,H,D,rope", [(400, 16, 192, 64), (1025, 1, 64, 64), (1024, 8, 64, 64), (30, 9, 64, 64), (30, 40, 24, 16), (30, 16, 128, 48), (30, 5, 128, 128)])
+def test_rotated_queries_do_not_depend_on_alignment(interleaved, T, H, D, rope):
     """Rows in 16-byte pieces and rows that start between them: the same bytes, those of a x cos - round(b x sin) and a x sin + round(b x cos)."""
     from batchgen_b200.ops import fused
 
-    T, H, D, rope = 400, 16, 192, 64
     g = torch.Generator(device="cuda").manual_seed(0)
     pos = torch.randint(0, 4096, (T,), device="cuda", dtype=torch.int32, generator=g)
     ang = torch.rand(4096, rope // 2, device="cuda", generator=g) * 6
